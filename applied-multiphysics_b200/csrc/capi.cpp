@@ -219,6 +219,7 @@ struct amp_factor_s {
   __nv_bfloat16 *dWhi = nullptr, *dWlo = nullptr;   // mixed LDL^T: BF16 split of L21 D
   CUtensorMap *dMaps = nullptr;                     // per supernode: TMA descriptors of the split A and B operands
   unsigned long long *dStatus = nullptr;
+  double *dLinv = nullptr;     // group panels: inverses of the 8 x 8 diagonal blocks of every pivot block (scratch)
   int *dGroupFlags = nullptr;  // group panels: flags of every item, then the ticket counter of every group step
   long long waitSpins = 0;  // bound of the device waits in polls (0 = the kernels' defaults)
   bool ok = false, hasValues = false;
@@ -465,7 +466,7 @@ void enqueue_factor(amp_factor *f) {
         timed(f, K_PANEL, sr.panelFlops, 0.0, [&] {
           amp::launch_group_panel<float>(f->plan->dGroupItems, f->plan->dStrips + sr.strip0,
                                          (int)(sr.strip1 - sr.strip0), tickets + sr.ticket, f->dGroupFlags, dp,
-                                         f->dL32, f->dStatus, f->dShi, f->dSlo, ld32, st);
+                                         f->dL32, f->dLinv, f->dStatus, f->dShi, f->dSlo, ld32, st);
         });
         la.trsm_done();
         la.before_part_a();
@@ -521,7 +522,7 @@ void enqueue_factor(amp_factor *f) {
       timed(f, K_PANEL, sr.panelFlops, 0.0, [&] {
         amp::launch_group_panel<double>(f->plan->dGroupItems, f->plan->dStrips + sr.strip0,
                                         (int)(sr.strip1 - sr.strip0), tickets + sr.ticket, f->dGroupFlags, dp, f->dLx,
-                                        f->dStatus, nullptr, nullptr, ld, st);
+                                        f->dLinv, f->dStatus, nullptr, nullptr, ld, st);
       });
       la.trsm_done();
       la.before_part_a();
@@ -938,7 +939,7 @@ void enqueue_cfactor(amp_factor *f) {
       timed(f, K_PANEL, 4.0 * sr.panelFlops, 0.0, [&] {
         amp::launch_group_panel<amp::cplx>(f->plan->dCxItems, f->plan->dCxStrips + sr.strip0,
                                            (int)(sr.strip1 - sr.strip0), tickets + sr.ticket, f->dCxFlags, dp,
-                                           f->dLc, f->dStatus, nullptr, nullptr, ld, st);
+                                           f->dLc, nullptr, f->dStatus, nullptr, nullptr, ld, st);
       });
       if (sr.tile1 > sr.tile0)
         timed(f, K_UPDATE, 4.0 * (sr.updateFlopsA + sr.updateFlopsB), 0.0, [&] {
@@ -1303,6 +1304,7 @@ int amp_factor_create(amp_plan *pl, const amp_factor_opts *opts, amp_factor **ou
       }
       f->dTickets = f->mem.alloc<int>(2);
       f->dGroupFlags = f->mem.alloc<int>((size_t)std::max(1, P.nGroupFlags + P.nGroupTickets));
+      f->dLinv = f->mem.alloc<double>((size_t)P.nGroupFlags / 2 * 512);
       f->dDone = f->mem.alloc<int>((size_t)kSlices * std::max(1, P.nsuper));
       f->dSolveStatus = f->mem.alloc<unsigned long long>(1);
       init_device_once(pl->device);

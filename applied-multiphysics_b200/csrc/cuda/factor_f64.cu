@@ -1,14 +1,13 @@
-// Multifrontal numeric factorization on sm_100a: Cholesky (FP64, or FP32 fronts for the mixed-precision path) and
-// LDL^T with static pivot perturbation (FP64).
+// Multifrontal numeric factorization on sm_100a: assembly, the FP64 and complex updates, the complex group panel.
 //
 // Per level of the supernodal tree (leaves first):
 //   k_assemble  zero the front, scatter A's entries (sparse.mjs:965-973) and extend-add the children's update
-//               matrices in the reference's child order (sparse.mjs:974-985). One CTA owns a block of 32 front
+//               matrices in the reference's child order (sparse.mjs:974-985). One CTA owns a block of 8 front
 //               columns, so every entry has a single writer and the summation order is the reference's.
 //   per group of up to kGroup pivot blocks of 64 columns:
-//     k_group_panel  one dataflow launch: POTRF (or LDL^T) of each 64 x 64 pivot block in registers, the rows below
-//                    it against it (TRSM, 64-row strips, one CTA each) and the update of the group's remaining
-//                    columns, ordered by flags between the strips of the launch.
+//     k_group_panel  (group_panel.cu; the complex factor's k_cgroup_panel is here) one dataflow launch: POTRF (or LDL^T)
+//                    of each 64 x 64 pivot block, the rows below it against it (TRSM, 64-row strips, one CTA each) and
+//                    the update of the group's remaining columns, ordered by flags between the strips of the launch.
 //     k_update       FP64 update F -= A B^T of the columns right of the group (A = L21, or L21 D for LDL^T; B = L21;
 //                    K = the group) on 128 x 64 tiles with the FP64 tensor-core MMA (mma.sync m16n8k16), covering
 //                    the remaining pivot columns (in Lx) and the update block (in the U arena). The mixed-precision
@@ -17,11 +16,10 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <cfloat>
-#include <type_traits>
 #include <cstdint>
 
 #include "devplan.cuh"
+#include "launch.hpp"
 #include "sync.cuh"
 #include "../host/plan.hpp"
 
@@ -31,36 +29,6 @@ template <class T>
 __device__ __forceinline__ T *front_addr(T *Lp, T *Up, int m, int nc, int i, int j) {
   // front entry (i, j), i >= j: first nc columns in the L panel (ld m), the rest in the U block (ld mu)
   return j < nc ? Lp + (int64_t)j * m + i : Up + (int64_t)(j - nc) * (m - nc) + (i - nc);
-}
-
-// 1/d by Newton-Raphson refinement of the FP32 reciprocal (x <- x + x (1 - d x), quadratic convergence: 2^-23 ->
-// 2^-46 -> full double precision). Not correctly rounded (within a few ulp of 1/d); used only for the trailing
-// update scale of the pivot block, where the factor's own rounding dominates. Finite nonzero d of either sign; other
-// values take the division.
-__device__ __forceinline__ double recip_nr(double d) {
-  const double a = fabs(d);
-  if (!(a > 1e-30 && a < 1e30)) return 1.0 / d;  // outside the float range of the first approximation
-  double x = (double)__frcp_rn((float)d);
-  double e = fma(-d, x, 1.0);
-  x = fma(x, e, x);
-  e = fma(-d, x, 1.0);
-  x = fma(x, e, x);
-  e = fma(-d, x, 1.0);
-  return fma(x, e, x);
-}
-
-// Static pivot perturbation of LDL^T (ldlt.mjs:513-522): |d| < tau (or NaN) becomes -tau / +tau by the sign of d,
-// a non-finite small pivot fails the factorization. flags: bit 0 negative pivot, bit 1 perturbed. false = failure.
-template <class T>
-__device__ __forceinline__ bool ldlt_pivot(T &d, T tau, unsigned char &flags) {
-  flags = 0;
-  if (!(fabs(d) >= tau)) {
-    if (!isfinite(d)) return false;
-    d = d < T(0) ? -tau : tau;
-    flags = 2;
-  }
-  if (d < T(0)) flags |= 1;
-  return true;
 }
 
 // Complex pivot of the complex-symmetric LDL^T (ldlt.mjs:715-730): a magnitude below tau (or not a number) becomes
@@ -79,20 +47,7 @@ __device__ __forceinline__ bool ldlt_pivot(cplx &d, double tau, unsigned char &f
   }
   return true;
 }
-// magnitude of a pivot
-__device__ __forceinline__ double pivot_mag(double d) { return fabs(d); }
-__device__ __forceinline__ double pivot_mag(float d) { return fabs((double)d); }
-__device__ __forceinline__ double pivot_mag(cplx d) { return hypot(d.re, d.im); }
-// Cholesky's pivot test and diagonal (real factors only; a complex factor is always LDL^T)
-template <class T>
-__device__ __forceinline__ bool chol_pivot_ok(T d) { return d > T(0); }
-__device__ __forceinline__ bool chol_pivot_ok(cplx) { return false; }
-template <class T>
-__device__ __forceinline__ T chol_sqrt(T d) { return sqrt(d); }
-__device__ __forceinline__ cplx chol_sqrt(cplx d) { return d; }
-// loads through L2 (data another CTA of the running launch wrote) and read-only loads, for every scalar type
-__device__ __forceinline__ double ldcg_v(const double *p) { return __ldcg(p); }
-__device__ __forceinline__ float ldcg_v(const float *p) { return __ldcg(p); }
+// loads through L2 (data another CTA of the running launch wrote) and read-only loads
 __device__ __forceinline__ cplx ldcg_v(const cplx *p) {
   const double2 v = __ldcg(reinterpret_cast<const double2 *>(p));
   return cplx(v.x, v.y);
@@ -211,71 +166,55 @@ __global__ void __launch_bounds__(256) k_assemble(const AsmTask *__restrict__ ta
   }
 }
 
-// Scale factors of the pivot block's right-looking update (not stored): FP64 as recip_nr, FP32 the hardware estimate.
-__device__ __forceinline__ double fast_recip(double d) { return recip_nr(d); }
-__device__ __forceinline__ float fast_recip(float d) { return __fdividef(1.0f, d); }
-__device__ __forceinline__ cplx fast_recip(cplx d) { return cplx(1.0) / d; }
-
 // ---------------------------------------------------------------------------------------------------------------
-// Group panel: the pivot blocks of a group of up to kGroup 64-column blocks of a front, factored in one dataflow
-// launch (POTRF of each pivot block, TRSM of the rows below it, and the update of the group's remaining columns).
+// Group panel of the complex-symmetric factor (the real factors': group_panel.cu): the pivot blocks of a group of
+// 64-column blocks of a front, factored in one dataflow launch (LDL^T of each pivot block, TRSM of the rows below it,
+// and the update of the group's remaining columns) on the CUDA cores.
 // ---------------------------------------------------------------------------------------------------------------
 
-// Pivot block: POTRF (or LDL^T) of the 64 x 64 diagonal block of a front, called by all 256 threads of a CTA, the
-// block in registers. T = double: the FP64 factor; T = float: the mixed-precision factor. src: the updated block in
-// shared memory, entry (i, j) at src[j lds + i]; Lp: the block's (0, 0) entry in the front (ld m), where the factor is
-// written; w <= 64 its columns. Thread t < 136 owns the 4 x 4 tile (ti, tj), ti >= tj, of the lower triangle.
-// Right-looking on the unscaled columns, four columns per step kb with two barriers: (1) the diagonal tile eliminates
-// its four columns (settling the pivots) and publishes them; (2) the tiles below it in column block kb eliminate the
-// same four columns against it and publish theirs; then every tile right of the block applies the rank-4 update
-// S(i, j) -= sum S(i, k) S(j, k) / d_k. Cholesky tests d > 0 (sparse.mjs:1151-1156); LDL^T (ld.scal != null,
-// ldlt.mjs:450-562) perturbs |d| < tau to +-tau and counts negative and perturbed pivots. At the end the columns are
-// scaled: Cholesky L = a / sqrt(d) with sqrt(d) on the diagonal, LDL^T L = a / d with a unit diagonal (D to ld.D).
-// Returns false (status set for the first failing column f + c0 + k) when a pivot failed; the block is then not
-// written back.
-// LB (the Bunch-Kaufman fast path): also returns 2, writing nothing, when a multiplier |L(i, k)| of the block exceeds
-// lbound or a pivot was perturbed.
-template <class T, class TC, bool LB = false>
-__device__ int potrf_core(const T *src, int lds, T *Lp, int m, int w, int f, int c0, int s,
-                          unsigned long long *status, const LdltArgs<T> &ld, double promoteBelow,
-                          double lbound = -1.0) {
-  __shared__ TC col[2][4][kPanel];  // per 4-column block (double-buffered): the block's unscaled columns, by row
-  __shared__ TC pd[kPanel], piv[2][4];
+// Pivot block: LDL^T of the 64 x 64 diagonal block of a front, called by all 256 threads of a CTA, the block in
+// registers. src: the updated block in shared memory, entry (i, j) at src[j lds + i]; Lp: the block's (0, 0) entry in
+// the front (ld m), where the factor is written; w <= 64 its columns. Thread t < 136 owns the 4 x 4 tile (ti, tj),
+// ti >= tj, of the lower triangle. Right-looking on the unscaled columns, four columns per step kb with two barriers:
+// (1) the diagonal tile eliminates its four columns (settling the pivots) and publishes them; (2) the tiles below it in
+// column block kb eliminate the same four columns against it and publish theirs; then every tile right of the block
+// applies the rank-4 update S(i, j) -= sum S(i, k) S(j, k) / d_k. A pivot of magnitude below tau is perturbed
+// (ldlt.mjs:715-730) and counted. At the end the columns are scaled: L = a / d with a unit diagonal (D to ld.D). When a
+// pivot failed (status set for the first failing column f + c0 + k) the block is not written back.
+__device__ void cpotrf_block(const cplx *src, int lds, cplx *Lp, int m, int w, int f, int c0, int s,
+                             unsigned long long *status, const LdltArgs<cplx> &ld) {
+  __shared__ cplx col[2][4][kPanel];  // per 4-column block (double-buffered): the block's unscaled columns, by row
+  __shared__ cplx pd[kPanel], piv[2][4];
   __shared__ unsigned char pflag[kPanel];
-  __shared__ int fail, promote;
+  __shared__ int fail;
   const int tid = threadIdx.x;
-  const bool ldlt = ld.scal != nullptr;
-  using RT = typename real_of<TC>::type;
-  const RT tau = ldlt ? (RT)ld.scal[1] : RT(0);
+  const double tau = ld.scal[1];
   // tile of this thread: row block ti, column block tj (ti >= tj), from tid by the triangular numbering
   int ti = 0;
   while ((ti + 1) * (ti + 2) / 2 <= tid) ti++;
   const int tj = tid - ti * (ti + 1) / 2;
   const bool owner = tid < 136;
   int myFail = -1;  // diagonal tiles only
-  TC a[4][4];
+  cplx a[4][4];
 #pragma unroll
   for (int r = 0; r < 4; r++)
 #pragma unroll
     for (int c = 0; c < 4; c++) {
       const int i = 4 * ti + r, j = 4 * tj + c;
-      a[r][c] = !owner || i < j ? TC(0) : (i < w ? (TC)src[j * lds + i] : (i == j ? TC(1) : TC(0)));
+      a[r][c] = !owner || i < j ? cplx(0) : (i < w ? src[j * lds + i] : (i == j ? cplx(1) : cplx(0)));
     }
-  if (tid == 0) {
-    fail = kPanel;  // none
-    promote = 0;
-  }
+  if (tid == 0) fail = kPanel;  // none
   for (int kb = 0; kb < kPanel / 4; kb++) {
     const int buf = kb & 1;
     if (owner && ti == kb && tj == kb) {
 #pragma unroll
       for (int kk = 0; kk < 4; kk++) {
         const int k = 4 * kb + kk;
-        TC d = a[kk][kk];
+        cplx d = a[kk][kk];
         unsigned char fl = 0;
-        const bool bad = k < w && (ldlt ? !ldlt_pivot(d, tau, fl) : !chol_pivot_ok(d));
+        const bool bad = k < w && !ldlt_pivot(d, tau, fl);
         if (bad && myFail < 0) myFail = k;  // first failing pivot of this diagonal tile
-        const TC iv = fast_recip(d);          // the update scale only; L is scaled with the exact 1 / d at the end
+        const cplx iv = cplx(1.0) / d;
         pd[k] = d;
         pflag[k] = fl;
         piv[buf][kk] = iv;
@@ -293,10 +232,10 @@ __device__ int potrf_core(const T *src, int lds, T *Lp, int m, int w, int f, int
     if (owner && tj == kb && ti > kb) {
 #pragma unroll
       for (int kk = 0; kk < 4; kk++) {
-        const TC iv = piv[buf][kk];
+        const cplx iv = piv[buf][kk];
 #pragma unroll
         for (int c = kk + 1; c < 4; c++) {
-          const TC cj = col[buf][kk][4 * kb + c] * iv;
+          const cplx cj = col[buf][kk][4 * kb + c] * iv;
 #pragma unroll
           for (int r = 0; r < 4; r++) a[r][c] -= a[r][kk] * cj;
         }
@@ -310,8 +249,8 @@ __device__ int potrf_core(const T *src, int lds, T *Lp, int m, int w, int f, int
     if (owner && tj > kb) {
 #pragma unroll
       for (int kk = 0; kk < 4; kk++) {
-        const TC iv = piv[buf][kk];
-        TC ci[4], cj[4];
+        const cplx iv = piv[buf][kk];
+        cplx ci[4], cj[4];
 #pragma unroll
         for (int r = 0; r < 4; r++) ci[r] = col[buf][kk][4 * ti + r];
 #pragma unroll
@@ -325,321 +264,63 @@ __device__ int potrf_core(const T *src, int lds, T *Lp, int m, int w, int f, int
     }
   }
   if (myFail >= 0) atomicMin(&fail, myFail);
-  if (promoteBelow > 0.0 && tid < w && !(pivot_mag(pd[tid]) >= promoteBelow)) promote = 1;
-  if constexpr (LB && !is_cplx<TC>::value) {
-    {  // every multiplier within the bound and no pivot perturbed, else redo with pivoting
-      if (tid < w && (pflag[tid] & 2)) promote = 1;
-      if (owner) {
-#pragma unroll
-        for (int r = 0; r < 4; r++)
-#pragma unroll
-          for (int c = 0; c < 4; c++) {
-            const int i = 4 * ti + r, j = 4 * tj + c;
-            if (i > j && i < w && !(fabs((double)a[r][c]) <= lbound * fabs((double)pd[j]))) promote = 1;
-          }
-      }
-    }
-  }
   __syncthreads();
-  if (promote) return 2;  // the caller redoes the block in higher precision (nothing written)
   if (fail < kPanel) {
-    if (tid == 0) atomicMin(status, status_word(f + c0 + fail, ldlt ? 2 : 1, s));
-    return 1;
+    if (tid == 0) atomicMin(status, status_word(f + c0 + fail, 2, s));
+    return;
   }
   if (owner) {
 #pragma unroll
     for (int c = 0; c < 4; c++) {
       const int j = 4 * tj + c;
-      const TC d = pd[j];
-      const TC lj = ldlt ? d : chol_sqrt(d);
-      const TC inv = TC(1) / lj;
+      const cplx inv = cplx(1) / pd[j];
 #pragma unroll
       for (int r = 0; r < 4; r++) {
         const int i = 4 * ti + r;
-        if (i >= j && i < w && j < w) Lp[(int64_t)j * m + i] = (T)(i == j ? (ldlt ? TC(1) : lj) : a[r][c] * inv);
+        if (i >= j && i < w && j < w) Lp[(int64_t)j * m + i] = i == j ? cplx(1) : a[r][c] * inv;
       }
     }
   }
-  if (ldlt) {
-    if (tid < w) ld.D[f + c0 + tid] = (typename LdltArgs<T>::DT)pd[tid];
-    if (tid == 0) {
-      int neg = 0, pert = 0;
-      for (int k = 0; k < w; k++) neg += pflag[k] & 1, pert += pflag[k] >> 1;
-      atomicAdd(ld.counts, neg);
-      atomicAdd(ld.counts + 1, pert);
-    }
-  }
-  return 0;
-}
-
-// POTRF / LDL^T of a pivot block (potrf_core in the factor's precision). An FP32 LDL^T block with a pivot of
-// magnitude below FLT_EPSILON x max_i |A(i, i)| (a pivot with no correct FP32 digit left) is factored again from the
-// same entries (src is left unchanged) in FP64 arithmetic (stored FP32): the small-pivot blocks of the mixed-precision
-// indefinite factor get FP64 pivots. Returns false when a pivot failed (status set).
-template <class T>
-__device__ bool potrf_block(const T *src, int lds, T *Lp, int m, int w, int f, int c0, int s,
-                            unsigned long long *status, const LdltArgs<T> &ld) {
-  if constexpr (std::is_same<T, float>::value) {
-    if (ld.scal != nullptr) {
-      const double amax = ld.scal[0] > 0.0 ? ld.scal[1] / ld.scal[0] : 0.0;
-      const int r = potrf_core<float, float>(src, lds, Lp, m, w, f, c0, s, status, ld, amax * (double)FLT_EPSILON);
-      if (r != 2) return r == 0;
-      return potrf_core<float, double>(src, lds, Lp, m, w, f, c0, s, status, ld, -1.0) == 0;
-    }
-  }
-  return potrf_core<T, T>(src, lds, Lp, m, w, f, c0, s, status, ld, -1.0) == 0;
-}
-
-// (value, index) of the largest value over the warp, the smallest index on ties (every lane gets the result)
-__device__ __forceinline__ void warp_argmax(double &v, int &i) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const double ov = __shfl_xor_sync(0xffffffffu, v, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, i, o);
-    if (ov > v || (ov == v && oi < i)) {
-      v = ov;
-      i = oi;
-    }
-  }
-}
-
-// Bunch-Kaufman LDL^T of a pivot block, the pivot search restricted to the block's w columns (so the supernode
-// partition and every row structure stay the reference's): at column k, with colmax = max_{i>k} |B(i, k)| (row r),
-// a 1 x 1 pivot k when |B(k, k)| >= alpha colmax or |B(k, k)| rowmax >= alpha colmax^2 (rowmax = max_{j != r}
-// |B(r, j)|), a 1 x 1 pivot r when |B(r, r)| >= alpha rowmax, else the 2 x 2 pivot (k, r); alpha = (1 + sqrt 17) / 8
-// (Bunch and Kaufman, Math. Comp. 31, 1977). Each interchange is applied to the block's whole rows, the L columns
-// already computed included, so that P B P^T = L D L^T with L unit lower triangular (L(k + 1, k) = 0 inside a 2 x 2
-// pivot, whose off-diagonal is D(k + 1, k)). A column with no entry at or above tau keeps the reference's static
-// perturbation (|d| < tau -> -+tau, a non-finite one fails; ldlt.mjs:513-522). FP64 arithmetic for every T.
-// S: 64 x 65 doubles of shared workspace (a full symmetric copy, S[j][i] = B(i, j)); src: the updated block (entry
-// (i, j), i >= j, at src[j lds + i]). Writes L to Lp (ld m), D, Doff and piv, adds the inertia (a 2 x 2 pivot with a
-// negative determinant has one negative eigenvalue, with a positive one two when its diagonal is negative) and the
-// perturbed count. Returns false (status set) on a non-finite pivot; nothing is written then. Called by every thread.
-template <class T>
-__device__ bool bk_block(const T *src, int lds, double (*S)[kPanel + 1], T *Lp, int m, int w, int f, int c0, int s,
-                         unsigned long long *status, const LdltArgs<T> &ld) {
-  __shared__ int sPerm[kPanel];
-  __shared__ double sD[kPanel], sE[kPanel], sC0[kPanel], sC1[kPanel];
-  __shared__ int sStep, sKp, sFail, sNeg, sPert;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = blockDim.x;
-  const double tau = ld.scal[1];
-  const double alpha = 0.64038820320220756;  // (1 + sqrt(17)) / 8
-  for (int e = tid; e < kPanel * kPanel; e += nthr) {
-    const int i = e & (kPanel - 1), j = e >> 6;
-    double v = i == j ? 1.0 : 0.0;
-    if (i < w && j < w) v = (double)(i >= j ? src[j * lds + i] : src[i * lds + j]);
-    S[j][i] = v;
-  }
-  if (tid < kPanel) {
-    sPerm[tid] = tid;
-    sD[tid] = 1.0;
-    sE[tid] = 0.0;
-  }
+  if (tid < w) ld.D[f + c0 + tid] = pd[tid];
   if (tid == 0) {
-    sFail = -1;
-    sNeg = 0;
-    sPert = 0;
+    int pert = 0;
+    for (int k = 0; k < w; k++) pert += pflag[k] >> 1;
+    atomicAdd(ld.counts + 1, pert);
   }
-  __syncthreads();
-  for (int k = 0; k < w;) {
-    if (warp == 0) {  // the pivot choice
-      double cm = -1.0;
-      int im = -1;
-      for (int i = k + 1 + lane; i < w; i += 32) {
-        const double a = fabs(S[k][i]);
-        if (a > cm) {
-          cm = a;
-          im = i;
-        }
-      }
-      warp_argmax(cm, im);
-      const double colmax = cm > 0.0 ? cm : 0.0, absakk = fabs(S[k][k]);
-      int step = 1, kp = k;
-      if (colmax > 0.0 && !(absakk >= alpha * colmax)) {  // (a NaN diagonal takes the 1 x 1 path and fails below)
-        double rm = 0.0;
-        for (int j = k + lane; j < w; j += 32)
-          if (j != im) rm = fmax(rm, fabs(S[j][im]));
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) rm = fmax(rm, __shfl_xor_sync(0xffffffffu, rm, o));
-        if (absakk * rm >= alpha * colmax * colmax) {
-          kp = k;
-        } else if (fabs(S[im][im]) >= alpha * rm) {
-          kp = im;
-        } else {
-          step = 2;
-          kp = im;
-        }
-      }
-      if (lane == 0) {
-        sStep = step;
-        sKp = kp;
-      }
-    }
-    __syncthreads();
-    const int step = sStep, kp = sKp, kk = k + step - 1, k1 = k + step;
-    if (kp != kk) {  // interchange kk and kp: whole rows (L columns included), then the trailing columns
-      if (tid < w) {
-        const double t = S[tid][kk];
-        S[tid][kk] = S[tid][kp];
-        S[tid][kp] = t;
-      }
-      __syncthreads();
-      if (tid >= k && tid < w) {
-        const double t = S[kk][tid];
-        S[kk][tid] = S[kp][tid];
-        S[kp][tid] = t;
-      }
-      if (tid == 0) {
-        const int t = sPerm[kk];
-        sPerm[kk] = sPerm[kp];
-        sPerm[kp] = t;
-      }
-      __syncthreads();
-    }
-    const int nt = w - k1;
-    if (step == 1) {
-      double d = S[k][k];
-      const bool small = !(fabs(d) >= tau);
-      if (small && isfinite(d)) d = d < 0.0 ? -tau : tau;
-      if (tid < w) sC0[tid] = S[k][tid];  // column k, unscaled
-      if (tid == 0) {
-        sD[k] = d;
-        if (!isfinite(d) && sFail < 0) sFail = k;
-        sNeg += d < 0.0 ? 1 : 0;
-        sPert += small ? 1 : 0;
-      }
-      __syncthreads();
-      if (sFail >= 0) break;  // block-uniform
-      const double inv = 1.0 / d;
-      for (int e = tid; e < nt * nt; e += nthr) {
-        const int i = k1 + e % nt, j = k1 + e / nt;
-        S[j][i] -= sC0[i] * (sC0[j] * inv);
-      }
-      if (tid >= k1 && tid < w) S[k][tid] = sC0[tid] * inv;  // L(i, k)
-    } else {
-      // D_k = e [[a, 1], [1, c]], D_k^-1 = (t / e) [[c, -1], [-1, a]] with a = d11 / e, c = d22 / e, t = 1 / (a c - 1)
-      const double d11 = S[k][k], e21 = S[k][k + 1], d22 = S[k + 1][k + 1];
-      const double a = d11 / e21, c = d22 / e21, te = (1.0 / (a * c - 1.0)) / e21;
-      if (tid < w) {
-        sC0[tid] = S[k][tid];
-        sC1[tid] = S[k + 1][tid];
-      }
-      if (tid == 0) {
-        sD[k] = d11;
-        sD[k + 1] = d22;
-        sE[k] = e21;
-        if (!(isfinite(te) && isfinite(a) && isfinite(c)) && sFail < 0) sFail = k;
-        sNeg += a * c - 1.0 < 0.0 ? 1 : (d11 < 0.0 ? 2 : 0);
-      }
-      __syncthreads();
-      if (sFail >= 0) break;  // block-uniform
-      for (int e = tid; e < nt * nt; e += nthr) {
-        const int i = k1 + e % nt, j = k1 + e / nt;
-        const double l1 = te * (c * sC0[i] - sC1[i]), l2 = te * (a * sC1[i] - sC0[i]);
-        S[j][i] -= l1 * sC0[j] + l2 * sC1[j];
-      }
-      if (tid >= k1 && tid < w) {
-        S[k][tid] = te * (c * sC0[tid] - sC1[tid]);  // L(i, k)
-        S[k + 1][tid] = te * (a * sC1[tid] - sC0[tid]);  // L(i, k + 1)
-      }
-      if (tid == 0) S[k][k + 1] = 0.0;  // L(k + 1, k)
-    }
-    __syncthreads();
-    k += step;
-  }
-  __syncthreads();
-  if (sFail >= 0) {
-    if (tid == 0) atomicMin(status, status_word(f + c0 + sFail, 2, s));
-    return false;
-  }
-  for (int e = tid; e < w * w; e += nthr) {
-    const int i = e % w, j = e / w;
-    if (i >= j) Lp[(int64_t)j * m + i] = (T)(i == j ? 1.0 : S[j][i]);
-  }
-  if (tid < w) {
-    ld.D[f + c0 + tid] = sD[tid];
-    ld.Doff[f + c0 + tid] = sE[tid];
-    ld.piv[f + c0 + tid] = sPerm[tid];
-  }
-  if (tid == 0) {
-    atomicAdd(ld.counts, sNeg);
-    atomicAdd(ld.counts + 1, sPert);
-  }
-  return true;
 }
 
 // TRSM of up to 64 rows [r0, r1) of a front (L: its column-major block, ld m) against its factored pivot block
-// [c0, c0 + w): x_k = (a_k - sum_{c<k} x_c M(k, c)) / M(k, k). Four threads per row, thread (row, q) holds columns
+// [c0, c0 + w): x_k = (a_k - sum_{c<k} x_c M(k, c)) / M(k, k), M(k, c) = L11(k, c) d_c, M(k, k) = d_k, x = L21, and
+// w = x D = L21 D (the update's A operand, written to ld.W). Four threads per row, thread (row, q) holds columns
 // 16 q .. 16 q + 15 in registers. Phase p: the threads of quarter p solve their 16 columns (the earlier quarters'
 // contributions already applied) and publish them; after a barrier the threads of the later quarters subtract
-// quarter p's contribution (16 x 16 products) from theirs. Cholesky: M = L11, x = L21. LDL^T: M(k, c) = L11(k, c) d_c,
-// M(k, k) = d_k, x = L21, and w = x D = L21 D (the update's A operand, written to ld.W for the FP64 factor). The rows
-// are also written as BF16 hi / lo pairs (hi = bf16(x), lo = bf16(x - hi)) into the split columns of the tensor-core
-// update (mixed precision). The pivot block and D come from another CTA of the launch: read through L2 (__ldcg).
+// quarter p's contribution (16 x 16 products) from theirs. The pivot block and D come from another CTA of the launch:
+// read through L2 (__ldcg).
 // x: this thread's 16 entries of its row (row r0 + tid % 64, columns c0 + 16 (tid / 64) + u), loaded by the caller
 // before it waited for the pivot block (the strip's own rows are final by then).
-// On return Ws[c][r] holds this strip's update operand (x, or x D for LDL^T) and M[c][r] the solved rows x
-// (c < w, r < r1 - r0; zero elsewhere): a diagonal strip's X_c for its own column block.
-template <class T, bool BK>
-__device__ void trsm_strip(T *L, int m, int f, int c0, int w, int r0, int r1, int64_t lxp, int64_t sp,
-                           __nv_bfloat16 *Shi, __nv_bfloat16 *Slo, const LdltArgs<T> &ld, T (*M)[kPanel + 1],
-                           T (*Ws)[kPanel + 1], T *invd, T *dv, T (&x)[16]) {
-  const bool ldlt = ld.scal != nullptr;
-  // Bunch-Kaufman pivots (real factors): the strip's columns are taken in the block's pivot order, solved against the
-  // unit L11 (W = x L11^-T, the update's operand), then L21 = W D^-1 with the block's 1 x 1 and 2 x 2 pivots:
-  // column c of L21 is dA[c] W_c + dB[c] W_dP[c] (dP[c] = the other column of its 2 x 2 pivot, dB = 0 for a 1 x 1)
-  constexpr bool bk = BK && !is_cplx<T>::value;
-  __shared__ double dA[kPanel], dB[kPanel];
-  __shared__ int dP[kPanel], sPiv[kPanel];
+// On return Ws[c][r] holds this strip's update operand x D and M[c][r] the solved rows x (c < w, r < r1 - r0; zero
+// elsewhere): a diagonal strip's X_c for its own column block.
+__device__ void ctrsm_strip(cplx *L, int m, int f, int c0, int w, int r0, int r1, int64_t lxp,
+                            const LdltArgs<cplx> &ld, cplx (*M)[kPanel + 1], cplx (*Ws)[kPanel + 1], cplx *invd,
+                            cplx *dv, cplx (&x)[16]) {
   const int tid = threadIdx.x, r = tid & (kPanel - 1), q = tid >> 6;
-  {  // the pivot block: thread (r, q) loads row r of columns 16 q .. 16 q + 15 (times their pivots for LDL^T), and
-     // thread r < 64 the pivot of column r, in one round trip
-    T v[16];
+  {  // the pivot block: thread (r, q) loads row r of columns 16 q .. 16 q + 15 times their pivots, and thread r < 64 the
+     // pivot of column r, in one round trip
+    cplx v[16];
 #pragma unroll
     for (int u = 0; u < 16; u++) {
       const int c = 16 * q + u;
-      v[u] = (r < w && c < r) ? ldcg_v(L + (int64_t)(c0 + c) * m + c0 + r) : T(0);
+      v[u] = (r < w && c < r) ? ldcg_v(L + (int64_t)(c0 + c) * m + c0 + r) : cplx(0);
     }
-    if (ldlt && !bk) {
 #pragma unroll
-      for (int u = 0; u < 16; u++) {
-        const int c = 16 * q + u;
-        v[u] = v[u] * (c < w ? (T)ldcg_v(ld.D + f + c0 + c) : T(1));
-      }
+    for (int u = 0; u < 16; u++) {
+      const int c = 16 * q + u;
+      v[u] = v[u] * (c < w ? ldcg_v(ld.D + f + c0 + c) : cplx(1));
     }
     if (tid < kPanel) {
-      if constexpr (bk) {
-        {
-          const int c = tid;
-          double a = 1.0, b = 0.0;
-          int pc = c;
-          if (c < w) {
-            const double d = ldcg_v(ld.D + f + c0 + c);
-            const double en = ldcg_v(ld.Doff + f + c0 + c), ep = c > 0 ? ldcg_v(ld.Doff + f + c0 + c - 1) : 0.0;
-            if (en != 0.0 || ep != 0.0) {  // 2 x 2 pivot (c, c + 1) or (c - 1, c): the inverse as in bk_block
-              const bool first = en != 0.0;
-              const double e = first ? en : ep;
-              const double d11 = first ? d : ldcg_v(ld.D + f + c0 + c - 1);
-              const double d22 = first ? ldcg_v(ld.D + f + c0 + c + 1) : d;
-              const double aa = d11 / e, cc = d22 / e, te = (1.0 / (aa * cc - 1.0)) / e;
-              a = te * (first ? cc : aa);
-              b = -te;
-              pc = first ? c + 1 : c - 1;
-            } else {
-              a = 1.0 / d;
-            }
-          }
-          dA[c] = a;
-          dB[c] = b;
-          dP[c] = pc;
-          sPiv[c] = c < w ? __ldcg(ld.piv + f + c0 + c) : c;
-        }
-      }
-      const T d = bk ? T(1)
-                     : tid < w ? (ldlt ? (T)ldcg_v(ld.D + f + c0 + tid) : ldcg_v(L + (int64_t)(c0 + tid) * m + c0 + tid))
-                               : T(1);
+      const cplx d = tid < w ? ldcg_v(ld.D + f + c0 + tid) : cplx(1);
       dv[tid] = d;
-      invd[tid] = T(1) / d;
+      invd[tid] = cplx(1) / d;
     }
 #pragma unroll
     for (int u = 0; u < 16; u++) M[r][16 * q + u] = v[u];
@@ -647,14 +328,6 @@ __device__ void trsm_strip(T *L, int m, int f, int c0, int w, int r0, int r1, in
   const int row = r0 + r;
   const bool active = row < r1;
   __syncthreads();
-  if constexpr (bk) {  // the strip's columns in the block's pivot order: x_new(c) = x(piv(c))
-#pragma unroll
-    for (int u = 0; u < 16; u++) Ws[16 * q + u][r] = x[u];
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < 16; u++) x[u] = Ws[sPiv[16 * q + u]][r];
-    __syncthreads();
-  }
   for (int p = 0; p < 4; p++) {
     if (q == p) {  // solve this quarter
 #pragma unroll
@@ -672,42 +345,22 @@ __device__ void trsm_strip(T *L, int m, int f, int c0, int w, int r0, int r1, in
 #pragma unroll 4
       for (int kk = 0; kk < 16; kk++) {
         const int k = 16 * p + kk;
-        const T xk = Ws[k][r];
+        const cplx xk = Ws[k][r];
 #pragma unroll
         for (int u = 0; u < 16; u++) x[u] -= xk * M[16 * q + u][k];
       }
     }
   }
   __syncthreads();  // every quarter read Ws: overwrite it with the update operand
-  const int ld8 = (m + 7) & ~7;
 #pragma unroll
   for (int u = 0; u < 16; u++) {
     const int cc = 16 * q + u;
-    T xv = x[u];
-    T wv = ldlt ? xv * dv[cc] : xv;
-    if constexpr (bk) {
-      {  // x[u] is W (already in Ws, zero outside the strip and the block); L21 = W D^-1
-        wv = x[u];
-        xv = (T)(dA[cc] * (double)x[u] + dB[cc] * (double)Ws[dP[cc]][r]);
-      }
-    }
-    if (!bk) Ws[cc][r] = active && cc < w ? wv : T(0);
-    M[cc][r] = active && cc < w ? xv : T(0);  // the pivot block in M is no longer read
+    const cplx xv = x[u], wv = xv * dv[cc];
+    Ws[cc][r] = active && cc < w ? wv : cplx(0);
+    M[cc][r] = active && cc < w ? xv : cplx(0);  // the pivot block in M is no longer read
     if (!active || cc >= w) continue;
     L[(int64_t)(c0 + cc) * m + row] = xv;
-    if (ldlt && ld.W) ld.W[lxp + (int64_t)(c0 + cc) * m + row] = wv;
-    if constexpr (!is_cplx<T>::value)
-    if (Shi) {
-      const int64_t g = sp + (int64_t)(c0 + cc) * ld8 + row;
-      const __nv_bfloat16 hi = __float2bfloat16_rn((float)xv);
-      Shi[g] = hi;
-      Slo[g] = __float2bfloat16_rn((float)xv - __bfloat162float(hi));
-      if (ldlt) {
-        const __nv_bfloat16 whi = __float2bfloat16_rn((float)wv);
-        ld.Whi[g] = whi;
-        ld.Wlo[g] = __float2bfloat16_rn((float)wv - __bfloat162float(whi));
-      }
-    }
+    ld.W[lxp + (int64_t)(c0 + cc) * m + row] = wv;
   }
   __syncthreads();
 }
@@ -756,21 +409,16 @@ __device__ __forceinline__ void panel_release(int *p, int v) {
 // launch cannot deadlock whatever the number of resident CTAs. The columns right of the group receive the group's
 // update afterwards (k_update / k_update_mx, K = the group). Failure (a pivot, a bounded wait) sets the status and
 // releases P[b], so every waiter leaves.
-constexpr int kGroupSmem = 3 * kPanel * (kPanel + 1) * (int)sizeof(double);
-// two CTAs per SM for the real factors (registers capped at 128); the complex one is held to one by its shared memory
-template <class T>
-constexpr int group_min_blocks() { return is_cplx<T>::value ? 1 : 2; }
-template <class T, bool BK>
-__global__ void __launch_bounds__(256, group_min_blocks<T>()) k_group_panel(const GroupItem *__restrict__ items,
-                                                     const StripTask *__restrict__ strips, int nstrips, int *ticket,
-                                                     int *flags, DevPlan P, T *__restrict__ Lx,
-                                                     unsigned long long *status, __nv_bfloat16 *__restrict__ Shi,
-                                                     __nv_bfloat16 *__restrict__ Slo, LdltArgs<T> ld) {
+constexpr int kCGroupSmem = 3 * kPanel * (kPanel + 1) * (int)sizeof(cplx);  // one CTA per SM
+__global__ void __launch_bounds__(256, 1) k_cgroup_panel(const GroupItem *__restrict__ items,
+                                                         const StripTask *__restrict__ strips, int nstrips,
+                                                         int *ticket, int *flags, DevPlan P, cplx *__restrict__ Lx,
+                                                         unsigned long long *status, LdltArgs<cplx> ld) {
   extern __shared__ __align__(16) unsigned char gp_raw[];
-  T(*M)[kPanel + 1] = reinterpret_cast<T(*)[kPanel + 1]>(gp_raw);  // pivot block (TRSM), then the X_c chunk
-  T(*Ws)[kPanel + 1] = reinterpret_cast<T(*)[kPanel + 1]>(gp_raw + kPanel * (kPanel + 1) * sizeof(T));
-  T(*Ds)[kPanel + 1] = reinterpret_cast<T(*)[kPanel + 1]>(gp_raw + 2 * kPanel * (kPanel + 1) * sizeof(T));
-  __shared__ T invd[kPanel], dv[kPanel];
+  cplx(*M)[kPanel + 1] = reinterpret_cast<cplx(*)[kPanel + 1]>(gp_raw);  // pivot block (TRSM), then the X_c chunk
+  cplx(*Ws)[kPanel + 1] = reinterpret_cast<cplx(*)[kPanel + 1]>(gp_raw + kPanel * (kPanel + 1) * sizeof(cplx));
+  cplx(*Ds)[kPanel + 1] = reinterpret_cast<cplx(*)[kPanel + 1]>(gp_raw + 2 * kPanel * (kPanel + 1) * sizeof(cplx));
+  __shared__ cplx invd[kPanel], dv[kPanel];
   __shared__ int sTicket;
   if (threadIdx.x == 0) sTicket = failed(status) ? nstrips : atomicAdd(ticket, 1);
   __syncthreads();
@@ -783,7 +431,7 @@ __global__ void __launch_bounds__(256, group_min_blocks<T>()) k_group_panel(cons
   const int nb = (g1 - g0 + kPanel - 1) / kPanel;
   const int r0 = st.r0, r1 = st.r1, jd = st.diag;
   const int bmax = jd >= 0 ? jd : nb;  // pivot blocks whose rows below include this strip
-  T *L = Lx + P.snLxp[s];
+  cplx *L = Lx + P.snLxp[s];
   int *Pf = flags + it.flag0, *Df = Pf + nb;
   const int tid = threadIdx.x, tr = tid & 15, tc = tid >> 4;
   // A diagonal strip keeps its own pivot block (columns [r0, r1), lower part) in shared memory while it updates it
@@ -791,24 +439,24 @@ __global__ void __launch_bounds__(256, group_min_blocks<T>()) k_group_panel(cons
   if (jd >= 0) {
     for (int e = tid; e < kPanel * kPanel; e += blockDim.x) {
       const int i = e & 63, j = e >> 6;
-      Ds[j][i] = (r0 + i < r1 && j <= i) ? L[(int64_t)(r0 + j) * m + r0 + i] : T(0);
+      Ds[j][i] = (r0 + i < r1 && j <= i) ? L[(int64_t)(r0 + j) * m + r0 + i] : cplx(0);
     }
   }
   for (int b = 0; b < bmax; b++) {
     const int c0 = g0 + b * kPanel, w = min(kPanel, g1 - c0), c1 = c0 + w;
-    T x[16];  // this thread's part of the strip's rows of block b, loaded while the pivot block is not yet ready
+    cplx x[16];  // this thread's part of the strip's rows of block b, loaded while the pivot block is not yet ready
     {
       const int xr = r0 + (tid & (kPanel - 1)), xq = tid >> 6;
 #pragma unroll
       for (int u = 0; u < 16; u++) {
         const int c = 16 * xq + u;
-        x[u] = xr < r1 && c < w ? L[(int64_t)(c0 + c) * m + xr] : T(0);
+        x[u] = xr < r1 && c < w ? L[(int64_t)(c0 + c) * m + xr] : cplx(0);
       }
     }
     if (!panel_wait(Pf + b, 1, status, P.spin)) return;
-    trsm_strip<T, BK>(L, m, f, c0, w, r0, r1, P.snLxp[s], P.snSp[s], Shi, Slo, ld, M, Ws, invd, dv, x);
+    ctrsm_strip(L, m, f, c0, w, r0, r1, P.snLxp[s], ld, M, Ws, invd, dv, x);
     if (jd >= 0) panel_release(Df + jd, b + 1);
-    // Update with block b (C -= W_r X_c^T, K = w): a diagonal strip first its own pivot block (X_c = its solved rows,
+    // Update with block b (C -= W_r X_c^cplx, K = w): a diagonal strip first its own pivot block (X_c = its solved rows,
     // left in M by the TRSM; into Ds), then the blocks between block b and its own; a strip below every remaining
     // column block of the group.
     const int hi = jd >= 0 ? r0 : g1, nown = jd >= 0 ? 1 : 0;
@@ -820,17 +468,17 @@ __global__ void __launch_bounds__(256, group_min_blocks<T>()) k_group_panel(cons
         if (!panel_wait(Df + (cb - g0) / kPanel, b + 1, status, P.spin)) return;
         for (int e = tid; e < kPanel * kPanel; e += blockDim.x) {  // X_c[k][jj] = L(cb + jj, c0 + k)
           const int k = e >> 6, jj = e & 63;
-          M[k][jj] = (k < w && jj < ncol) ? ldcg_v(L + (int64_t)(c0 + k) * m + cb + jj) : T(0);
+          M[k][jj] = (k < w && jj < ncol) ? ldcg_v(L + (int64_t)(c0 + k) * m + cb + jj) : cplx(0);
         }
         __syncthreads();
       }
-      T acc[4][4];
+      cplx acc[4][4];
 #pragma unroll
       for (int a = 0; a < 4; a++)
 #pragma unroll
-        for (int bb = 0; bb < 4; bb++) acc[a][bb] = T(0);
+        for (int bb = 0; bb < 4; bb++) acc[a][bb] = cplx(0);
       for (int k = 0; k < w; k++) {
-        T wv[4], xv[4];
+        cplx wv[4], xv[4];
 #pragma unroll
         for (int a = 0; a < 4; a++) wv[a] = Ws[k][tr + 16 * a];
 #pragma unroll
@@ -848,7 +496,7 @@ __global__ void __launch_bounds__(256, group_min_blocks<T>()) k_group_panel(cons
           if (own) {
             if (jj <= i) Ds[jj][i] -= acc[a][bb];
           } else if (r0 + i < r1 && jj < ncol) {
-            T *cptr = L + (int64_t)(cb + jj) * m + r0 + i;
+            cplx *cptr = L + (int64_t)(cb + jj) * m + r0 + i;
             *cptr = *cptr - acc[a][bb];
           }
         }
@@ -858,21 +506,7 @@ __global__ void __launch_bounds__(256, group_min_blocks<T>()) k_group_panel(cons
   if (jd >= 0) {  // this strip's own pivot block, fully updated: factor it and publish it (also after a failure)
     const int c0 = g0 + jd * kPanel, w = min(kPanel, g1 - c0);
     __syncthreads();  // Ds complete (also when the strip had no earlier pivot block)
-    if constexpr (BK && !is_cplx<T>::value) {
-      // Bunch-Kaufman keeps every pivot of the block in place exactly when each multiplier is at most 1 / alpha in
-      // magnitude and no pivot needs the perturbation: try the unpivoted LDL^T first (it writes nothing unless it
-      // passes that test), else redo the block with pivots from the untouched entries
-      const int r = potrf_core<T, T, true>(&Ds[0][0], kPanel + 1, L + (int64_t)c0 * m + c0, m, w, f, c0, s, status, ld,
-                                           -1.0, 1.0 / 0.64038820320220756);
-      if (r == 2) {  // FP64 workspace in M (and Ws for FP32 fronts), both free here
-        bk_block<T>(&Ds[0][0], kPanel + 1, reinterpret_cast<double(*)[kPanel + 1]>(gp_raw),
-                    L + (int64_t)c0 * m + c0, m, w, f, c0, s, status, ld);
-      } else if (r == 0 && threadIdx.x < w) {  // the identity pivot order, 1 x 1 pivots
-        ld.piv[f + c0 + threadIdx.x] = threadIdx.x;
-        ld.Doff[f + c0 + threadIdx.x] = 0.0;
-      }
-    } else
-      potrf_block<T>(&Ds[0][0], kPanel + 1, L + (int64_t)c0 * m + c0, m, w, f, c0, s, status, ld);
+    cpotrf_block(&Ds[0][0], kPanel + 1, L + (int64_t)c0 * m + c0, m, w, f, c0, s, status, ld);
     panel_release(Pf + jd, 1);
   }
 }
@@ -1130,20 +764,15 @@ __global__ void k_permute_out(const double *__restrict__ y, double *__restrict__
 // ---------------------------------------------------------------------------------------------------------------
 static int g_num_sms = 148;
 
+cudaError_t init_group_panel_attributes();
 cudaError_t init_mixed_attributes();
 cudaError_t init_solve_attributes();
 cudaError_t init_solve_multi_attributes();
 cudaError_t init_front_small_attributes();
 cudaError_t init_kernel_attributes() {
   // function attributes belong to the current device's context: the caller runs this once per device
-  cudaError_t e =
-      cudaFuncSetAttribute(k_group_panel<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupSmem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_group_panel<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupSmem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_group_panel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupSmem / 2);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_group_panel<cplx, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupSmem * 2);
+  cudaError_t e = cudaFuncSetAttribute(k_cgroup_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCGroupSmem);
+  if (e == cudaSuccess) e = init_group_panel_attributes();
   if (e == cudaSuccess) e = init_mixed_attributes();
   if (e == cudaSuccess) e = init_solve_attributes();
   if (e == cudaSuccess) e = init_solve_multi_attributes();
@@ -1166,30 +795,14 @@ template void launch_assemble<float>(const AsmTask *, const ChildRange *, int64_
                                      float *, float *, const unsigned long long *, cudaStream_t);
 template void launch_assemble<cplx>(const AsmTask *, const ChildRange *, int64_t, const DevPlan &, const cplx *,
                                     cplx *, cplx *, const unsigned long long *, cudaStream_t);
-template <class T>
-void launch_group_panel(const GroupItem *items, const StripTask *strips, int nstrips, int *ticket, int *flags,
-                        const DevPlan &P, T *Lx, unsigned long long *status, __nv_bfloat16 *Shi, __nv_bfloat16 *Slo,
-                        const LdltArgs<T> &ld, cudaStream_t st) {
-  if (nstrips <= 0) return;
-  const size_t smem = 3 * kPanel * (kPanel + 1) * sizeof(T);
-  if constexpr (std::is_same<T, double>::value)  // Bunch-Kaufman pivot blocks (FP64 LDL^T with ld.piv set)
-    if (ld.piv) {
-      k_group_panel<T, true><<<(unsigned)nstrips, 256, smem, st>>>(items, strips, nstrips, ticket, flags, P, Lx, status,
-                                                                  Shi, Slo, ld);
-      return;
-    }
-  k_group_panel<T, false><<<(unsigned)nstrips, 256, smem, st>>>(items, strips, nstrips, ticket, flags, P, Lx, status, Shi,
-                                                               Slo, ld);
+template <>
+void launch_group_panel<cplx>(const GroupItem *items, const StripTask *strips, int nstrips, int *ticket, int *flags,
+                              const DevPlan &P, cplx *Lx, double *, unsigned long long *status, __nv_bfloat16 *,
+                              __nv_bfloat16 *, const LdltArgs<cplx> &ld, cudaStream_t st) {
+  if (nstrips > 0)
+    k_cgroup_panel<<<(unsigned)nstrips, 256, kCGroupSmem, st>>>(items, strips, nstrips, ticket, flags, P, Lx, status,
+                                                               ld);
 }
-template void launch_group_panel<double>(const GroupItem *, const StripTask *, int, int *, int *, const DevPlan &,
-                                         double *, unsigned long long *, __nv_bfloat16 *, __nv_bfloat16 *,
-                                         const LdltArgs<double> &, cudaStream_t);
-template void launch_group_panel<float>(const GroupItem *, const StripTask *, int, int *, int *, const DevPlan &,
-                                        float *, unsigned long long *, __nv_bfloat16 *, __nv_bfloat16 *,
-                                        const LdltArgs<float> &, cudaStream_t);
-template void launch_group_panel<cplx>(const GroupItem *, const StripTask *, int, int *, int *, const DevPlan &,
-                                       cplx *, unsigned long long *, __nv_bfloat16 *, __nv_bfloat16 *,
-                                       const LdltArgs<cplx> &, cudaStream_t);
 
 void launch_update_c(const TileTask *tasks, int64_t ntasks, cplx *Lx, cplx *U, const cplx *W,
                      const unsigned long long *status, cudaStream_t st) {

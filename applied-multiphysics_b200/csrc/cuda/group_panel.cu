@@ -1,0 +1,872 @@
+// Group panel of the real factors (FP64, or FP32 storage for the mixed-precision path; Cholesky, LDL^T with static pivot
+// perturbation, LDL^T with Bunch-Kaufman pivots inside each pivot block): the pivot blocks of a group of 64-column
+// blocks of a front factored in one dataflow launch -- POTRF of each pivot block, TRSM of the rows below it, and the
+// update of the group's remaining columns. All arithmetic is FP64, its products on the FP64 tensor cores
+// (mma.sync m8n8k4); an FP32 factor rounds once, when an entry is stored.
+//
+// What bounds it: the chain through the pivot blocks of the large fronts (POTRF of block b, then block b + 1's rows
+// against it, then their update and POTRF), one CTA at a time, so a block's latency is what counts: per block POTRF
+// 11,100 clocks, the flag and the loads behind it 3,400, TRSM 2,500, the block's own update 1,600 (FP64; 33,700 / - /
+// 10,400 / 7,100 with FMA tiles and a four-thread substitution per row). A 4,096-row front's group of two blocks takes
+// 32 us (66 before) in FP64 and 32 us (39) in FP32, eight of them at once 63 us (110) and 65 us (74). The split: warp w
+// of a strip owns 8 rows (row group rg(w)) of every 64 x 64 product, so a strip's TRSM runs inside each warp without a
+// barrier -- the C fragment of a solved 8 x 8 tile is the A fragment of the next product (its two registers are the k
+// indices 2 t and 2 t + 1, and the B fragment takes the same pair with one 16-byte load).
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include <type_traits>
+
+#include "../host/plan.hpp"
+#include "devplan.cuh"
+#include "sync.cuh"
+
+namespace amp {
+
+namespace {
+
+__device__ __forceinline__ bool panel_failed(const unsigned long long *st) {
+  return *(volatile const unsigned long long *)st != kStatusOk;
+}
+
+// D += A B on an 8 x 8 tile, K = 4: lane (g, t) = (lane / 4, lane % 4) holds A(g, t), B(t, g), D(g, 2 t) and D(g, 2 t + 1)
+__device__ __forceinline__ void mma884(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
+// 64 x 64 FP64 blocks in shared memory, row-major, the column pairs of row r permuted by a bijection of r mod 8 so that
+// the 16-byte accesses of a fragment (8 rows, 4 neighbouring pairs) and the 8-byte stores of the block loads (8 rows,
+// 4 columns) touch every bank equally often.
+__device__ __forceinline__ int sw(int r, int c) {
+  return r * kPanel + (((c >> 1) ^ (((r & 1) << 2) | ((r >> 1) & 3))) << 1) + (c & 1);
+}
+__device__ __forceinline__ double2 pair_at(const double *S, int r, int c) {  // entries (r, c), (r, c + 1), c even
+  return *reinterpret_cast<const double2 *>(S + sw(r, c));
+}
+__device__ __forceinline__ void set_pair(double *S, int r, int c, double x, double y) {
+  *reinterpret_cast<double2 *>(S + sw(r, c)) = make_double2(x, y);
+}
+
+// the 8-row group of a warp: the pairs of warps that share a scheduler (w, w + 4) get groups that sum to 7, so the
+// lower triangle's work is the same on all four
+__device__ __forceinline__ int row_group(int warp) { return warp < 4 ? warp : 11 - warp; }
+
+// Rows [i0, i0 + nr) x columns [j0, j0 + ncol) of a front's column-major block (ld m) into S; lower: only the entries
+// on and below the diagonal. The rest is zero, and with pad the diagonal entries from ncol on are one. Read through
+// L2 (another CTA of the running launch may have written them). 8 rows x 4 columns per warp access.
+template <class T>
+__device__ __forceinline__ void load_block(double *S, const T *L, int m, int i0, int nr, int j0, int ncol, bool lower,
+                                           bool pad) {
+  const int lane = threadIdx.x & 31, i = 8 * (threadIdx.x >> 5) + (lane >> 2), t = lane & 3;
+  T v[16];
+#pragma unroll
+  for (int e = 0; e < 16; e++) {
+    const int c = 4 * e + t;
+    v[e] = (i < nr && c < ncol && (!lower || c <= i)) ? __ldcg(L + (int64_t)(j0 + c) * m + i0 + i) : T(0);
+  }
+#pragma unroll
+  for (int e = 0; e < 16; e++) {
+    const int c = 4 * e + t;
+    S[sw(i, c)] = pad && i == c && i >= ncol ? 1.0 : (double)v[e];
+  }
+}
+
+// 1 / d as x f. FP64: Newton's iteration on the hardware estimate x (relative error e below 2^-20):
+// 1 / d = x / (1 - e) = x (1 + e)(1 + e^2) up to e^4, x and f apart, so that a product with x can run beside f's chain;
+// the estimate flushes results outside the normal range, so it returns false for |d| below 2^-975 or above 2^960 (an
+// integer test of the exponent, off the FP64 pipe). FP32: the hardware quotient estimate. Exact: the quotient.
+template <bool Exact>
+__device__ __forceinline__ bool recip_parts(double d, double &x, double &f) {
+  if constexpr (Exact) {
+    x = 1.0 / d;
+    f = 1.0;
+    return true;
+  }
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
+  const double e = fma(-d, x, 1.0), s = 1.0 + e;
+  f = fma(s, e * e, s);
+  return ((unsigned)__double2hiint(d) & 0x7fffffffu) - 0x03000000u <= 0x79000000u;
+}
+template <bool Exact>
+__device__ __forceinline__ bool recip_parts(float d, float &x, float &f) {
+  x = __fdividef(1.0f, d);
+  f = 1.0f;
+  return true;
+}
+
+// POTRF step buffers: 8 columns of 64 rows; row strides with 16-byte rows and few bank conflicts
+template <class TC>
+constexpr int col_ld() { return sizeof(TC) == 8 ? 10 : 12; }
+template <class TC>
+struct Vec2;  // two neighbouring entries
+template <>
+struct Vec2<double> { using type = double2; };
+template <>
+struct Vec2<float> { using type = float2; };
+
+// C(g, 2 t ..) -= A(g, .) B(., 2 t ..) on an 8 x 8 tile, K = 8: P the negated rows of A, Q the rows of B^T (stride ld)
+__device__ __forceinline__ void step_tile(double (&c)[2], const double *P, const double *Q, int ld, int g, int t) {
+  const double2 a = *reinterpret_cast<const double2 *>(P + g * ld + 2 * t);
+  const double2 b = *reinterpret_cast<const double2 *>(Q + g * ld + 2 * t);
+  mma884(c, a.x, b.x);
+  mma884(c, a.y, b.y);
+}
+__device__ __forceinline__ void step_tile(float (&c)[2], const float *P, const float *Q, int ld, int g, int t) {
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const float4 a = *reinterpret_cast<const float4 *>(P + g * ld + 4 * h);
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      const float4 b = *reinterpret_cast<const float4 *>(Q + (2 * t + u) * ld + 4 * h);
+      c[u] = fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, c[u]))));
+    }
+  }
+}
+
+// Pivot block: POTRF (or LDL^T) of the 64 x 64 diagonal block of a front, called by all 256 threads of a CTA, in TC
+// (FP64, or FP32 for the FP32 Cholesky factor, as the whole-front kernels). Ds: the updated block (lower part; identity from column w on), left unchanged; Lp: the block's
+// (0, 0) entry in the front (ld m), where the factor is written; w <= 64 its columns; scr: 11 step buffers; Linv:
+// the inverses of the eight 8 x 8 diagonal blocks of L (64 doubles each, row-major), for the strips' TRSM.
+// Right-looking on the unscaled columns in steps of eight. Step k: (1) the first two warps, one row per lane, factor the
+// 8 x 8 diagonal tile redundantly in registers -- so no value of the pivot chain crosses lanes -- and eliminate their
+// own row with it, publishing -a and a / d; (2) after a barrier the warps of the row groups below (C fragments of their
+// trailing tiles in registers) update their tile of the next eight columns and hand it over; (3) after a second barrier
+// they update the rest of the triangle while the first two warps go on with step k + 1. The chain per column is one
+// reciprocal (the hardware estimate and three dependent products) and two products, 58 clocks (FP64); a step's FP64
+// issue in a panel warp takes 790 clocks alone and 1,050-1,200 beside the trailing products. The pivots are tested, the
+// columns scaled and everything written after the last step. A block takes 11,100 clocks in FP64 and 9,100 in FP32
+// (33,700 and 13,000 with 4 x 4 register tiles, a diagonal thread per step and two barriers per four columns).
+// Cholesky tests d > 0 (sparse.mjs:1151-1156); LDL^T (ldlt.mjs:450-562) perturbs |d| < tau to +-tau by the sign of d (a
+// non-finite small pivot fails) and counts negative and perturbed pivots. Cholesky L = a / sqrt(d) with sqrt(d) on the
+// diagonal, LDL^T L = a / d with a unit diagonal (D to ld.D). Returns 0, or 1 (status set for the first failing column
+// f + c0 + k, nothing written) when a pivot failed. LB (the Bunch-Kaufman fast path): returns 2, writing nothing, when
+// a multiplier |L(i, k)| of the block exceeds lbound or a pivot was perturbed.
+template <class T, class TC, bool LDLT, bool LB>
+__device__ int potrf_block(const double *Ds, double *scr, T *Lp, double *Linv, int m, int w, int f, int c0, int s,
+                           unsigned long long *status, const LdltArgs<T> &ld, double lbound) {
+  using V2 = typename Vec2<TC>::type;
+  constexpr int CL = col_ld<TC>(), kStepBuf = kPanel * CL;
+  __shared__ double scale[kPanel], diag[kPanel];
+  __shared__ int failAt, redo, nNeg, nPert, inexact;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, rg = row_group(warp);
+  const TC tau = LDLT ? (TC)ld.scal[1] : TC(0);
+  TC *R = reinterpret_cast<TC *>(scr), *Q = R + kStepBuf, *P = R + 3 * kStepBuf;  // Q: two buffers; P: -a of every step
+  const int myRow = (8 * rg + g) * CL + 2 * t;
+  auto tile = [&](int cb, TC(&c)[2]) {  // this warp's tile (rg, cb) of the block
+    const double2 v = pair_at(Ds, 8 * rg + g, 8 * cb + 2 * t);
+    c[0] = (TC)v.x;
+    c[1] = (TC)v.y;
+  };
+  auto hand_over = [&](const TC(&c)[2]) {
+    V2 v;
+    v.x = c[0];
+    v.y = c[1];
+    *reinterpret_cast<V2 *>(R + myRow) = v;
+  };
+  // (1) of step k for this lane's row; Exact: the pivots' reciprocals by division. Returns false when one is out of the
+  // estimate's range.
+  auto eliminate = [&](int k, auto exact) {
+    const int r = min(8 * k + 32 * warp + lane, kPanel - 1);  // (lanes past the block repeat its last row)
+    TC *Pk = P + k * kStepBuf + r * CL, *Qk = Q + (k & 1) * kStepBuf + r * CL;
+    TC dg[8][8], a[8], iv[8];
+    bool fine = true;
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+      for (int j = 0; j <= i; j += 2) {
+        const V2 v = *reinterpret_cast<const V2 *>(R + (8 * k + i) * CL + j);
+        dg[i][j] = v.x;
+        dg[i][j + 1] = v.y;
+      }
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      const V2 v = *reinterpret_cast<const V2 *>(R + r * CL + j);
+      a[j] = v.x;
+      a[j + 1] = v.y;
+    }
+#pragma unroll
+    for (int kk = 0; kk < 8; kk++) {
+      TC d = dg[kk][kk], x, fr;
+      if (LDLT && !(fabs(d) >= tau)) d = d < TC(0) ? -tau : tau;
+      fine &= recip_parts<decltype(exact)::value>(d, x, fr);
+      iv[kk] = x * fr;
+#pragma unroll
+      for (int j = kk + 1; j < 8; j++) {
+        const TC lj = (dg[j][kk] * x) * fr;  // the update scale; L is scaled with the exact quotient below
+#pragma unroll
+        for (int i = j; i < 8; i++) dg[i][j] -= dg[i][kk] * lj;
+        a[j] -= a[kk] * lj;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      V2 v;
+      v.x = -a[j];
+      v.y = -a[j + 1];
+      *reinterpret_cast<V2 *>(Pk + j) = v;
+      v.x = a[j] * iv[j];
+      v.y = a[j + 1] * iv[j + 1];
+      *reinterpret_cast<V2 *>(Qk + j) = v;
+    }
+    return fine;
+  };
+  auto panel = [&](auto exact) {  // the first two warps
+    bool fine = true;
+    for (int k = 0; k < 8; k++) {
+      if (8 * k + 32 * warp < kPanel) fine &= eliminate(k, exact);
+      __syncthreads();
+      if (k == 0 && warp == 1) {  // row group 1's only trailing tile
+        TC c[2];
+        tile(1, c);
+        step_tile(c, P + 8 * CL, Q + 8 * CL, CL, g, t);
+        hand_over(c);
+      }
+      __syncthreads();
+    }
+    if (!fine) inexact = 1;
+  };
+  auto trailing = [&]() {  // the other warps
+    TC c[7][2];  // at step k: the tiles (rg, k + 1), (rg, k + 2), ...
+#pragma unroll
+    for (int j = 0; j < 7; j++) {
+      c[j][0] = c[j][1] = TC(0);
+      if (j < rg) tile(j + 1, c[j]);
+    }
+    for (int k = 0; k < 8; k++) {
+      __syncthreads();
+      const TC *Pk = P + k * kStepBuf + 8 * rg * CL, *Qk = Q + (k & 1) * kStepBuf;
+      if (rg > k) {
+        step_tile(c[0], Pk, Qk + 8 * (k + 1) * CL, CL, g, t);
+        hand_over(c[0]);
+      }
+      __syncthreads();
+      if (rg > k + 1) {
+#pragma unroll
+        for (int j = 1; j < 7; j++) {
+          if (k + 1 + j <= rg) step_tile(c[j], Pk, Qk + 8 * (k + 1 + j) * CL, CL, g, t);
+          c[j - 1][0] = c[j][0];
+          c[j - 1][1] = c[j][1];
+        }
+      }
+    }
+  };
+  for (int pass = 0; pass < 2; pass++) {
+    TC first[2];
+    tile(0, first);
+    hand_over(first);
+    if (tid == 0) {
+      failAt = kPanel;  // none
+      redo = nNeg = nPert = inexact = 0;
+    }
+    __syncthreads();
+    if (warp >= 2)
+      trailing();
+    else if (pass == 0)
+      panel(std::false_type());
+    else
+      panel(std::true_type());
+    __syncthreads();
+    if (!inexact) break;  // (the second pass sets it never)
+    __syncthreads();
+  }
+  // the pivots: test and count, the columns' scales
+  if (tid < kPanel) {
+    double d = -(double)P[(tid >> 3) * kStepBuf + tid * CL + (tid & 7)];
+    bool bad = false, small = false;
+    if (LDLT) {
+      small = tid < w && !(fabs(d) >= (double)tau);
+      bad = small && !isfinite(d);
+      if (small) d = d < 0.0 ? -(double)tau : (double)tau;
+      const int neg = __popc(__ballot_sync(0xffffffffu, tid < w && d < 0.0));
+      const int pert = __popc(__ballot_sync(0xffffffffu, small));
+      if (lane == 0) {
+        atomicAdd(&nNeg, neg);
+        atomicAdd(&nPert, pert);
+        if (LB && pert) redo = 1;
+      }
+    } else {
+      bad = tid < w && !(d > 0.0);
+    }
+    const unsigned mask = __ballot_sync(0xffffffffu, bad);
+    if (lane == 0 && mask) atomicMin(&failAt, 32 * warp + __ffs(mask) - 1);
+    const double dl = LDLT ? d : sqrt(d);
+    diag[tid] = dl;
+    scale[tid] = 1.0 / dl;
+  }
+  __syncthreads();
+  if (LB) {  // the multipliers a / d of the strictly lower part (a failed pivot exceeds the bound too)
+    for (int e = tid; e < kPanel * kPanel; e += 256) {
+      const int r = e & (kPanel - 1), j = e >> 6;
+      if (r > j && r < w && !(fabs((double)P[(j >> 3) * kStepBuf + r * CL + (j & 7)]) <= lbound * fabs(diag[j]))) redo = 1;
+    }
+    __syncthreads();
+    if (redo) return 2;
+  }
+  if (failAt < kPanel) {
+    if (tid == 0) atomicMin(status, status_word(f + c0 + failAt, LDLT ? 2 : 1, s));
+    return 1;
+  }
+  if (warp >= 2) {  // the columns: a lane per row, eight columns at a time
+    const int r = tid & (kPanel - 1);
+    for (int p = (tid >> 6) - 1; p < 8; p += 3) {
+      if (r < 8 * p || r >= w) continue;
+      const TC *Pr = P + p * kStepBuf + r * CL;
+      T *dst = Lp + (int64_t)(8 * p) * m + r;
+      T v[8];
+#pragma unroll
+      for (int u = 0; u < 8; u += 2) {
+        const V2 a = *reinterpret_cast<const V2 *>(Pr + u);
+        v[u] = (T)(-(double)a.x * scale[8 * p + u]);
+        v[u + 1] = (T)(-(double)a.y * scale[8 * p + u + 1]);
+      }
+#pragma unroll
+      for (int u = 0; u < 8; u++)
+        if (r >= 8 * p + u) dst[(int64_t)u * m] = r > 8 * p + u ? v[u] : LDLT ? T(1) : (T)diag[r];
+    }
+  } else {  // column j of inv(L_pp): forward substitution with the unit block, rows over the diagonal
+    const int p = tid >> 3, j = tid & 7;
+    const TC *Pp = P + p * kStepBuf + 8 * p * CL;
+    double x[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      double v = 0.0;
+#pragma unroll
+      for (int u = 0; u < i; u++) {
+        const double sc = scale[8 * p + u];
+        v += ((double)Pp[i * CL + u] * (LDLT ? sc : sc * sc)) * x[u];
+      }
+      x[i] = i < j ? 0.0 : i == j ? 1.0 : v;  // (P holds -a)
+      Linv[64 * p + 8 * i + j] = x[i] * (LDLT ? 1.0 : scale[8 * p + i]);
+    }
+  }
+  if (LDLT) {
+    if (tid < w) ld.D[f + c0 + tid] = diag[tid];
+    if (tid == 0) {
+      atomicAdd(ld.counts, nNeg);
+      atomicAdd(ld.counts + 1, nPert);
+    }
+  }
+  return 0;
+}
+
+// (value, index) of the largest value over the warp, the smallest index on ties (every lane gets the result)
+__device__ __forceinline__ void warp_argmax(double &v, int &i) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double ov = __shfl_xor_sync(0xffffffffu, v, o);
+    const int oi = __shfl_xor_sync(0xffffffffu, i, o);
+    if (ov > v || (ov == v && oi < i)) {
+      v = ov;
+      i = oi;
+    }
+  }
+}
+
+// Bunch-Kaufman LDL^T of a pivot block, the pivot search restricted to the block's w columns (so the supernode
+// partition and every row structure stay the reference's): at column k, with colmax = max_{i>k} |B(i, k)| (row r),
+// a 1 x 1 pivot k when |B(k, k)| >= alpha colmax or |B(k, k)| rowmax >= alpha colmax^2 (rowmax = max_{j != r}
+// |B(r, j)|), a 1 x 1 pivot r when |B(r, r)| >= alpha rowmax, else the 2 x 2 pivot (k, r); alpha = (1 + sqrt 17) / 8
+// (Bunch and Kaufman, Math. Comp. 31, 1977). Each interchange is applied to the block's whole rows, the L columns
+// already computed included, so that P B P^T = L D L^T with L unit lower triangular (L(k + 1, k) = 0 inside a 2 x 2
+// pivot, whose off-diagonal is D(k + 1, k)). A column with no entry at or above tau keeps the reference's static
+// perturbation (|d| < tau -> -+tau, a non-finite one fails; ldlt.mjs:513-522). FP64 arithmetic for every T.
+// S: 64 x 65 doubles of shared workspace (a full symmetric copy, S[j][i] = B(i, j)); Ds: the updated block (lower part).
+// Writes L to Lp (ld m), D, Doff and piv, adds the inertia (a 2 x 2 pivot with a
+// negative determinant has one negative eigenvalue, with a positive one two when its diagonal is negative) and the
+// perturbed count. Returns false (status set) on a non-finite pivot; nothing is written then. Called by every thread.
+template <class T>
+__device__ bool bk_block(const double *Ds, double (*S)[kPanel + 1], T *Lp, double *Linv, int m, int w, int f, int c0, int s,
+                         unsigned long long *status, const LdltArgs<T> &ld) {
+  __shared__ int sPerm[kPanel];
+  __shared__ double sD[kPanel], sE[kPanel], sC0[kPanel], sC1[kPanel];
+  __shared__ int sStep, sKp, sFail, sNeg, sPert;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = blockDim.x;
+  const double tau = ld.scal[1];
+  const double alpha = 0.64038820320220756;  // (1 + sqrt(17)) / 8
+  for (int e = tid; e < kPanel * kPanel; e += nthr) {
+    const int i = e & (kPanel - 1), j = e >> 6;
+    double v = i == j ? 1.0 : 0.0;
+    if (i < w && j < w) v = i >= j ? Ds[sw(i, j)] : Ds[sw(j, i)];
+    S[j][i] = v;
+  }
+  if (tid < kPanel) {
+    sPerm[tid] = tid;
+    sD[tid] = 1.0;
+    sE[tid] = 0.0;
+  }
+  if (tid == 0) {
+    sFail = -1;
+    sNeg = 0;
+    sPert = 0;
+  }
+  __syncthreads();
+  for (int k = 0; k < w;) {
+    if (warp == 0) {  // the pivot choice
+      double cm = -1.0;
+      int im = -1;
+      for (int i = k + 1 + lane; i < w; i += 32) {
+        const double a = fabs(S[k][i]);
+        if (a > cm) {
+          cm = a;
+          im = i;
+        }
+      }
+      warp_argmax(cm, im);
+      const double colmax = cm > 0.0 ? cm : 0.0, absakk = fabs(S[k][k]);
+      int step = 1, kp = k;
+      if (colmax > 0.0 && !(absakk >= alpha * colmax)) {  // (a NaN diagonal takes the 1 x 1 path and fails below)
+        double rm = 0.0;
+        for (int j = k + lane; j < w; j += 32)
+          if (j != im) rm = fmax(rm, fabs(S[j][im]));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) rm = fmax(rm, __shfl_xor_sync(0xffffffffu, rm, o));
+        if (absakk * rm >= alpha * colmax * colmax) {
+          kp = k;
+        } else if (fabs(S[im][im]) >= alpha * rm) {
+          kp = im;
+        } else {
+          step = 2;
+          kp = im;
+        }
+      }
+      if (lane == 0) {
+        sStep = step;
+        sKp = kp;
+      }
+    }
+    __syncthreads();
+    const int step = sStep, kp = sKp, kk = k + step - 1, k1 = k + step;
+    if (kp != kk) {  // interchange kk and kp: whole rows (L columns included), then the trailing columns
+      if (tid < w) {
+        const double t = S[tid][kk];
+        S[tid][kk] = S[tid][kp];
+        S[tid][kp] = t;
+      }
+      __syncthreads();
+      if (tid >= k && tid < w) {
+        const double t = S[kk][tid];
+        S[kk][tid] = S[kp][tid];
+        S[kp][tid] = t;
+      }
+      if (tid == 0) {
+        const int t = sPerm[kk];
+        sPerm[kk] = sPerm[kp];
+        sPerm[kp] = t;
+      }
+      __syncthreads();
+    }
+    const int nt = w - k1;
+    if (step == 1) {
+      double d = S[k][k];
+      const bool small = !(fabs(d) >= tau);
+      if (small && isfinite(d)) d = d < 0.0 ? -tau : tau;
+      if (tid < w) sC0[tid] = S[k][tid];  // column k, unscaled
+      if (tid == 0) {
+        sD[k] = d;
+        if (!isfinite(d) && sFail < 0) sFail = k;
+        sNeg += d < 0.0 ? 1 : 0;
+        sPert += small ? 1 : 0;
+      }
+      __syncthreads();
+      if (sFail >= 0) break;  // block-uniform
+      const double inv = 1.0 / d;
+      for (int e = tid; e < nt * nt; e += nthr) {
+        const int i = k1 + e % nt, j = k1 + e / nt;
+        S[j][i] -= sC0[i] * (sC0[j] * inv);
+      }
+      if (tid >= k1 && tid < w) S[k][tid] = sC0[tid] * inv;  // L(i, k)
+    } else {
+      // D_k = e [[a, 1], [1, c]], D_k^-1 = (t / e) [[c, -1], [-1, a]] with a = d11 / e, c = d22 / e, t = 1 / (a c - 1)
+      const double d11 = S[k][k], e21 = S[k][k + 1], d22 = S[k + 1][k + 1];
+      const double a = d11 / e21, c = d22 / e21, te = (1.0 / (a * c - 1.0)) / e21;
+      if (tid < w) {
+        sC0[tid] = S[k][tid];
+        sC1[tid] = S[k + 1][tid];
+      }
+      if (tid == 0) {
+        sD[k] = d11;
+        sD[k + 1] = d22;
+        sE[k] = e21;
+        if (!(isfinite(te) && isfinite(a) && isfinite(c)) && sFail < 0) sFail = k;
+        sNeg += a * c - 1.0 < 0.0 ? 1 : (d11 < 0.0 ? 2 : 0);
+      }
+      __syncthreads();
+      if (sFail >= 0) break;  // block-uniform
+      for (int e = tid; e < nt * nt; e += nthr) {
+        const int i = k1 + e % nt, j = k1 + e / nt;
+        const double l1 = te * (c * sC0[i] - sC1[i]), l2 = te * (a * sC1[i] - sC0[i]);
+        S[j][i] -= l1 * sC0[j] + l2 * sC1[j];
+      }
+      if (tid >= k1 && tid < w) {
+        S[k][tid] = te * (c * sC0[tid] - sC1[tid]);  // L(i, k)
+        S[k + 1][tid] = te * (a * sC1[tid] - sC0[tid]);  // L(i, k + 1)
+      }
+      if (tid == 0) S[k][k + 1] = 0.0;  // L(k + 1, k)
+    }
+    __syncthreads();
+    k += step;
+  }
+  __syncthreads();
+  if (sFail >= 0) {
+    if (tid == 0) atomicMin(status, status_word(f + c0 + sFail, 2, s));
+    return false;
+  }
+  for (int e = tid; e < w * w; e += nthr) {
+    const int i = e % w, j = e / w;
+    if (i >= j) Lp[(int64_t)j * m + i] = (T)(i == j ? 1.0 : S[j][i]);
+  }
+  if (tid < kPanel) {  // the inverses of the diagonal 8 x 8 blocks of the unit L, for the strips' TRSM
+    const int p = tid >> 3, j = tid & 7;
+    double x[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      double v = 0.0;
+#pragma unroll
+      for (int u = 0; u < i; u++) v += (8 * p + i < w ? S[8 * p + u][8 * p + i] : 0.0) * x[u];
+      x[i] = i < j ? 0.0 : i == j ? 1.0 : -v;
+      Linv[64 * p + 8 * i + j] = x[i];
+    }
+  }
+  if (tid < w) {
+    ld.D[f + c0 + tid] = sD[tid];
+    ld.Doff[f + c0 + tid] = sE[tid];
+    ld.piv[f + c0 + tid] = sPerm[tid];
+  }
+  if (tid == 0) {
+    atomicAdd(ld.counts, sNeg);
+    atomicAdd(ld.counts + 1, sPert);
+  }
+  return true;
+}
+
+// Wait (thread 0, bounded) until *p >= need; false when the factorization has failed (a pivot, or a wait that ran
+// out: status set). Thread 0 decides and the CTA follows it after the barrier, so every thread returns the same.
+__device__ __forceinline__ bool panel_wait(const int *p, int need, unsigned long long *status, long long limit) {
+  __shared__ int ok;
+  if (threadIdx.x == 0) {
+    long long spins = 0;
+    int v = 1;
+    while (ld_acquire(p) < need) {
+      if (panel_failed(status)) {
+        v = 0;
+        break;
+      }
+      if (++spins > limit) {
+        atomicMin(status, status_word(0x7fffffff, 3, 0));
+        v = 0;
+        break;
+      }
+      __nanosleep(32);
+    }
+    if (panel_failed(status)) v = 0;  // a failed pivot also releases its flag
+    ok = v;
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
+// Publish *p = v after this CTA's global writes: all threads pass the barrier first, and thread 0's release store
+// orders every write made before the barrier (by any thread of the CTA) before the flag, for a reader that acquires it.
+__device__ __forceinline__ void panel_release(int *p, int v) {
+  __syncthreads();
+  if (threadIdx.x == 0) st_release(p, v);
+}
+
+// C(8 x 64 of this warp) += N S^T: N the warp's A fragments (8 x 64), S a block in shared memory. Eight independent
+// accumulators between two products of one.
+__device__ __forceinline__ void update_row_group(double (&c)[8][2], const double (&n)[8][2], const double *S, int g,
+                                                 int t) {
+#pragma unroll
+  for (int q = 0; q < 8; q++) {
+    double2 v[8];
+#pragma unroll
+    for (int p = 0; p < 8; p++) v[p] = pair_at(S, 8 * p + g, 8 * q + 2 * t);
+#pragma unroll
+    for (int p = 0; p < 8; p++) mma884(c[p], n[q][0], v[p].x);
+#pragma unroll
+    for (int p = 0; p < 8; p++) mma884(c[p], n[q][1], v[p].y);
+  }
+}
+
+// One group of pivot blocks [g0, g1) of a front, a strip of up to 64 rows per CTA, CTAs ordered by an atomic ticket
+// (the diagonal strips of every item first, then the strips below the group). A strip takes the group's pivot blocks b
+// in order (a diagonal strip those before its own), left-looking:
+//   its rows of block b receive the earlier blocks q: C -= W_q X_q^T, with W_q its own solved rows and X_q the rows of
+//   diagonal strip b, waited for by D[b] >= q + 1 (the last W_q is still in registers, earlier ones are read back);
+//   then, after P[b], they are solved against the pivot block: W = C L_bb^-T by 8 x 8 blocks with the inverses of its
+//   diagonal blocks (Cholesky X = W; LDL^T with the unit L_bb, X = W D^-1; Bunch-Kaufman the columns in the block's
+//   pivot order first, then the 1 x 1 and 2 x 2 inverses of D).
+// A diagonal strip keeps its own pivot block in shared memory from the start, publishes D[j] = b + 1 after each solve,
+// subtracts W X^T from the block's lower part, and after its last solve factors it and publishes P[j].
+// Every wait is on a strip with a smaller ticket, which runs to completion without waiting on a larger one, so the
+// launch cannot deadlock whatever the number of resident CTAs. The columns right of the group receive the group's
+// update afterwards (k_update / k_update_mx, K = the group). Failure (a pivot, a bounded wait) sets the status and
+// releases P[b], so every waiter leaves.
+constexpr int kBlockElems = kPanel * kPanel;
+constexpr int kGroupSmem = 3 * kBlockElems * (int)sizeof(double);  // two CTAs per SM
+template <class T, bool LDLT, bool BK>
+__global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restrict__ items,
+                                                        const StripTask *__restrict__ strips, int nstrips, int *ticket,
+                                                        int *flags, DevPlan P, T *__restrict__ Lx,
+                                                        double *__restrict__ Linv, unsigned long long *status,
+                                                        __nv_bfloat16 *__restrict__ Shi, __nv_bfloat16 *__restrict__ Slo,
+                                                        LdltArgs<T> ld) {
+  extern __shared__ __align__(16) unsigned char gp_raw[];
+  double *Ls = reinterpret_cast<double *>(gp_raw);  // pivot block, rows of another diagonal strip, POTRF step buffers
+  double *Xs = Ls + kBlockElems;                    // this strip's solved rows (Bunch-Kaufman: column exchange)
+  double *Ds = Xs + kBlockElems;                    // a diagonal strip's own pivot block
+  __shared__ __align__(16) double Li[8 * 64];
+  __shared__ double dv[kPanel], dinv[kPanel];
+  __shared__ double dB[BK ? kPanel : 1];
+  __shared__ int dP[BK ? kPanel : 1], sPiv[BK ? kPanel : 1];
+  __shared__ int sTicket;
+  if (threadIdx.x == 0) sTicket = panel_failed(status) ? nstrips : atomicAdd(ticket, 1);
+  __syncthreads();
+  const int tk = sTicket;
+  if (tk >= nstrips) return;
+  const StripTask st = strips[tk];
+  const GroupItem it = items[st.item];
+  const int s = it.s, g0 = it.g0, g1 = it.g1;
+  const int f = P.snF[s], m = P.snM[s];
+  const int nb = (g1 - g0 + kPanel - 1) / kPanel;
+  const int r0 = st.r0, r1 = st.r1, jd = st.diag;
+  const int bmax = jd >= 0 ? jd : nb;  // pivot blocks whose rows below include this strip
+  const int64_t lxp = P.snLxp[s], sp = P.snSp[s];
+  T *L = Lx + lxp;
+  int *Pf = flags + it.flag0, *Df = Pf + nb;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int lr = 8 * row_group(warp) + g, row = r0 + lr;  // this lane's row of every fragment
+  const bool act = row < r1;
+  const int ld8 = (m + 7) & ~7;
+  if (jd >= 0) load_block(Ds, L, m, r0, r1 - r0, r0, r1 - r0, true, true);
+  double nx[8][2];  // -W of the block solved last
+#pragma unroll
+  for (int p = 0; p < 8; p++) nx[p][0] = nx[p][1] = 0.0;
+  for (int b = 0; b < bmax; b++) {
+    const int c0 = g0 + b * kPanel, w = min(kPanel, g1 - c0);
+    double x[8][2];  // the strip's rows of block b
+    const T *src = L + (int64_t)(c0 + 2 * t) * m + row;
+#pragma unroll
+    for (int p = 0; p < 8; p++)
+#pragma unroll
+      for (int u = 0; u < 2; u++)
+        x[p][u] = act && 8 * p + 2 * t + u < w ? (double)__ldcg(src + (int64_t)(8 * p + u) * m) : 0.0;
+    for (int q = 0; q < b; q++) {
+      const int cq = g0 + q * kPanel;
+      if (b > 1) {  // read the strip's solved rows back (with one earlier block they are still in registers)
+#pragma unroll
+        for (int p = 0; p < 8; p++)
+#pragma unroll
+          for (int u = 0; u < 2; u++) {
+            const int cc = cq + 8 * p + 2 * t + u;  // (every pivot block before the last of a group is full)
+            double v = 0.0;
+            if (act) {
+              const int64_t at = (int64_t)cc * m + row;
+              v = BK ? (double)__ldcg(ld.W + lxp + at) : (double)__ldcg(L + at);
+              if (LDLT && !BK) v *= __ldcg(ld.D + f + cc);
+            }
+            nx[p][u] = -v;
+          }
+      }
+      if (!panel_wait(Df + b, q + 1, status, P.spin)) return;
+      load_block(Ls, L, m, c0, w, cq, kPanel, false, false);
+      __syncthreads();
+      update_row_group(x, nx, Ls, g, t);
+    }
+    if (!panel_wait(Pf + b, 1, status, P.spin)) return;  // (its barrier: every warp is done with Ls)
+    load_block(Ls, L, m, c0, w, c0, w, true, true);
+    if (tid < kPanel) {
+      if constexpr (BK) {
+        double a = 1.0, bb = 0.0;
+        int pc = tid;
+        if (tid < w) {
+          const double *D = ld.D + f + c0, *E = ld.Doff + f + c0;
+          const double d = __ldcg(D + tid), en = __ldcg(E + tid), ep = tid > 0 ? __ldcg(E + tid - 1) : 0.0;
+          if (en != 0.0 || ep != 0.0) {  // 2 x 2 pivot (tid, tid + 1) or (tid - 1, tid): the inverse as in bk_block
+            const bool first = en != 0.0;
+            const double e = first ? en : ep;
+            const double d11 = first ? d : __ldcg(D + tid - 1), d22 = first ? __ldcg(D + tid + 1) : d;
+            const double aa = d11 / e, cc = d22 / e, te = (1.0 / (aa * cc - 1.0)) / e;
+            a = te * (first ? cc : aa);
+            bb = -te;
+            pc = first ? tid + 1 : tid - 1;
+          } else {
+            a = 1.0 / d;
+          }
+        }
+        dinv[tid] = a;
+        dB[tid] = bb;
+        dP[tid] = pc;
+        sPiv[tid] = tid < w ? __ldcg(ld.piv + f + c0 + tid) : tid;
+      } else if constexpr (LDLT) {
+        const double d = tid < w ? __ldcg(ld.D + f + c0 + tid) : 1.0;
+        dv[tid] = d;
+        dinv[tid] = 1.0 / d;
+      }
+    }
+    *reinterpret_cast<double2 *>(Li + 2 * tid) =
+        __ldcg(reinterpret_cast<const double2 *>(Linv + ((int64_t)(it.flag0 / 2) + b) * (8 * 64) + 2 * tid));
+    __syncthreads();
+    if constexpr (BK) {  // the strip's columns in the block's pivot order (each warp exchanges its own rows)
+#pragma unroll
+      for (int p = 0; p < 8; p++) set_pair(Xs, lr, 8 * p + 2 * t, x[p][0], x[p][1]);
+      __syncwarp();
+#pragma unroll
+      for (int p = 0; p < 8; p++)
+#pragma unroll
+        for (int u = 0; u < 2; u++) x[p][u] = Xs[sw(lr, sPiv[8 * p + 2 * t + u])];
+      __syncwarp();
+    }
+    // W = C L_bb^-T, right-looking over the 8-column blocks: solved with the block's inverse, then subtracted from the
+    // later ones
+#pragma unroll
+    for (int p = 0; p < 8; p++) {
+      const double2 iv = *reinterpret_cast<const double2 *>(Li + 64 * p + 8 * g + 2 * t);
+      double wv[2] = {0.0, 0.0};
+      mma884(wv, x[p][0], iv.x);
+      mma884(wv, x[p][1], iv.y);
+      x[p][0] = wv[0];
+      x[p][1] = wv[1];
+#pragma unroll
+      for (int p2 = p + 1; p2 < 8; p2++) {
+        const double2 l = pair_at(Ls, 8 * p2 + g, 8 * p + 2 * t);
+        mma884(x[p2], -wv[0], l.x);
+        mma884(x[p2], -wv[1], l.y);
+      }
+    }
+    if constexpr (BK) {
+#pragma unroll
+      for (int p = 0; p < 8; p++) set_pair(Xs, lr, 8 * p + 2 * t, x[p][0], x[p][1]);
+      __syncwarp();
+    }
+    // x := L21's entries, rounded to the storage; nx := -W (W = x D for LDL^T)
+#pragma unroll
+    for (int p = 0; p < 8; p++)
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const int cc = 8 * p + 2 * t + u;
+        const double wv = x[p][u];
+        double xv = wv;
+        if constexpr (BK)
+          xv = dinv[cc] * wv + dB[cc] * Xs[sw(lr, dP[cc])];
+        else if constexpr (LDLT)
+          xv = wv * dinv[cc];
+        x[p][u] = (double)(T)xv;
+        nx[p][u] = BK ? -wv : LDLT ? -x[p][u] * dv[cc] : -x[p][u];
+        if (BK && act && cc < w) ld.W[lxp + (int64_t)(c0 + cc) * m + row] = (T)wv;
+      }
+    if constexpr (BK) __syncwarp();
+#pragma unroll
+    for (int p = 0; p < 8; p++) set_pair(Xs, lr, 8 * p + 2 * t, x[p][0], x[p][1]);
+    __syncthreads();
+    // written column by column, a warp's lanes on consecutive rows (the fragments' 8-row pieces of a column cost FP32
+    // and BF16 stores a partial sector each)
+    for (int cc = warp; cc < w; cc += 8) {
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int r = lane + 32 * h;
+        if (r0 + r >= r1) continue;
+        const double xv = Xs[sw(r, cc)];
+        const int64_t at = (int64_t)(c0 + cc) * m + r0 + r;
+        L[at] = (T)xv;
+        if (LDLT && !BK && ld.W) ld.W[lxp + at] = (T)(xv * dv[cc]);
+        if constexpr (std::is_same<T, float>::value) {  // the BF16 hi / lo pairs of the tensor-core update's operands
+          const int64_t as = sp + (int64_t)(c0 + cc) * ld8 + r0 + r;
+          const float xt = (float)xv;
+          const __nv_bfloat16 hi = __float2bfloat16_rn(xt);
+          Shi[as] = hi;
+          Slo[as] = __float2bfloat16_rn(xt - __bfloat162float(hi));
+          if (LDLT) {
+            const float wt = (float)(xv * dv[cc]);
+            const __nv_bfloat16 whi = __float2bfloat16_rn(wt);
+            ld.Whi[as] = whi;
+            ld.Wlo[as] = __float2bfloat16_rn(wt - __bfloat162float(whi));
+          }
+        }
+      }
+    }
+    if (jd < 0) continue;
+    panel_release(Df + jd, b + 1);
+    // the strip's own pivot block: tiles (rg, 0 .. rg) of D -= W X^T, two at a time
+    for (int nt = 0; nt <= lr >> 3; nt += 2) {
+      const bool two = nt + 1 <= lr >> 3;
+      const int nb2 = two ? nt + 1 : nt;
+      const double2 va = pair_at(Ds, lr, 8 * nt + 2 * t), vb = pair_at(Ds, lr, 8 * nb2 + 2 * t);
+      double ca[2] = {va.x, va.y}, cb[2] = {vb.x, vb.y};
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const double2 xa = pair_at(Xs, 8 * nt + g, 8 * q + 2 * t), xb = pair_at(Xs, 8 * nb2 + g, 8 * q + 2 * t);
+        mma884(ca, nx[q][0], xa.x);
+        if (two) mma884(cb, nx[q][0], xb.x);
+        mma884(ca, nx[q][1], xa.y);
+        if (two) mma884(cb, nx[q][1], xb.y);
+      }
+      set_pair(Ds, lr, 8 * nt + 2 * t, ca[0], ca[1]);
+      if (two) set_pair(Ds, lr, 8 * nt + 8 + 2 * t, cb[0], cb[1]);
+    }
+  }
+  if (jd >= 0) {  // this strip's own pivot block, fully updated: factor it and publish it (also after a failure)
+    const int c0 = g0 + jd * kPanel, w = min(kPanel, g1 - c0);
+    T *Lp = L + (int64_t)c0 * m + c0;
+    double *Lb = Linv + ((int64_t)(it.flag0 / 2) + jd) * (8 * 64);
+    __syncthreads();  // Ds complete (also when the strip had no earlier pivot block); Ls and Xs free
+    if constexpr (BK) {
+      // Bunch-Kaufman keeps every pivot of the block in place exactly when each multiplier is at most 1 / alpha in
+      // magnitude and no pivot needs the perturbation: try the unpivoted LDL^T first, else redo the block with pivots
+      // from its untouched entries
+      const int r = potrf_block<T, double, true, true>(Ds, Ls, Lp, Lb, m, w, f, c0, s, status, ld, 1.0 / 0.64038820320220756);
+      if (r == 2) {
+        bk_block<T>(Ds, reinterpret_cast<double(*)[kPanel + 1]>(gp_raw), Lp, Lb, m, w, f, c0, s, status, ld);
+      } else if (r == 0 && tid < w) {  // the identity pivot order, 1 x 1 pivots
+        ld.piv[f + c0 + tid] = tid;
+        ld.Doff[f + c0 + tid] = 0.0;
+      }
+    } else {
+      using TC = typename std::conditional<LDLT, double, T>::type;
+      potrf_block<T, TC, LDLT, false>(Ds, Ls, Lp, Lb, m, w, f, c0, s, status, ld, -1.0);
+    }
+    panel_release(Pf + jd, 1);
+  }
+}
+
+}  // namespace
+
+template <class T, bool LDLT, bool BK>
+static cudaError_t init_one() {
+  return cudaFuncSetAttribute(k_group_panel<T, LDLT, BK>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupSmem);
+}
+cudaError_t init_group_panel_attributes() {
+  cudaError_t e = init_one<double, false, false>();
+  if (e == cudaSuccess) e = init_one<double, true, false>();
+  if (e == cudaSuccess) e = init_one<double, true, true>();
+  if (e == cudaSuccess) e = init_one<float, false, false>();
+  if (e == cudaSuccess) e = init_one<float, true, false>();
+  return e;
+}
+
+template <class T>
+void launch_group_panel(const GroupItem *items, const StripTask *strips, int nstrips, int *ticket, int *flags,
+                        const DevPlan &P, T *Lx, double *Linv, unsigned long long *status, __nv_bfloat16 *Shi,
+                        __nv_bfloat16 *Slo, const LdltArgs<T> &ld, cudaStream_t st) {
+  if (nstrips <= 0) return;
+  auto run = [&](auto kernel) {
+    kernel<<<(unsigned)nstrips, 256, kGroupSmem, st>>>(items, strips, nstrips, ticket, flags, P, Lx, Linv, status, Shi,
+                                                       Slo, ld);
+  };
+  if constexpr (std::is_same<T, double>::value)
+    if (ld.piv) return run(k_group_panel<T, true, true>);  // Bunch-Kaufman pivot blocks
+  if (ld.scal)
+    run(k_group_panel<T, true, false>);
+  else
+    run(k_group_panel<T, false, false>);
+}
+template void launch_group_panel<double>(const GroupItem *, const StripTask *, int, int *, int *, const DevPlan &,
+                                         double *, double *, unsigned long long *, __nv_bfloat16 *, __nv_bfloat16 *,
+                                         const LdltArgs<double> &, cudaStream_t);
+template void launch_group_panel<float>(const GroupItem *, const StripTask *, int, int *, int *, const DevPlan &,
+                                         float *, double *, unsigned long long *, __nv_bfloat16 *, __nv_bfloat16 *,
+                                         const LdltArgs<float> &, cudaStream_t);
+
+}  // namespace amp
