@@ -105,3 +105,18 @@ def test_first_failing_column(bad):
     num = A.NumericFactor(sym)
     assert not num.factor(v)
     assert num.failColumn == bad
+
+
+@pytest.mark.parametrize("border", [63, 640, 2101])
+def test_update_block_tiles(border):
+    """Update launches of few tiles (half a task per CTA) and of more than the CTAs in flight (whole tasks)."""
+    M = bordered([130, 151], border, 11)
+    n = M.shape[0]
+    pat, v = dense_csr(M)
+    sym = A.analyze(pat, perm=np.arange(n, dtype=np.int32))
+    num = A.NumericFactor(sym)
+    assert num.factor(v)
+    b = np.random.default_rng(2).uniform(-1, 1, n)
+    x = num.solve_block(b[None, :])[0]
+    ref = np.linalg.solve(M, b)
+    assert np.max(np.abs(x - ref)) <= 10 * 10 * n * EPS[A.FP64] * np.max(np.abs(ref))
