@@ -203,6 +203,8 @@ struct amp_factor_s {
   cudaStream_t side = nullptr;                      // look-ahead: part B of the panel steps' updates
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t evPanel = nullptr, evSide = nullptr;  // look-ahead ordering between the two streams
+  cudaStream_t front[2] = {nullptr, nullptr};       // a level's small fronts beside its large ones (SmallFork)
+  cudaEvent_t evFork = nullptr, evFront[2] = {nullptr, nullptr};
   DevMem mem;
   double *dLx = nullptr, *dU = nullptr, *dD = nullptr, *dValues = nullptr;
   float *dL32 = nullptr, *dU32 = nullptr;           // mixed precision: FP32 factor and update arena
@@ -277,6 +279,11 @@ struct amp_factor_s {
     if (evPanel) cudaEventDestroy(evPanel);
     if (evSide) cudaEventDestroy(evSide);
     if (side) cudaStreamDestroy(side);
+    if (evFork) cudaEventDestroy(evFork);
+    for (int k = 0; k < 2; k++) {
+      if (evFront[k]) cudaEventDestroy(evFront[k]);
+      if (front[k]) cudaStreamDestroy(front[k]);
+    }
     if (stream) cudaStreamDestroy(stream);
   }
 };
@@ -412,19 +419,50 @@ struct LookAhead {
   }
 };
 
-// the small fronts of level L (whole fronts, one warp or one CTA each)
+// The small fronts of level L (whole fronts, one warp or one CTA each). They depend on the levels below only, like the
+// level's large fronts, so the kinds that a level has run beside one another: the warp fronts on the first of two more
+// streams, the CTA fronts on the second when the level also has large fronts (on the factor's stream). A level's kinds
+// one after another took their sum, e.g. 44 us for 34 tiny and 14 small fronts of a 2D mesh whose longest takes 15.
+// join() makes the factor's stream wait for them (before the next level).
 template <class T>
-void enqueue_small_fronts(amp_factor *f, int L, T *Lx, T *U, const amp::LdltArgs<T> &la) {
-  const amp::Plan &P = f->plan->P;
-  const int64_t t0 = P.tinyPtr[L], t1 = P.tinyPtr[L + 1], s0 = P.smallPtr[L], s1 = P.smallPtr[L + 1];
-  if (t1 == t0 && s1 == s0) return;
-  const double scale = sizeof(T) / 8.0;
-  timed(f, K_FRONTS, 2.0 * P.frontLvlFlops[L], P.frontLvlBytes[L] * scale, [&] {
-    return amp::launch_fronts_small<T>(f->plan->dTinySn + t0, (int)(t1 - t0), (int)(P.tinyMid[L] - t0),
-                                       f->plan->dSmallSn + s0, (int)(s1 - s0), P.smallMaxM[L], f->plan->dp,
-                                       f->dValues, Lx, U, f->dStatus, la, f->stream);
-  });
-}
+struct SmallFork {
+  amp_factor *f;
+  bool used[2] = {false, false};
+  void launch(int L, T *Lx, T *U, const amp::LdltArgs<T> &la) {
+    const amp::Plan &P = f->plan->P;
+    const int64_t t0 = P.tinyPtr[L], t1 = P.tinyPtr[L + 1], s0 = P.smallPtr[L], s1 = P.smallPtr[L + 1];
+    const int64_t sm = P.smallMid[L];
+    const bool large = P.asmLvlPtr[L + 1] > P.asmLvlPtr[L];
+    if (t1 == t0 && s1 == s0) return;
+    const int *small = f->plan->dSmallSn;
+    const amp::SmallClass none{nullptr, 0, 0, 0};
+    const amp::SmallClass half{small + s0, (int)(sm - s0), P.smallMaxM[2 * L], P.smallMaxNc[2 * L]};
+    const amp::SmallClass full{small + sm, (int)(s1 - sm), P.smallMaxM[2 * L + 1], P.smallMaxNc[2 * L + 1]};
+    const bool forkTiny = t1 > t0 && (large || s1 > s0), forkSmall = s1 > s0 && large;
+    if (forkTiny || forkSmall) ck(cudaEventRecord(f->evFork, f->stream), "event");
+    const double scale = sizeof(T) / 8.0, tot = (double)(t1 - t0 + s1 - s0);
+    auto run = [&](int k, bool fork, const amp::SmallFronts &fr, double count) {
+      const cudaStream_t st = fork ? f->front[k] : f->stream;
+      if (fork) ck(cudaStreamWaitEvent(st, f->evFork, 0), "wait");
+      timed_on(f, st, K_FRONTS, 2.0 * P.frontLvlFlops[L] * count / tot, P.frontLvlBytes[L] * scale * count / tot, [&] {
+        return amp::launch_fronts_small<T>(fr, f->plan->dp, f->dValues, Lx, U, f->dStatus, la, st);
+      });
+      if (fork) {
+        ck(cudaEventRecord(f->evFront[k], st), "event");
+        used[k] = true;
+      }
+    };
+    if (t1 > t0)
+      run(0, forkTiny, {f->plan->dTinySn + t0, (int)(t1 - t0), (int)(P.tinyMid[L] - t0), none, none}, (double)(t1 - t0));
+    if (s1 > s0) run(1, forkSmall, {nullptr, 0, 0, half, full}, (double)(s1 - s0));
+  }
+  void join() {
+    for (int k = 0; k < 2; k++) {
+      if (used[k]) ck(cudaStreamWaitEvent(f->stream, f->evFront[k], 0), "wait");
+      used[k] = false;
+    }
+  }
+};
 
 // chain matrices of consecutive diagonal blocks for the one-vector sweeps (after the inverses)
 template <class T>
@@ -454,7 +492,8 @@ void enqueue_factor(amp_factor *f) {
       amp::launch_ldlt_tau(f->dValues, dp, f->dScal, st);
     }
     for (int L = 0; L < P.nlevels; L++) {
-      enqueue_small_fronts<float>(f, L, f->dL32, f->dU32, ld32);
+      SmallFork<float> small{f};
+      small.launch(L, f->dL32, f->dU32, ld32);
       if (P.asmLvlPtr[L + 1] > P.asmLvlPtr[L])
         timed(f, K_ASSEMBLE, 0.0, P.asmLvlBytes[L] / 2, [&] {
           amp::launch_assemble<float>(f->plan->dAsm + P.asmLvlPtr[L], f->plan->dAsmCh, P.asmLvlPtr[L + 1] - P.asmLvlPtr[L], dp,
@@ -488,6 +527,7 @@ void enqueue_factor(amp_factor *f) {
           amp::launch_update_mx(f->plan->dMixU + u0, u1 - u0, f->dMaps, f->dL32, f->dU32, f->dStatus,
                                 amp::num_sms(), st, 256, f->waitSpins);
         });
+      small.join();
     }
     if (P.nflags)
       timed(f, K_DIAGINV, 0.0, 8.0 * (double)inv_elems(P),
@@ -510,7 +550,8 @@ void enqueue_factor(amp_factor *f) {
     amp::launch_ldlt_tau(f->dValues, dp, f->dScal, st);
   }
   for (int L = 0; L < P.nlevels; L++) {
-    enqueue_small_fronts<double>(f, L, f->dLx, f->dU, ld);
+    SmallFork<double> small{f};
+    small.launch(L, f->dLx, f->dU, ld);
     if (P.asmLvlPtr[L + 1] > P.asmLvlPtr[L])
       timed(f, K_ASSEMBLE, 0.0, P.asmLvlBytes[L], [&] {
         amp::launch_assemble<double>(f->plan->dAsm + P.asmLvlPtr[L], f->plan->dAsmCh, P.asmLvlPtr[L + 1] - P.asmLvlPtr[L], dp,
@@ -543,6 +584,7 @@ void enqueue_factor(amp_factor *f) {
         amp::launch_update(f->plan->dUTile + P.uLvlPtr[L], P.uLvlPtr[L + 1] - P.uLvlPtr[L], dp, f->dLx, f->dU, ld.W,
                            f->dStatus, st);
       });
+    small.join();
   }
   if (P.nflags)
     timed(f, K_DIAGINV, 0.0, 16.0 * (double)inv_elems(P),
@@ -1256,6 +1298,11 @@ int amp_factor_create(amp_plan *pl, const amp_factor_opts *opts, amp_factor **ou
       ck(cudaStreamCreateWithFlags(&f->side, cudaStreamNonBlocking), "cudaStreamCreate");
       ck(cudaEventCreateWithFlags(&f->evPanel, cudaEventDisableTiming), "cudaEventCreate");
       ck(cudaEventCreateWithFlags(&f->evSide, cudaEventDisableTiming), "cudaEventCreate");
+      ck(cudaEventCreateWithFlags(&f->evFork, cudaEventDisableTiming), "cudaEventCreate");
+      for (int k = 0; k < 2; k++) {
+        ck(cudaStreamCreateWithFlags(&f->front[k], cudaStreamNonBlocking), "cudaStreamCreate");
+        ck(cudaEventCreateWithFlags(&f->evFront[k], cudaEventDisableTiming), "cudaEventCreate");
+      }
       ck(cudaEventCreate(&f->ev0), "cudaEventCreate");
       ck(cudaEventCreate(&f->ev1), "cudaEventCreate");
       const amp::Plan &P = pl->P;

@@ -1,5 +1,5 @@
 // Small fronts: one warp (m <= 32, four or eight fronts per CTA) or one CTA (32 < m <= 128) per front does all of the
-// front's work for its level in shared memory, in one launch per level and size class:
+// front's work for its level, in one launch per level and size class:
 //   zero the front, add A's entries of the pivot columns (sparse.mjs:965-973), extend-add the children's update
 //   matrices in the reference's child order (sparse.mjs:974-985), factor the nc pivot columns right-looking over the
 //   whole trailing triangle (Cholesky sparse.mjs:995-1098; LDL^T with static pivot perturbation ldlt.mjs:450-562, or
@@ -7,14 +7,20 @@
 //   write the first nc columns to L (the reference layout) and the rest to the update matrix U (the arena).
 // Such fronts dominate 2D problems (the batched heat set: median m = 5, 97% with m <= 32), where the general path's
 // 64 x 64 pivot-block kernels and 128-row tiles would spend almost all of their work on padding, one launch per step.
+// What bounds them is the latency of one front, level after level: a 99-row root front took 144 us with a barrier and
+// two quotients per pivot column, 17 us now; a 76-row front with 15 pivots and two children 39 us, 17 now (about 5 us of
+// it the launch); the small fronts of a 64 x 64 heat problem 1,344 us, 620 now.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <type_traits>
 
 #include "../host/plan.hpp"
 #include "devplan.cuh"
+#include "launch.hpp"
+#include "pivot_steps.cuh"
 
 namespace amp {
 
@@ -24,6 +30,16 @@ namespace amp {
 template <int MAXM>
 constexpr int tiny_warps() {
   return MAXM <= kTinyMid ? 8 : 4;
+}
+// entries per lane in flight during the assembly, and CTAs per SM that the registers are held to: the m <= 16 class is
+// bound by the warps in flight (157,000 leaves of a batch: 262 us at 98 registers and two CTAs per SM)
+template <int MAXM>
+constexpr int tiny_batch() {
+  return MAXM <= kTinyMid ? 8 : 16;
+}
+template <int MAXM>
+constexpr int tiny_ctas() {
+  return MAXM <= kTinyMid ? 4 : 5;
 }
 
 template <int G>
@@ -50,96 +66,168 @@ __device__ __forceinline__ bool small_ldlt_pivot(T &d, T tau, int &neg, int &per
   return true;
 }
 
-// Children of one front whose metadata a group holds at a time (fetched in parallel, applied in the reference's order)
+// Children of one front whose metadata and row maps a CTA holds at a time (fetched in parallel, applied in the
+// reference's order); a map's entries are front positions below 128
 constexpr int kChildChunk = 32;
 struct ChildMeta {
   int muc[kChildChunk];
-  int64_t ea[kChildChunk], uo[kChildChunk];
+  int64_t uo[kChildChunk], ea[kChildChunk];
+  unsigned char map[kChildChunk][kSmallFront];
 };
 
-// Zero F (m x m), add A's entries of the pivot columns and the children's update matrices in the reference's order.
-template <class T, class TC, int G>
-__device__ void assemble_front(int s, const DevPlan &P, const double *__restrict__ values, const T *__restrict__ U,
-                               TC *F, int t, ChildMeta *cm) {
-  const int warp = t >> 5, lane = t & 31;
+// The latency of a front's assembly is its chain of dependent loads (the children's metadata, their maps, their update
+// matrices, one child after another), so the update matrices are read a batch ahead: while a batch of entries is
+// added to the front, the next one (of the same child or of the next) is in flight, up to 16 entries per lane.
+
+// Zero F (m x m, column-major), add A's entries of the pivot columns and the children's update matrices in the
+// reference's order. One warp, m <= 32: a lane per row of the child.
+template <class T, class TC, int kBatch>
+__device__ void assemble_warp(int s, const DevPlan &P, const double *__restrict__ values, const T *__restrict__ U,
+                              TC *F, int lane) {
   const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s];
-  for (int e = t; e < m * m; e += G) F[e] = TC(0);
-  group_sync<G>();
+  const int q0 = P.chPtr[s], nch = P.chPtr[s + 1] - q0;
+  const int p0 = P.asmColPtr[f], p1 = P.asmColPtr[f + nc];
+  for (int e = lane; e < m * m; e += 32) F[e] = TC(0);
+  __syncwarp();
   // A's entries of all nc pivot columns (one contiguous CSR range): slot dst = j m + i of the L panel, each (i, j) once
-  {
-    const int p0 = P.asmColPtr[f], p1 = P.asmColPtr[f + nc];
-    for (int p = p0 + t; p < p1; p += G) F[P.asmDst[p]] += (TC)(T)__ldg(values + P.asmSrc[p]);
-  }
-  group_sync<G>();
-  // children's update matrices, one after another (the map is injective within a child); the metadata of up to
-  // kChildChunk children is fetched at once, one child per thread
-  const int q0 = P.chPtr[s], q1 = P.chPtr[s + 1];
-  for (int qb = q0; qb < q1; qb += kChildChunk) {
-    const int nq = min(kChildChunk, q1 - qb);
+  for (int p = p0 + lane; p < p1; p += 32) F[P.asmDst[p]] += (TC)(T)__ldg(values + P.asmSrc[p]);
+  for (int qb = 0; qb < nch; qb += 32) {  // the metadata of up to 32 children, one per lane
+    const int nq = min(32, nch - qb);
     int muc = 0;
     int64_t ea = 0, uo = 0;
-    if (warp == 0 && lane < nq) {
-      const int c = P.chList[qb + lane];
+    if (lane < nq) {
+      const int c = P.chList[q0 + qb + lane];
       muc = P.snM[c] - P.snNc[c];
       ea = P.eaPtr[c];
       uo = P.snUoff[c];
     }
-    if constexpr (G > 32) {
-      if (qb > q0) __syncthreads();  // the previous chunk's metadata is read by all warps before it is replaced
-      if (warp == 0 && lane < nq) {
-        cm->muc[lane] = muc;
-        cm->ea[lane] = ea;
-        cm->uo[lane] = uo;
-      }
-      __syncthreads();
-    }
-    for (int q = 0; q < nq; q++) {
-      int mq;
-      int64_t eq, uq;
-      if constexpr (G == 32) {
-        mq = __shfl_sync(0xffffffffu, muc, q);
-        eq = __shfl_sync(0xffffffffu, ea, q);
-        uq = __shfl_sync(0xffffffffu, uo, q);
-      } else {
-        mq = cm->muc[q];
-        eq = cm->ea[q];
-        uq = cm->uo[q];
-      }
-      if (mq <= 0) continue;  // group-uniform
-      const int *map = P.eaMap + eq;
+    // batch (q, b0): columns [b0, b0 + kBatch) of child q, row a = lane; pos: the child row's front position
+    auto fetch = [&](int q, int b0, T(&v)[kBatch], int &mq, int &pos) {
+      mq = __shfl_sync(0xffffffffu, muc, q);
+      const int64_t eq = __shfl_sync(0xffffffffu, ea, q), uq = __shfl_sync(0xffffffffu, uo, q);
+      pos = lane < mq ? P.eaMap[eq + lane] : 0;
       const T *Uc = U + uq;
-      for (int e = t; e < mq * mq; e += G) {
-        const int b = e / mq, a = e - b * mq;
-        if (a >= b) F[map[b] * m + map[a]] += (TC)Uc[e];
+#pragma unroll
+      for (int i = 0; i < kBatch; i++)
+        v[i] = lane < mq && b0 + i <= lane ? Uc[(b0 + i) * mq + lane] : T(0);
+    };
+    T v[kBatch], vn[kBatch];
+    int mq = 0, pos = 0, mn = 0, pn = 0;
+    fetch(0, 0, v, mq, pos);
+    for (int q = 0, b0 = 0; q < nq;) {
+      const int qn = b0 + kBatch < mq ? q : q + 1, bn = qn == q ? b0 + kBatch : 0;
+      if (qn < nq) fetch(qn, bn, vn, mn, pn);
+#pragma unroll
+      for (int i = 0; i < kBatch; i++) {
+        const int col = __shfl_sync(0xffffffffu, pos, min(b0 + i, 31));
+        if (lane < mq && b0 + i <= lane) F[col * m + pos] += (TC)v[i];
       }
-      group_sync<G>();
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < kBatch; i++) v[i] = vn[i];
+      mq = mn;
+      pos = pn;
+      q = qn;
+      b0 = bn;
     }
   }
+  __syncwarp();
 }
 
-// The whole front of supernode s by a group of G threads (thread t) over the shared m x m column-major tile F, in the
-// compute type TC (the storage type T of L and U, or FP64: an FP32 LDL^T factor's small fronts are computed in FP64
-// and rounded once when stored, since the indefinite factor's pivots cancel). cm: the group's child metadata (G > 32;
-// a warp passes its child metadata by shuffles).
+// The same by a CTA of NT threads (m <= 128): warps over the child's columns, lanes over its rows. Ends with a barrier.
+template <class T, class TC, int NT>
+__device__ void assemble_cta(int s, const DevPlan &P, const double *__restrict__ values, const T *__restrict__ U, TC *F,
+                             ChildMeta *cm) {
+  constexpr int NW = NT / 32;
+  constexpr int kBatch = 16;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s];
+  const int q0 = P.chPtr[s], nch = P.chPtr[s + 1] - q0;
+  const int p0 = P.asmColPtr[f], p1 = P.asmColPtr[f + nc];
+  auto metadata = [&](int qb, int nq) {
+    if (t < nq) {
+      const int c = P.chList[q0 + qb + t];
+      cm->muc[t] = P.snM[c] - P.snNc[c];
+      cm->ea[t] = P.eaPtr[c];
+      cm->uo[t] = P.snUoff[c];
+    }
+  };
+  metadata(0, min(kChildChunk, nch));
+  for (int e = t; e < m * m; e += NT) F[e] = TC(0);
+  __syncthreads();
+  for (int p = p0 + t; p < p1; p += NT) F[P.asmDst[p]] += (TC)(T)__ldg(values + P.asmSrc[p]);
+  for (int qb = 0; qb < nch; qb += kChildChunk) {
+    const int nq = min(kChildChunk, nch - qb);
+    if (qb > 0) {
+      metadata(qb, nq);  // (the last chunk's data is consumed: barrier below)
+      __syncthreads();
+    }
+    // batch (q, i): rows [128 i' ..) of 4 of the warp's columns of child q: columns b = warp + NW (4 i + j), j < 4, rows
+    // b + lane + 32 h, h < 4
+    auto fetch = [&](int q, int i, T(&v)[kBatch]) {
+      const int mq = cm->muc[q];
+      const T *Uc = U + cm->uo[q];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int b = warp + NW * (4 * i + j);
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+          const int a = b + lane + 32 * h;
+          v[4 * j + h] = a < mq ? Uc[b * mq + a] : T(0);
+        }
+      }
+    };
+    T v[kBatch], vn[kBatch];
+    fetch(0, 0, v);
+    for (int e = t; e < nq * kSmallFront; e += NT) {
+      const int q = e / kSmallFront, a = e % kSmallFront;
+      if (a < cm->muc[q]) cm->map[q][a] = (unsigned char)P.eaMap[cm->ea[q] + a];
+    }
+    __syncthreads();  // the maps; A's entries
+    for (int q = 0, i = 0; q < nq;) {
+      const int mq = cm->muc[q];
+      const int qn = 4 * NW * (i + 1) < mq ? q : q + 1, in = qn == q ? i + 1 : 0;
+      if (qn < nq) fetch(qn, in, vn);
+      const unsigned char *map = cm->map[q];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int b = warp + NW * (4 * i + j);
+        if (b >= mq) continue;
+        TC *col = F + map[b] * m;
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+          const int a = b + lane + 32 * h;
+          if (a < mq) col[map[a]] += (TC)v[4 * j + h];
+        }
+      }
+      if (qn != q) __syncthreads();  // the next child adds to the same entries from other warps
+#pragma unroll
+      for (int j = 0; j < kBatch; j++) v[j] = vn[j];
+      q = qn;
+      i = in;
+    }
+  }
+  __syncthreads();
+}
+
+// The whole front of supernode s by one warp (m <= 32) over the shared m x m column-major tile F, in the compute type TC
+// (the storage type T of L and U, or FP64: an FP32 LDL^T factor's small fronts are computed in FP64 and rounded once when
+// stored, since the indefinite factor's pivots cancel).
 //
-// Column k of the elimination is one phase with one barrier: every thread reads the pivot F(k, k) (final since the
+// Column k of the elimination is one phase with one barrier: every lane reads the pivot F(k, k) (final since the
 // previous barrier), computes the same pivot decision and scale, writes its share of L's column k straight to Lx and
 // updates its share of the trailing triangle from the unscaled column k, which nobody writes in the phase. The
 // arithmetic is the column-scaled form's: l_i = F(i, k) / r (Cholesky, r = sqrt F(k, k)) or F(i, k) / d (LDL^T), and
 // F(i, j) -= l_i (l_j d) with d = 1 for Cholesky.
-template <class T, class TC, int G>
-__device__ void factor_front(int s, const DevPlan &P, const double *__restrict__ values, T *__restrict__ Lx,
-                             T *__restrict__ U, TC *F, unsigned long long *status, const LdltArgs<T> &la, int t,
-                             ChildMeta *cm) {
-  constexpr int NW = G / 32;
-  const int warp = t >> 5, lane = t & 31;
+template <class T, class TC, int MAXM>
+__device__ void factor_front_warp(int s, const DevPlan &P, const double *__restrict__ values, T *__restrict__ Lx,
+                                  T *__restrict__ U, TC *F, unsigned long long *status, const LdltArgs<T> &la,
+                                  int lane) {
   const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s], mu = m - nc;
   const bool ldlt = la.scal != nullptr;
   const TC tau = ldlt ? (TC)(T)la.scal[1] : TC(0);
-  assemble_front<T, TC, G>(s, P, values, U, F, t, cm);
-  // partial factorization of the nc pivot columns, one barrier per column; warps over the trailing columns j, lanes
-  // over the rows i >= j
-  int neg = 0, pert = 0;  // thread 0
+  assemble_warp<T, TC, tiny_batch<MAXM>()>(s, P, values, U, F, lane);
+  int neg = 0, pert = 0;  // lane 0
   T *Lp = Lx + P.snLxp[s];
   for (int k = 0; k < nc; k++) {
     TC d = F[k * m + k], inv, dk, diag;
@@ -147,10 +235,10 @@ __device__ void factor_front(int s, const DevPlan &P, const double *__restrict__
       int n1 = 0, p1 = 0;
       const bool ok = small_ldlt_pivot(d, tau, n1, p1);
       if (!ok) {
-        if (t == 0) atomicMin(status, status_word(f + k, 2, s));
-        return;  // group-uniform: every thread saw the same pivot
+        if (lane == 0) atomicMin(status, status_word(f + k, 2, s));
+        return;  // warp-uniform: every lane saw the same pivot
       }
-      if (t == 0) {
+      if (lane == 0) {
         neg += n1;
         pert += p1;
         la.D[f + k] = (double)(T)d;
@@ -160,8 +248,8 @@ __device__ void factor_front(int s, const DevPlan &P, const double *__restrict__
       diag = TC(1);
     } else {
       if (!(d > TC(0))) {
-        if (t == 0) atomicMin(status, status_word(f + k, 1, s));
-        return;  // group-uniform
+        if (lane == 0) atomicMin(status, status_word(f + k, 1, s));
+        return;  // warp-uniform
       }
       const TC r = sqrt(d);
       dk = TC(1);
@@ -169,26 +257,246 @@ __device__ void factor_front(int s, const DevPlan &P, const double *__restrict__
       diag = r;
     }
     const TC *Fk = F + k * m;
-    T *Lk = Lp + (int64_t)k * m;
-    for (int i = k + t; i < m; i += G) Lk[i] = (T)(i == k ? diag : Fk[i] * inv);
-    const int w = m - k - 1;
-    for (int jj = warp; jj < w; jj += NW) {
-      const int j = k + 1 + jj;
-      const TC lj = (Fk[j] * inv) * dk;
-      TC *Fj = F + j * m;
-      for (int i = j + lane; i < m; i += 32) Fj[i] -= (Fk[i] * inv) * lj;
+    const int i = lane;  // the lane's row
+    const TC li = i < m ? Fk[i] * inv : TC(0);
+    if (i >= k && i < m) Lp[(int64_t)k * m + i] = (T)(i == k ? diag : li);
+#pragma unroll 4
+    for (int j = k + 1; j < m; j++) {
+      const TC lj = __shfl_sync(0xffffffffu, li, j) * dk;
+      if (i >= j && i < m) F[j * m + i] -= li * lj;
     }
-    group_sync<G>();
+    __syncwarp();
   }
-  if (ldlt && t == 0 && (neg | pert)) {
+  if (ldlt && lane == 0 && (neg | pert)) {
     atomicAdd(la.counts, neg);
     atomicAdd(la.counts + 1, pert);
   }
-  if (mu > 0) {
-    T *Up = U + P.snUoff[s];
-    for (int e = t; e < mu * mu; e += G) {
-      const int jj = e / mu, ii = e - jj * mu;
-      if (ii >= jj) Up[e] = (T)F[(nc + jj) * m + nc + ii];
+  T *Up = U + P.snUoff[s];
+  for (int jj = 0; jj < mu; jj++) {
+    const int ii = jj + lane;
+    if (ii < mu) Up[(int64_t)jj * mu + ii] = (T)F[(nc + jj) * m + nc + ii];
+  }
+}
+
+// The whole front of supernode s (32 < m <= MAXM, 64 or 128) by one CTA, in TC (as above). The front is assembled in
+// shared memory and then held in registers, as C fragments of its 8 x 8 tiles: eight warps own the row groups (w, and
+// for 128 rows also 15 - w), MAXM / 32 more warps take the pivot columns, a row per lane (pivot_steps.cuh). Eight pivot
+// columns per step with two barriers: the panel warps eliminate them; the others update their tiles of the next eight
+// columns and hand them over, then the rest of the triangle while the panel warps go on. What bounds it is latency: a
+// step takes about 1,300 clocks, where a barrier and a rank-1 update of the shared front per column took 2,000 each.
+// The steps' columns stay in shared memory (over the front, which is dead by then) until they are scaled and written.
+template <int MAXM>
+constexpr int small_threads() { return 32 * (8 + MAXM / 32); }
+// shared memory (entries of TC) for fronts of at most m rows and nc pivot columns: the front, or the steps' columns over
+// it, and three step buffers
+template <class TC>
+__host__ __device__ constexpr int small_main(int m, int nc) {
+  const int f = m * m, p = (nc + 7) / 8 * ((m + 7) / 8 * 8) * col_ld<TC>();
+  return ((f > p ? f : p) + 3) & ~3;
+}
+template <class TC>
+constexpr int small_elems(int m, int nc) { return small_main<TC>(m, nc) + 3 * ((m + 7) / 8 * 8) * col_ld<TC>(); }
+
+template <class T, class TC, bool LDLT, int MAXM>
+__global__ void __launch_bounds__(small_threads<MAXM>(), MAXM == 64 ? 2 : 1)
+    k_front_small(const int *__restrict__ fronts, int mainElems, DevPlan P, const double *__restrict__ values,
+                  T *__restrict__ Lx, T *__restrict__ U, unsigned long long *status, LdltArgs<T> la) {
+  using V2 = typename Vec2<TC>::type;
+  constexpr int NT = small_threads<MAXM>(), NP = MAXM / 32, CL = col_ld<TC>(), NG = MAXM / 64;
+  extern __shared__ __align__(16) unsigned char fs_dyn[];
+  __shared__ ChildMeta cm;
+  __shared__ double scale[MAXM], diag[MAXM];
+  __shared__ int failAt, inexact, nNeg, nPert;
+  if (status_failed(status)) return;
+  const int s = fronts[blockIdx.x];
+  const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s], mu = m - nc;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int rows = (m + 7) & ~7, RB = rows / 8, steps = (nc + 7) / 8, pst = rows * CL;
+  TC *F = reinterpret_cast<TC *>(fs_dyn), *R = F + mainElems, *Q = R + pst, *Pc = F;  // Pc: -a of every step
+  T *Lp = Lx + P.snLxp[s];
+  T *Up = U + (mu > 0 ? P.snUoff[s] : 0);
+  const TC tau = LDLT ? (TC)(T)la.scal[1] : TC(0);
+  assemble_cta<T, TC, NT>(s, P, values, U, F, &cm);
+  // the front's tiles: row group rg[h], tile column cb
+  const int rg[2] = {warp, NG == 2 ? 15 - warp : -1};
+  auto tile = [&](int rb, int cb, TC(&c)[2]) {
+    const int i = 8 * rb + g;
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      const int j = 8 * cb + 2 * t + u;
+      c[u] = i < m && j <= i ? F[j * m + i] : i == j ? TC(1) : TC(0);
+    }
+  };
+  auto hand_over = [&](int rb, const TC(&c)[2]) {
+    V2 v;
+    v.x = c[0];
+    v.y = c[1];
+    *reinterpret_cast<V2 *>(R + (8 * rb + g) * CL + 2 * t) = v;
+  };
+  if (warp < 8) {
+#pragma unroll
+    for (int h = 0; h < NG; h++) {
+      TC c0[2];
+      if (rg[h] < RB) {
+        tile(rg[h], 0, c0);
+        hand_over(rg[h], c0);
+      }
+    }
+  }
+  if (tid == 0) {
+    failAt = 0x7fffffff;
+    inexact = nNeg = nPert = 0;
+  }
+  if (warp >= 8) {
+    __syncthreads();  // the front is in registers: Pc may overwrite it
+    for (int k = 0; k < steps; k++) {
+      TC *Pk = Pc + k * pst, *Qk = Q + (k & 1) * pst;
+      const int r = min(8 * k + 32 * (warp - 8) + lane, rows - 1), w = nc - 8 * k;
+      const bool mine = 8 * k + 32 * (warp - 8) < rows;
+      if (mine) {
+        const bool fine = w >= 8 ? eliminate8<false, LDLT, false>(R, Pk, Qk, 8 * k, r, 8, tau)
+                                 : eliminate8<false, LDLT, true>(R, Pk, Qk, 8 * k, r, w, tau);
+        if (!fine) inexact = 1;
+      }
+      __syncthreads();
+      if (inexact) {  // R is unchanged: the step again with exact quotients
+        if (mine) eliminate8<true, LDLT, true>(R, Pk, Qk, 8 * k, r, w, tau);
+        __syncthreads();
+        if (tid == 256) inexact = 0;
+      }
+      __syncthreads();
+    }
+  } else {
+    TC ca[7][2], cb[NG == 2 ? 15 : 1][2];  // at step k: the tiles (rg[h], k + 1), (rg[h], k + 2), ...
+#pragma unroll
+    for (int j = 0; j < 7; j++)
+      if (rg[0] < RB && j < rg[0]) tile(rg[0], j + 1, ca[j]);
+    if constexpr (NG == 2) {
+#pragma unroll
+      for (int j = 0; j < 15; j++)
+        if (rg[1] < RB && j < rg[1]) tile(rg[1], j + 1, cb[j]);
+    }
+    __syncthreads();
+    for (int k = 0; k < steps; k++) {
+      __syncthreads();
+      if (inexact) __syncthreads();
+      const TC *Pk = Pc + k * pst, *Qk = Q + (k & 1) * pst;
+      const bool on0 = rg[0] > k && rg[0] < RB, on1 = NG == 2 && rg[1] > k && rg[1] < RB;
+      if (on0) {
+        step_tile(ca[0], Pk + 8 * rg[0] * CL, Qk + 8 * (k + 1) * CL, CL, g, t);
+        hand_over(rg[0], ca[0]);
+      }
+      if (on1) {
+        step_tile(cb[0], Pk + 8 * rg[1] * CL, Qk + 8 * (k + 1) * CL, CL, g, t);
+        hand_over(rg[1], cb[0]);
+      }
+      __syncthreads();
+      const bool last = k + 1 == steps;  // the tiles from column k + 1 on are then the update block's
+      if (on0) {
+#pragma unroll
+        for (int j = 1; j < 7; j++)
+          if (k + 1 + j <= rg[0]) step_tile(ca[j], Pk + 8 * rg[0] * CL, Qk + 8 * (k + 1 + j) * CL, CL, g, t);
+        if (!last) {
+#pragma unroll
+          for (int j = 1; j < 7; j++) {
+            ca[j - 1][0] = ca[j][0];
+            ca[j - 1][1] = ca[j][1];
+          }
+        }
+      }
+      if constexpr (NG == 2) {
+        if (on1) {
+#pragma unroll
+          for (int j = 1; j < 15; j++)
+            if (k + 1 + j <= rg[1]) step_tile(cb[j], Pk + 8 * rg[1] * CL, Qk + 8 * (k + 1 + j) * CL, CL, g, t);
+          if (!last) {
+#pragma unroll
+            for (int j = 1; j < 15; j++) {
+              cb[j - 1][0] = cb[j][0];
+              cb[j - 1][1] = cb[j][1];
+            }
+          }
+        }
+      }
+    }
+    // the update block (of a failed front too: nobody reads it)
+    auto put = [&](int rb, int tc, const TC(&c)[2]) {
+      const int i = 8 * rb + g;
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const int j = 8 * tc + 2 * t + u;
+        if (i < m && j <= i) Up[(int64_t)(j - nc) * mu + i - nc] = (T)c[u];
+      }
+    };
+    if (rg[0] < RB) {
+#pragma unroll
+      for (int j = 0; j < 7; j++)
+        if (steps + j <= rg[0]) put(rg[0], steps + j, ca[j]);
+    }
+    if constexpr (NG == 2) {
+      if (rg[1] < RB) {
+#pragma unroll
+        for (int j = 0; j < 15; j++)
+          if (steps + j <= rg[1]) put(rg[1], steps + j, cb[j]);
+      }
+    }
+  }
+  // the pivots: test and count, the columns' scales
+  if (tid < MAXM) {
+    double d = tid < nc ? -(double)Pc[(tid >> 3) * pst + tid * CL + (tid & 7)] : 1.0;
+    bool bad = false, small = false;
+    if (LDLT) {
+      small = tid < nc && !(fabs(d) >= (double)tau);
+      bad = small && !isfinite(d);
+      if (small) d = d < 0.0 ? -(double)tau : (double)tau;
+      const int neg = __popc(__ballot_sync(0xffffffffu, tid < nc && d < 0.0));
+      const int pert = __popc(__ballot_sync(0xffffffffu, small));
+      if (lane == 0) {
+        atomicAdd(&nNeg, neg);
+        atomicAdd(&nPert, pert);
+      }
+    } else {
+      bad = tid < nc && !(d > 0.0);
+    }
+    const unsigned mask = __ballot_sync(0xffffffffu, bad);
+    if (lane == 0 && mask) atomicMin(&failAt, 32 * warp + __ffs(mask) - 1);
+    const double dl = LDLT ? d : sqrt(d);
+    diag[tid] = dl;
+    scale[tid] = 1.0 / dl;
+  }
+  __syncthreads();
+  if (failAt < MAXM) {
+    if (tid == 0) atomicMin(status, status_word(f + failAt, LDLT ? 2 : 1, s));
+    return;  // block-uniform
+  }
+  {  // L, and the update block's part of the last step's columns: a lane per row, eight columns at a time
+    const int r = tid & (MAXM - 1);
+    for (int p = tid / MAXM; p < steps && tid < NT / MAXM * MAXM; p += NT / MAXM) {
+      if (r < 8 * p || r >= m) continue;
+      const TC *Pr = Pc + p * pst + r * CL;
+      TC v[8];
+#pragma unroll
+      for (int u = 0; u < 8; u += 2) {
+        const V2 x = *reinterpret_cast<const V2 *>(Pr + u);
+        v[u] = -x.x;
+        v[u + 1] = -x.y;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const int col = 8 * p + u;
+        if (r < col) continue;
+        if (col < nc)
+          Lp[(int64_t)col * m + r] = (T)(r == col ? (LDLT ? 1.0 : diag[col]) : (double)v[u] * scale[col]);
+        else
+          Up[(int64_t)(col - nc) * mu + r - nc] = (T)v[u];
+      }
+    }
+  }
+  if (LDLT) {
+    if (tid < nc) la.D[f + tid] = (double)(T)diag[tid];
+    if (tid == 0 && (nNeg | nPert)) {
+      atomicAdd(la.counts, nNeg);
+      atomicAdd(la.counts + 1, nPert);
     }
   }
 }
@@ -224,7 +532,10 @@ __device__ void factor_front_bk(int s, const DevPlan &P, const double *__restric
   const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s], mu = m - nc;
   const double tau = la.scal[1];
   const double alpha = 0.64038820320220756;  // (1 + sqrt(17)) / 8
-  assemble_front<T, double, G>(s, P, values, U, F, t, cm);
+  if constexpr (G == 32)
+    assemble_warp<T, double, 16>(s, P, values, U, F, t);
+  else
+    assemble_cta<T, double, G>(s, P, values, U, F, cm);
   auto at = [&](int i, int j) -> double & { return F[j * m + i]; };  // entry (i, j), i >= j
   int neg = 0, pert = 0;  // thread 0
   int perm[64];           // thread 0: the current block's pivot order
@@ -370,7 +681,7 @@ __device__ void factor_front_bk(int s, const DevPlan &P, const double *__restric
 // m <= MAXM (16 or 32): one warp per front, tiny_warps<MAXM>() fronts per CTA
 // BK: Bunch-Kaufman pivots (FP64 factors with la.piv set)
 template <class T, class TC, int MAXM, bool BK>
-__global__ void __launch_bounds__(32 * tiny_warps<MAXM>()) k_front_tiny(const int *__restrict__ fronts, int count,
+__global__ void __launch_bounds__(32 * tiny_warps<MAXM>(), BK ? 1 : tiny_ctas<MAXM>()) k_front_tiny(const int *__restrict__ fronts, int count,
                                                                          DevPlan P, const double *__restrict__ values,
                                                                          T *__restrict__ Lx, T *__restrict__ U,
                                                                          unsigned long long *status, LdltArgs<T> la) {
@@ -383,37 +694,37 @@ __global__ void __launch_bounds__(32 * tiny_warps<MAXM>()) k_front_tiny(const in
   if constexpr (BK)
     factor_front_bk<T, 32>(fronts[idx], P, values, Lx, U, F[warp], status, la, lane, nullptr);
   else
-    factor_front<T, TC, 32>(fronts[idx], P, values, Lx, U, F[warp], status, la, lane, nullptr);
+    factor_front_warp<T, TC, MAXM>(fronts[idx], P, values, Lx, U, F[warp], status, la, lane);
 }
 
-// 32 < m <= 128: one CTA per front; dynamic shared memory = the launch's largest m squared
-template <class T, class TC, bool BK>
-__global__ void __launch_bounds__(256) k_front_small(const int *__restrict__ fronts, int count, DevPlan P,
-                                                     const double *__restrict__ values, T *__restrict__ Lx,
-                                                     T *__restrict__ U, unsigned long long *status, LdltArgs<T> la) {
+// 32 < m <= 128 with Bunch-Kaufman pivots: one CTA per front; dynamic shared memory = the launch's largest m squared
+template <class T>
+__global__ void __launch_bounds__(256) k_front_small_bk(const int *__restrict__ fronts, DevPlan P,
+                                                        const double *__restrict__ values, T *__restrict__ Lx,
+                                                        T *__restrict__ U, unsigned long long *status, LdltArgs<T> la) {
   extern __shared__ __align__(16) unsigned char fs_dyn[];
   __shared__ ChildMeta cm;
   if (status_failed(status)) return;
-  if constexpr (BK)
-    factor_front_bk<T, 256>(fronts[blockIdx.x], P, values, Lx, U, reinterpret_cast<double *>(fs_dyn), status, la,
-                            threadIdx.x, &cm);
-  else
-    factor_front<T, TC, 256>(fronts[blockIdx.x], P, values, Lx, U, reinterpret_cast<TC *>(fs_dyn), status, la,
-                             threadIdx.x, &cm);
+  factor_front_bk<T, 256>(fronts[blockIdx.x], P, values, Lx, U, reinterpret_cast<double *>(fs_dyn), status, la,
+                          threadIdx.x, &cm);
 }
 
+template <class T, class TC, bool LDLT>
+static cudaError_t init_small() {
+  const int bytes = small_elems<TC>(kSmallFront, kSmallFront) * (int)sizeof(TC);
+  cudaError_t e = cudaFuncSetAttribute(k_front_small<T, TC, LDLT, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       bytes);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_front_small<T, TC, LDLT, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  return e;
+}
 cudaError_t init_front_small_attributes() {
-  cudaError_t e = cudaFuncSetAttribute(k_front_small<double, double, false>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       kSmallFront * kSmallFront * (int)sizeof(double));
+  cudaError_t e = init_small<double, double, false>();
+  if (e == cudaSuccess) e = init_small<double, double, true>();
+  if (e == cudaSuccess) e = init_small<float, float, false>();
+  if (e == cudaSuccess) e = init_small<float, double, true>();
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_front_small<float, float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kSmallFront * kSmallFront * (int)sizeof(float));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_front_small<float, double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kSmallFront * kSmallFront * (int)sizeof(double));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_front_small<double, double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(k_front_small_bk<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              kSmallFront * kSmallFront * (int)sizeof(double));
   return e;
 }
@@ -428,35 +739,54 @@ static int launch_tiny(const int *fronts, int count, const DevPlan &P, const dou
   return 1;
 }
 
-template <class T, class TC, bool BK>
-static int launch_fronts_tc(const int *tiny, int ntiny, int ntinyMid, const int *small, int nsmall, int maxM,
-                            const DevPlan &P, const double *values, T *Lx, T *U, unsigned long long *status,
-                            const LdltArgs<T> &la, cudaStream_t st) {
-  int k = launch_tiny<T, TC, kTinyMid, BK>(tiny, ntinyMid, P, values, Lx, U, status, la, st);
-  k += launch_tiny<T, TC, kTinyFront, BK>(tiny + ntinyMid, ntiny - ntinyMid, P, values, Lx, U, status, la, st);
-  if (nsmall > 0)
-    k_front_small<T, TC, BK><<<nsmall, 256, (size_t)maxM * maxM * sizeof(TC), st>>>(small, nsmall, P, values, Lx, U,
-                                                                                    status, la);
-  return k + (nsmall > 0 ? 1 : 0);
+template <class T, class TC, bool LDLT, int MAXM>
+static int launch_small(const SmallClass &c, const DevPlan &P, const double *values, T *Lx, T *U,
+                        unsigned long long *status, const LdltArgs<T> &la, cudaStream_t st) {
+  if (c.count <= 0) return 0;
+  k_front_small<T, TC, LDLT, MAXM>
+      <<<c.count, small_threads<MAXM>(), small_elems<TC>(c.maxM, c.maxNc) * sizeof(TC), st>>>(
+          c.sn, small_main<TC>(c.maxM, c.maxNc), P, values, Lx, U, status, la);
+  return 1;
+}
+template <class T, class TC, bool LDLT, bool BK>
+static int launch_fronts_tc(const SmallFronts &fr, const DevPlan &P, const double *values, T *Lx, T *U,
+                            unsigned long long *status, const LdltArgs<T> &la, cudaStream_t st) {
+  // a class of its own only where the GPU would otherwise not hold the level's fronts at once: two launches one after
+  // the other take twice a front's latency
+  const int mid = fr.ntiny <= num_sms() * tiny_warps<kTinyFront>() ? 0 : fr.ntinyMid;
+  SmallClass half = fr.half, full = fr.full;
+  if (half.count + full.count <= num_sms() && half.count > 0 && full.count > 0) {  // (the two lists are one)
+    full = SmallClass{half.sn, half.count + full.count, full.maxM, std::max(half.maxNc, full.maxNc)};
+    half.count = 0;
+  }
+  int k = launch_tiny<T, TC, kTinyMid, BK>(fr.tiny, mid, P, values, Lx, U, status, la, st);
+  k += launch_tiny<T, TC, kTinyFront, BK>(fr.tiny + mid, fr.ntiny - mid, P, values, Lx, U, status, la, st);
+  if constexpr (BK) {
+    for (const SmallClass &c : {half, full})
+      if (c.count > 0) {
+        k_front_small_bk<T><<<c.count, 256, (size_t)c.maxM * c.maxM * sizeof(TC), st>>>(c.sn, P, values, Lx, U, status,
+                                                                                        la);
+        k++;
+      }
+  } else {
+    k += launch_small<T, TC, LDLT, 64>(half, P, values, Lx, U, status, la, st);
+    k += launch_small<T, TC, LDLT, 128>(full, P, values, Lx, U, status, la, st);
+  }
+  return k;
 }
 template <class T>
-int launch_fronts_small(const int *tiny, int ntiny, int ntinyMid, const int *small, int nsmall, int maxM,
-                        const DevPlan &P, const double *values, T *Lx, T *U, unsigned long long *status,
-                        const LdltArgs<T> &la, cudaStream_t st) {
+int launch_fronts_small(const SmallFronts &fr, const DevPlan &P, const double *values, T *Lx, T *U,
+                        unsigned long long *status, const LdltArgs<T> &la, cudaStream_t st) {
   if constexpr (std::is_same<T, double>::value)
     if (la.piv != nullptr)  // Bunch-Kaufman pivots (FP64)
-      return launch_fronts_tc<T, double, true>(tiny, ntiny, ntinyMid, small, nsmall, maxM, P, values, Lx, U, status,
-                                               la, st);
+      return launch_fronts_tc<T, double, true, true>(fr, P, values, Lx, U, status, la, st);
   if (la.scal != nullptr)  // LDL^T: FP64 arithmetic whatever the storage
-    return launch_fronts_tc<T, double, false>(tiny, ntiny, ntinyMid, small, nsmall, maxM, P, values, Lx, U, status,
-                                              la, st);
-  return launch_fronts_tc<T, T, false>(tiny, ntiny, ntinyMid, small, nsmall, maxM, P, values, Lx, U, status, la, st);
+    return launch_fronts_tc<T, double, true, false>(fr, P, values, Lx, U, status, la, st);
+  return launch_fronts_tc<T, T, false, false>(fr, P, values, Lx, U, status, la, st);
 }
-template int launch_fronts_small<double>(const int *, int, int, const int *, int, int, const DevPlan &,
-                                         const double *, double *, double *, unsigned long long *,
-                                         const LdltArgs<double> &, cudaStream_t);
-template int launch_fronts_small<float>(const int *, int, int, const int *, int, int, const DevPlan &,
-                                        const double *, float *, float *, unsigned long long *,
-                                        const LdltArgs<float> &, cudaStream_t);
+template int launch_fronts_small<double>(const SmallFronts &, const DevPlan &, const double *, double *, double *,
+                                         unsigned long long *, const LdltArgs<double> &, cudaStream_t);
+template int launch_fronts_small<float>(const SmallFronts &, const DevPlan &, const double *, float *, float *,
+                                        unsigned long long *, const LdltArgs<float> &, cudaStream_t);
 
 }  // namespace amp

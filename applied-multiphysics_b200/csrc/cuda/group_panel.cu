@@ -19,6 +19,7 @@
 
 #include "../host/plan.hpp"
 #include "devplan.cuh"
+#include "pivot_steps.cuh"
 #include "sync.cuh"
 
 namespace amp {
@@ -27,13 +28,6 @@ namespace {
 
 __device__ __forceinline__ bool panel_failed(const unsigned long long *st) {
   return *(volatile const unsigned long long *)st != kStatusOk;
-}
-
-// D += A B on an 8 x 8 tile, K = 4: lane (g, t) = (lane / 4, lane % 4) holds A(g, t), B(t, g), D(g, 2 t) and D(g, 2 t + 1)
-__device__ __forceinline__ void mma884(double (&c)[2], double a, double b) {
-  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
 }
 
 // 64 x 64 FP64 blocks in shared memory, row-major, the column pairs of row r permuted by a bijection of r mod 8 so that
@@ -70,58 +64,6 @@ __device__ __forceinline__ void load_block(double *S, const T *L, int m, int i0,
   for (int e = 0; e < 16; e++) {
     const int c = 4 * e + t;
     S[sw(i, c)] = pad && i == c && i >= ncol ? 1.0 : (double)v[e];
-  }
-}
-
-// 1 / d as x f. FP64: Newton's iteration on the hardware estimate x (relative error e below 2^-20):
-// 1 / d = x / (1 - e) = x (1 + e)(1 + e^2) up to e^4, x and f apart, so that a product with x can run beside f's chain;
-// the estimate flushes results outside the normal range, so it returns false for |d| below 2^-975 or above 2^960 (an
-// integer test of the exponent, off the FP64 pipe). FP32: the hardware quotient estimate. Exact: the quotient.
-template <bool Exact>
-__device__ __forceinline__ bool recip_parts(double d, double &x, double &f) {
-  if constexpr (Exact) {
-    x = 1.0 / d;
-    f = 1.0;
-    return true;
-  }
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
-  const double e = fma(-d, x, 1.0), s = 1.0 + e;
-  f = fma(s, e * e, s);
-  return ((unsigned)__double2hiint(d) & 0x7fffffffu) - 0x03000000u <= 0x79000000u;
-}
-template <bool Exact>
-__device__ __forceinline__ bool recip_parts(float d, float &x, float &f) {
-  x = __fdividef(1.0f, d);
-  f = 1.0f;
-  return true;
-}
-
-// POTRF step buffers: 8 columns of 64 rows; row strides with 16-byte rows and few bank conflicts
-template <class TC>
-constexpr int col_ld() { return sizeof(TC) == 8 ? 10 : 12; }
-template <class TC>
-struct Vec2;  // two neighbouring entries
-template <>
-struct Vec2<double> { using type = double2; };
-template <>
-struct Vec2<float> { using type = float2; };
-
-// C(g, 2 t ..) -= A(g, .) B(., 2 t ..) on an 8 x 8 tile, K = 8: P the negated rows of A, Q the rows of B^T (stride ld)
-__device__ __forceinline__ void step_tile(double (&c)[2], const double *P, const double *Q, int ld, int g, int t) {
-  const double2 a = *reinterpret_cast<const double2 *>(P + g * ld + 2 * t);
-  const double2 b = *reinterpret_cast<const double2 *>(Q + g * ld + 2 * t);
-  mma884(c, a.x, b.x);
-  mma884(c, a.y, b.y);
-}
-__device__ __forceinline__ void step_tile(float (&c)[2], const float *P, const float *Q, int ld, int g, int t) {
-#pragma unroll
-  for (int h = 0; h < 2; h++) {
-    const float4 a = *reinterpret_cast<const float4 *>(P + g * ld + 4 * h);
-#pragma unroll
-    for (int u = 0; u < 2; u++) {
-      const float4 b = *reinterpret_cast<const float4 *>(Q + (2 * t + u) * ld + 4 * h);
-      c[u] = fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, c[u]))));
-    }
   }
 }
 
@@ -165,57 +107,12 @@ __device__ int potrf_block(const double *Ds, double *scr, T *Lp, double *Linv, i
     v.y = c[1];
     *reinterpret_cast<V2 *>(R + myRow) = v;
   };
-  // (1) of step k for this lane's row; Exact: the pivots' reciprocals by division. Returns false when one is out of the
-  // estimate's range.
-  auto eliminate = [&](int k, auto exact) {
-    const int r = min(8 * k + 32 * warp + lane, kPanel - 1);  // (lanes past the block repeat its last row)
-    TC *Pk = P + k * kStepBuf + r * CL, *Qk = Q + (k & 1) * kStepBuf + r * CL;
-    TC dg[8][8], a[8], iv[8];
-    bool fine = true;
-#pragma unroll
-    for (int i = 0; i < 8; i++)
-#pragma unroll
-      for (int j = 0; j <= i; j += 2) {
-        const V2 v = *reinterpret_cast<const V2 *>(R + (8 * k + i) * CL + j);
-        dg[i][j] = v.x;
-        dg[i][j + 1] = v.y;
-      }
-#pragma unroll
-    for (int j = 0; j < 8; j += 2) {
-      const V2 v = *reinterpret_cast<const V2 *>(R + r * CL + j);
-      a[j] = v.x;
-      a[j + 1] = v.y;
-    }
-#pragma unroll
-    for (int kk = 0; kk < 8; kk++) {
-      TC d = dg[kk][kk], x, fr;
-      if (LDLT && !(fabs(d) >= tau)) d = d < TC(0) ? -tau : tau;
-      fine &= recip_parts<decltype(exact)::value>(d, x, fr);
-      iv[kk] = x * fr;
-#pragma unroll
-      for (int j = kk + 1; j < 8; j++) {
-        const TC lj = (dg[j][kk] * x) * fr;  // the update scale; L is scaled with the exact quotient below
-#pragma unroll
-        for (int i = j; i < 8; i++) dg[i][j] -= dg[i][kk] * lj;
-        a[j] -= a[kk] * lj;
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 8; j += 2) {
-      V2 v;
-      v.x = -a[j];
-      v.y = -a[j + 1];
-      *reinterpret_cast<V2 *>(Pk + j) = v;
-      v.x = a[j] * iv[j];
-      v.y = a[j + 1] * iv[j + 1];
-      *reinterpret_cast<V2 *>(Qk + j) = v;
-    }
-    return fine;
-  };
-  auto panel = [&](auto exact) {  // the first two warps
+  auto panel = [&](auto exact) {  // the first two warps, a row per lane
     bool fine = true;
     for (int k = 0; k < 8; k++) {
-      if (8 * k + 32 * warp < kPanel) fine &= eliminate(k, exact);
+      if (8 * k + 32 * warp < kPanel)
+        fine &= eliminate8<decltype(exact)::value, LDLT, false>(R, P + k * kStepBuf, Q + (k & 1) * kStepBuf, 8 * k,
+                                                               min(8 * k + 32 * warp + lane, kPanel - 1), 8, tau);
       __syncthreads();
       if (k == 0 && warp == 1) {  // row group 1's only trailing tile
         TC c[2];

@@ -28,11 +28,20 @@ void launch_ldlt_tau(const double *values, const DevPlan &P, double *scal, cudaS
 void launch_update_c(const TileTask *tasks, int64_t ntasks, cplx *Lx, cplx *U, const cplx *W,
                      const unsigned long long *status, cudaStream_t st);
 // whole small fronts of one level: tiny (m <= 32, warp per front; sorted by m, the first ntinyMid with m <= 16) and
-// small (m <= 128, CTA per front; maxM = their largest m); returns the kernels launched
+// small (a CTA per front: half 32 < m <= 64, full 64 < m <= 128, with the largest m and pivot column count of each
+// class); returns the kernels launched
+struct SmallClass {
+  const int *sn;
+  int count, maxM, maxNc;
+};
+struct SmallFronts {
+  const int *tiny;
+  int ntiny, ntinyMid;
+  SmallClass half, full;
+};
 template <class T>
-int launch_fronts_small(const int *tiny, int ntiny, int ntinyMid, const int *small, int nsmall, int maxM,
-                        const DevPlan &P, const double *values, T *Lx, T *U, unsigned long long *status,
-                        const LdltArgs<T> &la, cudaStream_t st);
+int launch_fronts_small(const SmallFronts &fr, const DevPlan &P, const double *values, T *Lx, T *U,
+                        unsigned long long *status, const LdltArgs<T> &la, cudaStream_t st);
 // width: the tiles' columns, 256, or 128 / 64 (tasks whose columns are one 128- / 64-column group)
 // spin: bound of each role's wait in polls (0 = the default, about 0.5 s)
 void launch_update_mx(const MixTask *tasks, int64_t ntasks, const CUtensorMap *maps, float *L32, float *U32,

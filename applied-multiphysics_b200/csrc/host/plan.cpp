@@ -403,7 +403,6 @@ void build_plan(const Symbolic &S, Plan &P, const Tuning &tune) {
   std::vector<int> appliedB(ns, 0);  // per front: pivot columns whose update every column beyond the next group has
   for (int L = 0; L < P.nlevels; L++) {
     // small fronts: the whole front in one kernel; the rest go through the steps below
-    int maxM = 0;
     double ff = 0, fb = 0;
     for (int q = P.lvlPtr[L]; q < P.lvlPtr[L + 1]; q++) {
       const int s = P.lvlSn[q];
@@ -419,7 +418,6 @@ void build_plan(const Symbolic &S, Plan &P, const Tuning &tune) {
         P.tinySn.push_back(s);
       } else {
         P.smallSn.push_back(s);
-        maxM = std::max(maxM, P.snM[s]);
       }
     }
     {
@@ -429,8 +427,24 @@ void build_plan(const Symbolic &S, Plan &P, const Tuning &tune) {
                           P.tinySn.begin());
     }
     P.tinyPtr.push_back((int64_t)P.tinySn.size());
+    {
+      auto s0 = P.smallSn.begin() + P.smallPtr.back();
+      std::stable_sort(s0, P.smallSn.end(), [&](int a, int b) { return P.snM[a] < P.snM[b]; });
+      const auto mid = std::partition_point(s0, P.smallSn.end(), [&](int a) { return P.snM[a] <= kSmallHalf; });
+      P.smallMid.push_back(mid - P.smallSn.begin());
+      auto largest = [&](auto from, auto to) {
+        int maxM = 0, maxNc = 0;
+        for (auto q = from; q != to; ++q) {
+          maxM = std::max(maxM, P.snM[*q]);
+          maxNc = std::max(maxNc, P.snNc[*q]);
+        }
+        P.smallMaxM.push_back(maxM);
+        P.smallMaxNc.push_back(maxNc);
+      };
+      largest(s0, mid);
+      largest(mid, P.smallSn.end());
+    }
     P.smallPtr.push_back((int64_t)P.smallSn.size());
-    P.smallMaxM.push_back(maxM);
     P.frontLvlFlops.push_back(ff);
     P.frontLvlBytes.push_back(fb);
     int maxSteps = 0;

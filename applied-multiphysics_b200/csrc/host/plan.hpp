@@ -25,6 +25,7 @@ constexpr int kAsmCols = 8;    // front columns per assembly task (one per warp)
 constexpr int kTrsmRows = 64;  // panel rows per TRSM task
 constexpr int kTinyFront = 32;    // fronts with m <= 32: one warp per front does the whole front (front_small.cu)
 constexpr int kTinyMid = 16;      // the smaller tiny class (m <= 16: 16 x 16 tiles, eight fronts per CTA)
+constexpr int kSmallHalf = 64;    // the smaller class of those: half the registers and a quarter of the shared memory
 constexpr int kSmallFront = 128;  // fronts with 32 < m <= 128: one CTA per front does the whole front
 constexpr int kSolveGroup = 4;    // supernodes with m <= kTinyFront per solve task (one warp each)
 constexpr int kWholeFront = 512;  // one-vector forward: supernodes with nc <= 64 and m <= 512 are one task each
@@ -135,9 +136,11 @@ struct Plan {
   std::vector<double> uLvlFlops;
   std::vector<StepRange> steps;
   // small fronts of each level, done whole by one warp (tiny) or one CTA (small) per front: tiny fronts of level L
-  // are tinySn[tinyPtr[L] .. tinyPtr[L + 1]), small ones smallSn[smallPtr[L] ..], the largest m of those smallMaxM[L]
-  std::vector<int> tinySn, smallSn, smallMaxM;
-  std::vector<int64_t> tinyPtr, smallPtr;
+  // are tinySn[tinyPtr[L] .. tinyPtr[L + 1]), small ones smallSn[smallPtr[L] ..], sorted by m, those from smallMid[L]
+  // on with m > kSmallHalf; the largest m and pivot column count of level L's two small classes (m <= kSmallHalf first)
+  // are smallMaxM[2 L], smallMaxM[2 L + 1] and smallMaxNc[2 L], smallMaxNc[2 L + 1]
+  std::vector<int> tinySn, smallSn, smallMaxM, smallMaxNc;
+  std::vector<int64_t> tinyPtr, smallPtr, smallMid;
   std::vector<int64_t> tinyMid;  // each level's tiny fronts are sorted by m; those from tinyMid[L] on have m > kTinyMid
   std::vector<double> frontLvlFlops, frontLvlBytes;  // algorithmic work of each level's small fronts
   // solve: rows below of each supernode (Si[Sp[s] + nc ..]) and the perm
