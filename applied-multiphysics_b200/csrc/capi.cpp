@@ -160,8 +160,8 @@ struct amp_plan_s {
   amp::StripTask *dStrips = nullptr;
   amp::TileTask *dTile = nullptr, *dUTile = nullptr;
   amp::MixTask *dMixTile = nullptr, *dMixU = nullptr;
-  int4 *dFwdTasks = nullptr, *dBwdTasks = nullptr, *dBwdAll = nullptr;
-  int4 *dFwdTasks1 = nullptr;  // the one-vector forward's list (with whole-supernode tasks)
+  int4 *dFwdTasks1 = nullptr, *dBwdAll = nullptr;  // the one-vector sweeps' lists (join_small)
+  int nFwd1 = 0, nBwd1 = 0;
   // the multi-vector lists with every block task expanded into ns vector slices, built on first use (index ns - 1)
   int4 *dFwdSl[kSlices] = {}, *dBwdSl[kSlices] = {};
   int nFwdSl[kSlices] = {}, nBwdSl[kSlices] = {};
@@ -203,8 +203,7 @@ struct amp_factor_s {
   cudaStream_t side = nullptr;                      // look-ahead: part B of the panel steps' updates
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t evPanel = nullptr, evSide = nullptr;  // look-ahead ordering between the two streams
-  cudaStream_t front[2] = {nullptr, nullptr};       // a level's small fronts beside its large ones (SmallFork)
-  cudaEvent_t evFork = nullptr, evFront[2] = {nullptr, nullptr};
+  cudaEvent_t evFork = nullptr, evFront = nullptr;  // a level's small fronts on the side stream (SmallFork)
   DevMem mem;
   double *dLx = nullptr, *dU = nullptr, *dD = nullptr, *dValues = nullptr;
   float *dL32 = nullptr, *dU32 = nullptr;           // mixed precision: FP32 factor and update arena
@@ -280,15 +279,35 @@ struct amp_factor_s {
     if (evSide) cudaEventDestroy(evSide);
     if (side) cudaStreamDestroy(side);
     if (evFork) cudaEventDestroy(evFork);
-    for (int k = 0; k < 2; k++) {
-      if (evFront[k]) cudaEventDestroy(evFront[k]);
-      if (front[k]) cudaStreamDestroy(front[k]);
-    }
+    if (evFront) cudaEventDestroy(evFront);
     if (stream) cudaStreamDestroy(stream);
   }
 };
 
 namespace {
+
+// A solve task list as it is launched: neighbouring one-warp tasks (kind 2) over consecutive supernodes joined to one
+// of up to kSolveWarps warps (a CTA's; the schedule's own tasks use half of them). several: for the multi-vector
+// sweeps, whose front vectors limit the larger tasks to supernodes with m <= kTinyMid.
+std::vector<int> join_small(const amp::Plan &P, const std::vector<int> &tasks, bool several) {
+  std::vector<int> out;
+  out.reserve(tasks.size());
+  auto fits = [&](int first, int count) {
+    for (int i = first; several && i < first + count; i++)
+      if (P.snM[P.solveSmall[i]] > amp::kTinyMid) return false;
+    return true;
+  };
+  for (size_t i = 0; i < tasks.size(); i += 4) {
+    const int *t = &tasks[i];
+    int *last = out.empty() ? nullptr : &out[out.size() - 4];
+    if (t[2] == 2 && last && last[2] == 2 && last[0] + last[1] == t[0] && last[1] + t[1] <= amp::kSolveWarps &&
+        fits(last[0], last[1]) && fits(t[0], t[1]))
+      last[1] += t[1];
+    else
+      out.insert(out.end(), t, t + 4);
+  }
+  return out;
+}
 
 void upload_plan(amp_plan *pl) {
   const amp::Plan &P = pl->P;
@@ -323,6 +342,8 @@ void upload_plan(amp_plan *pl) {
   d.invOff = m.upload(P.invOff);
   d.diagSlot = m.upload(P.diagSlot);
   d.solveSmall = m.upload(P.solveSmall);
+  d.gatherOff = m.upload(P.gatherOff);
+  d.gatherRange = (const int2 *)m.upload(P.gatherRange);
   pl->dAsm = m.upload(P.asmTasks);
   pl->dAsmCh = m.upload(P.asmCh);
   pl->dGroupItems = m.upload(P.groupItems);
@@ -331,10 +352,11 @@ void upload_plan(amp_plan *pl) {
   pl->dUTile = m.upload(P.uTasks);
   pl->dMixTile = m.upload(P.mixTiles);
   pl->dMixU = m.upload(P.mixUTasks);
-  pl->dFwdTasks = (int4 *)m.upload(P.fwdTasks);
-  pl->dFwdTasks1 = (int4 *)m.upload(P.fwdTasks1);
-  pl->dBwdTasks = (int4 *)m.upload(P.bwdTasks);
-  pl->dBwdAll = (int4 *)m.upload(P.bwdAll);
+  const std::vector<int> fwd1 = join_small(P, P.fwdTasks1, false), bwd1 = join_small(P, P.bwdAll, false);
+  pl->nFwd1 = (int)(fwd1.size() / 4);
+  pl->nBwd1 = (int)(bwd1.size() / 4);
+  pl->dFwdTasks1 = (int4 *)m.upload(fwd1);
+  pl->dBwdAll = (int4 *)m.upload(bwd1);
   pl->dTinySn = m.upload(P.tinySn);
   pl->dSmallSn = m.upload(P.smallSn);
   pl->dChain = (int2 *)m.upload(P.chainTasks);
@@ -420,14 +442,14 @@ struct LookAhead {
 };
 
 // The small fronts of level L (whole fronts, one warp or one CTA each). They depend on the levels below only, like the
-// level's large fronts, so the kinds that a level has run beside one another: the warp fronts on the first of two more
-// streams, the CTA fronts on the second when the level also has large fronts (on the factor's stream). A level's kinds
-// one after another took their sum, e.g. 44 us for 34 tiny and 14 small fronts of a 2D mesh whose longest takes 15.
-// join() makes the factor's stream wait for them (before the next level).
+// level's large fronts, so they run beside these on the side stream (its look-ahead updates come later in a level); in a
+// level without large fronts the warp fronts run there and the CTA fronts on the factor's stream. One after another they
+// took the sum, e.g. 44 us for 34 warp and 14 CTA fronts of a 2D mesh whose longest takes 15. join() makes the factor's
+// stream wait for them (before the next level).
 template <class T>
 struct SmallFork {
   amp_factor *f;
-  bool used[2] = {false, false};
+  bool used = false;
   void launch(int L, T *Lx, T *U, const amp::LdltArgs<T> &la) {
     const amp::Plan &P = f->plan->P;
     const int64_t t0 = P.tinyPtr[L], t1 = P.tinyPtr[L + 1], s0 = P.smallPtr[L], s1 = P.smallPtr[L + 1];
@@ -438,29 +460,26 @@ struct SmallFork {
     const amp::SmallClass none{nullptr, 0, 0, 0};
     const amp::SmallClass half{small + s0, (int)(sm - s0), P.smallMaxM[2 * L], P.smallMaxNc[2 * L]};
     const amp::SmallClass full{small + sm, (int)(s1 - sm), P.smallMaxM[2 * L + 1], P.smallMaxNc[2 * L + 1]};
-    const bool forkTiny = t1 > t0 && (large || s1 > s0), forkSmall = s1 > s0 && large;
-    if (forkTiny || forkSmall) ck(cudaEventRecord(f->evFork, f->stream), "event");
+    used = large || (t1 > t0 && s1 > s0);
+    if (used) {
+      ck(cudaEventRecord(f->evFork, f->stream), "event");
+      ck(cudaStreamWaitEvent(f->side, f->evFork, 0), "wait");
+    }
     const double scale = sizeof(T) / 8.0, tot = (double)(t1 - t0 + s1 - s0);
-    auto run = [&](int k, bool fork, const amp::SmallFronts &fr, double count) {
-      const cudaStream_t st = fork ? f->front[k] : f->stream;
-      if (fork) ck(cudaStreamWaitEvent(st, f->evFork, 0), "wait");
+    auto run = [&](cudaStream_t st, const amp::SmallFronts &fr, double count) {
       timed_on(f, st, K_FRONTS, 2.0 * P.frontLvlFlops[L] * count / tot, P.frontLvlBytes[L] * scale * count / tot, [&] {
         return amp::launch_fronts_small<T>(fr, f->plan->dp, f->dValues, Lx, U, f->dStatus, la, st);
       });
-      if (fork) {
-        ck(cudaEventRecord(f->evFront[k], st), "event");
-        used[k] = true;
-      }
     };
     if (t1 > t0)
-      run(0, forkTiny, {f->plan->dTinySn + t0, (int)(t1 - t0), (int)(P.tinyMid[L] - t0), none, none}, (double)(t1 - t0));
-    if (s1 > s0) run(1, forkSmall, {nullptr, 0, 0, half, full}, (double)(s1 - s0));
+      run(used ? f->side : f->stream,
+          {f->plan->dTinySn + t0, (int)(t1 - t0), (int)(P.tinyMid[L] - t0), none, none}, (double)(t1 - t0));
+    if (s1 > s0) run(large ? f->side : f->stream, {nullptr, 0, 0, half, full}, (double)(s1 - s0));
+    if (used) ck(cudaEventRecord(f->evFront, f->side), "event");
   }
   void join() {
-    for (int k = 0; k < 2; k++) {
-      if (used[k]) ck(cudaStreamWaitEvent(f->stream, f->evFront[k], 0), "wait");
-      used[k] = false;
-    }
+    if (used) ck(cudaStreamWaitEvent(f->stream, f->evFront, 0), "wait");
+    used = false;
   }
 };
 
@@ -612,7 +631,7 @@ void device_solve_permuted(amp_factor *f) {
   ck(cudaMemsetAsync(f->dDone, 0, sizeof(int) * std::max(1, P.nsuper), st), "memset done");
   ck(cudaMemsetAsync(f->dSolveStatus, 0xff, sizeof(unsigned long long), st), "memset status");
   const int efwd = 2 * (++f->solveEpoch) - 1, ebwd = 2 * f->solveEpoch;
-  const int nf = (int)(P.fwdTasks1.size() / 4), nb = (int)(P.bwdAll.size() / 4);
+  const int nf = f->plan->nFwd1, nb = f->plan->nBwd1;
   const bool ldlt = f->kind == AMP_LDLT;
   const double *Dp = ldlt && !f->bk ? f->dD : nullptr;  // a Bunch-Kaufman factor's D solve runs between the sweeps
   timed(f, K_FORWARD, 2.0 * (double)P.nnzLStored, lbytes, [&] {
@@ -664,16 +683,24 @@ void device_solve(amp_factor *f, const double *dB, double *dX) {
 // uploaded once per plan and ns.
 constexpr int kWideBlocks = 2;
 static std::vector<int> expand_slices(const amp::Plan &P, const std::vector<int> &tasks, size_t ntasks, int ns,
-                                      bool wide) {
+                                      bool wide, bool forward) {
   std::vector<int> out;
   out.reserve(4 * ntasks * (size_t)ns);
+  auto put = [&](int s, int blk, int kind) {
+    if (wide && (P.snNc[s] + 63) / 64 <= kWideBlocks)
+      out.insert(out.end(), {s, blk, kind, -1});
+    else
+      for (int sl = 0; sl < ns; sl++) out.insert(out.end(), {s, blk, kind, sl});
+  };
+  auto whole = [&](int s) { return forward && !wide && P.snNc[s] <= 64 && P.snM[s] <= amp::whole_multi_rows(); };
   for (size_t i = 0; i < ntasks; i++) {
     const int *t = &tasks[4 * i];
-    if (t[2] == 2 || (wide && (P.snNc[t[0]] + 63) / 64 <= kWideBlocks)) {
-      out.insert(out.end(), {t[0], t[1], t[2], t[2] == 2 ? 0 : -1});
-      continue;
-    }
-    for (int sl = 0; sl < ns; sl++) out.insert(out.end(), {t[0], t[1], t[2], sl});
+    if (t[2] == 2)
+      out.insert(out.end(), {t[0], t[1], 2, 0});
+    else if (!whole(t[0]))
+      put(t[0], t[1], t[2]);
+    else if (t[2] == 0)  // its tasks below are part of it
+      for (int sl = 0; sl < ns; sl++) out.insert(out.end(), {t[0], 0, 3, sl});
   }
   return out;
 }
@@ -689,8 +716,8 @@ static void slice_lists(amp_plan *pl, int ns) {
     if ((P.snNc[sn] + 63) / 64 <= kWideBlocks) lSmall += e;
   }
   const bool wide = ns > 1 && lAll > 0 && 2 * lSmall >= lAll;
-  const std::vector<int> fw = expand_slices(P, P.fwdTasks, nf, ns, wide);
-  const std::vector<int> bw = expand_slices(P, P.bwdAll, P.bwdAll.size() / 4, ns, wide);
+  const std::vector<int> fw = join_small(P, expand_slices(P, P.fwdTasks, nf, ns, wide, true), true);
+  const std::vector<int> bw = join_small(P, expand_slices(P, P.bwdAll, P.bwdAll.size() / 4, ns, wide, false), true);
   pl->wideSl[ns - 1] = wide;
   pl->dBwdSl[ns - 1] = (int4 *)pl->mem.upload(bw);
   pl->nBwdSl[ns - 1] = (int)(bw.size() / 4);
@@ -1299,10 +1326,7 @@ int amp_factor_create(amp_plan *pl, const amp_factor_opts *opts, amp_factor **ou
       ck(cudaEventCreateWithFlags(&f->evPanel, cudaEventDisableTiming), "cudaEventCreate");
       ck(cudaEventCreateWithFlags(&f->evSide, cudaEventDisableTiming), "cudaEventCreate");
       ck(cudaEventCreateWithFlags(&f->evFork, cudaEventDisableTiming), "cudaEventCreate");
-      for (int k = 0; k < 2; k++) {
-        ck(cudaStreamCreateWithFlags(&f->front[k], cudaStreamNonBlocking), "cudaStreamCreate");
-        ck(cudaEventCreateWithFlags(&f->evFront[k], cudaEventDisableTiming), "cudaEventCreate");
-      }
+      ck(cudaEventCreateWithFlags(&f->evFront, cudaEventDisableTiming), "cudaEventCreate");
       ck(cudaEventCreate(&f->ev0), "cudaEventCreate");
       ck(cudaEventCreate(&f->ev1), "cudaEventCreate");
       const amp::Plan &P = pl->P;

@@ -22,6 +22,8 @@ struct DevPlan {
   const int *rowBlk;       // 64-column diagonal block holding column i (n; the flag a backward reader of row i waits for)
   const int64_t *invOff;   // offset of the inverse of each diagonal block (w x w, column-major)
   const int *diagSlot;     // CSR slot of A(i, i), original row i (the LDL^T pivot scale)
+  const int64_t *gatherOff;  // forward gathers: entry gatherOff[s] + b children(s) + q of gatherRange holds the entries
+  const int2 *gatherRange;   // [x, y) of child q's pass-up vector that map into 64-row block b of supernode s
   const int *solveSmall;   // supernodes solved whole by one warp (solve tasks of kind 2 index this list)
   long long spin;          // bound of every inter-CTA wait of the solve sweeps, in polls (kSpinLimit by default)
   // Bunch-Kaufman LDL^T factor (null otherwise): the pivot order inside every 64-column pivot block of every

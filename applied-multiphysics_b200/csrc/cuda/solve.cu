@@ -183,7 +183,7 @@ constexpr int kChPre = 64;  // children located and waited for at once by a forw
 // y_b = w_b - M_b y_{b-1}.
 template <class TL>
 __global__ void __launch_bounds__(256, 3) k_fwd_blocks(const int4 *__restrict__ tasks, int ntasks, int *__restrict__ ticket,
-                                                    DevPlan P, const TL *__restrict__ Lx, const TL *__restrict__ Inv,
+                                                    const __grid_constant__ DevPlan P, const TL *__restrict__ Lx, const TL *__restrict__ Inv,
                                                     const TL *__restrict__ Mch, double *__restrict__ y,
                                                     double *__restrict__ T, int *__restrict__ flags,
                                                     unsigned long long *__restrict__ hand, int epoch,
@@ -196,6 +196,33 @@ __global__ void __launch_bounds__(256, 3) k_fwd_blocks(const int4 *__restrict__ 
   __shared__ int2 chA[kChPre];
   __shared__ int64_t chMap[kChPre], chT[kChPre];
   __shared__ double vs[kWholeFront];
+  // v[map(a) - r0] += the pass-up entries a in [chA.x, chA.y) of the nq staged children, one child after another; a
+  // child's entries (two per thread) are read while the one before it is added
+  auto add_children = [&](const int nq, const int r0, double *v) {
+    const int tid = threadIdx.x;
+    auto fetch = [&](int q, double(&x)[2], int(&dst)[2]) {
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const int a = chA[q].x + tid + 256 * u;
+        const bool in = a < chA[q].y;
+        dst[u] = in ? P.eaMap[chMap[q] + a] - r0 : -1;
+        x[u] = in ? __ldcg(T + chT[q] + a) : 0.0;
+      }
+    };
+    double x[2], xn[2] = {0.0, 0.0};
+    int dst[2], dn[2] = {-1, -1};
+    fetch(0, x, dst);
+    for (int q = 0; q < nq; q++) {
+      if (q + 1 < nq) fetch(q + 1, xn, dn);
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        if (dst[u] >= 0) v[dst[u]] += x[u];
+        x[u] = xn[u];
+        dst[u] = dn[u];
+      }
+      __syncthreads();
+    }
+  };
   // kind 3: the whole supernode s (nc <= 64, m <= kWholeFront): gather its front vector v (all m rows) in shared
   // memory, y = X v[0:nc), then u = v - L[rows below, :] y in 64-row chunks (L values loaded a chunk ahead, the first
   // chunk before the waits); the same arithmetic, term by term, as a diagonal task and its below tasks
@@ -233,12 +260,7 @@ __global__ void __launch_bounds__(256, 3) k_fwd_blocks(const int4 *__restrict__ 
         ok = wait_count(done + c, (muc + kSB - 1) / kSB, status, s, P.spin);
       }
       if (!__syncthreads_and(ok)) return false;  // block-uniform
-      for (int q = 0; q < nq; q++) {
-        const int *map = P.eaMap + chMap[q];
-        const double *tc = T + chT[q];
-        for (int a = tid; a < chA[q].y; a += blockDim.x) vs[map[a]] += __ldcg(tc + a);
-        __syncthreads();
-      }
+      add_children(nq, 0, vs);
     }
     if (q0 == q1) __syncthreads();
     {  // y = X v[0:nc): thread (row, part) sums columns part, part + 4, ... <= row
@@ -283,7 +305,7 @@ __global__ void __launch_bounds__(256, 3) k_fwd_blocks(const int4 *__restrict__ 
   auto run = [&](const int tkv) -> bool {
     const int4 t = tasks[tkv];
     if (t.z == 3) return whole(t.x);
-    if (t.z == 2) {  // up to kSolveGroup supernodes with m <= 32, one warp each
+    if (t.z == 2) {  // up to kSolveWarps supernodes with m <= 32, one warp each
       const int warp = threadIdx.x >> 5;
       if (threadIdx.x == 0) waitOk = 1;
       __syncthreads();
@@ -310,11 +332,12 @@ __global__ void __launch_bounds__(256, 3) k_fwd_blocks(const int4 *__restrict__ 
       for (int e = tid; e < rows * rows; e += blockDim.x) Xs[e % rows][e / rows] = (double)X[e];
     }
     // this task's rows of v: pivot rows start from y; the children's entries mapping to rows [r0, r0 + rows) are added
-    // in child order (the map is increasing, so they form one range per child). Up to kChPre children at a time, one
-    // per thread: the thread locates the child's range (static) and then waits for the child, so that the searches
-    // and the waits of all children overlap.
+    // in child order (the map is increasing, so they form one range per child, found with the schedule: searching the
+    // map on the device was two chains of dependent loads per task). Up to kChPre children at a time, one per thread,
+    // so that the waits of all children overlap.
     if (tid < kSB) rk[tid] = (tid < rows && r0 + tid < nc) ? y[f + r0 + tid] : 0.0;
     const int q0 = P.chPtr[s], q1 = P.chPtr[s + 1];
+    const int64_t range0 = P.gatherOff[s] + (int64_t)((below ? (nc + kSB - 1) / kSB : 0) + blk) * (q1 - q0);
     for (int qb = q0; qb < q1; qb += kChPre) {
       const int nq = min(kChPre, q1 - qb);
       if (qb > q0) __syncthreads();  // the previous chunk's ranges are consumed
@@ -322,30 +345,13 @@ __global__ void __launch_bounds__(256, 3) k_fwd_blocks(const int4 *__restrict__ 
       if (tid < nq) {
         const int c = P.chList[qb + tid];
         const int muc = P.snM[c] - P.snNc[c];
-        const int *map = P.eaMap + P.eaPtr[c];
-        int lo = 0, hi = muc;
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          if (map[mid] < r0) lo = mid + 1; else hi = mid;
-        }
-        const int a0 = lo;
-        hi = muc;
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          if (map[mid] < r0 + rows) lo = mid + 1; else hi = mid;
-        }
-        chA[tid] = make_int2(a0, lo);
+        chA[tid] = P.gatherRange[range0 + qb - q0 + tid];
         chMap[tid] = P.eaPtr[c];
         chT[tid] = P.snTOff[c];
         ok = wait_count(done + c, (muc + kSB - 1) / kSB, status, s, P.spin);
       }
       if (!__syncthreads_and(ok)) return false;  // block-uniform
-      for (int q = 0; q < nq; q++) {
-        const int *map = P.eaMap + chMap[q];
-        const double *tc = T + chT[q];
-        for (int a = chA[q].x + tid; a < chA[q].y; a += blockDim.x) rk[map[a] - r0] += __ldcg(tc + a);
-        __syncthreads();
-      }
+      add_children(nq, r0, rk);
     }
     if (q0 == q1) __syncthreads();
     const double vreg = tid < kSB ? rk[tid] : 0.0;
@@ -459,7 +465,7 @@ __global__ void __launch_bounds__(256, 3) k_fwd_blocks(const int4 *__restrict__ 
 constexpr int kBwdSmem = 2 * kSB * (kSB + 1) * (int)sizeof(double);
 template <class TL>
 __global__ void __launch_bounds__(256, 3) k_bwd_blocks(const int4 *__restrict__ tasks, int ntasks, int *__restrict__ ticket,
-                                                    DevPlan P, const TL *__restrict__ Lx, const TL *__restrict__ Inv,
+                                                    const __grid_constant__ DevPlan P, const TL *__restrict__ Lx, const TL *__restrict__ Inv,
                                                     const TL *__restrict__ Gch, const double *__restrict__ Dpiv,
                                                     double *__restrict__ y, int *__restrict__ flags,
                                                     unsigned long long *__restrict__ hand, int epoch,
@@ -475,7 +481,7 @@ __global__ void __launch_bounds__(256, 3) k_bwd_blocks(const int4 *__restrict__ 
   double(*Gt)[kSB + 1] = reinterpret_cast<double(*)[kSB + 1]>(bwd_dyn + kSB * (kSB + 1));  // G_b, [r][c]
   auto run = [&](const int tkv) -> bool {
     const int4 t = tasks[tkv];
-    if (t.z == 2) {  // up to kSolveGroup supernodes with m <= 32, one warp each
+    if (t.z == 2) {  // up to kSolveWarps supernodes with m <= 32, one warp each
       const int warp = threadIdx.x >> 5;
       if (threadIdx.x == 0) waitOk = 1;
       __syncthreads();

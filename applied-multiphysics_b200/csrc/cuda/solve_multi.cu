@@ -16,11 +16,24 @@
 // each, not expanded) solve all q vectors and count/release every slice.
 //
 // A task is a small GEMM on the FP64 tensor cores (mma.sync m16n8k16): out (64 rows x 16 vectors) = sum over a
-// reduction index of A (64 x 32 chunk, FP32 factors widened on the shared-memory store) times B (32 x 16), 8 warps
-// as 4 (16-row blocks) x 2 (16-wide halves of the chunk), the halves summed through shared memory at the end.
+// reduction index of A (64 rows x a chunk, FP32 factors widened as they are read) times B (chunk x 16), 8 warps as 4
+// 16-row blocks x 2 vector halves, each with the whole reduction of its tile (no sum over warps).
 // Forward: A = L[block rows, pivot columns so far], B = y[those columns]. Backward: A = the block's columns of L over
-// the rows below the block (transposed on load), B = x[those rows]. Then the 64 x 64 inverse of the diagonal block,
-// prefetched into shared memory by cp.async when the task starts, is applied the same way.
+// the rows below the block, B = x[those rows]. Then the 64 x 64 inverse of the diagonal block, prefetched into shared
+// memory by cp.async when the task starts, is applied the same way.
+//
+// What bounds a task is latency, not bandwidth: the factor's chunks, the flags, the values behind the flags and the
+// children's rows were read one after the other, each a trip to L2 or HBM. So A streams through a ring of four
+// cp.async stages (16 FP64 or 32 FP32 columns each; two in flight while one is multiplied, small enough for three
+// CTAs per SM), the flags of up to 32 blocks (8 ancestor chunks) are polled at once, the values are read one block
+// ahead of the products, and the children's rows are read ahead of their maps (solve_small.cuh). 16 vectors
+// of the quadratic heat system with 32 elements per edge (FP32 factors), five sweeps each way: forward 15.4 -> 11.6 ms,
+// backward 10.4 -> 8.7 ms; FP64 LDL^T factors of the edge-element system with 24: 5.25 -> 3.82 and 3.73 -> 3.20 ms.
+//
+// Supernodes with one pivot block and at most kWholeMulti rows (in plans that are not WIDE) are one task per slice
+// (kind 3, run_whole): their block tasks did a few products each and paid a hand-off through flags in between. A batch
+// of 64 systems of 4,225 unknowns, where most supernodes are of this size: forward 4.05 -> 2.39 ms, backward 3.10 ->
+// 2.20 ms.
 //
 // Backward order: the rows below the supernode are summed from the last chunk down, each chunk after the flags of the
 // ancestor blocks that hold its rows (rowBlk), so a task works while its ancestors are still being solved (the
@@ -37,22 +50,34 @@
 
 namespace amp {
 
-constexpr int kMB = 64;              // rows of a block task
-constexpr int kKC = 32;              // reduction chunk
-constexpr int kQS = 16;              // vectors per slice (one slice per task)
-constexpr int kMQ = 64;              // vectors per pass (the host splits larger sets)
-constexpr int kLdKM = kMB + 4;       // A stored [k][m] (m contiguous): 68 doubles, == 4 mod 16 (conflict-free fragments)
-constexpr int kLdMK = kKC + 4;       // A chunk stored [m][k]: 36
-constexpr int kLdX = kMB + 4;        // inverse block stored [k][m] or [m][k], 64 x 64: 68
-constexpr int kLdB = kQS + 4;        // B stored [k][n]: 20
-constexpr int kMultiThreads = 256;
-constexpr int kMultiCtas = 3;      // resident CTAs per SM of the persistent sweeps (registers capped at 80)
-constexpr int kAElems = kMB * kLdMK;  // >= kKC * kLdKM; also the halves' reduction buffer (64 x 17)
-static_assert(kAElems >= kKC * kLdKM && kAElems >= kMB * (kQS + 1), "A tile buffer");
+constexpr int kMB = 64;   // rows of a block task
+constexpr int kQS = 16;   // vectors per slice (one slice per task)
+constexpr int kMQ = 64;   // vectors per pass (the host splits larger sets)
+// A operands stream through a ring of stages, a chunk of the reduction index each: 16 FP64 or 32 FP32 columns
 template <class TL>
+constexpr int chunk_k() { return sizeof(TL) == 8 ? 16 : 32; }
+constexpr int kStages = 4;
+constexpr int kLdKM = kMB + 4;  // a chunk stored [k][m] (m contiguous): 4 mod 16 doubles, 4 mod 32 floats
+template <class TL>
+constexpr int ld_mk() { return chunk_k<TL>() + 4; }  // a chunk stored [m][k]: 20 doubles, 36 floats (conflict-free)
+constexpr int kLdB = kQS + 4;  // B and R stored [k][n]: 20
+constexpr int kMultiThreads = 256;
+constexpr int kMultiCtas = 3;  // resident CTAs per SM of the persistent sweeps (registers capped at 80)
+constexpr int kWholeMulti = 256;  // supernodes with one pivot block and at most this many rows are one task per slice
+constexpr int kRingBytes = kStages * kMB * ld_mk<double>() * (int)sizeof(double);  // the largest stage: FP64 [m][k]
+static_assert(kMB * ld_mk<float>() * 4 <= kMB * ld_mk<double>() * 8 && chunk_k<double>() * kLdKM <= kMB * ld_mk<double>() &&
+                  chunk_k<float>() * kLdKM * 4 <= kMB * ld_mk<double>() * 8,
+              "ring stage");
+static_assert(kWholeMulti * kLdB * 8 <= kRingBytes && 2 * chunk_k<double>() * kLdKM * 8 <= 2 * kMB * kLdB * 8 &&
+                  2 * chunk_k<float>() * kLdKM * 4 <= 2 * kMB * kLdB * 8,
+              "whole-supernode tasks: the front vector in the ring, two stages in Bs");
+int whole_multi_rows() { return kWholeMulti; }
+// front vectors of one warp of a kind 2 task of `count` supernodes (more than kSolveGroup: m <= kTinyMid)
+__host__ __device__ constexpr int small_stride(int count) { return (count > kSolveGroup ? kTinyMid : kTinyFront) * kMQ; }
 constexpr int multi_smem() {
-  const int own = (kAElems + 2 * kMB * kLdB) * (int)sizeof(double) + kMB * kLdX * (int)sizeof(TL);
-  const int small = kSolveGroup * 32 * kMQ * (int)sizeof(double);  // kind 2 tasks: 32 x 64 front vectors per warp
+  const int own = kRingBytes + 3 * kMB * kLdB * (int)sizeof(double);
+  const int small = kSolveGroup * small_stride(kSolveGroup) * (int)sizeof(double);
+  static_assert(kSolveWarps * small_stride(kSolveWarps) <= kSolveGroup * small_stride(kSolveGroup), "kind 2 tasks");
   const int wide = (2 * 32 + kMB) * 66 * (int)sizeof(double);        // all-vector tasks (kWideSmem)
   const int m1 = own > small ? own : small;
   return m1 > wide ? m1 : wide;
@@ -69,49 +94,30 @@ __device__ __forceinline__ void dmma16816(double (&c)[4], const double (&a)[8], 
 
 // Fragment layouts of the m16n8k16 FP64 MMA (g = lane / 4, t = lane % 4): A (m = g + 8 (v & 1), k = t + 4 (v >> 1)),
 // B (n = g, k = t + 4 v), C (m = g + 8 (v >> 1), n = 2 t + (v & 1)).
-// c[nb] += A[16 mw .. +16, k0 .. k0 + 16) B[k0 .. k0 + 16, 8 nb .. 8 nb + 8) for both n halves; A element (m, k) at
-// A[k * lda + m] (KM) or A[m * lda + k] (MK), B element (k, n) at B[k * kLdB + n].
-template <bool KM, class TA>
-__device__ __forceinline__ void mma_k16(const TA *__restrict__ A, int lda, const double *__restrict__ B, int k0,
-                                        int mw, int lane, double (&c)[2][4]) {
-  const int g = lane >> 2, t = lane & 3;
-  double a[8];
+// One chunk: c += A[16 mw .. +16, 0 .. K) B[0 .. K, 8 nv .. 8 nv + 8) with K = chunk_k; A element (m, k) at A[k * kLdKM + m]
+// (KM) or A[m * ld_mk + k], widened to FP64 as it is read; B element (k, n) at B[k * kLdB + n]. 8 warps: mw = warp % 4 the
+// 16-row blocks, nv = warp / 4 the vector halves, so a tile needs no sum over warps.
+template <bool KM, class TL>
+__device__ __forceinline__ void mma_chunk(const TL *__restrict__ A, const double *__restrict__ B, int warp, int lane,
+                                          double (&c)[4]) {
+  const int g = lane >> 2, t = lane & 3, m0 = 16 * (warp & 3), n = 8 * (warp >> 2) + g;
 #pragma unroll
-  for (int v = 0; v < 8; v++) {
-    const int m = 16 * mw + g + 8 * (v & 1), k = k0 + t + 4 * (v >> 1);
-    a[v] = (double)(KM ? A[k * lda + m] : A[m * lda + k]);
-  }
+  for (int k0 = 0; k0 < chunk_k<TL>(); k0 += 16) {
+    double a[8], b[4];
 #pragma unroll
-  for (int nb = 0; nb < 2; nb++) {
-    double b[4];
+    for (int v = 0; v < 8; v++) {
+      const int m = m0 + g + 8 * (v & 1), k = k0 + t + 4 * (v >> 1);
+      a[v] = (double)(KM ? A[k * kLdKM + m] : A[m * ld_mk<TL>() + k]);
+    }
 #pragma unroll
-    for (int v = 0; v < 4; v++) b[v] = B[(k0 + t + 4 * v) * kLdB + 8 * nb + g];
-    dmma16816(c[nb], a, b);
-  }
-}
-
-// The two halves of the reduction index: warps 4-7 add their partial tile into warps 0-3's (red: 64 x 17 doubles).
-// On return warps 0-3 hold the sum; red is free after the caller's next barrier.
-__device__ __forceinline__ void halves_sum(double (&c)[2][4], double *red, int warp, int lane) {
-  const int mw = warp & 3, g = lane >> 2, t = lane & 3;
-  if (warp >= 4) {
-#pragma unroll
-    for (int nb = 0; nb < 2; nb++)
-#pragma unroll
-      for (int v = 0; v < 4; v++) red[(16 * mw + g + 8 * (v >> 1)) * (kQS + 1) + 8 * nb + 2 * t + (v & 1)] = c[nb][v];
-  }
-  __syncthreads();
-  if (warp < 4) {
-#pragma unroll
-    for (int nb = 0; nb < 2; nb++)
-#pragma unroll
-      for (int v = 0; v < 4; v++) c[nb][v] += red[(16 * mw + g + 8 * (v >> 1)) * (kQS + 1) + 8 * nb + 2 * t + (v & 1)];
+    for (int v = 0; v < 4; v++) b[v] = B[(k0 + t + 4 * v) * kLdB + n];
+    dmma16816(c, a, b);
   }
 }
 
-// row / vector of accumulator element (nb, v) of this lane (warps 0-3)
+// row / vector of accumulator element v of this lane
 __device__ __forceinline__ int acc_row(int warp, int lane, int v) { return 16 * (warp & 3) + (lane >> 2) + 8 * (v >> 1); }
-__device__ __forceinline__ int acc_vec(int lane, int nb, int v) { return 8 * nb + 2 * (lane & 3) + (v & 1); }
+__device__ __forceinline__ int acc_vec(int warp, int lane, int v) { return 8 * (warp >> 2) + 2 * (lane & 3) + (v & 1); }
 
 __device__ __forceinline__ void cp_async_el(void *smem, const void *gmem, int bytes, bool valid) {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
@@ -120,6 +126,11 @@ __device__ __forceinline__ void cp_async_el(void *smem, const void *gmem, int by
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(gmem), "r"(n) : "memory");
   else
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(sa), "l"(gmem), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 __device__ __forceinline__ void cp_async_all() {
   asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -139,25 +150,30 @@ __device__ __forceinline__ void ticket_loop(int *ticket, int ntasks, Run &&run) 
   }
 }
 
-// This task's rows [r0, r0 + rows) of the front vector v_s = [y(f .. f + nc); 0] + the children's pass-up vectors,
-// vectors [vb, vb + qs) of q, into Rs (row r at Rs[r LDR], QW >= qs columns; zero outside): the pivot rows from y,
-// then each child's entries that map into these rows, in the reference's child order. Up to kGatherCh children at a
-// time, one per thread: the thread locates the child's entries for these rows (the map is increasing, so they form
-// one range) and waits for the child's pass-up vectors of slices [sl0, sl0 + nsl), so the searches and the waits of
-// all children overlap and every task of the supernode gathers its own rows in parallel. false: a wait gave up.
+// This task's rows [r0, r0 + rows) of the front vector v_s = [y(f .. f + nc); 0] + the children's pass-up vectors (rb:
+// their 64-row block), vectors [vb, vb + qs) of q, into Rs (row r at Rs[r LDR], QW >= qs columns; zero outside): the
+// pivot rows from y, then each child's entries that map into these rows (the schedule's gatherRange), in the
+// reference's child order. Up to kGatherCh children at a time, one per thread, are waited for (their pass-up vectors of
+// slices [sl0, sl0 + nsl)), so the waits of all children overlap; a child's entries are read while the one before it is
+// added. Every task of the supernode gathers its own rows in parallel. false: a wait gave up.
 constexpr int kGatherCh = 64;
+// whole: rb is not used, the rows are the whole front (r0 = 0) and every child's vector is taken whole. Rs is cleared up
+// to the next multiple of kMB rows.
 template <int QW, int LDR>
-__device__ bool gather_front_rows(const DevPlan &P, int s, int r0, int rows, const double *__restrict__ y,
+__device__ __forceinline__ bool gather_front_rows(const DevPlan &P, int s, bool whole, int rb, int r0, int rows,
+                                                  const double *__restrict__ y,
                                   const double *__restrict__ T, int *done, int sl0, int nsl, int q, int vb, int qs,
                                   unsigned long long *status, double *Rs) {
   __shared__ int2 chA[kGatherCh];
   __shared__ int64_t chMap[kGatherCh], chT[kGatherCh];
+  constexpr int N = 4;  // entries per thread read ahead
   const int tid = threadIdx.x, f = P.snF[s], nc = P.snNc[s];
-  for (int e = tid; e < kMB * QW; e += blockDim.x) {
+  for (int e = tid; e < (rows + kMB - 1) / kMB * kMB * QW; e += blockDim.x) {
     const int row = e / QW, k = e % QW;
     Rs[row * LDR + k] = (row < rows && k < qs && r0 + row < nc) ? y[(int64_t)(f + r0 + row) * q + vb + k] : 0.0;
   }
   const int q0 = P.chPtr[s], q1 = P.chPtr[s + 1];
+  const int64_t range0 = P.gatherOff[s] + (int64_t)rb * (q1 - q0);
   for (int qb = q0; qb < q1; qb += kGatherCh) {
     const int nq = min(kGatherCh, q1 - qb);
     if (qb > q0) __syncthreads();  // the previous chunk's ranges are consumed
@@ -165,34 +181,46 @@ __device__ bool gather_front_rows(const DevPlan &P, int s, int r0, int rows, con
     if (tid < nq) {
       const int c = P.chList[qb + tid];
       const int muc = P.snM[c] - P.snNc[c];
-      const int *map = P.eaMap + P.eaPtr[c];
-      int lo = 0, hi = muc;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (map[mid] < r0) lo = mid + 1; else hi = mid;
-      }
-      const int a0 = lo;
-      hi = muc;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (map[mid] < r0 + rows) lo = mid + 1; else hi = mid;
-      }
-      chA[tid] = make_int2(a0, lo);
+      chA[tid] = whole ? make_int2(0, muc) : P.gatherRange[range0 + qb - q0 + tid];
       chMap[tid] = P.eaPtr[c];
       chT[tid] = P.snTOff[c];
       const int need = (muc + kMB - 1) / kMB;
       for (int sl = sl0; sl < sl0 + nsl && ok; sl++) ok = wait_count(done + (int64_t)sl * P.nsuper + c, need, status, s, P.spin);
     }
     if (!__syncthreads_and(ok)) return false;  // block-uniform
-    for (int qq = 0; qq < nq; qq++) {
-      const int *map = P.eaMap + chMap[qq];
-      const double *tc = T + chT[qq] * q + vb;
+    // the first N entries per thread of child qq (row a0 + e / QW of its vector, vector e % QW), and where they go
+    auto fetch = [&](int qq, double(&v)[N], int(&dst)[N]) {
       const int a0 = chA[qq].x, na = chA[qq].y - a0;
-      for (int e = tid; e < na * QW; e += blockDim.x) {
+#pragma unroll
+      for (int u = 0; u < N; u++) {
+        const int e = tid + (int)blockDim.x * u, a = a0 + e / QW, k = e % QW;
+        dst[u] = -1;
+        v[u] = 0.0;
+        if (e < na * QW && k < qs) {
+          dst[u] = (P.eaMap[chMap[qq] + a] - r0) * LDR + k;
+          v[u] = __ldcg(T + (chT[qq] + a) * q + vb + k);
+        }
+      }
+    };
+    double v[N], vn[N];
+    int dst[N], dn[N];
+    fetch(0, v, dst);
+    for (int qq = 0; qq < nq; qq++) {
+      if (qq + 1 < nq) fetch(qq + 1, vn, dn);
+#pragma unroll
+      for (int u = 0; u < N; u++)
+        if (dst[u] >= 0) Rs[dst[u]] += v[u];
+      const int a0 = chA[qq].x, na = chA[qq].y - a0;
+      for (int e = tid + (int)blockDim.x * N; e < na * QW; e += blockDim.x) {
         const int a = a0 + e / QW, k = e % QW;
-        if (k < qs) Rs[(map[a] - r0) * LDR + k] += __ldcg(tc + (int64_t)a * q + k);
+        if (k < qs) Rs[(P.eaMap[chMap[qq] + a] - r0) * LDR + k] += __ldcg(T + (chT[qq] + a) * q + vb + k);
       }
       __syncthreads();
+#pragma unroll
+      for (int u = 0; u < N; u++) {
+        v[u] = vn[u];
+        dst[u] = dn[u];
+      }
     }
   }
   if (q0 == q1) __syncthreads();
@@ -242,7 +270,7 @@ __device__ __forceinline__ bool fwd_wide_task(const int4 t, const DevPlan &P, co
   const int ncols = below ? nc : blk * kMB;
   int *myflags = flags + P.blkOff[s];  // the slice-0 set: this supernode releases every slice at once
   // this task's rows of v_s, every vector, into Rs (every slice of each child done)
-  if (!gather_front_rows<kMQ, kWLd>(P, s, r0, rows, y, T, done, 0, ns, q, 0, q, status, Rs)) return false;
+  if (!gather_front_rows<kMQ, kWLd>(P, s, false, (below ? (nc + kMB - 1) / kMB : 0) + blk, r0, rows, y, T, done, 0, ns, q, 0, q, status, Rs)) return false;
   double acc[4][4];
 #pragma unroll
   for (int i = 0; i < 4; i++)
@@ -474,17 +502,18 @@ __device__ __forceinline__ bool bwd_wide_task(const int4 t, const DevPlan &P, co
 // chunk, the reduction and the inverse product.
 template <class TL, bool WIDE>
 __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_fwd_multi(const int4 *__restrict__ tasks, int ntasks, int ns,
-                                                                int *__restrict__ ticket, DevPlan P,
+                                                                int *__restrict__ ticket, const __grid_constant__ DevPlan P,
                                                                 const TL *__restrict__ Lx, const TL *__restrict__ Inv,
                                                                 const TL *__restrict__ Mch, double *__restrict__ y,
                                                                 double *__restrict__ T, int *__restrict__ flags,
                                                                 int nflags, int epoch, int *__restrict__ done, int q,
                                                                 unsigned long long *status) {
   extern __shared__ double msm[];
-  double *As = msm, *Bs = As + kAElems, *Rs = Bs + kMB * kLdB;
-  TL *Xs = reinterpret_cast<TL *>(Rs + kMB * kLdB);
-  __shared__ int waitOk;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, mw = warp & 3, kh = warp >> 2;
+  constexpr int KC = chunk_k<TL>(), PB = kMB / KC;  // reduction chunk, chunks per 64-column block
+  TL *ring = reinterpret_cast<TL *>(msm);
+  double *Bs = msm + kRingBytes / sizeof(double), *Rs = Bs + 2 * kMB * kLdB;  // two blocks of y values; v_s, then R
+  __shared__ int waitOk, sReady;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   auto bail = [] {  // a wait gave up: drain this thread's copies into shared memory before the CTA leaves
     cp_async_all();
     return false;
@@ -494,176 +523,230 @@ __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_fwd_multi(const i
     const int s = t.x, blk = t.y, below = t.z;
     const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s], mu = m - nc;
     const int vb = sl * kQS, qs = min(kQS, q - vb);
-    const TL *Lp = Lx + P.snLxp[s];
     const int r0 = below ? nc + blk * kMB : blk * kMB;
     const int rows = below ? min(kMB, mu - blk * kMB) : min(kMB, nc - blk * kMB);
     const bool chain = Mch != nullptr && !below && blk > 0;  // block b - 1 enters through M_b after the last wait
     const int ncols = below ? nc : (chain ? blk - 1 : blk) * kMB;
     int *myflags = flags + (int64_t)sl * nflags + P.blkOff[s];
     int *mydone = done + (int64_t)sl * P.nsuper;
-    if (!below) {  // the inverse of the diagonal block, [k][m], arrives while the task sums
-      const TL *X = Inv + P.invOff[P.blkOff[s] + blk];
-      for (int e = tid; e < kMB * kMB; e += kMultiThreads) {
-        const int i = e & (kMB - 1), k = e >> 6;
-        const bool ok = i < rows && k < rows;
-        cp_async_el(Xs + k * kLdX + i, ok ? X + (int64_t)k * rows + i : X, (int)sizeof(TL), ok);
-      }
-      asm volatile("cp.async.commit_group;\n" ::: "memory");
-    }
-    // this task's rows of v_s (this slice) into Rs, gathered by every task of the supernode in parallel
-    if (!gather_front_rows<kQS, kLdB>(P, s, r0, rows, y, T, done, sl, 1, q, vb, qs, status, Rs)) return bail();
-    double c[2][4];
+    // The task's A operands, chunk after chunk: L[block rows, the columns summed], then (diagonal) the block's inverse X
+    // and M_b. None depends on another task of the sweep, so they stream through the ring kStages - 1 chunks ahead.
+    const int nL = (ncols + KC - 1) / KC, nX = below ? 0 : (rows + KC - 1) / KC, nM = chain ? PB : 0;
+    const TL *Lb = Lx + P.snLxp[s] + r0;
+    const TL *Xb = Inv + (below ? 0 : P.invOff[P.blkOff[s] + blk]);
+    const TL *Mb = chain ? Mch + (int64_t)(P.blkOff[s] - s + blk - 1) * kMB * kMB : Xb;
+    auto issue = [&](int i) {  // [k][m]: chunk i's element (row, column k0 + cc) at [cc kLdKM + row]
+      const bool isL = i < nL, isX = !isL && i < nL + nX;
+      const TL *src = isL ? Lb : isX ? Xb : Mb;
+      const int ld = isL ? m : isX ? rows : kMB, lim = isL ? ncols : isX ? rows : kMB;
+      const int k0 = (isL ? i : isX ? i - nL : i - nL - nX) * KC;
+      TL *dst = ring + (i % kStages) * (KC * kLdKM);
+      if (i < nL + nX + nM) {
 #pragma unroll
-    for (int nb = 0; nb < 2; nb++)
-#pragma unroll
-      for (int v = 0; v < 4; v++) c[nb][v] = 0.0;
-    // L chunk, [k][m]: As[cc][row] = L(r0 + row, cb + cc); thread elements e = tid + 256 u: row = e & 63, cc = e >> 6
-    TL lr[8];
-    auto loadL = [&](int cb) {
-#pragma unroll
-      for (int u = 0; u < 8; u++) {
-        const int e = tid + kMultiThreads * u, row = e & (kMB - 1), cc = e >> 6;
-        lr[u] = (row < rows && cb + cc < ncols) ? Lp[(int64_t)(cb + cc) * m + r0 + row] : (TL)0;
-      }
-    };
-    const int nch = (ncols + kKC - 1) / kKC;
-    if (nch > 0) loadL(0);
-    for (int ch = 0; ch < nch; ch++) {
-      const int cb = ch * kKC, cw = min(kKC, ncols - cb);
-      const double *Bc = Bs + (cb & (kMB - 1)) * kLdB;  // this chunk's rows of the block's y values
-      if ((cb & (kMB - 1)) == 0) {  // first chunk of a pivot block: its y values final? Then all 64 rows at once
-        if (tid == 0) waitOk = wait_flag(myflags + cb / kMB, epoch, status, s, P.spin);
-        __syncthreads();
-        if (!waitOk) return bail();
-        for (int e = tid; e < kMB * kQS; e += kMultiThreads) {
-          const int k = e >> 4, n = e & (kQS - 1);
-          Bs[k * kLdB + n] = (cb + k < ncols && n < qs) ? __ldcg(y + (int64_t)(f + cb + k) * q + vb + n) : 0.0;
+        for (int u = 0; u < KC * kMB / kMultiThreads; u++) {
+          const int e = tid + kMultiThreads * u, row = e & (kMB - 1), cc = e >> 6;
+          const bool ok = row < rows && k0 + cc < lim;
+          cp_async_el(dst + cc * kLdKM + row, ok ? src + (int64_t)(k0 + cc) * ld + row : src, (int)sizeof(TL), ok);
         }
       }
+      cp_async_commit();
+    };
+    for (int i = 0; i < kStages - 1; i++) issue(i);
+    // this task's rows of v_s (this slice) into Rs, gathered by every task of the supernode in parallel
+    if (!gather_front_rows<kQS, kLdB>(P, s, false, (below ? (nc + kMB - 1) / kMB : 0) + blk, r0, rows, y, T, done, sl, 1, q, vb,
+                                      qs, status, Rs))
+      return bail();
+    double c[4] = {0.0, 0.0, 0.0, 0.0};
+    // y values of a pivot block (64 x 16, four per thread): read one block ahead when that block is known final. ready:
+    // the leading blocks known final, found for up to 32 blocks at a time.
+    double yr[4];
+    auto load_y = [&](int cb) {
 #pragma unroll
-      for (int u = 0; u < 8; u++) {
-        const int e = tid + kMultiThreads * u;
-        As[(e >> 6) * kLdKM + (e & (kMB - 1))] = (double)lr[u];
+      for (int u = 0; u < 4; u++) {
+        const int e = tid + kMultiThreads * u, k = e >> 4, n = e & (kQS - 1);
+        yr[u] = (cb + k < ncols && n < qs) ? __ldcg(y + (int64_t)(f + cb + k) * q + vb + n) : 0.0;
       }
-      __syncthreads();
-      if (ch + 1 < nch) loadL(cb + kKC);
-      if (16 * kh < cw) mma_k16<true>(As, kLdKM, Bc, 16 * kh, mw, lane, c);
-      __syncthreads();
-    }
-    halves_sum(c, As, warp, lane);
-    // R = v[block] - acc (the task's rows of v in Rs)
-    if (below) {
-      if (warp < 4) {
-        double *to = T + (P.snTOff[s] + (int64_t)blk * kMB) * q + vb;
-#pragma unroll
-        for (int nb = 0; nb < 2; nb++)
-#pragma unroll
-          for (int v = 0; v < 4; v++) {
-            const int row = acc_row(warp, lane, v), n = acc_vec(lane, nb, v);
-            if (row < rows && n < qs) to[(int64_t)row * q + n] = Rs[row * kLdB + n] - c[nb][v];
+    };
+    int ready = 0;
+    bool ahead = false;
+    for (int i = 0; i < nL; i++) {
+      const int cb = i * KC, j = cb / kMB;
+      const bool first = (cb & (kMB - 1)) == 0;
+      double *Bj = Bs + (j & 1) * kMB * kLdB;
+      if (first) {
+        if (!ahead) {
+          if (ready <= j) {
+            if (warp == 0) {
+              const bool fin = (j + lane) * kMB < ncols && ld_acquire(myflags + j + lane) == epoch;
+              int run = __ffs(~__ballot_sync(0xffffffffu, fin)) - 1;
+              if (run < 0) run = 32;
+              if (run == 0) {
+                int ok = 1;
+                if (lane == 0) ok = wait_flag(myflags + j, epoch, status, s, P.spin);
+                run = __shfl_sync(0xffffffffu, ok, 0) ? 1 : -1;
+              }
+              if (lane == 0) sReady = run < 0 ? -1 : j + run;
+            }
+            __syncthreads();
+            ready = sReady;
+            if (ready < 0) return bail();
           }
+          load_y(cb);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const int e = tid + kMultiThreads * u;
+          Bj[(e >> 4) * kLdB + (e & (kQS - 1))] = yr[u];
+        }
+      }
+      cp_async_wait<kStages - 2>();
+      __syncthreads();  // chunk i and its y values have arrived; every warp is done with chunk i - 1
+      if (first) {
+        ahead = ready > j + 1 && cb + kMB < ncols;
+        if (ahead) load_y(cb + kMB);
+      }
+      issue(i + kStages - 1);
+      mma_chunk<true>(ring + (i % kStages) * (KC * kLdKM), Bj + (cb & (kMB - 1)) * kLdB, warp, lane, c);
+    }
+    // R = v[block] - the sum (the task's rows of v in Rs)
+    if (below) {
+      double *to = T + (P.snTOff[s] + (int64_t)blk * kMB) * q + vb;
+#pragma unroll
+      for (int v = 0; v < 4; v++) {
+        const int row = acc_row(warp, lane, v), n = acc_vec(warp, lane, v);
+        if (row < rows && n < qs) to[(int64_t)row * q + n] = Rs[row * kLdB + n] - c[v];
       }
       __syncthreads();
       if (tid == 0) red_release_add(mydone + s, 1);
       return true;
     }
-    if (warp < 4) {
 #pragma unroll
-      for (int nb = 0; nb < 2; nb++)
-#pragma unroll
-        for (int v = 0; v < 4; v++) {
-          const int row = acc_row(warp, lane, v), n = acc_vec(lane, nb, v);
-          Rs[row * kLdB + n] = (row < rows && n < qs) ? Rs[row * kLdB + n] - c[nb][v] : 0.0;
-        }
+    for (int v = 0; v < 4; v++) {
+      const int at = acc_row(warp, lane, v) * kLdB + acc_vec(warp, lane, v);
+      Rs[at] = (acc_row(warp, lane, v) < rows && acc_vec(warp, lane, v) < qs) ? Rs[at] - c[v] : 0.0;
+      c[v] = 0.0;
     }
-#pragma unroll
-    for (int nb = 0; nb < 2; nb++)
-#pragma unroll
-      for (int v = 0; v < 4; v++) c[nb][v] = 0.0;
-    cp_async_all();
-    __syncthreads();
-    // y[block] = X R: k = 0 .. 63 of X as four k16 steps, two per warp half
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const int k0 = 32 * h + 16 * kh;
-      if (k0 < rows) mma_k16<true>(Xs, kLdX, Rs, k0, mw, lane, c);
+    // y[block] = X R
+    for (int i = nL; i < nL + nX; i++) {
+      cp_async_wait<kStages - 2>();
+      __syncthreads();
+      issue(i + kStages - 1);
+      mma_chunk<true>(ring + (i % kStages) * (KC * kLdKM), Rs + (i - nL) * KC * kLdB, warp, lane, c);
     }
-    halves_sum(c, As, warp, lane);
-    if (chain) {
-      // W stays in Rs (its R was consumed by the product); M_b arrives in Xs while the task waits for block b - 1
-      if (warp < 4) {
+    if (chain) {  // y[block] = W - M_b y[block b - 1]; M_b's chunks all fit the ring now
+      double wv[4];
 #pragma unroll
-        for (int nb = 0; nb < 2; nb++)
-#pragma unroll
-          for (int v = 0; v < 4; v++) {
-            const int row = acc_row(warp, lane, v), n = acc_vec(lane, nb, v);
-            Rs[row * kLdB + n] = c[nb][v];
-          }
+      for (int v = 0; v < 4; v++) {
+        wv[v] = c[v];
+        c[v] = 0.0;
       }
-#pragma unroll
-      for (int nb = 0; nb < 2; nb++)
-#pragma unroll
-        for (int v = 0; v < 4; v++) c[nb][v] = 0.0;
-      __syncthreads();  // every warp is done with X in Xs
-      {  // M_b (rows x 64, column-major), [k][m] like X
-        const TL *M = Mch + (int64_t)(P.blkOff[s] - s + blk - 1) * kMB * kMB;
-        for (int e = tid; e < kMB * kMB; e += kMultiThreads) {
-          const int i = e & (kMB - 1), k = e >> 6;
-          const bool ok = i < rows;
-          cp_async_el(Xs + k * kLdX + i, ok ? M + (int64_t)k * kMB + i : M, (int)sizeof(TL), ok);
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-      }
+      __syncthreads();  // every warp is done with X
+      for (int i = nL + nX + kStages - 1; i < nL + nX + nM; i++) issue(i);
       if (tid == 0) waitOk = wait_flag(myflags + blk - 1, epoch, status, s, P.spin);
       __syncthreads();
       if (!waitOk) return bail();
       const int cp = (blk - 1) * kMB;  // block b - 1: 64 columns (not the last block)
-      for (int e = tid; e < kMB * kQS; e += kMultiThreads) {
-        const int k = e >> 4, n = e & (kQS - 1);
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int e = tid + kMultiThreads * u, k = e >> 4, n = e & (kQS - 1);
         Bs[k * kLdB + n] = n < qs ? __ldcg(y + (int64_t)(f + cp + k) * q + vb + n) : 0.0;
       }
-      cp_async_all();
+      cp_async_wait<0>();
       __syncthreads();
 #pragma unroll
-      for (int h = 0; h < 2; h++) mma_k16<true>(Xs, kLdX, Bs, 32 * h + 16 * kh, mw, lane, c);
-      halves_sum(c, As, warp, lane);
-      if (warp < 4) {
+      for (int i = 0; i < PB; i++)
+        mma_chunk<true>(ring + ((nL + nX + i) % kStages) * (KC * kLdKM), Bs + i * KC * kLdB, warp, lane, c);
 #pragma unroll
-        for (int nb = 0; nb < 2; nb++)
-#pragma unroll
-          for (int v = 0; v < 4; v++) {
-            const int row = acc_row(warp, lane, v), n = acc_vec(lane, nb, v);
-            if (row < rows && n < qs) y[(int64_t)(f + r0 + row) * q + vb + n] = Rs[row * kLdB + n] - c[nb][v];
-          }
-      }
-      __syncthreads();
-      if (tid == 0) st_release(myflags + blk, epoch);
-      return true;
+      for (int v = 0; v < 4; v++) c[v] = wv[v] - c[v];
     }
-    if (warp < 4) {
 #pragma unroll
-      for (int nb = 0; nb < 2; nb++)
-#pragma unroll
-        for (int v = 0; v < 4; v++) {
-          const int row = acc_row(warp, lane, v), n = acc_vec(lane, nb, v);
-          if (row < rows && n < qs) y[(int64_t)(f + r0 + row) * q + vb + n] = c[nb][v];
-        }
+    for (int v = 0; v < 4; v++) {
+      const int row = acc_row(warp, lane, v), n = acc_vec(warp, lane, v);
+      if (row < rows && n < qs) y[(int64_t)(f + r0 + row) * q + vb + n] = c[v];
     }
     __syncthreads();
     if (tid == 0) st_release(myflags + blk, epoch);
     return true;
   };
+  // kind 3: the whole supernode s (nc <= 64, m <= kWholeMulti) for vector slice sl: its front vector v (all m rows) where
+  // the ring is, y = X v[0:nc), then u = v - L[rows below, :] y in 64-row blocks. Most supernodes are this small, and
+  // one task for each replaces a diagonal task and up to four below it, whose latencies (ticket, gather, flag) were all
+  // their time.
+  auto run_whole = [&](const int s, const int sl) -> bool {
+    const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s], mu = m - nc;
+    const int vb = sl * kQS, qs = min(kQS, q - vb);
+    double *V = msm;
+    TL *stage = reinterpret_cast<TL *>(Bs);
+    const int nK = (nc + KC - 1) / KC, nbel = (mu + kMB - 1) / kMB, total = nK + nbel * nK;
+    const TL *Lb = Lx + P.snLxp[s] + nc, *Xb = Inv + P.invOff[P.blkOff[s]];
+    auto issue = [&](int i) {  // chunk i: of X, then of each block of rows below; [k][m]
+      if (i < total) {
+        const int j = i / nK - 1, k0 = (i % nK) * KC;  // j < 0: X
+        const TL *src = j < 0 ? Xb : Lb + kMB * j;
+        const int ld = j < 0 ? nc : m, rows = j < 0 ? nc : min(kMB, mu - kMB * j);
+        TL *dst = stage + (i & 1) * (KC * kLdKM);
+#pragma unroll
+        for (int u = 0; u < KC * kMB / kMultiThreads; u++) {
+          const int e = tid + kMultiThreads * u, row = e & (kMB - 1), cc = e >> 6;
+          const bool ok = row < rows && k0 + cc < nc;
+          cp_async_el(dst + cc * kLdKM + row, ok ? src + (int64_t)(k0 + cc) * ld + row : src, (int)sizeof(TL), ok);
+        }
+      }
+      cp_async_commit();
+    };
+    issue(0);
+    if (!gather_front_rows<kQS, kLdB>(P, s, true, 0, 0, m, y, T, done, sl, 1, q, vb, qs, status, V)) return bail();
+    for (int e = tid; e < kMB * kQS; e += kMultiThreads) {  // R = v[0:nc)
+      const int row = e >> 4, n = e & (kQS - 1);
+      Rs[row * kLdB + n] = row < nc ? V[row * kLdB + n] : 0.0;
+    }
+    double c[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int i = 0; i < total; i++) {
+      const int j = i / nK - 1, kk = i % nK;
+      cp_async_wait<0>();
+      __syncthreads();  // chunk i has arrived (and R, or y, is complete); every warp is done with chunk i - 1
+      issue(i + 1);
+      mma_chunk<true>(stage + (i & 1) * (KC * kLdKM), Rs + kk * KC * kLdB, warp, lane, c);
+      if (kk + 1 < nK) continue;
+      if (j < 0) {  // y: to memory, and over R for the products below
+        __syncthreads();  // every warp is done with R
+#pragma unroll
+        for (int v = 0; v < 4; v++) {
+          const int row = acc_row(warp, lane, v), n = acc_vec(warp, lane, v);
+          Rs[row * kLdB + n] = row < nc ? c[v] : 0.0;
+          if (row < nc && n < qs) y[(int64_t)(f + row) * q + vb + n] = c[v];
+          c[v] = 0.0;
+        }
+      } else {
+        double *to = T + (P.snTOff[s] + (int64_t)j * kMB) * q + vb;
+        const double *Vj = V + (nc + j * kMB) * kLdB;
+#pragma unroll
+        for (int v = 0; v < 4; v++) {
+          const int row = acc_row(warp, lane, v), n = acc_vec(warp, lane, v);
+          if (row < mu - j * kMB && n < qs) to[(int64_t)row * q + n] = Vj[row * kLdB + n] - c[v];
+          c[v] = 0.0;
+        }
+      }
+    }
+    __syncthreads();
+    if (tid == 0) {  // after the barrier: the CTA's stores of y and T are ordered before both
+      st_release(flags + (int64_t)sl * nflags + P.blkOff[s], epoch);
+      if (nbel > 0) red_release_add(done + (int64_t)sl * P.nsuper + s, nbel);
+    }
+    return true;
+  };
   auto run = [&](const int tkv) -> bool {
     const int4 t = tasks[tkv];
-    if (t.z == 2) {  // up to kSolveGroup supernodes with m <= 32, one warp each, all q vectors
+    if (t.z == 2) {  // up to kSolveGroup supernodes with m <= 32, or kSolveWarps with m <= 16, one warp each, all vectors
       if (tid == 0) waitOk = 1;
       __syncthreads();
       if (warp < t.y && !small_fwd_warp_multi<TL>(P.solveSmall[t.x + warp], P, Lx, y, T, done, q, ns, status,
-                                                  msm + 32 * kMQ * warp))
+                                                  msm + small_stride(t.y) * warp))
         waitOk = 0;
       __syncthreads();
       return waitOk != 0;
     }
+    if (t.z == 3) return run_whole(t.x, t.w);
     if constexpr (WIDE) {
       if (t.w < 0) return fwd_wide_task<TL>(t, P, Lx, Inv, y, T, flags, nflags, epoch, done, q, ns, status, msm, waitOk);
     }
@@ -678,7 +761,7 @@ __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_fwd_multi(const i
 // after its flag as x[block] = W - G_b^T x[block b + 1], W = X^T (y[block] - the other rows' terms).
 template <class TL, bool WIDE>
 __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_bwd_multi(const int4 *__restrict__ tasks, int ntasks, int ns,
-                                                                int *__restrict__ ticket, DevPlan P,
+                                                                int *__restrict__ ticket, const __grid_constant__ DevPlan P,
                                                                 const TL *__restrict__ Lx, const TL *__restrict__ Inv,
                                                                 const TL *__restrict__ Gch,
                                                                 const double *__restrict__ Dpiv,
@@ -686,10 +769,12 @@ __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_bwd_multi(const i
                                                                 int nflags, int epoch, int q,
                                                                 unsigned long long *status) {
   extern __shared__ double msm[];
-  double *As = msm, *Bs = As + kAElems, *Rs = Bs + kMB * kLdB;
-  TL *Xs = reinterpret_cast<TL *>(Rs + kMB * kLdB);
-  __shared__ int waitOk;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, mw = warp & 3, kh = warp >> 2;
+  constexpr int KC = chunk_k<TL>(), PB = kMB / KC, LD = ld_mk<TL>();  // reduction chunk, chunks per block, [m][k] stride
+  constexpr int NY = KC * kQS / kMultiThreads;                          // x values per thread and chunk
+  TL *ring = reinterpret_cast<TL *>(msm);
+  double *Bs = msm + kRingBytes / sizeof(double), *Rs = Bs + 2 * kMB * kLdB;  // x values; R
+  __shared__ int waitOk, sReady, sFin[8];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   auto bail = [] {  // a wait gave up: drain this thread's copies into shared memory before the CTA leaves
     cp_async_all();
     return false;
@@ -699,190 +784,195 @@ __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_bwd_multi(const i
     const int s = t.x, blk = t.y;
     const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s];
     const int vb = sl * kQS, qs = min(kQS, q - vb);
-    const TL *Lp = Lx + P.snLxp[s];
     const int *rowsOf = P.Si + P.Sp[s];
     const int c0 = blk * kMB, w = min(kMB, nc - c0), nb = (nc + kMB - 1) / kMB;
     int *sflags = flags + (int64_t)sl * nflags;
     int *myflags = sflags + P.blkOff[s];
-    {  // X^T: Xs[i][j] = X(j, i) = X[i w + j] ([m][k] with m = i), arriving while the task sums
-      const TL *X = Inv + P.invOff[P.blkOff[s] + blk];
-      for (int e = tid; e < kMB * kMB; e += kMultiThreads) {
-        const int j = e & (kMB - 1), i = e >> 6;
-        const bool ok = i < w && j < w;
-        cp_async_el(Xs + i * kLdX + j, ok ? X + (int64_t)i * w + j : X, (int)sizeof(TL), ok);
-      }
-      asm volatile("cp.async.commit_group;\n" ::: "memory");
-    }
-    double c[2][4];
-#pragma unroll
-    for (int nb2 = 0; nb2 < 2; nb2++)
-#pragma unroll
-      for (int v = 0; v < 4; v++) c[nb2][v] = 0.0;
-    // chunks: the rows below the supernode [nc, m) in kKC steps from the last down, then pivot blocks nb - 1 .. blk + 1
-    // (two chunks each)
+    // chunks of the reduction: the rows below the supernode [nc, m) in KC steps from the last down, then pivot blocks
+    // nb - 1 .. blk + 1 (PB chunks each), then X^T and G_b^T; none of these A operands depends on another task of the
+    // sweep, so they stream through the ring kStages - 1 chunks ahead
     const bool chain = Gch != nullptr && blk + 1 < nb;  // block b + 1 enters through G_b after its flag
-    const int nanc = (m - nc + kKC - 1) / kKC;
-    const int npiv = (nb - 1 - blk - (chain ? 1 : 0)) * (kMB / kKC);
-    const int nch = nanc + npiv;
-    auto chunk = [&](int ch, int &rb, int &rw) {
+    const int nanc = (m - nc + KC - 1) / KC;
+    const int nS = nanc + (nb - 1 - blk - (chain ? 1 : 0)) * PB;  // summed chunks
+    const int nX = (w + KC - 1) / KC, nG = chain ? PB : 0;
+    const int rn = (blk + 1) * kMB, wn = chain ? min(kMB, nc - rn) : 0;  // the next pivot block
+    auto chunk_rows = [&](int ch, int &rb, int &rw) {
       if (ch < nanc) {
-        rb = nc + (nanc - 1 - ch) * kKC;
-        rw = min(kKC, m - rb);
+        rb = nc + (nanc - 1 - ch) * KC;
+        rw = min(KC, m - rb);
       } else {
-        const int p = ch - nanc, pb = nb - 1 - p / 2;  // pivot block, from the last down
-        rb = pb * kMB + (p & 1) * kKC;
-        rw = max(0, min(kKC, nc - rb));
+        const int p = ch - nanc, pb = nb - 1 - p / PB;  // pivot block, from the last down
+        rb = pb * kMB + (p % PB) * KC;
+        rw = max(0, min(KC, nc - rb));
       }
     };
-    // L chunk, [m][k]: As[cc][rr] = L(rb + rr, c0 + cc); elements e = tid + 256 u: rr = e & 31, cc = e >> 5
-    TL lr[8];
-    auto loadL = [&](int rb, int rw) {
+    const TL *Lb = Lx + P.snLxp[s] + (int64_t)c0 * m;
+    const TL *Xb = Inv + P.invOff[P.blkOff[s] + blk];
+    const TL *Gb = chain ? Gch + (int64_t)(P.blkOff[s] - s + blk) * kMB * kMB : Xb;
+    auto issue = [&](int i) {  // [m][k]: chunk i's element (k0 + rr, column cc) at [cc LD + rr]
+      if (i < nS + nX + nG) {
+        const TL *src = Lb;
+        int ld = m, k0, lim;
+        if (i < nS) {
+          int rw;
+          chunk_rows(i, k0, rw);
+          lim = k0 + rw;
+        } else if (i < nS + nX) {
+          src = Xb;
+          ld = lim = w;
+          k0 = (i - nS) * KC;
+        } else {
+          src = Gb;
+          ld = kMB;
+          lim = wn;
+          k0 = (i - nS - nX) * KC;
+        }
+        TL *dst = ring + (i % kStages) * (kMB * LD);
 #pragma unroll
-      for (int u = 0; u < 8; u++) {
-        const int e = tid + kMultiThreads * u, rr = e & (kKC - 1), cc = e >> 5;
-        lr[u] = (rr < rw && cc < w) ? Lp[(int64_t)(c0 + cc) * m + rb + rr] : (TL)0;
+        for (int u = 0; u < KC * kMB / kMultiThreads; u++) {
+          const int e = tid + kMultiThreads * u, rr = e % KC, cc = e / KC;
+          const bool ok = cc < w && k0 + rr < lim;
+          cp_async_el(dst + cc * LD + rr, ok ? src + (int64_t)cc * ld + k0 + rr : src, (int)sizeof(TL), ok);
+        }
+      }
+      cp_async_commit();
+    };
+    for (int i = 0; i < kStages - 1; i++) issue(i);
+    double c[4] = {0.0, 0.0, 0.0, 0.0};
+    // x values of a chunk (KC x 16): read one chunk ahead when its rows are known final (ready: the chunks known final,
+    // found for up to eight chunks of ancestors' rows, a warp each, or 32 pivot blocks at a time); ix: the row numbers of
+    // the chunk to be read next, themselves read when the one before it was
+    double yr[NY];
+    int ix[NY];
+    auto row_index = [&](int ch) {
+      int rb, rw;
+      chunk_rows(ch, rb, rw);
+#pragma unroll
+      for (int u = 0; u < NY; u++) {
+        const int rr = (tid + kMultiThreads * u) >> 4;
+        ix[u] = rr >= rw ? -1 : ch < nanc ? rowsOf[rb + rr] : f + rb + rr;
       }
     };
-    int rb = 0, rw = 0;
-    if (nch > 0) {
-      chunk(0, rb, rw);
-      loadL(rb, rw);
-    }
-    for (int ch = 0; ch < nch; ch++) {
-      const bool anc = ch < nanc;
-      if (anc) {  // the ancestor blocks holding this chunk's rows final? (one lane per row, each distinct block once)
-        if (warp == 0) {
-          const int fb = lane < rw ? P.rowBlk[rowsOf[rb + lane]] : -1;
-          const int prev = __shfl_up_sync(0xffffffffu, fb, 1);
-          int ok = 1;
-          if (fb >= 0 && (lane == 0 || fb != prev)) ok = wait_flag(sflags + fb, epoch, status, s, P.spin);
-          ok = __all_sync(0xffffffffu, ok);
-          if (lane == 0) waitOk = ok;
-        }
-        __syncthreads();
-        if (!waitOk) return bail();
-      } else if (((ch - nanc) & 1) == 0) {  // first chunk of a pivot block: its x values final?
-        if (tid == 0) waitOk = wait_flag(myflags + rb / kMB, epoch, status, s, P.spin);
-        __syncthreads();
-        if (!waitOk) return bail();
-      }
-      for (int e = tid; e < kKC * kQS; e += kMultiThreads) {
-        const int rr = e >> 4, n = e & (kQS - 1);
-        double v = 0.0;
-        if (rr < rw && n < qs) {
-          const int gi = anc ? rowsOf[rb + rr] : f + rb + rr;
-          v = __ldcg(y + (int64_t)gi * q + vb + n);
-        }
-        Bs[rr * kLdB + n] = v;
-      }
+    auto load_x = [&]() {
 #pragma unroll
-      for (int u = 0; u < 8; u++) {
+      for (int u = 0; u < NY; u++) {
+        const int n = tid & (kQS - 1);
+        yr[u] = ix[u] >= 0 && n < qs ? __ldcg(y + (int64_t)ix[u] * q + vb + n) : 0.0;
+      }
+    };
+    int ready = 0;
+    bool ahead = false;
+    if (nS > 0) row_index(0);
+    for (int i = 0; i < nS; i++) {
+      if (!ahead) {
+        if (ready <= i) {
+          if (i < nanc) {
+            const int ch = i + warp;
+            int rb, rw;
+            bool fin = false;
+            if (ch < nanc) {
+              chunk_rows(ch, rb, rw);
+              fin = lane >= rw || ld_acquire(sflags + P.rowBlk[rowsOf[rb + lane]]) == epoch;
+            }
+            fin = __all_sync(0xffffffffu, fin);
+            if (lane == 0) sFin[warp] = fin;
+            __syncthreads();
+            if (warp == 0) {
+              const unsigned bits = __ballot_sync(0xffffffffu, lane < 8 && sFin[lane & 7]);
+              int run = __ffs(~bits) - 1;
+              if (run == 0) {  // the ancestor blocks of this chunk's rows: one lane per row, each distinct block once
+                chunk_rows(i, rb, rw);
+                const int fb = lane < rw ? P.rowBlk[rowsOf[rb + lane]] : -1;
+                const int prev = __shfl_up_sync(0xffffffffu, fb, 1);
+                int ok = 1;
+                if (fb >= 0 && (lane == 0 || fb != prev)) ok = wait_flag(sflags + fb, epoch, status, s, P.spin);
+                run = __all_sync(0xffffffffu, ok) ? 1 : -1;
+              }
+              if (lane == 0) sReady = run < 0 ? -1 : i + run;
+            }
+          } else if (warp == 0) {  // pivot blocks from pb down
+            const int p = i - nanc, pb = nb - 1 - p / PB;
+            const bool fin = pb - lane > blk && ld_acquire(myflags + pb - lane) == epoch;
+            int run = __ffs(~__ballot_sync(0xffffffffu, fin)) - 1;
+            if (run < 0) run = 32;
+            if (run == 0) {
+              int ok = 1;
+              if (lane == 0) ok = wait_flag(myflags + pb, epoch, status, s, P.spin);
+              run = __shfl_sync(0xffffffffu, ok, 0) ? 1 : -1;
+            }
+            if (lane == 0) sReady = run < 0 ? -1 : i - p % PB + run * PB;
+          }
+          __syncthreads();
+          ready = sReady;
+          if (ready < 0) return bail();
+        }
+        load_x();
+        if (i + 1 < nS) row_index(i + 1);
+      }
+      double *Bi = Bs + (i & 1) * kMB * kLdB;
+#pragma unroll
+      for (int u = 0; u < NY; u++) {
         const int e = tid + kMultiThreads * u;
-        As[(e >> 5) * kLdMK + (e & (kKC - 1))] = (double)lr[u];
+        Bi[(e >> 4) * kLdB + (e & (kQS - 1))] = yr[u];
       }
-      __syncthreads();
-      const int cw = rw;
-      if (ch + 1 < nch) {
-        chunk(ch + 1, rb, rw);
-        loadL(rb, rw);
+      cp_async_wait<kStages - 2>();
+      __syncthreads();  // chunk i and its x values have arrived; every warp is done with chunk i - 1
+      ahead = i + 1 < nS && ready > i + 1;
+      if (ahead) {
+        load_x();
+        if (i + 2 < nS) row_index(i + 2);
       }
-      if (16 * kh < cw) mma_k16<false>(As, kLdMK, Bs, 16 * kh, mw, lane, c);
-      __syncthreads();
+      issue(i + kStages - 1);
+      mma_chunk<false>(ring + (i % kStages) * (kMB * LD), Bi, warp, lane, c);
     }
-    halves_sum(c, As, warp, lane);
-    // R = y[block] (/ D) - acc
-    if (warp < 4) {
+    // R = y[block] (/ D) - the sum
 #pragma unroll
-      for (int nb2 = 0; nb2 < 2; nb2++)
-#pragma unroll
-        for (int v = 0; v < 4; v++) {
-          const int cc = acc_row(warp, lane, v), n = acc_vec(lane, nb2, v);
-          double r = 0.0;
-          if (cc < w && n < qs) {
-            const double yv = y[(int64_t)(f + c0 + cc) * q + vb + n];
-            r = (Dpiv ? yv / Dpiv[f + c0 + cc] : yv) - c[nb2][v];  // LDL^T: y /= D before the backward sweep (ldlt.mjs:629)
-          }
-          Rs[cc * kLdB + n] = r;
-          c[nb2][v] = 0.0;
-        }
+    for (int v = 0; v < 4; v++) {
+      const int cc = acc_row(warp, lane, v), n = acc_vec(warp, lane, v);
+      double r = 0.0;
+      if (cc < w && n < qs) {
+        const double yv = y[(int64_t)(f + c0 + cc) * q + vb + n];
+        r = (Dpiv ? yv / Dpiv[f + c0 + cc] : yv) - c[v];  // LDL^T: y /= D before the backward sweep (ldlt.mjs:629)
+      }
+      Rs[cc * kLdB + n] = r;
+      c[v] = 0.0;
     }
-    if (warp >= 4) {
-#pragma unroll
-      for (int nb2 = 0; nb2 < 2; nb2++)
-#pragma unroll
-        for (int v = 0; v < 4; v++) c[nb2][v] = 0.0;
-    }
-    cp_async_all();
-    __syncthreads();
     // x[block] = X^T R
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const int k0 = 32 * h + 16 * kh;
-      if (k0 < w) mma_k16<false>(Xs, kLdX, Rs, k0, mw, lane, c);
+    for (int i = nS; i < nS + nX; i++) {
+      cp_async_wait<kStages - 2>();
+      __syncthreads();
+      issue(i + kStages - 1);
+      mma_chunk<false>(ring + (i % kStages) * (kMB * LD), Rs + (i - nS) * KC * kLdB, warp, lane, c);
     }
-    halves_sum(c, As, warp, lane);
-    if (chain) {
-      // W stays in Rs; G_b^T arrives in Xs while the task waits for block b + 1
-      const int rn = (blk + 1) * kMB, wn = min(kMB, nc - rn);
-      if (warp < 4) {
+    if (chain) {  // x[block] = W - G_b^T x[block b + 1]; G_b's chunks all fit the ring now
+      double wv[4];
 #pragma unroll
-        for (int nb2 = 0; nb2 < 2; nb2++)
-#pragma unroll
-          for (int v = 0; v < 4; v++) {
-            const int cc = acc_row(warp, lane, v), n = acc_vec(lane, nb2, v);
-            Rs[cc * kLdB + n] = c[nb2][v];
-          }
+      for (int v = 0; v < 4; v++) {
+        wv[v] = c[v];
+        c[v] = 0.0;
       }
-#pragma unroll
-      for (int nb2 = 0; nb2 < 2; nb2++)
-#pragma unroll
-        for (int v = 0; v < 4; v++) c[nb2][v] = 0.0;
-      __syncthreads();  // every warp is done with X^T in Xs
-      {  // G_b^T ([m][k]): Xs[i][r] = G(r, i) = G[i 64 + r], G (wn x w, column-major)
-        const TL *G = Gch + (int64_t)(P.blkOff[s] - s + blk) * kMB * kMB;
-        for (int e = tid; e < kMB * kMB; e += kMultiThreads) {
-          const int r = e & (kMB - 1), i = e >> 6;
-          const bool ok = i < w && r < wn;
-          cp_async_el(Xs + i * kLdX + r, ok ? G + (int64_t)i * kMB + r : G, (int)sizeof(TL), ok);
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-      }
+      __syncthreads();  // every warp is done with X^T
+      for (int i = nS + nX + kStages - 1; i < nS + nX + nG; i++) issue(i);
       if (tid == 0) waitOk = wait_flag(myflags + blk + 1, epoch, status, s, P.spin);
       __syncthreads();
       if (!waitOk) return bail();
-      for (int e = tid; e < kMB * kQS; e += kMultiThreads) {
-        const int r = e >> 4, n = e & (kQS - 1);
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int e = tid + kMultiThreads * u, r = e >> 4, n = e & (kQS - 1);
         Bs[r * kLdB + n] = (r < wn && n < qs) ? __ldcg(y + (int64_t)(f + rn + r) * q + vb + n) : 0.0;
       }
-      cp_async_all();
+      cp_async_wait<0>();
       __syncthreads();
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int k0 = 32 * h + 16 * kh;
-        if (k0 < wn) mma_k16<false>(Xs, kLdX, Bs, k0, mw, lane, c);
-      }
-      halves_sum(c, As, warp, lane);
-      if (warp < 4) {
+      for (int i = 0; i < PB; i++)
+        mma_chunk<false>(ring + ((nS + nX + i) % kStages) * (kMB * LD), Bs + i * KC * kLdB, warp, lane, c);
 #pragma unroll
-        for (int nb2 = 0; nb2 < 2; nb2++)
-#pragma unroll
-          for (int v = 0; v < 4; v++) {
-            const int cc = acc_row(warp, lane, v), n = acc_vec(lane, nb2, v);
-            if (cc < w && n < qs) y[(int64_t)(f + c0 + cc) * q + vb + n] = Rs[cc * kLdB + n] - c[nb2][v];
-          }
-      }
-      __syncthreads();
-      if (tid == 0) st_release(myflags + blk, epoch);
-      return true;
+      for (int v = 0; v < 4; v++) c[v] = wv[v] - c[v];
     }
-    if (warp < 4) {
 #pragma unroll
-      for (int nb2 = 0; nb2 < 2; nb2++)
-#pragma unroll
-        for (int v = 0; v < 4; v++) {
-          const int cc = acc_row(warp, lane, v), n = acc_vec(lane, nb2, v);
-          if (cc < w && n < qs) y[(int64_t)(f + c0 + cc) * q + vb + n] = c[nb2][v];
-        }
+    for (int v = 0; v < 4; v++) {
+      const int cc = acc_row(warp, lane, v), n = acc_vec(warp, lane, v);
+      if (cc < w && n < qs) y[(int64_t)(f + c0 + cc) * q + vb + n] = c[v];
     }
     __syncthreads();
     if (tid == 0) st_release(myflags + blk, epoch);
@@ -890,11 +980,11 @@ __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_bwd_multi(const i
   };
   auto run = [&](const int tkv) -> bool {
     const int4 t = tasks[tkv];
-    if (t.z == 2) {  // up to kSolveGroup supernodes with m <= 32, one warp each, all q vectors
+    if (t.z == 2) {  // up to kSolveGroup supernodes with m <= 32, or kSolveWarps with m <= 16, one warp each, all vectors
       if (tid == 0) waitOk = 1;
       __syncthreads();
       if (warp < t.y && !small_bwd_warp_multi<TL>(P.solveSmall[t.x + warp], P, Lx, Dpiv, y, flags, nflags, epoch, q,
-                                                  ns, status, msm + 32 * kMQ * warp))
+                                                  ns, status, msm + small_stride(t.y) * warp))
         waitOk = 0;
       __syncthreads();
       return waitOk != 0;
@@ -1031,9 +1121,9 @@ __global__ void __launch_bounds__(256) k_residual_multi(int n, const int *__rest
 template <class TL, bool WIDE>
 static cudaError_t set_multi_smem() {
   cudaError_t e =
-      cudaFuncSetAttribute(k_fwd_multi<TL, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, multi_smem<TL>());
+      cudaFuncSetAttribute(k_fwd_multi<TL, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, multi_smem());
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_bwd_multi<TL, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, multi_smem<TL>());
+    e = cudaFuncSetAttribute(k_bwd_multi<TL, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, multi_smem());
   return e;
 }
 cudaError_t init_solve_multi_attributes() {
@@ -1057,7 +1147,7 @@ void launch_fwd_multi(const int4 *tasks, int ntasks, bool wide, int *ticket, con
   const int ns = multi_slices(q);
   if (ntasks <= 0) return;
   auto k = wide ? k_fwd_multi<TL, true> : k_fwd_multi<TL, false>;
-  k<<<multi_grid(ntasks), kMultiThreads, multi_smem<TL>(), st>>>(tasks, ntasks, ns, ticket, P, Lx, Inv, Mch, y, T,
+  k<<<multi_grid(ntasks), kMultiThreads, multi_smem(), st>>>(tasks, ntasks, ns, ticket, P, Lx, Inv, Mch, y, T,
                                                                   flags, nflags, epoch, done, q, status);
 }
 template <class TL>
@@ -1067,7 +1157,7 @@ void launch_bwd_multi(const int4 *tasks, int ntasks, bool wide, int *ticket, con
   const int ns = multi_slices(q);
   if (ntasks <= 0) return;
   auto k = wide ? k_bwd_multi<TL, true> : k_bwd_multi<TL, false>;
-  k<<<multi_grid(ntasks), kMultiThreads, multi_smem<TL>(), st>>>(tasks, ntasks, ns, ticket, P, Lx, Inv, Gch, Dpiv, y,
+  k<<<multi_grid(ntasks), kMultiThreads, multi_smem(), st>>>(tasks, ntasks, ns, ticket, P, Lx, Inv, Gch, Dpiv, y,
                                                                   flags, nflags, epoch, q, status);
 }
 void launch_to_interleaved(const double *B, double *Yil, int n, int q, cudaStream_t st) {

@@ -29,15 +29,28 @@ __device__ __forceinline__ bool warp_wait(const int *p, int v, bool eq, unsigned
   return ok != 0;
 }
 
-// children of s complete in the forward sweep (their pass-up vectors written)
-__device__ __forceinline__ bool warp_wait_children(const DevPlan &P, int s, const int *done,
-                                                   unsigned long long *status) {
-  for (int qq = P.chPtr[s]; qq < P.chPtr[s + 1]; qq++) {
-    const int c = P.chList[qq];
-    const int need = (P.snM[c] - P.snNc[c] + 63) / 64;
-    if (!warp_wait(done + c, need, false, status, s, P.spin)) return false;
+// The children of s, 32 at a time, one per lane: their pass-up vectors' lengths, offsets and maps (mu, to, ea), each waited
+// for by its own lane (ns vector slices), so that neither the loads nor the waits of several children follow one another.
+struct ChildLanes {
+  int mu;
+  int64_t to, ea;
+};
+__device__ __forceinline__ bool warp_children(const DevPlan &P, int s, int qb, int nq, const int *done, int ns,
+                                              unsigned long long *status, ChildLanes &ch) {
+  const int lane = threadIdx.x & 31;
+  int ok = 1;
+  ch = ChildLanes{0, 0, 0};
+  if (lane < nq) {
+    const int c = P.chList[qb + lane];
+    ch.mu = P.snM[c] - P.snNc[c];
+    ch.to = P.snTOff[c];
+    ch.ea = P.eaPtr[c];
+    const int need = (ch.mu + 63) / 64;
+    for (int sl = 0; sl < ns && ok; sl++) ok = wait_count(done + (int64_t)sl * P.nsuper + c, need, status, s, P.spin);
   }
-  return true;
+  ok = __all_sync(0xffffffffu, ok);
+  __syncwarp();  // orders the other lanes' later loads after each lane's acquire
+  return ok != 0;
 }
 
 // ---- one right-hand side --------------------------------------------------------------------------------------------
@@ -47,21 +60,35 @@ __device__ bool small_fwd_warp(int s, const DevPlan &P, const TL *__restrict__ L
                                double *__restrict__ T, int *done, unsigned long long *status, double *vs) {
   const int lane = threadIdx.x & 31;
   const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s];
-  if (!warp_wait_children(P, s, done, status)) return false;
+  const TL *Lp = Lx + P.snLxp[s];
+  double lk = lane < m ? (double)Lp[lane] : 0.0;  // column 0
   vs[lane] = lane < nc ? y[f + lane] : 0.0;
   __syncwarp();
-  for (int qq = P.chPtr[s]; qq < P.chPtr[s + 1]; qq++) {
-    const int c = P.chList[qq];
-    const int muc = P.snM[c] - P.snNc[c];
-    const int *map = P.eaMap + P.eaPtr[c];
-    const double *tc = T + P.snTOff[c];
-    for (int a = lane; a < muc; a += 32) vs[map[a]] += __ldcg(tc + a);
-    __syncwarp();
+  const int q0 = P.chPtr[s], q1 = P.chPtr[s + 1];
+  for (int qb = q0; qb < q1; qb += 32) {
+    const int nq = min(32, q1 - qb);
+    ChildLanes ch;
+    if (!warp_children(P, s, qb, nq, done, 1, status, ch)) return false;
+    // child q's entry of this lane (muc <= m <= 32), read while the child before it is added
+    auto fetch = [&](int q, double &v, int &dst) {
+      const int mu = __shfl_sync(0xffffffffu, ch.mu, q);
+      const int64_t to = __shfl_sync(0xffffffffu, ch.to, q), ea = __shfl_sync(0xffffffffu, ch.ea, q);
+      dst = lane < mu ? P.eaMap[ea + lane] : -1;
+      v = lane < mu ? __ldcg(T + to + lane) : 0.0;
+    };
+    double v, vn = 0.0;
+    int dst, dn = -1;
+    fetch(0, v, dst);
+    for (int q = 0; q < nq; q++) {
+      if (q + 1 < nq) fetch(q + 1, vn, dn);
+      if (dst >= 0) vs[dst] += v;
+      __syncwarp();
+      v = vn;
+      dst = dn;
+    }
   }
   double v = vs[lane];
   if (P.lpiv) v = __shfl_sync(0xffffffffu, v, lane < nc ? P.lpiv[f + lane] : lane);  // Bunch-Kaufman pivot order
-  const TL *Lp = Lx + P.snLxp[s];
-  double lk = lane < m ? (double)Lp[lane] : 0.0;  // column 0
   for (int k = 0; k < nc; k++) {
     const double ln = (k + 1 < nc && lane < m) ? (double)Lp[(int64_t)(k + 1) * m + lane] : 0.0;
     const double yk = __shfl_sync(0xffffffffu, lane == k ? v / lk : 0.0, k);
@@ -86,21 +113,24 @@ __device__ bool small_bwd_warp(int s, const DevPlan &P, const TL *__restrict__ L
   const int lane = threadIdx.x & 31;
   const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s];
   const int par = P.snParent[s];
+  const TL *Lp = Lx + P.snLxp[s];
+  double lk = (lane >= nc - 1 && lane < m) ? (double)Lp[(int64_t)(nc - 1) * m + lane] : 0.0;  // the last column
+  const int row = lane >= nc && lane < m ? P.Si[P.Sp[s] + lane] : 0;
   if (par >= 0 && m > nc && !warp_wait(flags + P.blkOff[par], epoch, true, status, s, P.spin)) return false;
   double x = 0.0;
   if (lane >= nc && lane < m) {
-    x = __ldcg(y + P.Si[P.Sp[s] + lane]);
+    x = __ldcg(y + row);
   } else if (lane < nc) {
     x = y[f + lane];
     if (Dpiv) x = x / Dpiv[f + lane];  // LDL^T: y /= D before the backward sweep (ldlt.mjs:629)
   }
-  const TL *Lp = Lx + P.snLxp[s];
   for (int k = nc - 1; k >= 0; k--) {
-    const double lk = (lane >= k && lane < m) ? (double)Lp[(int64_t)k * m + lane] : 0.0;
+    const double ln = (k > 0 && lane >= k - 1 && lane < m) ? (double)Lp[(int64_t)(k - 1) * m + lane] : 0.0;
     double p = lane > k ? lk * x : 0.0;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
     if (lane == k) x = (x - p) / lk;
+    lk = ln;
   }
   if (lane < nc) y[f + (P.lpiv ? P.lpiv[f + lane] : lane)] = x;  // back to the original order (Bunch-Kaufman)
   __syncwarp();  // orders the warp's stores before the release
@@ -118,21 +148,39 @@ __device__ bool small_fwd_warp_multi(int s, const DevPlan &P, const TL *__restri
   const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s];
   const int k0 = lane, k1 = lane + 32;
   const bool v0 = k0 < q, v1 = k1 < q;
-  for (int sl = 0; sl < ns; sl++)  // every vector slice of the children done
-    if (!warp_wait_children(P, s, done + (int64_t)sl * P.nsuper, status)) return false;
+  const TL *Lp = Lx + P.snLxp[s];
+  double lcol = lane < m ? (double)Lp[lane] : 0.0;  // column 0 (below)
+#pragma unroll 4
   for (int r = 0; r < m; r++) {
     if (v0) Vs[64 * r + k0] = r < nc ? y[(int64_t)(f + r) * q + k0] : 0.0;
     if (v1) Vs[64 * r + k1] = r < nc ? y[(int64_t)(f + r) * q + k1] : 0.0;
   }
-  for (int qq = P.chPtr[s]; qq < P.chPtr[s + 1]; qq++) {  // each lane touches only its own vectors: no barrier
-    const int c = P.chList[qq];
-    const int muc = P.snM[c] - P.snNc[c];
-    const int *map = P.eaMap + P.eaPtr[c];
-    const double *tc = T + P.snTOff[c] * q;
-    for (int a = 0; a < muc; a++) {
-      const int r = map[a];
-      if (v0) Vs[64 * r + k0] += __ldcg(tc + (int64_t)a * q + k0);
-      if (v1) Vs[64 * r + k1] += __ldcg(tc + (int64_t)a * q + k1);
+  const int q0 = P.chPtr[s], q1 = P.chPtr[s + 1];
+  for (int qb = q0; qb < q1; qb += 32) {  // each lane touches only its own vectors: no barrier
+    const int nq = min(32, q1 - qb);
+    ChildLanes ch;
+    if (!warp_children(P, s, qb, nq, done, ns, status, ch)) return false;
+    for (int qq = 0; qq < nq; qq++) {
+      const int mu = __shfl_sync(0xffffffffu, ch.mu, qq);
+      const int64_t to = __shfl_sync(0xffffffffu, ch.to, qq), ea = __shfl_sync(0xffffffffu, ch.ea, qq);
+      const int map = lane < mu ? P.eaMap[ea + lane] : 0;  // the child's front positions, one per lane
+      const double *tc = T + to * q;
+      for (int a0 = 0; a0 < mu; a0 += 4) {  // four rows in flight
+        double t0[4], t1[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          t0[u] = v0 && a0 + u < mu ? __ldcg(tc + (int64_t)(a0 + u) * q + k0) : 0.0;
+          t1[u] = v1 && a0 + u < mu ? __ldcg(tc + (int64_t)(a0 + u) * q + k1) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const int r = __shfl_sync(0xffffffffu, map, min(a0 + u, 31));
+          if (a0 + u < mu) {
+            if (v0) Vs[64 * r + k0] += t0[u];
+            if (v1) Vs[64 * r + k1] += t1[u];
+          }
+        }
+      }
     }
   }
   if (P.lpiv) {  // Bunch-Kaufman pivot order of the pivot rows (each lane permutes its own vectors)
@@ -148,8 +196,6 @@ __device__ bool small_fwd_warp_multi(int s, const DevPlan &P, const TL *__restri
     }
   }
   // column k of L is held one row per lane (loaded one column ahead) and broadcast by shuffles
-  const TL *Lp = Lx + P.snLxp[s];
-  double lcol = lane < m ? (double)Lp[lane] : 0.0;
   for (int k = 0; k < nc; k++) {
     const double lnext = (k + 1 < nc && lane < m) ? (double)Lp[(int64_t)(k + 1) * m + lane] : 0.0;
     const double lkk = __shfl_sync(0xffffffffu, lcol, k);
@@ -182,12 +228,17 @@ __device__ bool small_bwd_warp_multi(int s, const DevPlan &P, const TL *__restri
   const int k0 = lane, k1 = lane + 32;
   const bool v0 = k0 < q, v1 = k1 < q;
   const int par = P.snParent[s];
-  if (par >= 0 && m > nc)
-    for (int sl = 0; sl < ns; sl++)  // the parent's every vector slice final
-      if (!warp_wait(flags + (int64_t)sl * nflags + P.blkOff[par], epoch, true, status, s, P.spin)) return false;
-  const int *rowsOf = P.Si + P.Sp[s];
+  const int rowOf = lane < nc ? f + lane : lane < m ? P.Si[P.Sp[s] + lane] : 0;  // the front's rows, one per lane
+  const TL *Lp = Lx + P.snLxp[s];
+  double lcol = (nc > 0 && lane < m) ? (double)Lp[(int64_t)(nc - 1) * m + lane] : 0.0;  // the last column (below)
+  if (par >= 0 && m > nc) {  // the parent's every vector slice final, a lane each
+    const int ok = lane >= ns || wait_flag(flags + (int64_t)lane * nflags + P.blkOff[par], epoch, status, s, P.spin);
+    if (!__all_sync(0xffffffffu, ok)) return false;
+    __syncwarp();
+  }
+#pragma unroll 4
   for (int r = 0; r < m; r++) {
-    const int64_t gi = r < nc ? f + r : rowsOf[r];
+    const int64_t gi = __shfl_sync(0xffffffffu, rowOf, r);
     const double d = (r < nc && Dpiv) ? Dpiv[f + r] : 1.0;
     if (v0) {
       const double xv = r < nc ? y[gi * q + k0] : __ldcg(y + gi * q + k0);
@@ -199,8 +250,6 @@ __device__ bool small_bwd_warp_multi(int s, const DevPlan &P, const TL *__restri
     }
   }
   // column k of L one row per lane (loaded one column ahead), broadcast by shuffles
-  const TL *Lp = Lx + P.snLxp[s];
-  double lcol = (nc > 0 && lane < m) ? (double)Lp[(int64_t)(nc - 1) * m + lane] : 0.0;
   for (int k = nc - 1; k >= 0; k--) {
     const double lnext = (k > 0 && lane < m) ? (double)Lp[(int64_t)(k - 1) * m + lane] : 0.0;
     double s0 = 0.0, s1 = 0.0;

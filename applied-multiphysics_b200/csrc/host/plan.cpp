@@ -558,6 +558,28 @@ void build_plan(const Symbolic &S, Plan &P, const Tuning &tune) {
   P.blkOff.assign(ns + 1, 0);
   for (int s = 0; s < ns; s++) P.blkOff[s + 1] = P.blkOff[s] + (P.snNc[s] + B - 1) / B;
   P.nflags = P.blkOff[ns];
+  P.gatherOff.assign(ns + 1, 0);
+  for (int s = 0; s < ns; s++) {
+    const int nc = P.snNc[s], m = P.snM[s], nch = P.chPtr[s + 1] - P.chPtr[s];
+    const int nb = (nc + B - 1) / B, nbelow = (m - nc + B - 1) / B;
+    P.gatherOff[s + 1] = P.gatherOff[s];
+    if (m <= kTinyFront || nch == 0) continue;
+    P.gatherOff[s + 1] += (int64_t)(nb + nbelow) * nch;
+    P.gatherRange.resize(2 * (size_t)P.gatherOff[s + 1]);
+    int *out = P.gatherRange.data() + 2 * (size_t)P.gatherOff[s];
+    for (int q = 0; q < nch; q++) {
+      const int c = P.chList[P.chPtr[s] + q], muc = P.snM[c] - P.snNc[c];
+      const int *map = P.eaMap.data() + P.eaPtr[c];  // increasing
+      int a = 0;
+      for (int b = 0; b < nb + nbelow; b++) {
+        const int end = b < nb ? std::min(nc, (b + 1) * B) : std::min(m, nc + (b - nb + 1) * B);
+        int *r = out + 2 * ((size_t)b * nch + q);
+        r[0] = a;
+        a = (int)(std::lower_bound(map + a, map + muc, end) - map);
+        r[1] = a;
+      }
+    }
+  }
   P.rowBlk.assign(S.n, 0);
   for (int s = 0; s < ns; s++)
     for (int c = 0; c < P.snNc[s]; c++) P.rowBlk[P.snF[s] + c] = P.blkOff[s] + c / B;

@@ -28,6 +28,7 @@ constexpr int kTinyMid = 16;      // the smaller tiny class (m <= 16: 16 x 16 ti
 constexpr int kSmallHalf = 64;    // the smaller class of those: half the registers and a quarter of the shared memory
 constexpr int kSmallFront = 128;  // fronts with 32 < m <= 128: one CTA per front does the whole front
 constexpr int kSolveGroup = 4;    // supernodes with m <= kTinyFront per solve task (one warp each)
+constexpr int kSolveWarps = 8;    // the same in a task of the launched lists, where neighbouring tasks are joined
 constexpr int kWholeFront = 512;  // one-vector forward: supernodes with nc <= 64 and m <= 512 are one task each
 
 struct GroupItem {  // pivot columns [g0, g1) (up to kGroup pivot blocks) of supernode s, factored by one group-panel
@@ -147,6 +148,11 @@ struct Plan {
   std::vector<int> perm, Sp, Si;
   int64_t solveBufDoubles = 0;      // sum of mu (per RHS) for the forward update vectors
   std::vector<int64_t> snTOff;      // offset of supernode s's forward update vector (per RHS)
+  // The forward gathers: the entries [a0, a1) of child q's pass-up vector that map into 64-row block b of supernode s
+  // (its pivot blocks, then its blocks of rows below) are gatherRange[2 (gatherOff[s] + b children(s) + q)] and the next
+  // (supernodes with m > kTinyFront; the others are gathered whole)
+  std::vector<int64_t> gatherOff;
+  std::vector<int> gatherRange;
   // block tasks of the solves ({supernode, block, kind, 0}); ready flags per 64-row pivot block
   std::vector<int> blkOff;          // first flag of supernode s
   std::vector<int> rowBlk;          // flag (64-column diagonal block) holding each column, permuted order (n)
