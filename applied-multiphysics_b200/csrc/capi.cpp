@@ -58,6 +58,12 @@ void ck(cudaError_t e, const char *what) {
   }
 }
 
+// A blocking copy from pageable host memory may return once the data is staged, before the copy to the device has ended,
+// and a blocking memset or device-to-device copy returns at once: both are ordered on the legacy stream only, which the
+// factors' streams (non-blocking) do not wait for. So whoever issues one calls this before its data is used on another
+// stream.
+void settle() { ck(cudaStreamSynchronize(cudaStreamLegacy), "legacy stream"); }
+
 // Device buffer list owned by a handle.
 struct DevMem {
   std::vector<void *> ptrs;
@@ -71,6 +77,7 @@ struct DevMem {
     bytes += (int64_t)b;
     return (T *)p;
   }
+  // settle() before first use
   template <class T>
   T *upload(const std::vector<T> &v) {
     T *p = alloc<T>(v.size());
@@ -722,7 +729,9 @@ static void slice_lists(amp_plan *pl, int ns) {
   pl->dBwdSl[ns - 1] = (int4 *)pl->mem.upload(bw);
   pl->nBwdSl[ns - 1] = (int)(bw.size() / 4);
   pl->nFwdSl[ns - 1] = (int)(fw.size() / 4);
-  pl->dFwdSl[ns - 1] = (int4 *)pl->mem.upload(fw);
+  int4 *const dfw = (int4 *)pl->mem.upload(fw);
+  settle();
+  pl->dFwdSl[ns - 1] = dfw;
 }
 // y (permuted order, interleaved) := A^-1 y in place
 void device_solve_multi_permuted(amp_factor *f, int q) {
@@ -1379,6 +1388,7 @@ int amp_factor_create(amp_plan *pl, const amp_factor_opts *opts, amp_factor **ou
       f->dDone = f->mem.alloc<int>((size_t)kSlices * std::max(1, P.nsuper));
       f->dSolveStatus = f->mem.alloc<unsigned long long>(1);
       init_device_once(pl->device);
+      settle();  // the schedule's uploads and the memsets above
     } catch (...) {
       delete f;
       throw;
@@ -1569,6 +1579,7 @@ int amp_factor_set_row_groups(amp_factor *f, int32_t ngroups, const int64_t *off
     ck(cudaSetDevice(f->plan->device), "cudaSetDevice");
     f->groupMem.release();
     f->dRowGroup = f->groupMem.upload(gid);
+    settle();
     f->dGroupNorms = f->groupMem.alloc<double>((size_t)2 * ngroups * amp::multi_max_vectors());
     f->ngroups = ngroups;
     return (int)AMP_OK;
@@ -1848,6 +1859,7 @@ int amp_cfactor_create(amp_plan *pl, amp_factor **out) {
       f->dStatus = f->mem.alloc<unsigned long long>(1);
       f->dCxFlags = f->mem.alloc<int>((size_t)std::max(1, pl->cx.nGroupFlags + pl->cx.nGroupTickets));
       init_device_once(pl->device);
+      settle();  // the schedule's uploads and the memsets above
     } catch (...) {
       delete f;
       throw;
@@ -2072,6 +2084,7 @@ int amp_assembly_create(int kind, int32_t n, const int32_t *rowptr, const int32_
       a->dKe = a->mem.alloc<double>((size_t)nelem * nd * nd);
       a->dCoef = a->mem.alloc<double>((size_t)nelem * a->ncoef);
       a->dValues = a->mem.alloc<double>((size_t)nnz);
+      settle();
     } catch (...) {
       delete a;
       throw;
@@ -2119,6 +2132,7 @@ int amp_factor_set_mass(amp_factor *f, const double *mvalues, int64_t nvalues, i
     if (nvalues)
       ck(cudaMemcpy(f->dMass, mvalues, sizeof(double) * nvalues,
                     on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice), "copy mass");
+    settle();
     return (int)AMP_OK;
   });
 }
@@ -2139,7 +2153,7 @@ int amp_shift_invert_apply(amp_factor *f, const double *X, int32_t m, double *Y,
     double *dY = Y;
     if (!on_device) {
       double *a = tmp.alloc<double>(len), *b = tmp.alloc<double>(len);
-      ck(cudaMemcpy(a, X, sizeof(double) * len, cudaMemcpyHostToDevice), "copy X");
+      ck(cudaMemcpyAsync(a, X, sizeof(double) * len, cudaMemcpyHostToDevice, f->stream), "copy X");
       dX = a;
       dY = b;
     }
@@ -2191,7 +2205,8 @@ int amp_eigen_block_arnoldi(amp_factor *f, const amp_eigen_opts *opts, double *m
         s = s * 1664525u + 1013904223u;
         v = (double)s / 4294967296.0 - 0.5;
       }
-      ck(cudaMemcpy(V, x0.data(), sizeof(double) * x0.size(), cudaMemcpyHostToDevice), "start block");
+      ck(cudaMemcpyAsync(V, x0.data(), sizeof(double) * x0.size(), cudaMemcpyHostToDevice, st), "start block");
+      ck(cudaStreamSynchronize(st), "start block");  // x0 ends here
     }
     int opVectors = 0;
     // M-orthonormalise the b vectors at X (M X at MX): X <- X R^-1 with R^T R = X^T M X; R to Rout (b x b,
@@ -2334,6 +2349,7 @@ int amp_eigen_block_arnoldi(amp_factor *f, const amp_eigen_opts *opts, double *m
         ew.combine(U, V, coef, pc);
         ck(cudaMemcpy(vecs + (int64_t)k * n, U, sizeof(double) * n,
                       on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost), "copy Ritz vector");
+        settle();  // the next vector overwrites U
       }
     }
     if (stats) {
