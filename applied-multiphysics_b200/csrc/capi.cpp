@@ -182,6 +182,7 @@ struct amp_plan_s {
   bool uploaded = false;
   // the dense schedule of every front, for complex-symmetric factors (built and uploaded by the first of them)
   amp::DenseSched cx;
+  std::vector<amp::CSolveLevel> cxSolve;  // the sweeps' launches, leaves first
   bool cxUploaded = false;
   amp::AsmTask *dCxAsm = nullptr;
   amp::ChildRange *dCxAsmCh = nullptr;
@@ -980,7 +981,17 @@ namespace {
 
 void upload_cx(amp_plan *pl) {
   if (pl->cxUploaded) return;
-  amp::build_dense_all(pl->P, pl->cx);
+  const amp::Plan &P = pl->P;
+  amp::build_dense_all(P, pl->cx);
+  for (int L = 0; L < P.nlevels; L++) {
+    int maxNc = 0, maxM = 0;
+    for (int i = P.lvlPtr[L]; i < P.lvlPtr[L + 1]; i++) {
+      maxNc = std::max(maxNc, P.snNc[P.lvlSn[i]]);
+      maxM = std::max(maxM, P.snM[P.lvlSn[i]]);
+    }
+    if (P.lvlPtr[L + 1] > P.lvlPtr[L])
+      pl->cxSolve.push_back(amp::csolve_level(P.lvlPtr[L], P.lvlPtr[L + 1] - P.lvlPtr[L], maxNc, maxM));
+  }
   DevMem &m = pl->mem;
   pl->dCxAsm = m.upload(pl->cx.asmTasks);
   pl->dCxAsmCh = m.upload(pl->cx.asmCh);
@@ -1037,7 +1048,7 @@ void enqueue_cfactor(amp_factor *f) {
 void csolve_permuted(amp_factor *f, amp::cplx *y) {
   const amp::Plan &P = f->plan->P;
   timed(f, K_FORWARD, 8.0 * (double)P.nnzLStored, 16.0 * (double)P.nnzLStored, [&] {
-    return amp::launch_csolve_permuted(f->plan->dp, P.lvlPtr.data(), P.nlevels, f->dLc, f->dDc, y, f->stream);
+    return amp::launch_csolve_permuted(f->plan->dp, f->plan->cxSolve, f->dLc, f->dDc, y, f->stream);
   });
 }
 

@@ -782,6 +782,7 @@ cudaError_t init_kernel_attributes() {
   if (e == cudaSuccess) e = init_solve_attributes();
   if (e == cudaSuccess) e = init_solve_multi_attributes();
   if (e == cudaSuccess) e = init_front_small_attributes();
+  if (e == cudaSuccess) e = init_csolve();
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_update<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, upd_smem<128>());
   if (e == cudaSuccess)

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <vector>
 
 #include "../host/plan.hpp"
 #include "devplan.cuh"
@@ -101,8 +102,15 @@ void launch_cpermute_in(int n, const double *br, const double *bi, const int *pe
 void launch_cpermute_out(int n, const cplx *y, const int *perm, double *xr, double *xi, cudaStream_t st);
 void launch_cpermute_vec(int n, const cplx *src, const int *perm, cplx *dst, bool gather, cudaStream_t st);
 void launch_caxpy(int n, cplx *x, const cplx *dx, cudaStream_t st);
-int launch_csolve_permuted(const DevPlan &P, const int *lvlPtr, int nlevels, const cplx *L, const cplx *D, cplx *y,
+struct CSolveLevel {
+  int first, count;  // supernodes (positions in the level order)
+  int cluster;       // CTAs per supernode
+  int ld, tri, smem; // a staged triangle's leading dimension and entries; dynamic shared memory (bytes)
+};
+CSolveLevel csolve_level(int first, int count, int maxNc, int maxM);
+int launch_csolve_permuted(const DevPlan &P, const std::vector<CSolveLevel> &levels, const cplx *L, const cplx *D, cplx *y,
                            cudaStream_t st);
+cudaError_t init_csolve();
 void launch_cresidual(int n, const int *rowptr, const int *colidx, const cplx *val, const cplx *x, const cplx *b,
                       cplx *r, double *norms, cudaStream_t st);
 
