@@ -1028,7 +1028,7 @@ void enqueue_cfactor(amp_factor *f) {
       timed(f, K_PANEL, 4.0 * sr.panelFlops, 0.0, [&] {
         amp::launch_group_panel<amp::cplx>(f->plan->dCxItems, f->plan->dCxStrips + sr.strip0,
                                            (int)(sr.strip1 - sr.strip0), tickets + sr.ticket, f->dCxFlags, dp,
-                                           f->dLc, nullptr, f->dStatus, nullptr, nullptr, ld, st);
+                                           f->dLc, f->dLinv, f->dStatus, nullptr, nullptr, ld, st);
       });
       if (sr.tile1 > sr.tile0)
         timed(f, K_UPDATE, 4.0 * (sr.updateFlopsA + sr.updateFlopsB), 0.0, [&] {
@@ -1868,6 +1868,7 @@ int amp_cfactor_create(amp_plan *pl, amp_factor **out) {
       f->dScal = f->mem.alloc<double>(2);
       f->dCounts = f->mem.alloc<int>(2);
       f->dStatus = f->mem.alloc<unsigned long long>(1);
+      f->dLinv = f->mem.alloc<double>((size_t)pl->cx.nGroupFlags / 2 * 1024);
       f->dCxFlags = f->mem.alloc<int>((size_t)std::max(1, pl->cx.nGroupFlags + pl->cx.nGroupTickets));
       init_device_once(pl->device);
       settle();  // the schedule's uploads and the memsets above

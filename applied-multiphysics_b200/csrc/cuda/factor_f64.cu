@@ -1,11 +1,11 @@
-// Multifrontal numeric factorization on sm_100a: assembly, the FP64 and complex updates, the complex group panel.
+// Multifrontal numeric factorization on sm_100a: assembly, the FP64 and complex updates.
 //
 // Per level of the supernodal tree (leaves first):
 //   k_assemble  zero the front, scatter A's entries (sparse.mjs:965-973) and extend-add the children's update
 //               matrices in the reference's child order (sparse.mjs:974-985). One CTA owns a block of 8 front
 //               columns, so every entry has a single writer and the summation order is the reference's.
 //   per group of up to kGroup pivot blocks of 64 columns:
-//     k_group_panel  (group_panel.cu; the complex factor's k_cgroup_panel is here) one dataflow launch: POTRF (or LDL^T)
+//     k_group_panel  (group_panel.cu, cgroup_panel.cu for the complex factor) one dataflow launch: POTRF (or LDL^T)
 //                    of each 64 x 64 pivot block, the rows below it against it (TRSM, 64-row strips, one CTA each) and
 //                    the update of the group's remaining columns, ordered by flags between the strips of the launch.
 //     k_update       FP64 update F -= A B^T of the columns right of the group (A = L21, or L21 D for LDL^T; B = L21;
@@ -31,27 +31,6 @@ __device__ __forceinline__ T *front_addr(T *Lp, T *Up, int m, int nc, int i, int
   return j < nc ? Lp + (int64_t)j * m + i : Up + (int64_t)(j - nc) * (m - nc) + (i - nc);
 }
 
-// Complex pivot of the complex-symmetric LDL^T (ldlt.mjs:715-730): a magnitude below tau (or not a number) becomes
-// tau, keeping the pivot's phase (tau itself when d = 0); a non-finite small magnitude fails the factorization.
-// flags: bit 1 perturbed (a complex factor has no inertia).
-__device__ __forceinline__ bool ldlt_pivot(cplx &d, double tau, unsigned char &flags) {
-  flags = 0;
-  const double mag = hypot(d.re, d.im);
-  if (!(mag >= tau)) {
-    if (!isfinite(mag)) return false;
-    if (mag == 0)
-      d.re = tau;
-    else
-      d = cplx(d.re * (tau / mag), d.im * (tau / mag));
-    flags = 2;
-  }
-  return true;
-}
-// loads through L2 (data another CTA of the running launch wrote) and read-only loads
-__device__ __forceinline__ cplx ldcg_v(const cplx *p) {
-  const double2 v = __ldcg(reinterpret_cast<const double2 *>(p));
-  return cplx(v.x, v.y);
-}
 __device__ __forceinline__ double ldg_v(const double *p) { return __ldg(p); }
 __device__ __forceinline__ cplx ldg_v(const cplx *p) {
   const double2 v = __ldg(reinterpret_cast<const double2 *>(p));
@@ -163,351 +142,6 @@ __global__ void __launch_bounds__(256) k_assemble(const AsmTask *__restrict__ ta
       }
     }
     __syncthreads();
-  }
-}
-
-// ---------------------------------------------------------------------------------------------------------------
-// Group panel of the complex-symmetric factor (the real factors': group_panel.cu): the pivot blocks of a group of
-// 64-column blocks of a front, factored in one dataflow launch (LDL^T of each pivot block, TRSM of the rows below it,
-// and the update of the group's remaining columns) on the CUDA cores.
-// ---------------------------------------------------------------------------------------------------------------
-
-// Pivot block: LDL^T of the 64 x 64 diagonal block of a front, called by all 256 threads of a CTA, the block in
-// registers. src: the updated block in shared memory, entry (i, j) at src[j lds + i]; Lp: the block's (0, 0) entry in
-// the front (ld m), where the factor is written; w <= 64 its columns. Thread t < 136 owns the 4 x 4 tile (ti, tj),
-// ti >= tj, of the lower triangle. Right-looking on the unscaled columns, four columns per step kb with two barriers:
-// (1) the diagonal tile eliminates its four columns (settling the pivots) and publishes them; (2) the tiles below it in
-// column block kb eliminate the same four columns against it and publish theirs; then every tile right of the block
-// applies the rank-4 update S(i, j) -= sum S(i, k) S(j, k) / d_k. A pivot of magnitude below tau is perturbed
-// (ldlt.mjs:715-730) and counted. At the end the columns are scaled: L = a / d with a unit diagonal (D to ld.D). When a
-// pivot failed (status set for the first failing column f + c0 + k) the block is not written back.
-__device__ void cpotrf_block(const cplx *src, int lds, cplx *Lp, int m, int w, int f, int c0, int s,
-                             unsigned long long *status, const LdltArgs<cplx> &ld) {
-  __shared__ cplx col[2][4][kPanel];  // per 4-column block (double-buffered): the block's unscaled columns, by row
-  __shared__ cplx pd[kPanel], piv[2][4];
-  __shared__ unsigned char pflag[kPanel];
-  __shared__ int fail;
-  const int tid = threadIdx.x;
-  const double tau = ld.scal[1];
-  // tile of this thread: row block ti, column block tj (ti >= tj), from tid by the triangular numbering
-  int ti = 0;
-  while ((ti + 1) * (ti + 2) / 2 <= tid) ti++;
-  const int tj = tid - ti * (ti + 1) / 2;
-  const bool owner = tid < 136;
-  int myFail = -1;  // diagonal tiles only
-  cplx a[4][4];
-#pragma unroll
-  for (int r = 0; r < 4; r++)
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-      const int i = 4 * ti + r, j = 4 * tj + c;
-      a[r][c] = !owner || i < j ? cplx(0) : (i < w ? src[j * lds + i] : (i == j ? cplx(1) : cplx(0)));
-    }
-  if (tid == 0) fail = kPanel;  // none
-  for (int kb = 0; kb < kPanel / 4; kb++) {
-    const int buf = kb & 1;
-    if (owner && ti == kb && tj == kb) {
-#pragma unroll
-      for (int kk = 0; kk < 4; kk++) {
-        const int k = 4 * kb + kk;
-        cplx d = a[kk][kk];
-        unsigned char fl = 0;
-        const bool bad = k < w && !ldlt_pivot(d, tau, fl);
-        if (bad && myFail < 0) myFail = k;  // first failing pivot of this diagonal tile
-        const cplx iv = cplx(1.0) / d;
-        pd[k] = d;
-        pflag[k] = fl;
-        piv[buf][kk] = iv;
-#pragma unroll
-        for (int r = kk + 1; r < 4; r++)
-#pragma unroll
-          for (int c = kk + 1; c <= r; c++) a[r][c] -= a[r][kk] * (a[c][kk] * iv);
-      }
-#pragma unroll
-      for (int kk = 0; kk < 4; kk++)
-#pragma unroll
-        for (int r = 0; r < 4; r++) col[buf][kk][4 * kb + r] = a[r][kk];
-    }
-    __syncthreads();
-    if (owner && tj == kb && ti > kb) {
-#pragma unroll
-      for (int kk = 0; kk < 4; kk++) {
-        const cplx iv = piv[buf][kk];
-#pragma unroll
-        for (int c = kk + 1; c < 4; c++) {
-          const cplx cj = col[buf][kk][4 * kb + c] * iv;
-#pragma unroll
-          for (int r = 0; r < 4; r++) a[r][c] -= a[r][kk] * cj;
-        }
-      }
-#pragma unroll
-      for (int kk = 0; kk < 4; kk++)
-#pragma unroll
-        for (int r = 0; r < 4; r++) col[buf][kk][4 * ti + r] = a[r][kk];
-    }
-    __syncthreads();
-    if (owner && tj > kb) {
-#pragma unroll
-      for (int kk = 0; kk < 4; kk++) {
-        const cplx iv = piv[buf][kk];
-        cplx ci[4], cj[4];
-#pragma unroll
-        for (int r = 0; r < 4; r++) ci[r] = col[buf][kk][4 * ti + r];
-#pragma unroll
-        for (int c = 0; c < 4; c++) cj[c] = col[buf][kk][4 * tj + c] * iv;
-#pragma unroll
-        for (int r = 0; r < 4; r++)
-#pragma unroll
-          for (int c = 0; c < 4; c++)
-            if (ti > tj || c <= r) a[r][c] -= ci[r] * cj[c];
-      }
-    }
-  }
-  if (myFail >= 0) atomicMin(&fail, myFail);
-  __syncthreads();
-  if (fail < kPanel) {
-    if (tid == 0) atomicMin(status, status_word(f + c0 + fail, 2, s));
-    return;
-  }
-  if (owner) {
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-      const int j = 4 * tj + c;
-      const cplx inv = cplx(1) / pd[j];
-#pragma unroll
-      for (int r = 0; r < 4; r++) {
-        const int i = 4 * ti + r;
-        if (i >= j && i < w && j < w) Lp[(int64_t)j * m + i] = i == j ? cplx(1) : a[r][c] * inv;
-      }
-    }
-  }
-  if (tid < w) ld.D[f + c0 + tid] = pd[tid];
-  if (tid == 0) {
-    int pert = 0;
-    for (int k = 0; k < w; k++) pert += pflag[k] >> 1;
-    atomicAdd(ld.counts + 1, pert);
-  }
-}
-
-// TRSM of up to 64 rows [r0, r1) of a front (L: its column-major block, ld m) against its factored pivot block
-// [c0, c0 + w): x_k = (a_k - sum_{c<k} x_c M(k, c)) / M(k, k), M(k, c) = L11(k, c) d_c, M(k, k) = d_k, x = L21, and
-// w = x D = L21 D (the update's A operand, written to ld.W). Four threads per row, thread (row, q) holds columns
-// 16 q .. 16 q + 15 in registers. Phase p: the threads of quarter p solve their 16 columns (the earlier quarters'
-// contributions already applied) and publish them; after a barrier the threads of the later quarters subtract
-// quarter p's contribution (16 x 16 products) from theirs. The pivot block and D come from another CTA of the launch:
-// read through L2 (__ldcg).
-// x: this thread's 16 entries of its row (row r0 + tid % 64, columns c0 + 16 (tid / 64) + u), loaded by the caller
-// before it waited for the pivot block (the strip's own rows are final by then).
-// On return Ws[c][r] holds this strip's update operand x D and M[c][r] the solved rows x (c < w, r < r1 - r0; zero
-// elsewhere): a diagonal strip's X_c for its own column block.
-__device__ void ctrsm_strip(cplx *L, int m, int f, int c0, int w, int r0, int r1, int64_t lxp,
-                            const LdltArgs<cplx> &ld, cplx (*M)[kPanel + 1], cplx (*Ws)[kPanel + 1], cplx *invd,
-                            cplx *dv, cplx (&x)[16]) {
-  const int tid = threadIdx.x, r = tid & (kPanel - 1), q = tid >> 6;
-  {  // the pivot block: thread (r, q) loads row r of columns 16 q .. 16 q + 15 times their pivots, and thread r < 64 the
-     // pivot of column r, in one round trip
-    cplx v[16];
-#pragma unroll
-    for (int u = 0; u < 16; u++) {
-      const int c = 16 * q + u;
-      v[u] = (r < w && c < r) ? ldcg_v(L + (int64_t)(c0 + c) * m + c0 + r) : cplx(0);
-    }
-#pragma unroll
-    for (int u = 0; u < 16; u++) {
-      const int c = 16 * q + u;
-      v[u] = v[u] * (c < w ? ldcg_v(ld.D + f + c0 + c) : cplx(1));
-    }
-    if (tid < kPanel) {
-      const cplx d = tid < w ? ldcg_v(ld.D + f + c0 + tid) : cplx(1);
-      dv[tid] = d;
-      invd[tid] = cplx(1) / d;
-    }
-#pragma unroll
-    for (int u = 0; u < 16; u++) M[r][16 * q + u] = v[u];
-  }
-  const int row = r0 + r;
-  const bool active = row < r1;
-  __syncthreads();
-  for (int p = 0; p < 4; p++) {
-    if (q == p) {  // solve this quarter
-#pragma unroll
-      for (int u = 0; u < 16; u++) {
-        const int c = 16 * p + u;
-        x[u] *= invd[c];
-#pragma unroll
-        for (int u2 = u + 1; u2 < 16; u2++) x[u2] -= x[u] * M[16 * p + u2][c];
-      }
-#pragma unroll
-      for (int u = 0; u < 16; u++) Ws[16 * p + u][r] = x[u];
-    }
-    __syncthreads();
-    if (q > p) {  // subtract quarter p's contribution
-#pragma unroll 4
-      for (int kk = 0; kk < 16; kk++) {
-        const int k = 16 * p + kk;
-        const cplx xk = Ws[k][r];
-#pragma unroll
-        for (int u = 0; u < 16; u++) x[u] -= xk * M[16 * q + u][k];
-      }
-    }
-  }
-  __syncthreads();  // every quarter read Ws: overwrite it with the update operand
-#pragma unroll
-  for (int u = 0; u < 16; u++) {
-    const int cc = 16 * q + u;
-    const cplx xv = x[u], wv = xv * dv[cc];
-    Ws[cc][r] = active && cc < w ? wv : cplx(0);
-    M[cc][r] = active && cc < w ? xv : cplx(0);  // the pivot block in M is no longer read
-    if (!active || cc >= w) continue;
-    L[(int64_t)(c0 + cc) * m + row] = xv;
-    ld.W[lxp + (int64_t)(c0 + cc) * m + row] = wv;
-  }
-  __syncthreads();
-}
-
-// Wait (thread 0, bounded) until *p >= need; false when the factorization has failed (a pivot, or a wait that ran
-// out: status set). Thread 0 decides and the CTA follows it after the barrier, so every thread returns the same.
-__device__ __forceinline__ bool panel_wait(const int *p, int need, unsigned long long *status, long long limit) {
-  __shared__ int ok;
-  if (threadIdx.x == 0) {
-    long long spins = 0;
-    int v = 1;
-    while (ld_acquire(p) < need) {
-      if (failed(status)) {
-        v = 0;
-        break;
-      }
-      if (++spins > limit) {
-        atomicMin(status, status_word(0x7fffffff, 3, 0));
-        v = 0;
-        break;
-      }
-      __nanosleep(64);
-    }
-    if (failed(status)) v = 0;  // a failed pivot also releases its flag
-    ok = v;
-  }
-  __syncthreads();
-  return ok != 0;
-}
-
-// Publish *p = v after this CTA's global writes: all threads pass the barrier first, and thread 0's release store
-// orders every write made before the barrier (by any thread of the CTA) before the flag, for a reader that acquires it.
-__device__ __forceinline__ void panel_release(int *p, int v) {
-  __syncthreads();
-  if (threadIdx.x == 0) st_release(p, v);
-}
-
-// One group of pivot blocks [g0, g1) of a front, a strip of up to 64 rows per CTA, CTAs ordered by an atomic ticket
-// (the diagonal strips of every item first, then the strips below the group). Per pivot block b of the group:
-//   the diagonal strip of block b (rows [c0, c0 + w)) factors it once its own updates are done and publishes P[b];
-//   every strip with rows below block b waits for P[b], solves its rows against the block (TRSM) and, when it is a
-//   diagonal strip, publishes D[j] = b + 1; then it updates its rows of the group's remaining columns [c0 + w, g1)
-//   with block b (C -= W_r X_c^T, K = w; X_c: the rows of those columns, from the diagonal strips' TRSM, waited for
-//   by D[j] >= b + 1; a diagonal strip updates only the lower part, columns up to its own rows).
-// Every wait is on a strip with a smaller ticket, which runs to completion without waiting on a larger one, so the
-// launch cannot deadlock whatever the number of resident CTAs. The columns right of the group receive the group's
-// update afterwards (k_update / k_update_mx, K = the group). Failure (a pivot, a bounded wait) sets the status and
-// releases P[b], so every waiter leaves.
-constexpr int kCGroupSmem = 3 * kPanel * (kPanel + 1) * (int)sizeof(cplx);  // one CTA per SM
-__global__ void __launch_bounds__(256, 1) k_cgroup_panel(const GroupItem *__restrict__ items,
-                                                         const StripTask *__restrict__ strips, int nstrips,
-                                                         int *ticket, int *flags, DevPlan P, cplx *__restrict__ Lx,
-                                                         unsigned long long *status, LdltArgs<cplx> ld) {
-  extern __shared__ __align__(16) unsigned char gp_raw[];
-  cplx(*M)[kPanel + 1] = reinterpret_cast<cplx(*)[kPanel + 1]>(gp_raw);  // pivot block (TRSM), then the X_c chunk
-  cplx(*Ws)[kPanel + 1] = reinterpret_cast<cplx(*)[kPanel + 1]>(gp_raw + kPanel * (kPanel + 1) * sizeof(cplx));
-  cplx(*Ds)[kPanel + 1] = reinterpret_cast<cplx(*)[kPanel + 1]>(gp_raw + 2 * kPanel * (kPanel + 1) * sizeof(cplx));
-  __shared__ cplx invd[kPanel], dv[kPanel];
-  __shared__ int sTicket;
-  if (threadIdx.x == 0) sTicket = failed(status) ? nstrips : atomicAdd(ticket, 1);
-  __syncthreads();
-  const int t = sTicket;
-  if (t >= nstrips) return;
-  const StripTask st = strips[t];
-  const GroupItem it = items[st.item];
-  const int s = it.s, g0 = it.g0, g1 = it.g1;
-  const int f = P.snF[s], m = P.snM[s];
-  const int nb = (g1 - g0 + kPanel - 1) / kPanel;
-  const int r0 = st.r0, r1 = st.r1, jd = st.diag;
-  const int bmax = jd >= 0 ? jd : nb;  // pivot blocks whose rows below include this strip
-  cplx *L = Lx + P.snLxp[s];
-  int *Pf = flags + it.flag0, *Df = Pf + nb;
-  const int tid = threadIdx.x, tr = tid & 15, tc = tid >> 4;
-  // A diagonal strip keeps its own pivot block (columns [r0, r1), lower part) in shared memory while it updates it
-  // (Ds[j][i] = block (i, j)), and its POTRF reads it from there: no round trip through the front.
-  if (jd >= 0) {
-    for (int e = tid; e < kPanel * kPanel; e += blockDim.x) {
-      const int i = e & 63, j = e >> 6;
-      Ds[j][i] = (r0 + i < r1 && j <= i) ? L[(int64_t)(r0 + j) * m + r0 + i] : cplx(0);
-    }
-  }
-  for (int b = 0; b < bmax; b++) {
-    const int c0 = g0 + b * kPanel, w = min(kPanel, g1 - c0), c1 = c0 + w;
-    cplx x[16];  // this thread's part of the strip's rows of block b, loaded while the pivot block is not yet ready
-    {
-      const int xr = r0 + (tid & (kPanel - 1)), xq = tid >> 6;
-#pragma unroll
-      for (int u = 0; u < 16; u++) {
-        const int c = 16 * xq + u;
-        x[u] = xr < r1 && c < w ? L[(int64_t)(c0 + c) * m + xr] : cplx(0);
-      }
-    }
-    if (!panel_wait(Pf + b, 1, status, P.spin)) return;
-    ctrsm_strip(L, m, f, c0, w, r0, r1, P.snLxp[s], ld, M, Ws, invd, dv, x);
-    if (jd >= 0) panel_release(Df + jd, b + 1);
-    // Update with block b (C -= W_r X_c^cplx, K = w): a diagonal strip first its own pivot block (X_c = its solved rows,
-    // left in M by the TRSM; into Ds), then the blocks between block b and its own; a strip below every remaining
-    // column block of the group.
-    const int hi = jd >= 0 ? r0 : g1, nown = jd >= 0 ? 1 : 0;
-    const int nchunk = nown + (hi > c1 ? (hi - c1 + kPanel - 1) / kPanel : 0);
-    for (int ch = 0; ch < nchunk; ch++) {
-      const bool own = ch < nown;
-      const int cb = own ? r0 : c1 + (ch - nown) * kPanel, ncol = own ? r1 - r0 : min(kPanel, hi - cb);
-      if (!own) {
-        if (!panel_wait(Df + (cb - g0) / kPanel, b + 1, status, P.spin)) return;
-        for (int e = tid; e < kPanel * kPanel; e += blockDim.x) {  // X_c[k][jj] = L(cb + jj, c0 + k)
-          const int k = e >> 6, jj = e & 63;
-          M[k][jj] = (k < w && jj < ncol) ? ldcg_v(L + (int64_t)(c0 + k) * m + cb + jj) : cplx(0);
-        }
-        __syncthreads();
-      }
-      cplx acc[4][4];
-#pragma unroll
-      for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int bb = 0; bb < 4; bb++) acc[a][bb] = cplx(0);
-      for (int k = 0; k < w; k++) {
-        cplx wv[4], xv[4];
-#pragma unroll
-        for (int a = 0; a < 4; a++) wv[a] = Ws[k][tr + 16 * a];
-#pragma unroll
-        for (int bb = 0; bb < 4; bb++) xv[bb] = M[k][tc + 16 * bb];
-#pragma unroll
-        for (int a = 0; a < 4; a++)
-#pragma unroll
-          for (int bb = 0; bb < 4; bb++) acc[a][bb] += wv[a] * xv[bb];
-      }
-#pragma unroll
-      for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int bb = 0; bb < 4; bb++) {
-          const int i = tr + 16 * a, jj = tc + 16 * bb;
-          if (own) {
-            if (jj <= i) Ds[jj][i] -= acc[a][bb];
-          } else if (r0 + i < r1 && jj < ncol) {
-            cplx *cptr = L + (int64_t)(cb + jj) * m + r0 + i;
-            *cptr = *cptr - acc[a][bb];
-          }
-        }
-      __syncthreads();  // M is reloaded by the next chunk, or by the next TRSM
-    }
-  }
-  if (jd >= 0) {  // this strip's own pivot block, fully updated: factor it and publish it (also after a failure)
-    const int c0 = g0 + jd * kPanel, w = min(kPanel, g1 - c0);
-    __syncthreads();  // Ds complete (also when the strip had no earlier pivot block)
-    cpotrf_block(&Ds[0][0], kPanel + 1, L + (int64_t)c0 * m + c0, m, w, f, c0, s, status, ld);
-    panel_release(Pf + jd, 1);
   }
 }
 
@@ -770,14 +404,15 @@ __global__ void k_permute_out(const double *__restrict__ y, double *__restrict__
 static int g_num_sms = 148;
 
 cudaError_t init_group_panel_attributes();
+cudaError_t init_cgroup_panel_attributes();
 cudaError_t init_mixed_attributes();
 cudaError_t init_solve_attributes();
 cudaError_t init_solve_multi_attributes();
 cudaError_t init_front_small_attributes();
 cudaError_t init_kernel_attributes() {
   // function attributes belong to the current device's context: the caller runs this once per device
-  cudaError_t e = cudaFuncSetAttribute(k_cgroup_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCGroupSmem);
-  if (e == cudaSuccess) e = init_group_panel_attributes();
+  cudaError_t e = init_group_panel_attributes();
+  if (e == cudaSuccess) e = init_cgroup_panel_attributes();
   if (e == cudaSuccess) e = init_mixed_attributes();
   if (e == cudaSuccess) e = init_solve_attributes();
   if (e == cudaSuccess) e = init_solve_multi_attributes();
@@ -804,15 +439,6 @@ template void launch_assemble<float>(const AsmTask *, const ChildRange *, int64_
                                      float *, float *, const unsigned long long *, cudaStream_t);
 template void launch_assemble<cplx>(const AsmTask *, const ChildRange *, int64_t, const DevPlan &, const cplx *,
                                     cplx *, cplx *, const unsigned long long *, cudaStream_t);
-template <>
-void launch_group_panel<cplx>(const GroupItem *items, const StripTask *strips, int nstrips, int *ticket, int *flags,
-                              const DevPlan &P, cplx *Lx, double *, unsigned long long *status, __nv_bfloat16 *,
-                              __nv_bfloat16 *, const LdltArgs<cplx> &ld, cudaStream_t st) {
-  if (nstrips > 0)
-    k_cgroup_panel<<<(unsigned)nstrips, 256, kCGroupSmem, st>>>(items, strips, nstrips, ticket, flags, P, Lx, status,
-                                                               ld);
-}
-
 void launch_update_c(const TileTask *tasks, int64_t ntasks, cplx *Lx, cplx *U, const cplx *W,
                      const unsigned long long *status, cudaStream_t st) {
   if (ntasks > 0) k_update_c<<<(unsigned)ntasks, 256, 0, st>>>(tasks, Lx, U, W, status);

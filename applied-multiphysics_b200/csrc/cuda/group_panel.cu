@@ -19,33 +19,12 @@
 
 #include "../host/plan.hpp"
 #include "devplan.cuh"
+#include "panel_blocks.cuh"
 #include "pivot_steps.cuh"
-#include "sync.cuh"
 
 namespace amp {
 
 namespace {
-
-__device__ __forceinline__ bool panel_failed(const unsigned long long *st) {
-  return *(volatile const unsigned long long *)st != kStatusOk;
-}
-
-// 64 x 64 FP64 blocks in shared memory, row-major, the column pairs of row r permuted by a bijection of r mod 8 so that
-// the 16-byte accesses of a fragment (8 rows, 4 neighbouring pairs) and the 8-byte stores of the block loads (8 rows,
-// 4 columns) touch every bank equally often.
-__device__ __forceinline__ int sw(int r, int c) {
-  return r * kPanel + (((c >> 1) ^ (((r & 1) << 2) | ((r >> 1) & 3))) << 1) + (c & 1);
-}
-__device__ __forceinline__ double2 pair_at(const double *S, int r, int c) {  // entries (r, c), (r, c + 1), c even
-  return *reinterpret_cast<const double2 *>(S + sw(r, c));
-}
-__device__ __forceinline__ void set_pair(double *S, int r, int c, double x, double y) {
-  *reinterpret_cast<double2 *>(S + sw(r, c)) = make_double2(x, y);
-}
-
-// the 8-row group of a warp: the pairs of warps that share a scheduler (w, w + 4) get groups that sum to 7, so the
-// lower triangle's work is the same on all four
-__device__ __forceinline__ int row_group(int warp) { return warp < 4 ? warp : 11 - warp; }
 
 // Rows [i0, i0 + nr) x columns [j0, j0 + ncol) of a front's column-major block (ld m) into S; lower: only the entries
 // on and below the diagonal. The rest is zero, and with pad the diagonal entries from ncol on are one. Read through
@@ -93,6 +72,7 @@ __device__ int potrf_block(const double *Ds, double *scr, T *Lp, double *Linv, i
   __shared__ double scale[kPanel], diag[kPanel];
   __shared__ int failAt, redo, nNeg, nPert, inexact;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, rg = row_group(warp);
+  const int nk = (w + 7) >> 3;  // steps: the columns from w on are the identity's
   const TC tau = LDLT ? (TC)ld.scal[1] : TC(0);
   TC *R = reinterpret_cast<TC *>(scr), *Q = R + kStepBuf, *P = R + 3 * kStepBuf;  // Q: two buffers; P: -a of every step
   const int myRow = (8 * rg + g) * CL + 2 * t;
@@ -109,7 +89,7 @@ __device__ int potrf_block(const double *Ds, double *scr, T *Lp, double *Linv, i
   };
   auto panel = [&](auto exact) {  // the first two warps, a row per lane
     bool fine = true;
-    for (int k = 0; k < 8; k++) {
+    for (int k = 0; k < nk; k++) {
       if (8 * k + 32 * warp < kPanel)
         fine &= eliminate8<decltype(exact)::value, LDLT, false>(R, P + k * kStepBuf, Q + (k & 1) * kStepBuf, 8 * k,
                                                                min(8 * k + 32 * warp + lane, kPanel - 1), 8, tau);
@@ -131,7 +111,7 @@ __device__ int potrf_block(const double *Ds, double *scr, T *Lp, double *Linv, i
       c[j][0] = c[j][1] = TC(0);
       if (j < rg) tile(j + 1, c[j]);
     }
-    for (int k = 0; k < 8; k++) {
+    for (int k = 0; k < nk; k++) {
       __syncthreads();
       const TC *Pk = P + k * kStepBuf + 8 * rg * CL, *Qk = Q + (k & 1) * kStepBuf;
       if (rg > k) {
@@ -223,7 +203,7 @@ __device__ int potrf_block(const double *Ds, double *scr, T *Lp, double *Linv, i
         if (r >= 8 * p + u) dst[(int64_t)u * m] = r > 8 * p + u ? v[u] : LDLT ? T(1) : (T)diag[r];
     }
   } else {  // column j of inv(L_pp): forward substitution with the unit block, rows over the diagonal
-    const int p = tid >> 3, j = tid & 7;
+    const int p = min(tid >> 3, nk - 1), j = tid & 7;  // (the strips use the first nk blocks)
     const TC *Pp = P + p * kStepBuf + 8 * p * CL;
     double x[8];
 #pragma unroll
@@ -438,39 +418,6 @@ __device__ bool bk_block(const double *Ds, double (*S)[kPanel + 1], T *Lp, doubl
   return true;
 }
 
-// Wait (thread 0, bounded) until *p >= need; false when the factorization has failed (a pivot, or a wait that ran
-// out: status set). Thread 0 decides and the CTA follows it after the barrier, so every thread returns the same.
-__device__ __forceinline__ bool panel_wait(const int *p, int need, unsigned long long *status, long long limit) {
-  __shared__ int ok;
-  if (threadIdx.x == 0) {
-    long long spins = 0;
-    int v = 1;
-    while (ld_acquire(p) < need) {
-      if (panel_failed(status)) {
-        v = 0;
-        break;
-      }
-      if (++spins > limit) {
-        atomicMin(status, status_word(0x7fffffff, 3, 0));
-        v = 0;
-        break;
-      }
-      __nanosleep(32);
-    }
-    if (panel_failed(status)) v = 0;  // a failed pivot also releases its flag
-    ok = v;
-  }
-  __syncthreads();
-  return ok != 0;
-}
-
-// Publish *p = v after this CTA's global writes: all threads pass the barrier first, and thread 0's release store
-// orders every write made before the barrier (by any thread of the CTA) before the flag, for a reader that acquires it.
-__device__ __forceinline__ void panel_release(int *p, int v) {
-  __syncthreads();
-  if (threadIdx.x == 0) st_release(p, v);
-}
-
 // C(8 x 64 of this warp) += N S^T: N the warp's A fragments (8 x 64), S a block in shared memory. Eight independent
 // accumulators between two products of one.
 __device__ __forceinline__ void update_row_group(double (&c)[8][2], const double (&n)[8][2], const double *S, int g,
@@ -620,6 +567,7 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
     // later ones
 #pragma unroll
     for (int p = 0; p < 8; p++) {
+      if (8 * p >= w) break;  // x is zero from column w on
       const double2 iv = *reinterpret_cast<const double2 *>(Li + 64 * p + 8 * g + 2 * t);
       double wv[2] = {0.0, 0.0};
       mma884(wv, x[p][0], iv.x);
@@ -628,6 +576,7 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
       x[p][1] = wv[1];
 #pragma unroll
       for (int p2 = p + 1; p2 < 8; p2++) {
+        if (8 * p2 >= w) break;
         const double2 l = pair_at(Ls, 8 * p2 + g, 8 * p + 2 * t);
         mma884(x[p2], -wv[0], l.x);
         mma884(x[p2], -wv[1], l.y);
