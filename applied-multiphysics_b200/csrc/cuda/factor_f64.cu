@@ -20,6 +20,7 @@
 
 #include "devplan.cuh"
 #include "launch.hpp"
+#include "pivot_steps.cuh"
 #include "sync.cuh"
 #include "../host/plan.hpp"
 
@@ -320,63 +321,113 @@ __global__ void __launch_bounds__(128, ROWS == 128 ? 2 : 3)
 
 
 // Complex-symmetric update tiles (no conjugation): F[i0:i0+128, j0:j0+64] -= W B^T with W = L21 D (the A operand of
-// the LDL^T update) and B = L21, K = the task's pivot columns, on the CUDA cores (four FP64 products per complex
-// product). One CTA per tile: 256 threads as 32 (rows) x 8 (columns), 4 x 8 outputs each; K in chunks of 8 staged
-// in shared memory. Same tiles and masks as k_update.
-__global__ void __launch_bounds__(256) k_update_c(const TileTask *__restrict__ tasks, cplx *__restrict__ Lx,
+// the LDL^T update) and B = L21, K = the task's pivot columns, four FP64 tensor-core products (mma.sync m8n8k4) per complex
+// one. A task is split into TS x TS squares of its tile, one CTA of 4 warps (2 x 2, TS / 2 rows and columns each) per square;
+// the operands come through a ring of four cp.async stages of 16 pivot columns. What bounds it at the sizes of complex
+// systems is the latency of one square (the launches of a front's groups follow one another and have few tasks): 128 x 64
+// per CTA, 8 columns at a time copied and then multiplied, took 66 us per launch for the edge-element system with 10
+// elements per edge, now 15 us.
+constexpr int kCK = 16, kCStages = 4;
+template <int TS>
+constexpr int cupd_ld() { return TS + 2; }  // 2 mod 8 entries of 16 bytes: conflict-free fragment loads
+template <int TS>
+constexpr int cupd_smem() { return kCStages * 2 * kCK * cupd_ld<TS>() * (int)sizeof(cplx); }
+template <int TS>
+__global__ void __launch_bounds__(128) k_update_c(const TileTask *__restrict__ tasks, cplx *__restrict__ Lx,
                                                   cplx *__restrict__ U, const cplx *__restrict__ W,
                                                   const unsigned long long *status) {
+  constexpr int LD = cupd_ld<TS>(), PER = (kTileM / TS) * (kTile / TS), ROWS = kTileM / TS, MT = TS / 16;
+  extern __shared__ __align__(16) cplx cu_raw[];
+  const TileTask t = tasks[blockIdx.x / PER];
+  const int sub = blockIdx.x % PER, i0 = t.i0 + TS * (sub % ROWS), j0 = t.j0 + TS * (sub / ROWS);
+  const int m = t.m, nc = t.nc, jend = t.jend;
+  if (i0 >= m || j0 >= jend || i0 + TS <= j0) return;
   __shared__ int sOk;
-  if (threadIdx.x == 0) sOk = !failed(status);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
+  if (tid == 0) sOk = !failed(status);
+  const cplx *Ap = W + t.lp + (int64_t)t.c0 * m, *Bp = Lx + t.lp + (int64_t)t.c0 * m;
+  const int nchunk = (t.w + kCK - 1) / kCK;
+  auto stage = [&](int ch) {
+    cplx *As = cu_raw + (ch % kCStages) * 2 * kCK * LD, *Bs = As + kCK * LD;
+    if (ch < nchunk) {
+      const int i = tid & (TS - 1);
+#pragma unroll
+      for (int k = tid / TS; k < kCK; k += 128 / TS) {
+        const int c = ch * kCK + k;
+        const bool okA = c < t.w && i0 + i < m, okB = c < t.w && j0 + i < m;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
+                         (unsigned)__cvta_generic_to_shared(As + k * LD + i)),
+                     "l"(Ap + (okA ? (int64_t)c * m + i0 + i : 0)), "r"(okA ? 16 : 0)
+                     : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
+                         (unsigned)__cvta_generic_to_shared(Bs + k * LD + i)),
+                     "l"(Bp + (okB ? (int64_t)c * m + j0 + i : 0)), "r"(okB ? 16 : 0)
+                     : "memory");
+      }
+    }
+    cp_async_commit();
+  };
+  for (int ch = 0; ch < kCStages - 1; ch++) stage(ch);
   __syncthreads();
-  if (!sOk) return;
-  const TileTask t = tasks[blockIdx.x];
-  constexpr int KC = 8;
-  __shared__ cplx As[KC][kTileM], Bs[KC][kTile];
-  const int tid = threadIdx.x, tr = tid & 31, tc = tid >> 5;
-  const int m = t.m, nc = t.nc, mu = m - nc;
-  const cplx *Ap = W + t.lp, *Bp = Lx + t.lp;
-  cplx acc[4][8];
-#pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int b = 0; b < 8; b++) acc[a][b] = cplx(0.0);
-  for (int k0 = 0; k0 < t.w; k0 += KC) {
-    for (int e = tid; e < KC * kTileM; e += 256) {
-      const int k = e / kTileM, i = e % kTileM, r = t.i0 + i;
-      As[k][i] = (k0 + k < t.w && r < m) ? Ap[(int64_t)(t.c0 + k0 + k) * m + r] : cplx(0.0);
-    }
-    for (int e = tid; e < KC * kTile; e += 256) {
-      const int k = e / kTile, j = e % kTile, r = t.j0 + j;
-      Bs[k][j] = (k0 + k < t.w && r < m) ? Bp[(int64_t)(t.c0 + k0 + k) * m + r] : cplx(0.0);
-    }
-    __syncthreads();
-#pragma unroll 4
-    for (int k = 0; k < KC; k++) {
-      cplx av[4], bv[8];
-#pragma unroll
-      for (int a = 0; a < 4; a++) av[a] = As[k][tr + 32 * a];
-#pragma unroll
-      for (int b = 0; b < 8; b++) bv[b] = Bs[k][tc + 8 * b];
-#pragma unroll
-      for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 8; b++) acc[a][b] += av[a] * bv[b];
-    }
-    __syncthreads();
+  if (!sOk) {
+    cp_async_wait<0>();
+    return;
   }
+  const int wr = TS / 2 * (warp & 1), wc = TS / 2 * (warp >> 1);
+  double re[MT][MT][2], im[MT][MT][2];
+#pragma unroll
+  for (int a = 0; a < MT; a++)
+#pragma unroll
+    for (int b = 0; b < MT; b++) re[a][b][0] = re[a][b][1] = im[a][b][0] = im[a][b][1] = 0.0;
+  for (int ch = 0; ch < nchunk; ch++) {
+    cp_async_wait<kCStages - 2>();
+    __syncthreads();  // chunk ch has arrived, and everyone is done with chunk ch - 1
+    stage(ch + kCStages - 1);
+    const cplx *As = cu_raw + (ch % kCStages) * 2 * kCK * LD, *Bs = As + kCK * LD;
+#pragma unroll
+    for (int k = 0; k < kCK; k += 4) {
+      cplx av[MT], bv[MT];
+#pragma unroll
+      for (int a = 0; a < MT; a++) av[a] = As[(k + q) * LD + wr + 8 * a + g];
+#pragma unroll
+      for (int b = 0; b < MT; b++) bv[b] = Bs[(k + q) * LD + wc + 8 * b + g];
+#pragma unroll
+      for (int a = 0; a < MT; a++) {
+        const double ni = -av[a].im;
+#pragma unroll
+        for (int b = 0; b < MT; b++) mma884(re[a][b], av[a].re, bv[b].re);
+#pragma unroll
+        for (int b = 0; b < MT; b++) mma884(im[a][b], av[a].re, bv[b].im);
+#pragma unroll
+        for (int b = 0; b < MT; b++) mma884(re[a][b], ni, bv[b].im);
+#pragma unroll
+        for (int b = 0; b < MT; b++) mma884(im[a][b], av[a].im, bv[b].re);
+      }
+    }
+  }
+  cp_async_wait<0>();
   cplx *Lp = Lx + t.lp;
   cplx *Up = t.up >= 0 ? U + t.up : Lp;
 #pragma unroll
-  for (int a = 0; a < 4; a++)
+  for (int b = 0; b < MT; b++) {  // C -= the product, a column of squares' entries in flight together
+    cplx cv[MT][2];
 #pragma unroll
-    for (int b = 0; b < 8; b++) {
-      const int i = t.i0 + tr + 32 * a, j = t.j0 + tc + 8 * b;
-      if (i < m && j < t.jend && i >= j) {
-        cplx *c = j < nc ? Lp + (int64_t)j * m + i : Up + (int64_t)(j - nc) * mu + (i - nc);
-        *c = *c - acc[a][b];
+    for (int pass = 0; pass < 2; pass++)
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const int j = j0 + wc + 8 * b + 2 * q + u;
+        cplx *col = j < nc ? Lp + (int64_t)j * m : Up + (int64_t)(j - nc) * (m - nc) - nc;
+#pragma unroll
+        for (int a = 0; a < MT; a++) {
+          const int i = i0 + wr + 8 * a + g;
+          if (i >= m || i < j || j >= jend) continue;
+          if (pass == 0)
+            cv[a][u] = col[i];
+          else
+            col[i] = cplx(cv[a][u].re - re[a][b][u], cv[a][u].im - im[a][b][u]);
+        }
       }
-    }
+  }
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -422,6 +473,10 @@ cudaError_t init_kernel_attributes() {
     e = cudaFuncSetAttribute(k_update<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, upd_smem<128>());
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_update<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, upd_smem<64>());
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_update_c<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, cupd_smem<32>());
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_update_c<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, cupd_smem<64>());
   int dev = 0;
   if (e == cudaSuccess) e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
@@ -441,7 +496,13 @@ template void launch_assemble<cplx>(const AsmTask *, const ChildRange *, int64_t
                                     cplx *, cplx *, const unsigned long long *, cudaStream_t);
 void launch_update_c(const TileTask *tasks, int64_t ntasks, cplx *Lx, cplx *U, const cplx *W,
                      const unsigned long long *status, cudaStream_t st) {
-  if (ntasks > 0) k_update_c<<<(unsigned)ntasks, 256, 0, st>>>(tasks, Lx, U, W, status);
+  if (ntasks <= 0) return;
+  // squares of 32 while the tasks' squares of 64 are fewer than two per SM: a quarter of a square's latency, and four times
+  // the CTAs; beyond that squares of 64, which read each operand half as often
+  if (2 * ntasks <= 2 * g_num_sms)
+    k_update_c<32><<<(unsigned)(8 * ntasks), 128, cupd_smem<32>(), st>>>(tasks, Lx, U, W, status);
+  else
+    k_update_c<64><<<(unsigned)(2 * ntasks), 128, cupd_smem<64>(), st>>>(tasks, Lx, U, W, status);
 }
 void launch_ldlt_tau(const double *values, const DevPlan &P, double *scal, cudaStream_t st) {
   k_ldlt_tau<<<1, 1024, 0, st>>>(values, P.diagSlot, P.n, scal);
