@@ -515,7 +515,7 @@ __device__ __forceinline__ void front_warp_argmax(double &v, int &i) {
 }
 
 // The whole front with Bunch-Kaufman pivots inside each 64-column block of its pivot columns (AMP_LDLT_BK; the rule,
-// the 2 x 2 inverse and the outputs of bk_block in factor_f64.cu), FP64 arithmetic. At column k of block [c0, c1):
+// the 2 x 2 inverse and the outputs of bk_block in group_panel.cu), FP64 arithmetic. At column k of block [c0, c1):
 // colmax and rowmax over the block's rows only, computed by every warp with shuffles (the same values in the same
 // order, so every thread takes the same decision without sharing it); the interchange applied in lower storage to
 // the block's earlier columns (their rows) and to the whole trailing triangle (rows below the pivot columns
