@@ -72,6 +72,35 @@ __device__ __forceinline__ bool mx_wait(uint64_t *bar, uint32_t parity, MxShared
   return false;
 }
 
+// One row of a task's tile as an epilogue lane sees it
+struct MxRow {
+  float *row, *urow;  // entry (i, 0) of the front in L, and the place of column nc's entry in U less nc columns
+  int m, mu, nc, j0, jlo, jhi;  // columns [jlo, jhi) of the row are updated (none: jhi <= jlo)
+  __device__ __forceinline__ void set(const MixTask &tk, float *L32, float *U32, int r) {
+    const int i = tk.i0 + r;
+    m = tk.m;
+    nc = tk.nc;
+    mu = m - nc;
+    j0 = tk.j0;
+    jlo = tk.jlo;
+    jhi = i >= tk.ilo && i < m ? min(tk.jend, i + 1) : 0;
+    row = L32 + tk.lp + i;
+    urow = tk.up >= 0 ? U32 + tk.up + (i - nc) - (int64_t)nc * mu : row;
+  }
+  __device__ __forceinline__ float *at(int col) const {
+    const int j = j0 + col;
+    return j < nc ? row + (int64_t)j * m : urow + (int64_t)j * mu;
+  }
+  // the entries of columns [col0, col0 + 32) that are updated; returns their mask
+  __device__ __forceinline__ uint32_t load(int col0, float (&c)[32]) const {
+    const int a = max(jlo - j0 - col0, 0), b = min(jhi - j0 - col0, 32);
+    const uint32_t msk = b > a ? (0xffffffffu >> (32 - b)) & ~((1u << a) - 1) : 0u;
+#pragma unroll
+    for (int x = 0; x < 32; x++) c[x] = (msk >> x) & 1 ? *at(col0 + x) : 0.f;
+    return msk;
+  }
+};
+
 // N: tile columns, 256 (the general tiles), or 128 / 64 (the next group of the look-ahead when it is that wide)
 template <int N>
 __global__ void __launch_bounds__(kThreads, 1) k_update_mx(const MixTask *__restrict__ tasks, int ntasks,
@@ -182,44 +211,51 @@ __global__ void __launch_bounds__(kThreads, 1) k_update_mx(const MixTask *__rest
     __syncwarp();
   } else {  // ---- epilogue: quadrant q of the TMEM lanes (rows), column quarter h
     const int ew = warp - 2, q = warp & 3, h = ew >> 2;
+    constexpr int kChunks = kN / kEpiPerQuad / 32;
+    // One row of the front per lane, 32 columns at a time. The front's entries of the next 32 columns (the next tile's
+    // first ones after the last) are read before the accumulator's columns are waited for and stored: with reads that
+    // followed each accumulator, 32 KB per SM were in flight and the launches stayed at 4.7 TB/s.
+    MxRow cur;
+    float c[32];
+    uint32_t msk = 0;
+    if ((int)blockIdx.x < ntasks) {
+      cur.set(tasks[blockIdx.x], L32, U32, 32 * q + lane);
+      msk = cur.load(h * (kN / kEpiPerQuad), c);
+    }
     int tl = 0;
     for (int t = blockIdx.x; t < ntasks; t += gridDim.x, tl++) {
-      const MixTask tk = tasks[t];
       const int a = tl & 1;
       bool ok = true;
       if (lane == 0) ok = mx_wait(&sh.accFull[a], (tl >> 1) & 1, sh, status, spin);
       if (!__shfl_sync(0xffffffffu, ok ? 1 : 0, 0)) break;
       umma::tc_fence_after();
-      const int i = tk.i0 + 32 * q + lane, m = tk.m, nc = tk.nc, mu = m - nc;
-      const bool rowok = i >= tk.ilo && i < m;
-      float *Lp = L32 + tk.lp;
-      float *Up = tk.up >= 0 ? U32 + tk.up : Lp;
-      constexpr int kChunks = kN / kEpiPerQuad / 32;
 #pragma unroll 1
       for (int cc = 0; cc < kChunks; cc++) {
         const int col0 = h * (kN / kEpiPerQuad) + cc * 32;
+        const bool last = cc == kChunks - 1;
+        MxRow nxt = cur;
+        float cn[32];
+        uint32_t mskn = 0;
+        if (!last) {
+          mskn = nxt.load(col0 + 32, cn);
+        } else if (t + (int)gridDim.x < ntasks) {
+          nxt.set(tasks[t + gridDim.x], L32, U32, 32 * q + lane);
+          mskn = nxt.load(h * (kN / kEpiPerQuad), cn);
+        }
         float v[32];
         umma::tmem_ld32(tmem + a * kN + ((uint32_t)(32 * q) << 16) + col0, v);
-        if (cc == kChunks - 1) {  // accumulator fully read: hand it back to the MMA warp
+        if (last) {  // accumulator fully read: hand it back to the MMA warp
           umma::tc_fence_before();
           __syncwarp();
           if (lane == 0) umma::mbar_arrive(&sh.accEmpty[a]);
         }
-        if (!rowok) continue;
-        const int j0 = tk.j0 + col0;
-        const int jl = max(tk.jlo, j0), jh = min(min(tk.jend, i + 1), j0 + 32);  // columns of this row to update
-        if (jl >= jh) continue;
-        const uint32_t msk = (jh - j0 == 32 ? 0xffffffffu : ((1u << (jh - j0)) - 1)) & ~((1u << (jl - j0)) - 1);
-        auto addr = [&](int x) {
-          const int j = j0 + x;
-          return j < nc ? Lp + (int64_t)j * m + i : Up + (int64_t)(j - nc) * mu + (i - nc);
-        };
-        float c[32];
-#pragma unroll
-        for (int x = 0; x < 32; x++) c[x] = (msk >> x) & 1 ? *addr(x) : 0.f;
 #pragma unroll
         for (int x = 0; x < 32; x++)
-          if ((msk >> x) & 1) *addr(x) = c[x] - v[x];
+          if ((msk >> x) & 1) *cur.at(col0 + x) = c[x] - v[x];
+        cur = nxt;
+        msk = mskn;
+#pragma unroll
+        for (int x = 0; x < 32; x++) c[x] = cn[x];
       }
     }
   }
