@@ -33,6 +33,18 @@ namespace amp {
 
 constexpr int kSB = 64;  // solve block rows
 
+// Wait (a warp, bounded) until flag p[0] carries the epoch. The first poll also reads the flags p[step * lane], lane < n;
+// when p[0] is not set by then, lane 0 polls it alone (more polls slow the flags down for everyone). The mask of those
+// that carry the epoch, bit 0 among them; 0 on time-out (status set for s).
+__device__ __forceinline__ unsigned warp_flags(const int *p, int step, int n, int epoch, unsigned long long *status, int s,
+                                               long long limit) {
+  const int lane = threadIdx.x & 31;
+  unsigned mask = __ballot_sync(0xffffffffu, lane < n && ld_acquire(p + step * lane) == epoch);
+  if (!(mask & 1)) mask = __ballot_sync(0xffffffffu, lane == 0 && wait_flag(p, epoch, status, s, limit));
+  __syncwarp();  // orders the other lanes' later loads after each lane's acquire
+  return mask;
+}
+
 // ---- inverses of the diagonal blocks -----------------------------------------------------------------------------
 // One CTA per 64-column block b of the pivot columns (all supernodes): X = L_kk^-1, w x w column-major, lower part.
 // The block's lower triangle is staged in shared memory (coalesced column loads); then a group of 4 lanes computes
@@ -530,10 +542,18 @@ __global__ void __launch_bounds__(256, 3) k_bwd_blocks(const int4 *__restrict__ 
       const int fp = P.snF[par], ncp = P.snNc[par], nbp = (ncp + kSB - 1) / kSB;
       const int *pflags = flags + P.blkOff[par];
       int ready = nbp;  // the parent's blocks >= ready are known final (warp-uniform)
-      // the chunk's row indices and L values (static) are loaded one chunk ahead, so that a chunk waits for one load
-      // round trip (its x values) after its flag
+      // the chunk's L values (static) are loaded one chunk ahead, its row indices two, and its x values one chunk ahead
+      // when its rows are known final by then, so that a chunk of final rows waits for one round trip, that of L; the
+      // flags of up to 32 of the parent's blocks are read together
       int rb = nc + ((mu - 1) / 32) * 32;
       int idx = rb + lane < m ? rowsOf[rb + lane] : -1;
+      int idxn = rb - 32 >= nc ? rowsOf[rb - 32 + lane] : -1;
+      auto block_of = [&](int i) {  // of the chunk's first row, lane 0's (>= fp: every row below is one of the parent's front)
+        const int g0 = __shfl_sync(0xffffffffu, i, 0);
+        return g0 < fp + ncp ? max(0, g0 - fp) / kSB : nbp - 1;
+      };
+      double xr = 0.0;
+      bool have = false;  // xr holds the chunk's x values
       TL lc[8];
 #pragma unroll
       for (int u = 0; u < 8; u++) {
@@ -542,26 +562,32 @@ __global__ void __launch_bounds__(256, 3) k_bwd_blocks(const int4 *__restrict__ 
       }
       for (; rb >= nc; rb -= 32) {
         const int rbn = rb - 32;  // the next chunk (rows below rb, all < m)
-        const int idxn = rbn >= nc ? rowsOf[rbn + lane] : -1;
+        const int idx2 = rbn - 32 >= nc ? rowsOf[rbn - 32 + lane] : -1;
         TL ln[8];
 #pragma unroll
         for (int u = 0; u < 8; u++) {
           const int c = warp + 8 * u;
           ln[u] = (idxn >= 0 && c < w) ? Lp[(int64_t)(c0 + c) * m + rbn + lane] : (TL)0;
         }
-        // the chunk's first row, lane 0's (>= fp: every row below is a row of the parent's front)
-        const int g0 = __shfl_sync(0xffffffffu, idx, 0);
-        const int k = g0 < fp + ncp ? max(0, g0 - fp) / kSB : nbp - 1;
-        if (k < ready && wok) {
-          wok = warp_wait(pflags + k, epoch, true, status, s, P.spin);
-          ready = k;
+        if (!have) {
+          const int k = block_of(idx);
+          if (k < ready && wok) {
+            const unsigned mask = warp_flags(pflags + k, -1, k + 1, epoch, status, s, P.spin);
+            wok = mask != 0;
+            ready = k - (31 - __clz(mask | 1));  // a block's flag stands for the later ones too
+          }
+          if (idx >= 0 && wok) xr = __ldcg(y + idx);
         }
+        double xn = 0.0;
+        have = wok && rbn >= nc && block_of(idxn) >= ready;
+        if (have && idxn >= 0) xn = __ldcg(y + idxn);
         if (idx >= 0 && wok) {
-          const double xr = __ldcg(y + idx);
 #pragma unroll
           for (int u = 0; u < 8; u++) acc[u] += (double)lc[u] * xr;
         }
         idx = idxn;
+        idxn = idx2;
+        xr = xn;
 #pragma unroll
         for (int u = 0; u < 8; u++) lc[u] = ln[u];
       }
@@ -581,18 +607,35 @@ __global__ void __launch_bounds__(256, 3) k_bwd_blocks(const int4 *__restrict__ 
       }
     };
     load_block(nb - 1, lv);
+    int ready = nb;  // the blocks >= ready are known final (a block's flag stands for the later ones too)
+    double xr[2] = {0.0, 0.0};
+    bool have = false;  // xr holds block rb's values
     for (int rb = nb - 1; rb > rbLast; rb--) {
       TL ln[2][8];
       load_block(rb - 1, ln);
-      if (tid == 0) waitOk = wait_flag(myflags + rb, epoch, status, s, P.spin);
-      __syncthreads();
-      if (!waitOk) return false;  // block-uniform
+      if (rb < ready) {  // each warp by itself, the flags of up to 32 blocks together
+        const unsigned mask = warp_flags(myflags + rb, -1, rb - rbLast, epoch, status, s, P.spin);
+        wok = mask != 0;
+        if (!wok) break;
+        ready = rb - (31 - __clz(mask));
+      }
+      if (!have) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int r = rb * kSB + lane + 32 * h;
+          xr[h] = r < nc ? __ldcg(y + f + r) : 0.0;
+        }
+      }
+      have = rb - 1 > rbLast && rb - 1 >= ready;
+      double xn[2] = {0.0, 0.0};
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+        if (have) xn[h] = __ldcg(y + f + (rb - 1) * kSB + lane + 32 * h);
 #pragma unroll
       for (int h = 0; h < 2; h++) {
-        const int r = rb * kSB + lane + 32 * h;
-        const double xr = r < nc ? __ldcg(y + f + r) : 0.0;
 #pragma unroll
-        for (int u = 0; u < 8; u++) acc[u] += (double)lv[h][u] * xr;
+        for (int u = 0; u < 8; u++) acc[u] += (double)lv[h][u] * xr[h];
+        xr[h] = xn[h];
       }
 #pragma unroll
       for (int h = 0; h < 2; h++)
@@ -606,7 +649,7 @@ __global__ void __launch_bounds__(256, 3) k_bwd_blocks(const int4 *__restrict__ 
       for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
       if (lane == 0) red0[warp + 8 * u] = v;
     }
-    __syncthreads();
+    if (!__syncthreads_and(wok)) return false;  // block-uniform
     if (tid < kSB) {
       double yv = 0.0;  // LDL^T: y /= D before the backward sweep (ldlt.mjs:629)
       if (tid < w) yv = Dpiv ? y[f + c0 + tid] / Dpiv[f + c0 + tid] : y[f + c0 + tid];
