@@ -635,9 +635,7 @@ void device_solve_permuted(amp_factor *f) {
   const amp::DevPlan dp = solve_view(f);
   const double lbytes = (f->dL32 ? 4.0 : 8.0) * (double)P.nnzLStored;  // each sweep reads L once
   cudaStream_t st = f->stream;
-  ck(cudaMemsetAsync(f->dTickets, 0, sizeof(int) * 2, st), "memset tickets");
-  ck(cudaMemsetAsync(f->dDone, 0, sizeof(int) * std::max(1, P.nsuper), st), "memset done");
-  ck(cudaMemsetAsync(f->dSolveStatus, 0xff, sizeof(unsigned long long), st), "memset status");
+  amp::launch_sweep_begin(f->dSolveStatus, f->dTickets, f->dDone, P.nsuper, st);
   const int efwd = 2 * (++f->solveEpoch) - 1, ebwd = 2 * f->solveEpoch;
   const int nf = f->plan->nFwd1, nb = f->plan->nBwd1;
   const bool ldlt = f->kind == AMP_LDLT;
@@ -665,10 +663,11 @@ void device_solve_permuted(amp_factor *f) {
   });
 }
 
-// AMP_DEVICE_TIMEOUT when a bounded wait of the last solve gave up (the stream must be synchronised)
+// Waits for the factor's stream; AMP_DEVICE_TIMEOUT when a bounded wait of the last solve gave up
 int solve_status(amp_factor *f) {
   unsigned long long stw = 0;
-  ck(cudaMemcpy(&stw, f->dSolveStatus, sizeof stw, cudaMemcpyDeviceToHost), "copy solve status");
+  ck(cudaMemcpyAsync(&stw, f->dSolveStatus, sizeof stw, cudaMemcpyDeviceToHost, f->stream), "copy solve status");
+  ck(cudaStreamSynchronize(f->stream), "solve");
   if (stw != amp::kStatusOk) return fail(AMP_DEVICE_TIMEOUT, "solve: a device wait timed out");
   return AMP_OK;
 }
@@ -741,10 +740,8 @@ void device_solve_multi_permuted(amp_factor *f, int q) {
   const double lbytes = (f->dL32 ? 4.0 : 8.0) * (double)P.nnzLStored;  // each sweep reads L once for all q vectors
   const double flops = 2.0 * (double)P.nnzLStored * q;
   cudaStream_t st = f->stream;
-  ck(cudaMemsetAsync(f->dTickets, 0, sizeof(int) * 2, st), "memset tickets");
   const int nfl = std::max(1, P.nflags);
-  ck(cudaMemsetAsync(f->dDone, 0, sizeof(int) * kSlices * std::max(1, P.nsuper), st), "memset done");
-  ck(cudaMemsetAsync(f->dSolveStatus, 0xff, sizeof(unsigned long long), st), "memset status");
+  amp::launch_sweep_begin(f->dSolveStatus, f->dTickets, f->dDone, kSlices * P.nsuper, st);
   const int efwd = 2 * (++f->solveEpoch) - 1, ebwd = 2 * f->solveEpoch;
   const int ns = amp::multi_slices(q);
   slice_lists(f->plan, ns);
@@ -852,7 +849,6 @@ int solve_many(amp_factor *f, const double *b, int nrhs, double *x, bool on_devi
     }
   }
   ck(cudaGetLastError(), "kernel launch");
-  ck(cudaStreamSynchronize(st), "solve");
   if (int rc = solve_status(f)) return rc;
   if (stt) {
     stt->rel_residual = worst;
@@ -904,7 +900,6 @@ int device_shift_invert(amp_factor *f, const double *dX, int m, double *dY, doub
   ensure_solve_ws(f, 1);
   device_solve(f, dT, dY);
   ck(cudaGetLastError(), "kernel launch");
-  ck(cudaStreamSynchronize(st), "shift-invert");
   return solve_status(f);
 }
 
@@ -1499,7 +1494,6 @@ int amp_solve(amp_factor *f, const double *b, int32_t nrhs, double *x, int on_de
     device_solve(f, dB, dX);
     ck(cudaGetLastError(), "kernel launch");
     if (!on_device) ck(cudaMemcpyAsync(x, dX, bytes, cudaMemcpyDeviceToHost, f->stream), "copy x");
-    ck(cudaStreamSynchronize(f->stream), "solve");
     return solve_status(f);
   });
 }
@@ -1562,7 +1556,6 @@ int amp_solve_refined(amp_factor *f, const double *b, int32_t nrhs, double *x, i
     }
     ck(cudaGetLastError(), "kernel launch");
     if (!on_device) ck(cudaMemcpyAsync(x, dX, bytes, cudaMemcpyDeviceToHost, st), "copy x");
-    ck(cudaStreamSynchronize(st), "refine");
     if (int rc = solve_status(f)) return rc;
     stt.rel_residual = worst;
     stt.steps = steps;
@@ -1727,7 +1720,6 @@ int amp_solve_gmres(amp_factor *f, const double *b, double *x, int on_device, co
     res.converged = res.rel_residual <= std::max(o.tol * 10, 1e-14);
     ck(cudaMemcpyAsync(x, xb, sizeof(double) * n, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, st),
        "copy x");
-    ck(cudaStreamSynchronize(st), "gmres");
     if (int rc = solve_status(f)) return rc;
     if (stats) *stats = res;
     return (int)AMP_OK;

@@ -50,6 +50,8 @@ void launch_update_mx(const MixTask *tasks, int64_t ntasks, const CUtensorMap *m
 int num_sms();
 void launch_update(const TileTask *tasks, int64_t ntasks, const DevPlan &P, double *Lx, double *U, const double *W,
                    const unsigned long long *status, cudaStream_t st);
+// before a pair of sweeps: the status word, the two tickets, the done counts of nsuper supernodes (per slice)
+void launch_sweep_begin(unsigned long long *status, int *tickets, int *done, int nsuper, cudaStream_t st);
 void launch_permute_in(const double *b, double *y, const int *perm, int n, int q, cudaStream_t st);
 void launch_permute_out(const double *y, double *x, const int *perm, int n, int q, cudaStream_t st);
 // inverses of the diagonal blocks (with each block's pivot order folded in when P.lpiv is set)

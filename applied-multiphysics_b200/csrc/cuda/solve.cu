@@ -184,6 +184,17 @@ __global__ void __launch_bounds__(256) k_chain_mats(const int2 *__restrict__ tas
   }
 }
 
+__global__ void k_sweep_begin(unsigned long long *status, int *tickets, int *done, int nsuper) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < nsuper) done[i] = 0;
+  if (i < 2) tickets[i] = 0;
+  if (i == 0) *status = kStatusOk;
+}
+// one launch where three fills would follow one another, some 2 us each on the stream of a solve
+void launch_sweep_begin(unsigned long long *status, int *tickets, int *done, int nsuper, cudaStream_t st) {
+  k_sweep_begin<<<nsuper / 256 + 1, 256, 0, st>>>(status, tickets, done, nsuper);
+}
+
 // ---- forward block tasks -----------------------------------------------------------------------------------------
 constexpr int kChPre = 64;  // children located and waited for at once by a forward block task
 // task: .x supernode, .y block, .z kind (0 diagonal, 1 below, 2 small supernodes, 3 whole supernode: one-vector list)
