@@ -458,17 +458,20 @@ template <class T>
 struct SmallFork {
   amp_factor *f;
   bool used = false;
-  void launch(int L, T *Lx, T *U, const amp::LdltArgs<T> &la) {
+  // alone: the stream's last work is the small fronts of the level below (then this level's may start before they have
+  // ended, if they are alone too); returns the same for this level
+  bool launch(int L, T *Lx, T *U, const amp::LdltArgs<T> &la, bool alone) {
     const amp::Plan &P = f->plan->P;
     const int64_t t0 = P.tinyPtr[L], t1 = P.tinyPtr[L + 1], s0 = P.smallPtr[L], s1 = P.smallPtr[L + 1];
     const int64_t sm = P.smallMid[L];
     const bool large = P.asmLvlPtr[L + 1] > P.asmLvlPtr[L];
-    if (t1 == t0 && s1 == s0) return;
+    if (t1 == t0 && s1 == s0) return false;
     const int *small = f->plan->dSmallSn;
     const amp::SmallClass none{nullptr, 0, 0, 0};
     const amp::SmallClass half{small + s0, (int)(sm - s0), P.smallMaxM[2 * L], P.smallMaxNc[2 * L]};
     const amp::SmallClass full{small + sm, (int)(s1 - sm), P.smallMaxM[2 * L + 1], P.smallMaxNc[2 * L + 1]};
     used = large || (t1 > t0 && s1 > s0);
+    const bool after = alone && !used;
     if (used) {
       ck(cudaEventRecord(f->evFork, f->stream), "event");
       ck(cudaStreamWaitEvent(f->side, f->evFork, 0), "wait");
@@ -481,9 +484,10 @@ struct SmallFork {
     };
     if (t1 > t0)
       run(used ? f->side : f->stream,
-          {f->plan->dTinySn + t0, (int)(t1 - t0), (int)(P.tinyMid[L] - t0), none, none}, (double)(t1 - t0));
-    if (s1 > s0) run(large ? f->side : f->stream, {nullptr, 0, 0, half, full}, (double)(s1 - s0));
+          {f->plan->dTinySn + t0, (int)(t1 - t0), (int)(P.tinyMid[L] - t0), none, none, after}, (double)(t1 - t0));
+    if (s1 > s0) run(large ? f->side : f->stream, {nullptr, 0, 0, half, full, after}, (double)(s1 - s0));
     if (used) ck(cudaEventRecord(f->evFront, f->side), "event");
+    return !used;
   }
   void join() {
     if (used) ck(cudaStreamWaitEvent(f->stream, f->evFront, 0), "wait");
@@ -518,9 +522,10 @@ void enqueue_factor(amp_factor *f) {
       ck(cudaMemsetAsync(f->dCounts, 0, 2 * sizeof(int), st), "memset counts");
       amp::launch_ldlt_tau(f->dValues, dp, f->dScal, st);
     }
+    bool alone = false;  // (SmallFork::launch)
     for (int L = 0; L < P.nlevels; L++) {
       SmallFork<float> small{f};
-      small.launch(L, f->dL32, f->dU32, ld32);
+      alone = small.launch(L, f->dL32, f->dU32, ld32, alone);
       if (P.asmLvlPtr[L + 1] > P.asmLvlPtr[L])
         timed(f, K_ASSEMBLE, 0.0, P.asmLvlBytes[L] / 2, [&] {
           amp::launch_assemble<float>(f->plan->dAsm + P.asmLvlPtr[L], f->plan->dAsmCh, P.asmLvlPtr[L + 1] - P.asmLvlPtr[L], dp,
@@ -576,9 +581,10 @@ void enqueue_factor(amp_factor *f) {
     ck(cudaMemsetAsync(f->dCounts, 0, 2 * sizeof(int), st), "memset counts");
     amp::launch_ldlt_tau(f->dValues, dp, f->dScal, st);
   }
+  bool alone = false;  // (SmallFork::launch)
   for (int L = 0; L < P.nlevels; L++) {
     SmallFork<double> small{f};
-    small.launch(L, f->dLx, f->dU, ld);
+    alone = small.launch(L, f->dLx, f->dU, ld, alone);
     if (P.asmLvlPtr[L + 1] > P.asmLvlPtr[L])
       timed(f, K_ASSEMBLE, 0.0, P.asmLvlBytes[L], [&] {
         amp::launch_assemble<double>(f->plan->dAsm + P.asmLvlPtr[L], f->plan->dAsmCh, P.asmLvlPtr[L + 1] - P.asmLvlPtr[L], dp,

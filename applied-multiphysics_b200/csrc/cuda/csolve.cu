@@ -26,6 +26,7 @@
 #include "cplx.cuh"
 #include "devplan.cuh"
 #include "launch.hpp"
+#include "sync.cuh"
 
 namespace amp {
 
@@ -106,10 +107,6 @@ __device__ __forceinline__ cplx cluster_ld(const cplx *p, int k) {
   asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.re), "=d"(v.im) : "r"(a) : "memory");
   return v;
 }
-// programmatic dependent launch: the launch before this one has ended and its writes are visible; the next may start
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 constexpr int kCB = 64;  // columns of a block
 
 // the strictly lower part of a block's pivot triangle (columns [p0, p0 + w)) to T[c * ld + r]

@@ -21,6 +21,7 @@
 #include "devplan.cuh"
 #include "launch.hpp"
 #include "pivot_steps.cuh"
+#include "sync.cuh"
 
 namespace amp {
 
@@ -91,6 +92,7 @@ __device__ void assemble_warp(int s, const DevPlan &P, const double *__restrict_
   __syncwarp();
   // A's entries of all nc pivot columns (one contiguous CSR range): slot dst = j m + i of the L panel, each (i, j) once
   for (int p = p0 + lane; p < p1; p += 32) F[P.asmDst[p]] += (TC)(T)__ldg(values + P.asmSrc[p]);
+  pdl_wait();  // the children's level
   for (int qb = 0; qb < nch; qb += 32) {  // the metadata of up to 32 children, one per lane
     const int nq = min(32, nch - qb);
     int muc = 0;
@@ -156,6 +158,7 @@ __device__ void assemble_cta(int s, const DevPlan &P, const double *__restrict__
   for (int e = t; e < m * m; e += NT) F[e] = TC(0);
   __syncthreads();
   for (int p = p0 + t; p < p1; p += NT) F[P.asmDst[p]] += (TC)(T)__ldg(values + P.asmSrc[p]);
+  pdl_wait();  // the children's level
   for (int qb = 0; qb < nch; qb += kChildChunk) {
     const int nq = min(kChildChunk, nch - qb);
     if (qb > 0) {
@@ -227,6 +230,7 @@ __device__ void factor_front_warp(int s, const DevPlan &P, const double *__restr
   const bool ldlt = la.scal != nullptr;
   const TC tau = ldlt ? (TC)(T)la.scal[1] : TC(0);
   assemble_warp<T, TC, tiny_batch<MAXM>()>(s, P, values, U, F, lane);
+  if (status_failed(status)) return;
   int neg = 0, pert = 0;  // lane 0
   T *Lp = Lx + P.snLxp[s];
   for (int k = 0; k < nc; k++) {
@@ -307,7 +311,7 @@ __global__ void __launch_bounds__(small_threads<MAXM>(), MAXM == 64 ? 2 : 1)
   __shared__ ChildMeta cm;
   __shared__ double scale[MAXM], diag[MAXM];
   __shared__ int failAt, inexact, nNeg, nPert;
-  if (status_failed(status)) return;
+  pdl_next();
   const int s = fronts[blockIdx.x];
   const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s], mu = m - nc;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
@@ -317,6 +321,7 @@ __global__ void __launch_bounds__(small_threads<MAXM>(), MAXM == 64 ? 2 : 1)
   T *Up = U + (mu > 0 ? P.snUoff[s] : 0);
   const TC tau = LDLT ? (TC)(T)la.scal[1] : TC(0);
   assemble_cta<T, TC, NT>(s, P, values, U, F, &cm);
+  if (status_failed(status)) return;
   // the front's tiles: row group rg[h], tile column cb
   const int rg[2] = {warp, NG == 2 ? 15 - warp : -1};
   auto tile = [&](int rb, int cb, TC(&c)[2]) {
@@ -536,6 +541,7 @@ __device__ void factor_front_bk(int s, const DevPlan &P, const double *__restric
     assemble_warp<T, double, 16>(s, P, values, U, F, t);
   else
     assemble_cta<T, double, G>(s, P, values, U, F, cm);
+  if (status_failed(status)) return;
   auto at = [&](int i, int j) -> double & { return F[j * m + i]; };  // entry (i, j), i >= j
   int neg = 0, pert = 0;  // thread 0
   int perm[64];           // thread 0: the current block's pivot order
@@ -687,7 +693,7 @@ __global__ void __launch_bounds__(32 * tiny_warps<MAXM>(), BK ? 1 : tiny_ctas<MA
                                                                          unsigned long long *status, LdltArgs<T> la) {
   constexpr int W = tiny_warps<MAXM>();
   __shared__ TC F[W][MAXM * MAXM];
-  if (status_failed(status)) return;
+  pdl_next();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int idx = blockIdx.x * W + warp;
   if (idx >= count) return;  // warp-uniform; no CTA-wide barrier follows
@@ -704,7 +710,7 @@ __global__ void __launch_bounds__(256) k_front_small_bk(const int *__restrict__ 
                                                         T *__restrict__ U, unsigned long long *status, LdltArgs<T> la) {
   extern __shared__ __align__(16) unsigned char fs_dyn[];
   __shared__ ChildMeta cm;
-  if (status_failed(status)) return;
+  pdl_next();
   factor_front_bk<T, 256>(fronts[blockIdx.x], P, values, Lx, U, reinterpret_cast<double *>(fs_dyn), status, la,
                           threadIdx.x, &cm);
 }
@@ -729,23 +735,40 @@ cudaError_t init_front_small_attributes() {
   return e;
 }
 
+// after: the launch before it on the stream is the one of the level below, alone (SmallFronts): it then starts before that
+// one has ended, and assembles A's entries meanwhile
+template <class... KA, class... A>
+static void launch_level(void (*kernel)(KA...), bool after, int grid, int threads, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3((unsigned)grid);
+  c.blockDim = dim3((unsigned)threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = after ? 1 : 0;
+  cudaLaunchKernelEx(&c, kernel, KA(args)...);
+}
+
 template <class T, class TC, int MAXM, bool BK>
-static int launch_tiny(const int *fronts, int count, const DevPlan &P, const double *values, T *Lx, T *U,
+static int launch_tiny(bool after, const int *fronts, int count, const DevPlan &P, const double *values, T *Lx, T *U,
                        unsigned long long *status, const LdltArgs<T> &la, cudaStream_t st) {
   constexpr int W = tiny_warps<MAXM>();
   if (count <= 0) return 0;
-  k_front_tiny<T, TC, MAXM, BK><<<(count + W - 1) / W, 32 * W, 0, st>>>(fronts, count, P, values, Lx, U, status,
-                                                                        la);
+  launch_level(k_front_tiny<T, TC, MAXM, BK>, after, (count + W - 1) / W, 32 * W, 0, st, fronts, count, P, values, Lx, U, status,
+               la);
   return 1;
 }
 
 template <class T, class TC, bool LDLT, int MAXM>
-static int launch_small(const SmallClass &c, const DevPlan &P, const double *values, T *Lx, T *U,
+static int launch_small(bool after, const SmallClass &c, const DevPlan &P, const double *values, T *Lx, T *U,
                         unsigned long long *status, const LdltArgs<T> &la, cudaStream_t st) {
   if (c.count <= 0) return 0;
-  k_front_small<T, TC, LDLT, MAXM>
-      <<<c.count, small_threads<MAXM>(), small_elems<TC>(c.maxM, c.maxNc) * sizeof(TC), st>>>(
-          c.sn, small_main<TC>(c.maxM, c.maxNc), P, values, Lx, U, status, la);
+  launch_level(k_front_small<T, TC, LDLT, MAXM>, after, c.count, small_threads<MAXM>(),
+               small_elems<TC>(c.maxM, c.maxNc) * sizeof(TC), st, c.sn, small_main<TC>(c.maxM, c.maxNc), P, values, Lx, U,
+               status, la);
   return 1;
 }
 template <class T, class TC, bool LDLT, bool BK>
@@ -759,18 +782,18 @@ static int launch_fronts_tc(const SmallFronts &fr, const DevPlan &P, const doubl
     full = SmallClass{half.sn, half.count + full.count, full.maxM, std::max(half.maxNc, full.maxNc)};
     half.count = 0;
   }
-  int k = launch_tiny<T, TC, kTinyMid, BK>(fr.tiny, mid, P, values, Lx, U, status, la, st);
-  k += launch_tiny<T, TC, kTinyFront, BK>(fr.tiny + mid, fr.ntiny - mid, P, values, Lx, U, status, la, st);
+  int k = launch_tiny<T, TC, kTinyMid, BK>(fr.after, fr.tiny, mid, P, values, Lx, U, status, la, st);
+  k += launch_tiny<T, TC, kTinyFront, BK>(fr.after, fr.tiny + mid, fr.ntiny - mid, P, values, Lx, U, status, la, st);
   if constexpr (BK) {
     for (const SmallClass &c : {half, full})
       if (c.count > 0) {
-        k_front_small_bk<T><<<c.count, 256, (size_t)c.maxM * c.maxM * sizeof(TC), st>>>(c.sn, P, values, Lx, U, status,
-                                                                                        la);
+        launch_level(k_front_small_bk<T>, fr.after, c.count, 256, (size_t)c.maxM * c.maxM * sizeof(TC), st, c.sn, P, values,
+                     Lx, U, status, la);
         k++;
       }
   } else {
-    k += launch_small<T, TC, LDLT, 64>(half, P, values, Lx, U, status, la, st);
-    k += launch_small<T, TC, LDLT, 128>(full, P, values, Lx, U, status, la, st);
+    k += launch_small<T, TC, LDLT, 64>(fr.after, half, P, values, Lx, U, status, la, st);
+    k += launch_small<T, TC, LDLT, 128>(fr.after, full, P, values, Lx, U, status, la, st);
   }
   return k;
 }

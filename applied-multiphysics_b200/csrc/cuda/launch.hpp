@@ -39,6 +39,7 @@ struct SmallFronts {
   const int *tiny;
   int ntiny, ntinyMid;
   SmallClass half, full;
+  bool after;  // the stream's last launch is one of the level below, and no other stream holds any: start before it ends
 };
 template <class T>
 int launch_fronts_small(const SmallFronts &fr, const DevPlan &P, const double *values, T *Lx, T *U,

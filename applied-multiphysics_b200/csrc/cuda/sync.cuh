@@ -22,6 +22,10 @@ __device__ __forceinline__ void red_release_add(int *p, int v) {
   asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// programmatic dependent launch: the launch before this one has ended and its writes are visible; the next may start
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Tagged words: the high 32 bits carry the sweep's epoch, the low 32 bits half of a double. A strong 8-byte store is
 // seen whole, so a reader that finds its epoch in the tag holds the value without a separate flag round trip.
 __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long *p) {
