@@ -67,12 +67,19 @@ __device__ __forceinline__ bool failed(const unsigned long long *st) {
 // Assembly + extend-add
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int kAsmChildren = 64;  // children whose column ranges an assembly CTA stages in shared memory up front
-constexpr int kAsmInFlight = 4;   // extend-add entries per lane in flight
+// extend-add entries per lane and read-modify-write step; as many are read ahead
+template <class T>
+constexpr int asm_step() { return sizeof(T) == 4 ? 8 : 4; }
 
+// What bounds it is memory latency: an entry's map and value, then the front's entry behind the map. With four entries per
+// lane and nothing read ahead the large fronts' children came in at 2.4 TB/s; now the next entries (eight FP32, four
+// wider) are read while the current ones are added, four CTAs per SM (64 registers; with three or five the launches are
+// slower). 40^3 elasticity, FP32 fronts: 3.29 -> 2.73 ms (3 CTAs 3.05, 5 CTAs 3.33), FP64 4.59 -> 4.29; quadratic heat
+// with 32 elements per edge 4.38 -> 3.53 ms.
 // ranges[t.ch0 + q]: the columns of child q's update matrix that map into the task's front columns (computed with
 // the schedule, so a CTA starts without searching the children's maps)
 template <class T>
-__global__ void __launch_bounds__(256) k_assemble(const AsmTask *__restrict__ tasks, const ChildRange *__restrict__ ranges,
+__global__ void __launch_bounds__(256, 4) k_assemble(const AsmTask *__restrict__ tasks, const ChildRange *__restrict__ ranges,
                                                   DevPlan P, const value_of<T> *__restrict__ values, T *__restrict__ Lx,
                                                   T *__restrict__ U, const unsigned long long *status) {
   if (failed(status)) return;
@@ -115,6 +122,7 @@ __global__ void __launch_bounds__(256) k_assemble(const AsmTask *__restrict__ ta
   }
   __syncthreads();
   // 3. children, one after another (stack order of the reference)
+  constexpr int N = asm_step<T>();
   for (int q = 0; q < nch; q++) {
     const int c = P.chList[q0 + q];
     const int muc = P.snM[c] - P.snNc[c];
@@ -125,21 +133,31 @@ __global__ void __launch_bounds__(256) k_assemble(const AsmTask *__restrict__ ta
     for (int b = br.b0 + warp; b < br.b1; b += nwarps) {
       const int jj = map[b];
       const T *col = Uc + (int64_t)b * muc;
-      // kAsmInFlight entries per lane in flight: gather the child's values and target rows, then read-modify-write
-      for (int a = b + lane; a < muc; a += 32 * kAsmInFlight) {
-        T v[kAsmInFlight], cur[kAsmInFlight];
-        T *dst[kAsmInFlight];
+      T *to = jj < nc ? Lp + (int64_t)jj * m : Up + (int64_t)(jj - nc) * (m - nc) - nc;  // row i of front column jj
+      int dst[N], dn[N];
+      T v[N], vn[N];
+      auto fetch = [&](int a, int(&d)[N], T(&x)[N]) {
 #pragma unroll
-        for (int u = 0; u < kAsmInFlight; u++) {
+        for (int u = 0; u < N; u++) {
           const int aa = a + 32 * u;
-          dst[u] = aa < muc ? front_addr(Lp, Up, m, nc, __ldg(map + aa), jj) : nullptr;
-          v[u] = aa < muc ? col[aa] : T(0);
+          d[u] = aa < muc ? __ldg(map + aa) : -1;
+          x[u] = aa < muc ? col[aa] : T(0);
         }
+      };
+      fetch(b + lane, dst, v);
+      for (int a = b + lane; a - lane < muc; a += 32 * N) {
+        fetch(a + 32 * N, dn, vn);
+        T cur[N];
 #pragma unroll
-        for (int u = 0; u < kAsmInFlight; u++) cur[u] = dst[u] ? *dst[u] : T(0);
+        for (int u = 0; u < N; u++) cur[u] = dst[u] >= 0 ? to[dst[u]] : T(0);
 #pragma unroll
-        for (int u = 0; u < kAsmInFlight; u++)
-          if (dst[u]) *dst[u] = cur[u] + v[u];
+        for (int u = 0; u < N; u++)
+          if (dst[u] >= 0) to[dst[u]] = cur[u] + v[u];
+#pragma unroll
+        for (int u = 0; u < N; u++) {
+          dst[u] = dn[u];
+          v[u] = vn[u];
+        }
       }
     }
     __syncthreads();
