@@ -488,6 +488,8 @@ static int g_num_sms = 148;
 
 cudaError_t init_group_panel_attributes();
 cudaError_t init_cgroup_panel_attributes();
+cudaError_t init_group_panel_f32_attributes();
+cudaError_t init_front_small_f32_attributes();
 cudaError_t init_mixed_attributes();
 cudaError_t init_solve_attributes();
 cudaError_t init_solve_multi_attributes();
@@ -496,6 +498,8 @@ cudaError_t init_kernel_attributes() {
   // function attributes belong to the current device's context: the caller runs this once per device
   cudaError_t e = init_group_panel_attributes();
   if (e == cudaSuccess) e = init_cgroup_panel_attributes();
+  if (e == cudaSuccess) e = init_group_panel_f32_attributes();
+  if (e == cudaSuccess) e = init_front_small_f32_attributes();
   if (e == cudaSuccess) e = init_mixed_attributes();
   if (e == cudaSuccess) e = init_solve_attributes();
   if (e == cudaSuccess) e = init_solve_multi_attributes();

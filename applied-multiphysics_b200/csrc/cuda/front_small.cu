@@ -727,8 +727,6 @@ static cudaError_t init_small() {
 cudaError_t init_front_small_attributes() {
   cudaError_t e = init_small<double, double, false>();
   if (e == cudaSuccess) e = init_small<double, double, true>();
-  if (e == cudaSuccess) e = init_small<float, float, false>();
-  if (e == cudaSuccess) e = init_small<float, double, true>();
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_front_small_bk<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              kSmallFront * kSmallFront * (int)sizeof(double));
@@ -809,7 +807,5 @@ int launch_fronts_small(const SmallFronts &fr, const DevPlan &P, const double *v
 }
 template int launch_fronts_small<double>(const SmallFronts &, const DevPlan &, const double *, double *, double *,
                                          unsigned long long *, const LdltArgs<double> &, cudaStream_t);
-template int launch_fronts_small<float>(const SmallFronts &, const DevPlan &, const double *, float *, float *,
-                                        unsigned long long *, const LdltArgs<float> &, cudaStream_t);
 
 }  // namespace amp

@@ -1,14 +1,13 @@
-// Group panel of the real factors (FP64, or FP32 storage for the mixed-precision path; Cholesky, LDL^T with static pivot
-// perturbation, LDL^T with Bunch-Kaufman pivots inside each pivot block): the pivot blocks of a group of 64-column
-// blocks of a front factored in one dataflow launch -- POTRF of each pivot block, TRSM of the rows below it, and the
-// update of the group's remaining columns. All arithmetic is FP64, its products on the FP64 tensor cores
-// (mma.sync m8n8k4); an FP32 factor rounds once, when an entry is stored.
+// Group panel of the FP64 factors (the FP32 ones': group_panel_f32.cu; Cholesky, LDL^T with static pivot perturbation,
+// LDL^T with Bunch-Kaufman pivots inside each pivot block): the pivot blocks of a group of 64-column blocks of a front
+// factored in one dataflow launch -- POTRF of each pivot block, TRSM of the rows below it, and the update of the group's
+// remaining columns. The products run on the FP64 tensor cores (mma.sync m8n8k4).
 //
 // What bounds it: the chain through the pivot blocks of the large fronts (POTRF of block b, then block b + 1's rows
 // against it, then their update and POTRF), one CTA at a time, so a block's latency is what counts: per block POTRF
 // 11,100 clocks, the flag and the loads behind it 3,400, TRSM 2,500, the block's own update 1,600 (FP64; 33,700 / - /
 // 10,400 / 7,100 with FMA tiles and a four-thread substitution per row). A 4,096-row front's group of two blocks takes
-// 32 us (66 before) in FP64 and 32 us (39) in FP32, eight of them at once 63 us (110) and 65 us (74). The split: warp w
+// 32 us (66 before), eight of them at once 63 us (110). The split: warp w
 // of a strip owns 8 rows (row group rg(w)) of every 64 x 64 product, so a strip's TRSM runs inside each warp without a
 // barrier -- the C fragment of a solved 8 x 8 tile is the A fragment of the next product (its two registers are the k
 // indices 2 t and 2 t + 1, and the B fragment takes the same pair with one 16-byte load).
@@ -46,8 +45,8 @@ __device__ __forceinline__ void load_block(double *S, const T *L, int m, int i0,
   }
 }
 
-// Pivot block: POTRF (or LDL^T) of the 64 x 64 diagonal block of a front, called by all 256 threads of a CTA, in TC
-// (FP64, or FP32 for the FP32 Cholesky factor, as the whole-front kernels). Ds: the updated block (lower part; identity from column w on), left unchanged; Lp: the block's
+// Pivot block: POTRF (or LDL^T) of the 64 x 64 diagonal block of a front, called by all 256 threads of a CTA, in TC.
+// Ds: the updated block (lower part; identity from column w on), left unchanged; Lp: the block's
 // (0, 0) entry in the front (ld m), where the factor is written; w <= 64 its columns; scr: 11 step buffers; Linv:
 // the inverses of the eight 8 x 8 diagonal blocks of L (64 doubles each, row-major), for the strips' TRSM.
 // Right-looking on the unscaled columns in steps of eight. Step k: (1) the first two warps, one row per lane, factor the
@@ -57,8 +56,8 @@ __device__ __forceinline__ void load_block(double *S, const T *L, int m, int i0,
 // they update the rest of the triangle while the first two warps go on with step k + 1. The chain per column is one
 // reciprocal (the hardware estimate and three dependent products) and two products, 58 clocks (FP64); a step's FP64
 // issue in a panel warp takes 790 clocks alone and 1,050-1,200 beside the trailing products. The pivots are tested, the
-// columns scaled and everything written after the last step. A block takes 11,100 clocks in FP64 and 9,100 in FP32
-// (33,700 and 13,000 with 4 x 4 register tiles, a diagonal thread per step and two barriers per four columns).
+// columns scaled and everything written after the last step. A block takes 11,100 clocks
+// (33,700 with 4 x 4 register tiles, a diagonal thread per step and two barriers per four columns).
 // Cholesky tests d > 0 (sparse.mjs:1151-1156); LDL^T (ldlt.mjs:450-562) perturbs |d| < tau to +-tau by the sign of d (a
 // non-finite small pivot fails) and counts negative and perturbed pivots. Cholesky L = a / sqrt(d) with sqrt(d) on the
 // diagonal, LDL^T L = a / d with a unit diagonal (D to ld.D). Returns 0, or 1 (status set for the first failing column
@@ -469,7 +468,6 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
                                                         const StripTask *__restrict__ strips, int nstrips, int *ticket,
                                                         int *flags, DevPlan P, T *__restrict__ Lx,
                                                         double *__restrict__ Linv, unsigned long long *status,
-                                                        __nv_bfloat16 *__restrict__ Shi, __nv_bfloat16 *__restrict__ Slo,
                                                         LdltArgs<T> ld) {
   extern __shared__ __align__(16) unsigned char gp_raw[];
   double *Ls = reinterpret_cast<double *>(gp_raw);  // pivot block, rows of another diagonal strip, POTRF step buffers
@@ -491,13 +489,12 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
   const int nb = (g1 - g0 + kPanel - 1) / kPanel;
   const int r0 = st.r0, r1 = st.r1, jd = st.diag;
   const int bmax = jd >= 0 ? jd : nb;  // pivot blocks whose rows below include this strip
-  const int64_t lxp = P.snLxp[s], sp = P.snSp[s];
+  const int64_t lxp = P.snLxp[s];
   T *L = Lx + lxp;
   int *Pf = flags + it.flag0, *Df = Pf + nb;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int lr = 8 * row_group(warp) + g, row = r0 + lr;  // this lane's row of every fragment
   const bool act = row < r1;
-  const int ld8 = (m + 7) & ~7;
   if (jd >= 0) load_block(Ds, L, m, r0, r1 - r0, r0, r1 - r0, true, true);
   double nx[8][2];  // -W of the block solved last
 #pragma unroll
@@ -632,19 +629,6 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
         const int64_t at = (int64_t)(c0 + cc) * m + r0 + r;
         L[at] = (T)xv;
         if (LDLT && !BK && ld.W) ld.W[lxp + at] = (T)(xv * dv[cc]);
-        if constexpr (std::is_same<T, float>::value) {  // the BF16 hi / lo pairs of the tensor-core update's operands
-          const int64_t as = sp + (int64_t)(c0 + cc) * ld8 + r0 + r;
-          const float xt = (float)xv;
-          const __nv_bfloat16 hi = __float2bfloat16_rn(xt);
-          Shi[as] = hi;
-          Slo[as] = __float2bfloat16_rn(xt - __bfloat162float(hi));
-          if (LDLT) {
-            const float wt = (float)(xv * dv[cc]);
-            const __nv_bfloat16 whi = __float2bfloat16_rn(wt);
-            ld.Whi[as] = whi;
-            ld.Wlo[as] = __float2bfloat16_rn(wt - __bfloat162float(whi));
-          }
-        }
       }
     }
     if (jd < 0) continue;
@@ -701,19 +685,16 @@ cudaError_t init_group_panel_attributes() {
   cudaError_t e = init_one<double, false, false>();
   if (e == cudaSuccess) e = init_one<double, true, false>();
   if (e == cudaSuccess) e = init_one<double, true, true>();
-  if (e == cudaSuccess) e = init_one<float, false, false>();
-  if (e == cudaSuccess) e = init_one<float, true, false>();
   return e;
 }
 
 template <class T>
 void launch_group_panel(const GroupItem *items, const StripTask *strips, int nstrips, int *ticket, int *flags,
-                        const DevPlan &P, T *Lx, double *Linv, unsigned long long *status, __nv_bfloat16 *Shi,
-                        __nv_bfloat16 *Slo, const LdltArgs<T> &ld, cudaStream_t st) {
+                        const DevPlan &P, T *Lx, double *Linv, unsigned long long *status, __nv_bfloat16 *,
+                        __nv_bfloat16 *, const LdltArgs<T> &ld, cudaStream_t st) {
   if (nstrips <= 0) return;
   auto run = [&](auto kernel) {
-    kernel<<<(unsigned)nstrips, 256, kGroupSmem, st>>>(items, strips, nstrips, ticket, flags, P, Lx, Linv, status, Shi,
-                                                       Slo, ld);
+    kernel<<<(unsigned)nstrips, 256, kGroupSmem, st>>>(items, strips, nstrips, ticket, flags, P, Lx, Linv, status, ld);
   };
   if constexpr (std::is_same<T, double>::value)
     if (ld.piv) return run(k_group_panel<T, true, true>);  // Bunch-Kaufman pivot blocks
@@ -725,8 +706,5 @@ void launch_group_panel(const GroupItem *items, const StripTask *strips, int nst
 template void launch_group_panel<double>(const GroupItem *, const StripTask *, int, int *, int *, const DevPlan &,
                                          double *, double *, unsigned long long *, __nv_bfloat16 *, __nv_bfloat16 *,
                                          const LdltArgs<double> &, cudaStream_t);
-template void launch_group_panel<float>(const GroupItem *, const StripTask *, int, int *, int *, const DevPlan &,
-                                         float *, double *, unsigned long long *, __nv_bfloat16 *, __nv_bfloat16 *,
-                                         const LdltArgs<float> &, cudaStream_t);
 
 }  // namespace amp

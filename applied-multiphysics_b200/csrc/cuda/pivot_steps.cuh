@@ -18,7 +18,7 @@ __device__ __forceinline__ void mma884(double (&c)[2], double a, double b) {
 // 1 / d as x f. FP64: Newton's iteration on the hardware estimate x (relative error e below 2^-20):
 // 1 / d = x / (1 - e) = x (1 + e)(1 + e^2) up to e^4, x and f apart, so that a product with x can run beside f's chain;
 // the estimate flushes results outside the normal range, so it returns false for |d| below 2^-975 or above 2^960 (an
-// integer test of the exponent, off the FP64 pipe). FP32: one Newton step on the hardware quotient. Exact: the quotient.
+// integer test of the exponent, off the FP64 pipe). Exact: the quotient.
 template <bool Exact>
 __device__ __forceinline__ bool recip_parts(double d, double &x, double &f) {
   if constexpr (Exact) {
@@ -31,14 +31,6 @@ __device__ __forceinline__ bool recip_parts(double d, double &x, double &f) {
   f = fma(s, e * e, s);
   return ((unsigned)__double2hiint(d) & 0x7fffffffu) - 0x03000000u <= 0x79000000u;
 }
-template <bool Exact>
-__device__ __forceinline__ bool recip_parts(float d, float &x, float &f) {
-  const float y = __fdividef(1.0f, d);
-  x = fmaf(y, fmaf(-d, y, 1.0f), y);
-  f = 1.0f;
-  return true;
-}
-
 // POTRF step buffers: 8 columns of 64 rows; row strides with 16-byte rows and few bank conflicts
 template <class TC>
 constexpr int col_ld() { return sizeof(TC) == 8 ? 10 : 12; }
@@ -46,8 +38,6 @@ template <class TC>
 struct Vec2;  // two neighbouring entries
 template <>
 struct Vec2<double> { using type = double2; };
-template <>
-struct Vec2<float> { using type = float2; };
 
 // C(g, 2 t ..) -= A(g, .) B(., 2 t ..) on an 8 x 8 tile, K = 8: P the negated rows of A, Q the rows of B^T (stride ld)
 __device__ __forceinline__ void step_tile(double (&c)[2], const double *P, const double *Q, int ld, int g, int t) {
@@ -56,18 +46,6 @@ __device__ __forceinline__ void step_tile(double (&c)[2], const double *P, const
   mma884(c, a.x, b.x);
   mma884(c, a.y, b.y);
 }
-__device__ __forceinline__ void step_tile(float (&c)[2], const float *P, const float *Q, int ld, int g, int t) {
-#pragma unroll
-  for (int h = 0; h < 2; h++) {
-    const float4 a = *reinterpret_cast<const float4 *>(P + g * ld + 4 * h);
-#pragma unroll
-    for (int u = 0; u < 2; u++) {
-      const float4 b = *reinterpret_cast<const float4 *>(Q + (2 * t + u) * ld + 4 * h);
-      c[u] = fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, c[u]))));
-    }
-  }
-}
-
 // One pivot step for row r (one row per lane of the calling warps; rows past the block repeat its last one): the columns
 // [k8, k8 + 8) in R (row stride col_ld), their diagonal tile in R's rows k8 ... The first `pivots` columns are pivots
 // (all eight unless Partial); the others only take the pivots' updates. Writes -a to Pk and a / d (0 for a column that is
