@@ -100,7 +100,7 @@ __device__ int potrf_core(const T *src, int lds, T *Lp, int m, int w, int f, int
     fail = kPanel;  // none
     promote = 0;
   }
-  for (int kb = 0; kb < kPanel / 4; kb++) {
+  for (int kb = 0; kb < (w + 3) / 4; kb++) {  // the columns from w on are the identity's
     const int buf = kb & 1;
     if (owner && ti == kb && tj == kb) {
 #pragma unroll
@@ -257,7 +257,7 @@ __device__ void trsm_strip(T *L, int m, int f, int c0, int w, int r0, int r1, in
   const int row = r0 + r;
   const bool active = row < r1;
   __syncthreads();
-  for (int p = 0; p < 4; p++) {
+  for (int p = 0; p < (w + 15) / 16; p++) {  // (zero from column w on)
     if (q == p) {  // solve this quarter
 #pragma unroll
       for (int u = 0; u < 16; u++) {
