@@ -214,8 +214,7 @@ __device__ void assemble_cta(int s, const DevPlan &P, const double *__restrict__
 }
 
 // The whole front of supernode s by one warp (m <= 32) over the shared m x m column-major tile F, in the compute type TC
-// (the storage type T of L and U, or FP64: an FP32 LDL^T factor's small fronts are computed in FP64 and rounded once when
-// stored, since the indefinite factor's pivots cancel).
+// (FP64, as the storage type T: the FP32 factors' kernels are in front_small_f32.cu).
 //
 // Column k of the elimination is one phase with one barrier: every lane reads the pivot F(k, k) (final since the
 // previous barrier), computes the same pivot decision and scale, writes its share of L's column k straight to Lx and

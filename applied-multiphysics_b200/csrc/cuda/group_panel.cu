@@ -618,8 +618,7 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
 #pragma unroll
     for (int p = 0; p < 8; p++) set_pair(Xs, lr, 8 * p + 2 * t, x[p][0], x[p][1]);
     __syncthreads();
-    // written column by column, a warp's lanes on consecutive rows (the fragments' 8-row pieces of a column cost FP32
-    // and BF16 stores a partial sector each)
+    // written column by column, a warp's lanes on consecutive rows (the fragments hold 8-row pieces of a column)
     for (int cc = warp; cc < w; cc += 8) {
 #pragma unroll
       for (int h = 0; h < 2; h++) {
