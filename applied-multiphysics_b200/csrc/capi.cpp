@@ -1396,7 +1396,7 @@ int amp_factor_create(amp_plan *pl, const amp_factor_opts *opts, amp_factor **ou
       }
       f->dTickets = f->mem.alloc<int>(2);
       f->dGroupFlags = f->mem.alloc<int>((size_t)std::max(1, P.nGroupFlags + P.nGroupTickets));
-      f->dLinv = f->mem.alloc<double>((size_t)P.nGroupFlags / 2 * 512);
+      f->dLinv = f->mem.alloc<double>((size_t)P.nGroupFlags / 2 * amp::linv_stride(1));
       f->dDone = f->mem.alloc<int>((size_t)kSlices * std::max(1, P.nsuper));
       f->dSolveStatus = f->mem.alloc<unsigned long long>(1);
       init_device_once(pl->device);
@@ -1866,7 +1866,7 @@ int amp_cfactor_create(amp_plan *pl, amp_factor **out) {
       f->dScal = f->mem.alloc<double>(2);
       f->dCounts = f->mem.alloc<int>(2);
       f->dStatus = f->mem.alloc<unsigned long long>(1);
-      f->dLinv = f->mem.alloc<double>((size_t)pl->cx.nGroupFlags / 2 * 1024);
+      f->dLinv = f->mem.alloc<double>((size_t)pl->cx.nGroupFlags / 2 * amp::linv_stride(2));
       f->dCxFlags = f->mem.alloc<int>((size_t)std::max(1, pl->cx.nGroupFlags + pl->cx.nGroupTickets));
       init_device_once(pl->device);
       settle();  // the schedule's uploads and the memsets above

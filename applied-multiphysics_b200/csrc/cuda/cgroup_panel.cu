@@ -11,6 +11,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "../host/plan.hpp"
 #include "cplx.cuh"
 #include "devplan.cuh"
@@ -281,6 +283,21 @@ __device__ void cpotrf_block(const double *Ds, double *scr, cplx *Lp, double *Li
       Linv[64 * p + 8 * i + j] = x[i].re;
       Linv[512 + 64 * p + 8 * i + j] = x[i].im;
     }
+    // magnitudes by |re| + |im|, those of the pivots compared with by the larger part: both err towards substitution
+    auto mag = [](cplx z) { return fabs(z.re) + fabs(z.im); };
+    double r2 = mag(piv[8 * p + j]);  // squared norm of row j of the scaled block
+#pragma unroll
+    for (int u = 0; u < 7; u++) {
+      const cplx a = u < j ? cplx(Pp[j * kRowLd + u], Pp[kStepPlane + j * kRowLd + u]) : cplx(0.0);
+      r2 += mag(a) * mag(a * scale[8 * p + u]);
+    }
+    bool wild = false;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const double z = mag(x[i]);
+      wild |= !(z * z * r2 <= kInvBound * kInvBound * fmax(fabs(piv[8 * p + i].re), fabs(piv[8 * p + i].im)));
+    }
+    put_wild(Linv, 2, wild);
   }
   if (tid < w) ld.D[f + c0 + tid] = piv[tid];
   if (tid == 0) atomicAdd(ld.counts + 1, nPert);
@@ -307,6 +324,28 @@ __device__ __forceinline__ void cupdate_row_group(CTile (&c)[8], const CTile (&n
         for (int p = 0; p < 4; p++) mma884(c[ph + p].im, n[q].im[u], v[p].re[u]);
       }
     }
+}
+
+// as the real panel's substitute8, with the unit L_pp
+__device__ __forceinline__ void csubstitute8(const CTile &c, CTile &w, const double *Ls, int p, int g, int t) {
+  CTile x = c;
+#pragma unroll 1
+  for (int k = 0; k < 8; k++) {
+    const double vr = __shfl_sync(0xffffffffu, k & 1 ? x.re[1] : x.re[0], 4 * g + (k >> 1));
+    const double vi = __shfl_sync(0xffffffffu, k & 1 ? x.im[1] : x.im[0], 4 * g + (k >> 1));
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      if (2 * t + u == k) {
+        w.re[u] = vr;
+        w.im[u] = vi;
+      }
+      const cplx l = at(Ls, 8 * p + 2 * t + u, 8 * p + k);  // (nothing reads an entry after its own step)
+      x.re[u] = fma(-vr, l.re, x.re[u]);
+      x.re[u] = fma(vi, l.im, x.re[u]);
+      x.im[u] = fma(-vr, l.im, x.im[u]);
+      x.im[u] = fma(-vi, l.re, x.im[u]);
+    }
+  }
 }
 
 constexpr int kCGroupSmem = (3 * 2 * kPlane + 2 * 512) * (int)sizeof(double);  // one CTA per SM
@@ -383,30 +422,41 @@ __global__ void __launch_bounds__(256, 1) k_cgroup_panel(const GroupItem *__rest
       dv[tid] = d;
       dinv[tid] = cplx(1.0) / d;
     }
-    const double *Lb = Linv + ((int64_t)(it.flag0 / 2) + b) * 1024;
+    const double *Lb = Linv + ((int64_t)(it.flag0 / 2) + b) * linv_stride(2);
 #pragma unroll
     for (int h = 0; h < 2; h++)
       *reinterpret_cast<double2 *>(Li + 512 * h + 2 * tid) = __ldcg(reinterpret_cast<const double2 *>(Lb + 512 * h + 2 * tid));
+    const int wild = wild_blocks(Lb, 2);
     __syncthreads();
-    // W = C L_bb^-T, right-looking over the 8-column blocks: solved with the block's inverse, then subtracted from the
-    // later ones
+    // W = C L_bb^-T, right-looking over the 8-column blocks: solved with the block's inverse (by substitution where that is
+    // large), then subtracted from the later ones
+    auto solve = [&](auto some) {
 #pragma unroll
-    for (int p = 0; p < 8; p++) {
-      if (8 * p >= w) break;  // x is zero from column w on
-      const double2 vr = *reinterpret_cast<const double2 *>(Li + 64 * p + 8 * g + 2 * t);
-      const double2 vi = *reinterpret_cast<const double2 *>(Li + 512 + 64 * p + 8 * g + 2 * t);
-      CTile wv = {{0.0, 0.0}, {0.0, 0.0}};
-      cmma(wv, x[p].re[0], x[p].im[0], vr.x, vi.x);
-      cmma(wv, x[p].re[1], x[p].im[1], vr.y, vi.y);
-      x[p] = wv;
+      for (int p = 0; p < 8; p++) {
+        if (8 * p >= w) break;  // x is zero from column w on
+        CTile wv = {{0.0, 0.0}, {0.0, 0.0}};
+        if (decltype(some)::value && wild >> p & 1) {
+          csubstitute8(x[p], wv, Ls, p, g, t);
+        } else {
+          const double2 vr = *reinterpret_cast<const double2 *>(Li + 64 * p + 8 * g + 2 * t);
+          const double2 vi = *reinterpret_cast<const double2 *>(Li + 512 + 64 * p + 8 * g + 2 * t);
+          cmma(wv, x[p].re[0], x[p].im[0], vr.x, vi.x);
+          cmma(wv, x[p].re[1], x[p].im[1], vr.y, vi.y);
+        }
+        x[p] = wv;
 #pragma unroll
-      for (int p2 = p + 1; p2 < 8; p2++) {
-        if (8 * p2 >= w) break;
-        const CTile l = tile_at(Ls, 8 * p2 + g, 8 * p + 2 * t);
-        cmma(x[p2], -wv.re[0], -wv.im[0], l.re[0], l.im[0]);
-        cmma(x[p2], -wv.re[1], -wv.im[1], l.re[1], l.im[1]);
+        for (int p2 = p + 1; p2 < 8; p2++) {
+          if (8 * p2 >= w) break;
+          const CTile l = tile_at(Ls, 8 * p2 + g, 8 * p + 2 * t);
+          cmma(x[p2], -wv.re[0], -wv.im[0], l.re[0], l.im[0]);
+          cmma(x[p2], -wv.re[1], -wv.im[1], l.re[1], l.im[1]);
+        }
       }
-    }
+    };
+    if (wild == 0)
+      solve(std::false_type());
+    else
+      solve(std::true_type());
     // x := L21's entries; nx := -W, W = x D
 #pragma unroll
     for (int p = 0; p < 8; p++) {
@@ -455,7 +505,7 @@ __global__ void __launch_bounds__(256, 1) k_cgroup_panel(const GroupItem *__rest
   if (jd >= 0) {  // this strip's own pivot block, fully updated: factor it and publish it (also after a failure)
     const int c0 = g0 + jd * kPanel, w = min(kPanel, g1 - c0);
     __syncthreads();  // Ds complete (also when the strip had no earlier pivot block); Ls and Xs free
-    cpotrf_block(Ds, Ls, L + (int64_t)c0 * m + c0, Linv + ((int64_t)(it.flag0 / 2) + jd) * 1024, m, w, f, c0, s, status,
+    cpotrf_block(Ds, Ls, L + (int64_t)c0 * m + c0, Linv + ((int64_t)(it.flag0 / 2) + jd) * linv_stride(2), m, w, f, c0, s, status,
                  ld);
     panel_release(Pf + jd, 1);
   }

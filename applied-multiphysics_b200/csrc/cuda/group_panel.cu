@@ -214,8 +214,24 @@ __device__ int potrf_block(const double *Ds, double *scr, T *Lp, double *Linv, i
         v += ((double)Pp[i * CL + u] * (LDLT ? sc : sc * sc)) * x[u];
       }
       x[i] = i < j ? 0.0 : i == j ? 1.0 : v;  // (P holds -a)
-      Linv[64 * p + 8 * i + j] = x[i] * (LDLT ? 1.0 : scale[8 * p + i]);
     }
+    double r2 = 0.0;  // squared norm of row j of the scaled block
+#pragma unroll
+    for (int u = 0; u < 7; u++) {
+      const double a = u < j ? (double)Pp[j * CL + u] : 0.0, l = a * scale[8 * p + u];
+      r2 += LDLT ? fabs(a * l) : l * l;
+    }
+    r2 += LDLT ? fabs(diag[8 * p + j]) : diag[8 * p + j] * diag[8 * p + j];
+    unsigned top = 0;  // high word of the largest X(i, j)^2 / |d_i| (Cholesky: |X(i, j)|); above all numbers for NaN
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const double sc = scale[8 * p + i], z = LDLT ? x[i] : x[i] * sc;
+      Linv[64 * p + 8 * i + j] = z;
+      top = max(top, (unsigned)__double2hiint(LDLT ? z * (z * sc) : z) & 0x7fffffffu);
+    }
+    const double z2 = __hiloint2double((int)top, 0);
+    const bool wild = !((LDLT ? z2 : z2 * z2) * r2 <= kInvBound * kInvBound);
+    put_wild(Linv, 1, wild);
   }
   if (LDLT) {
     if (tid < w) ld.D[f + c0 + tid] = diag[tid];
@@ -418,6 +434,17 @@ __device__ bool bk_block(double *Ds, double (*S)[kPanel + 1], T *Lp, double *Lin
       x[ii] = ii < j ? 0.0 : ii == j ? 1.0 : -z;
       Linv[64 * p + 8 * ii + j] = x[ii];
     }
+    // multipliers are bounded here, so the block itself stands for its scaled form
+    double r2 = 1.0;
+    bool wild = false;
+#pragma unroll
+    for (int u = 0; u < 7; u++) {
+      const double l = u < j ? Ds[kPanel * (8 * p + u) + 8 * p + j] : 0.0;
+      r2 += l * l;
+    }
+#pragma unroll
+    for (int ii = 0; ii < 8; ii++) wild |= !(x[ii] * x[ii] * r2 <= kInvBound * kInvBound);
+    put_wild(Linv, 1, wild);
   }
   if (tid < w) {
     ld.D[f + c0 + tid] = sD[tid];
@@ -444,6 +471,21 @@ __device__ __forceinline__ void update_row_group(double (&c)[8][2], const double
     for (int p = 0; p < 8; p++) mma884(c[p], n[q][0], v[p].x);
 #pragma unroll
     for (int p = 0; p < 8; p++) mma884(c[p], n[q][1], v[p].y);
+  }
+}
+
+// Row g of w = c L_pp^-T by substitution, L_pp the p-th 8 x 8 diagonal block of the pivot block Ls, 1 / L(k, k) on the
+// diagonal of its inverse; lane t of the row holds entries 2 t and 2 t + 1.
+__device__ __forceinline__ void substitute8(const double (&c)[2], double (&w)[2], const double *Ls, const double *Li, int p,
+                                            int g, int t) {
+  double x0 = c[0], x1 = c[1];
+#pragma unroll 1
+  for (int k = 0; k < 8; k++) {
+    const double v = __shfl_sync(0xffffffffu, k & 1 ? x1 : x0, 4 * g + (k >> 1)) * Li[64 * p + 9 * k];
+    if (2 * t == k) w[0] = v;
+    if (2 * t + 1 == k) w[1] = v;
+    x0 -= v * Ls[sw(8 * p + 2 * t, 8 * p + k)];  // (nothing reads an entry after its own step)
+    x1 -= v * Ls[sw(8 * p + 2 * t + 1, 8 * p + k)];
   }
 }
 
@@ -477,7 +519,7 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
   __shared__ double dv[kPanel], dinv[kPanel];
   __shared__ double dB[BK ? kPanel : 1];
   __shared__ int dP[BK ? kPanel : 1], sPiv[BK ? kPanel : 1];
-  __shared__ int sTicket;
+  __shared__ int sTicket, sWild;
   if (threadIdx.x == 0) sTicket = panel_failed(status) ? nstrips : atomicAdd(ticket, 1);
   __syncthreads();
   const int tk = sTicket;
@@ -561,8 +603,9 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
         dinv[tid] = 1.0 / d;
       }
     }
-    *reinterpret_cast<double2 *>(Li + 2 * tid) =
-        __ldcg(reinterpret_cast<const double2 *>(Linv + ((int64_t)(it.flag0 / 2) + b) * (8 * 64) + 2 * tid));
+    const double *Lb = Linv + ((int64_t)(it.flag0 / 2) + b) * linv_stride(1);
+    *reinterpret_cast<double2 *>(Li + 2 * tid) = __ldcg(reinterpret_cast<const double2 *>(Lb + 2 * tid));
+    if (tid == 0) sWild = wild_blocks(Lb, 1);
     __syncthreads();
     if constexpr (BK) {  // the strip's columns in the block's pivot order (each warp exchanges its own rows)
 #pragma unroll
@@ -574,25 +617,35 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
         for (int u = 0; u < 2; u++) x[p][u] = Xs[sw(lr, sPiv[8 * p + 2 * t + u])];
       __syncwarp();
     }
-    // W = C L_bb^-T, right-looking over the 8-column blocks: solved with the block's inverse, then subtracted from the
-    // later ones
+    // W = C L_bb^-T, right-looking over the 8-column blocks: solved with the block's inverse (by substitution where that is
+    // large), then subtracted from the later ones
+    auto solve = [&](auto some, const int wild) {
 #pragma unroll
-    for (int p = 0; p < 8; p++) {
-      if (8 * p >= w) break;  // x is zero from column w on
-      const double2 iv = *reinterpret_cast<const double2 *>(Li + 64 * p + 8 * g + 2 * t);
-      double wv[2] = {0.0, 0.0};
-      mma884(wv, x[p][0], iv.x);
-      mma884(wv, x[p][1], iv.y);
-      x[p][0] = wv[0];
-      x[p][1] = wv[1];
+      for (int p = 0; p < 8; p++) {
+        if (8 * p >= w) break;  // x is zero from column w on
+        double wv[2] = {0.0, 0.0};
+        if (decltype(some)::value && wild >> p & 1) {
+          substitute8(x[p], wv, Ls, Li, p, g, t);
+        } else {
+          const double2 iv = *reinterpret_cast<const double2 *>(Li + 64 * p + 8 * g + 2 * t);
+          mma884(wv, x[p][0], iv.x);
+          mma884(wv, x[p][1], iv.y);
+        }
+        x[p][0] = wv[0];
+        x[p][1] = wv[1];
 #pragma unroll
-      for (int p2 = p + 1; p2 < 8; p2++) {
-        if (8 * p2 >= w) break;
-        const double2 l = pair_at(Ls, 8 * p2 + g, 8 * p + 2 * t);
-        mma884(x[p2], -wv[0], l.x);
-        mma884(x[p2], -wv[1], l.y);
+        for (int p2 = p + 1; p2 < 8; p2++) {
+          if (8 * p2 >= w) break;
+          const double2 l = pair_at(Ls, 8 * p2 + g, 8 * p + 2 * t);
+          mma884(x[p2], -wv[0], l.x);
+          mma884(x[p2], -wv[1], l.y);
+        }
       }
-    }
+    };
+    if (sWild == 0)
+      solve(std::false_type(), 0);
+    else
+      solve(std::true_type(), sWild);
     if constexpr (BK) {
 #pragma unroll
       for (int p = 0; p < 8; p++) set_pair(Xs, lr, 8 * p + 2 * t, x[p][0], x[p][1]);
@@ -653,7 +706,7 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
   if (jd >= 0) {  // this strip's own pivot block, fully updated: factor it and publish it (also after a failure)
     const int c0 = g0 + jd * kPanel, w = min(kPanel, g1 - c0);
     T *Lp = L + (int64_t)c0 * m + c0;
-    double *Lb = Linv + ((int64_t)(it.flag0 / 2) + jd) * (8 * 64);
+    double *Lb = Linv + ((int64_t)(it.flag0 / 2) + jd) * linv_stride(1);
     __syncthreads();  // Ds complete (also when the strip had no earlier pivot block); Ls and Xs free
     if constexpr (BK) {
       // Bunch-Kaufman keeps every pivot of the block in place exactly when each multiplier is at most 1 / alpha in

@@ -18,8 +18,8 @@ cudaError_t init_kernel_attributes();  // once per device (with that device curr
 template <class T>
 void launch_assemble(const AsmTask *tasks, const ChildRange *ranges, int64_t ntasks, const DevPlan &P,
                      const value_of<T> *values, T *Lx, T *U, const unsigned long long *status, cudaStream_t st);
-// one group of pivot blocks per item: nstrips strip tasks, ticket and flags zeroed before the factorization; Linv: 512
-// doubles per pivot block of the schedule (block b of an item at flag0 / 2 + b; complex: 1024), scratch of the launches
+// one group of pivot blocks per item: nstrips strip tasks, ticket and flags zeroed before the factorization; Linv: linv_stride
+// doubles per pivot block of the schedule (block b of an item at flag0 / 2 + b), scratch of the launches
 template <class T>
 void launch_group_panel(const GroupItem *items, const StripTask *strips, int nstrips, int *ticket, int *flags,
                         const DevPlan &P, T *Lx, double *Linv, unsigned long long *status, __nv_bfloat16 *Shi,

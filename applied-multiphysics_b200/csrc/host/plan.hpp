@@ -31,6 +31,10 @@ constexpr int kSolveGroup = 4;    // supernodes with m <= kTinyFront per solve t
 constexpr int kSolveWarps = 8;    // the same in a task of the launched lists, where neighbouring tasks are joined
 constexpr int kWholeFront = 512;  // one-vector forward: supernodes with nc <= 64 and m <= 512 are one task each
 
+// doubles of scratch per pivot block of the FP64 group panels (panel_blocks.cuh): eight 8 x 8 blocks in one plane, or two
+// (complex), and two ints; a multiple of 16 bytes
+constexpr int linv_stride(int planes) { return 512 * planes + 2; }
+
 struct GroupItem {  // pivot columns [g0, g1) (up to kGroup pivot blocks) of supernode s, factored by one group-panel
                     // launch; its flags start at flag0: one POTRF flag per pivot block, then one TRSM counter per
                     // diagonal strip
