@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(256, 1) k_cgroup_panel(const GroupItem *__rest
   double *Li = Ds + 2 * kPlane;                     // the pivot block's Linv
   __shared__ cplx dv[kPanel], dinv[kPanel];
   __shared__ int sTicket;
-  if (threadIdx.x == 0) sTicket = panel_failed(status) ? nstrips : atomicAdd(ticket, 1);
+  if (threadIdx.x == 0) sTicket = factor_failed(status) ? nstrips : atomicAdd(ticket, 1);
   __syncthreads();
   const int tk = sTicket;
   if (tk >= nstrips) return;

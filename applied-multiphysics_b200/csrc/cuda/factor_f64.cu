@@ -59,10 +59,6 @@ __global__ void __launch_bounds__(1024) k_ldlt_tau(const double *__restrict__ va
   }
 }
 
-__device__ __forceinline__ bool failed(const unsigned long long *st) {
-  return *(volatile const unsigned long long *)st != kStatusOk;
-}
-
 // ---------------------------------------------------------------------------------------------------------------
 // Assembly + extend-add
 // ---------------------------------------------------------------------------------------------------------------
@@ -82,7 +78,7 @@ template <class T>
 __global__ void __launch_bounds__(256, 4) k_assemble(const AsmTask *__restrict__ tasks, const ChildRange *__restrict__ ranges,
                                                   DevPlan P, const value_of<T> *__restrict__ values, T *__restrict__ Lx,
                                                   T *__restrict__ U, const unsigned long long *status) {
-  if (failed(status)) return;
+  if (cta_failed(status)) return;
   const AsmTask t = tasks[blockIdx.x];
   const int s = t.s, j0 = t.j0;
   const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s];
@@ -226,7 +222,7 @@ template <int ROWS>
 __global__ void __launch_bounds__(128, ROWS == 128 ? 2 : 3)
     k_update(const TileTask *__restrict__ tasks, int ntasks, double *__restrict__ Lx, double *__restrict__ U,
              const double *__restrict__ W, const unsigned long long *status) {
-  if (failed(status)) return;
+  if (cta_failed(status)) return;
   constexpr int SPLIT = kTileM / ROWS, MA = ROWS / 32;  // CTA tiles per task; 16-row fragments per warp
   const double *Ax = W ? W : Lx;                        // LDL^T: A = L21 D
   extern __shared__ double smem_upd[];
@@ -376,7 +372,7 @@ __global__ void __launch_bounds__(128) k_update_c(const TileTask *__restrict__ t
   if (i0 >= m || j0 >= jend || i0 + TS <= j0) return;
   __shared__ int sOk;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
-  if (tid == 0) sOk = !failed(status);
+  if (tid == 0) sOk = !factor_failed(status);
   const cplx *Ap = W + t.lp + (int64_t)t.c0 * m, *Bp = Lx + t.lp + (int64_t)t.c0 * m;
   const int nchunk = (t.w + kCK - 1) / kCK;
   auto stage = [&](int ch) {

@@ -30,6 +30,7 @@
 #include "../../../include/ampsolve.h"
 #include "../host/plan.hpp"
 #include "devplan.cuh"
+#include "sync.cuh"
 
 namespace amp {
 void set_last_error(const std::string &msg);
@@ -43,16 +44,12 @@ constexpr int kNoAllocBlocks = kNoAllocMaxFront / kPanel; // pivot blocks of the
 // [0] status word, [1 + k] readers of pivot block k: (1 + 256) x 8 bytes
 static __device__ __align__(256) unsigned long long g_front_scratch[1 + kNoAllocBlocks];
 
-__device__ __forceinline__ bool na_failed(const unsigned long long *st) {
-  return *(volatile const unsigned long long *)st != kStatusOk;
-}
-
 // One CTA per chunk of 256 rows below pivot block [c0, c0 + w): factor the block, solve the chunk; the last CTA to
 // have read the unfactored block writes it back.
 __global__ void __launch_bounds__(256) k_front_panel_na(double *__restrict__ F, int m, int nc, int c0,
                                                         unsigned long long *scratch) {
   unsigned long long *status = scratch;
-  if (na_failed(status)) return;
+  if (cta_failed(status)) return;
   const int w = min(kPanel, nc - c0), c1 = c0 + w;
   const int nchunks = c1 < m ? (m - c1 + kNaRows - 1) / kNaRows : 1;
   const int r0 = c1 + blockIdx.x * kNaRows, r1 = min(r0 + kNaRows, m);
@@ -132,7 +129,7 @@ constexpr int kNaLd = kTile + 4;
 // Trailing update after pivot block [c0, c0 + w): lower 64 x 64 tiles of [c1, m), tile (I, J) from blockIdx.
 __global__ void __launch_bounds__(128) k_front_update_na(double *__restrict__ F, int m, int nc, int c0,
                                                          const unsigned long long *scratch) {
-  if (na_failed(scratch)) return;
+  if (cta_failed(scratch)) return;
   const int w = min(kPanel, nc - c0), c1 = c0 + w, wp = (w + 3) & ~3;
   const int b = blockIdx.x;
   int I = (int)((sqrt(8.0 * b + 1.0) - 1.0) * 0.5);

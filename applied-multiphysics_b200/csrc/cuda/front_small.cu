@@ -51,10 +51,6 @@ __device__ __forceinline__ void group_sync() {
     __syncthreads();
 }
 
-__device__ __forceinline__ bool status_failed(const unsigned long long *st) {
-  return *(volatile const unsigned long long *)st != kStatusOk;
-}
-
 // |d| < tau (or NaN) becomes -tau / +tau by the sign of d; a non-finite small pivot fails (ldlt.mjs:513-522)
 template <class T>
 __device__ __forceinline__ bool small_ldlt_pivot(T &d, T tau, int &neg, int &pert) {
@@ -136,10 +132,11 @@ __device__ void assemble_warp(int s, const DevPlan &P, const double *__restrict_
   __syncwarp();
 }
 
-// The same by a CTA of NT threads (m <= 128): warps over the child's columns, lanes over its rows. Ends with a barrier.
+// The same by a CTA of NT threads (m <= 128): warps over the child's columns, lanes over its rows. Ends with a barrier;
+// false (in every thread) when the factorization has failed.
 template <class T, class TC, int NT>
-__device__ void assemble_cta(int s, const DevPlan &P, const double *__restrict__ values, const T *__restrict__ U, TC *F,
-                             ChildMeta *cm) {
+__device__ bool assemble_cta(int s, const DevPlan &P, const double *__restrict__ values, const T *__restrict__ U, TC *F,
+                             ChildMeta *cm, const unsigned long long *status) {
   constexpr int NW = NT / 32;
   constexpr int kBatch = 16;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -159,6 +156,7 @@ __device__ void assemble_cta(int s, const DevPlan &P, const double *__restrict__
   __syncthreads();
   for (int p = p0 + t; p < p1; p += NT) F[P.asmDst[p]] += (TC)(T)__ldg(values + P.asmSrc[p]);
   pdl_wait();  // the children's level
+  const bool bad = t == 0 && factor_failed(status);  // one read for the CTA (sync.cuh), in time for the last barrier
   for (int qb = 0; qb < nch; qb += kChildChunk) {
     const int nq = min(kChildChunk, nch - qb);
     if (qb > 0) {
@@ -210,7 +208,7 @@ __device__ void assemble_cta(int s, const DevPlan &P, const double *__restrict__
       i = in;
     }
   }
-  __syncthreads();
+  return !__syncthreads_or(bad);
 }
 
 // The whole front of supernode s by one warp (m <= 32) over the shared m x m column-major tile F, in the compute type TC
@@ -229,7 +227,7 @@ __device__ void factor_front_warp(int s, const DevPlan &P, const double *__restr
   const bool ldlt = la.scal != nullptr;
   const TC tau = ldlt ? (TC)(T)la.scal[1] : TC(0);
   assemble_warp<T, TC, tiny_batch<MAXM>()>(s, P, values, U, F, lane);
-  if (status_failed(status)) return;
+  if (warp_failed(status)) return;
   int neg = 0, pert = 0;  // lane 0
   T *Lp = Lx + P.snLxp[s];
   for (int k = 0; k < nc; k++) {
@@ -319,8 +317,7 @@ __global__ void __launch_bounds__(small_threads<MAXM>(), MAXM == 64 ? 2 : 1)
   T *Lp = Lx + P.snLxp[s];
   T *Up = U + (mu > 0 ? P.snUoff[s] : 0);
   const TC tau = LDLT ? (TC)(T)la.scal[1] : TC(0);
-  assemble_cta<T, TC, NT>(s, P, values, U, F, &cm);
-  if (status_failed(status)) return;
+  if (!assemble_cta<T, TC, NT>(s, P, values, U, F, &cm, status)) return;
   // the front's tiles: row group rg[h], tile column cb
   const int rg[2] = {warp, NG == 2 ? 15 - warp : -1};
   auto tile = [&](int rb, int cb, TC(&c)[2]) {
@@ -536,11 +533,12 @@ __device__ void factor_front_bk(int s, const DevPlan &P, const double *__restric
   const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s], mu = m - nc;
   const double tau = la.scal[1];
   const double alpha = 0.64038820320220756;  // (1 + sqrt(17)) / 8
-  if constexpr (G == 32)
+  if constexpr (G == 32) {
     assemble_warp<T, double, 16>(s, P, values, U, F, t);
-  else
-    assemble_cta<T, double, G>(s, P, values, U, F, cm);
-  if (status_failed(status)) return;
+    if (warp_failed(status)) return;
+  } else {
+    if (!assemble_cta<T, double, G>(s, P, values, U, F, cm, status)) return;
+  }
   auto at = [&](int i, int j) -> double & { return F[j * m + i]; };  // entry (i, j), i >= j
   int neg = 0, pert = 0;  // thread 0
   int perm[64];           // thread 0: the current block's pivot order

@@ -11,6 +11,7 @@
 #include "../host/plan.hpp"
 #include "devplan.cuh"
 #include "launch.hpp"
+#include "sync.cuh"
 
 namespace amp {
 
@@ -30,10 +31,6 @@ __device__ __forceinline__ void group_sync() {
     __syncwarp();
   else
     __syncthreads();
-}
-
-__device__ __forceinline__ bool status_failed(const unsigned long long *st) {
-  return *(volatile const unsigned long long *)st != kStatusOk;
 }
 
 // |d| < tau (or NaN) becomes -tau / +tau by the sign of d; a non-finite small pivot fails (ldlt.mjs:513-522)
@@ -201,7 +198,7 @@ __global__ void __launch_bounds__(32 * tiny_warps<MAXM>()) k_front_tiny_f32(cons
                                                                          unsigned long long *status, LdltArgs<T> la) {
   constexpr int W = tiny_warps<MAXM>();
   __shared__ TC F[W][MAXM * MAXM];
-  if (status_failed(status)) return;
+  if (warp_failed(status)) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int idx = blockIdx.x * W + warp;
   if (idx >= count) return;  // warp-uniform; no CTA-wide barrier follows
@@ -215,7 +212,7 @@ __global__ void __launch_bounds__(256) k_front_small_f32(const int *__restrict__
                                                      T *__restrict__ U, unsigned long long *status, LdltArgs<T> la) {
   extern __shared__ __align__(16) unsigned char fs_dyn[];
   __shared__ ChildMeta cm;
-  if (status_failed(status)) return;
+  if (cta_failed(status)) return;
   factor_front<T, TC, 256>(fronts[blockIdx.x], P, values, Lx, U, reinterpret_cast<TC *>(fs_dyn), status, la,
                              threadIdx.x, &cm);
 }

@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
   __shared__ double dB[BK ? kPanel : 1];
   __shared__ int dP[BK ? kPanel : 1], sPiv[BK ? kPanel : 1];
   __shared__ int sTicket, sWild;
-  if (threadIdx.x == 0) sTicket = panel_failed(status) ? nstrips : atomicAdd(ticket, 1);
+  if (threadIdx.x == 0) sTicket = factor_failed(status) ? nstrips : atomicAdd(ticket, 1);
   __syncthreads();
   const int tk = sTicket;
   if (tk >= nstrips) return;

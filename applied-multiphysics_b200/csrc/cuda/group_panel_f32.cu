@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(256, 2) k_group_panel_f32(const GroupItem *__r
   T(*Ds)[kPanel + 1] = reinterpret_cast<T(*)[kPanel + 1]>(gp_raw + 2 * kPanel * (kPanel + 1) * sizeof(T));
   __shared__ T invd[kPanel], dv[kPanel];
   __shared__ int sTicket;
-  if (threadIdx.x == 0) sTicket = panel_failed(status) ? nstrips : atomicAdd(ticket, 1);
+  if (threadIdx.x == 0) sTicket = factor_failed(status) ? nstrips : atomicAdd(ticket, 1);
   __syncthreads();
   const int t = sTicket;
   if (t >= nstrips) return;

@@ -9,10 +9,6 @@
 
 namespace amp {
 
-__device__ __forceinline__ bool panel_failed(const unsigned long long *st) {
-  return *(volatile const unsigned long long *)st != kStatusOk;
-}
-
 // 64 x 64 FP64 blocks in shared memory, row-major, the column pairs of row r permuted by a bijection of r mod 8 so that
 // the 16-byte accesses of a fragment (8 rows, 4 neighbouring pairs) and the 8-byte stores of the block loads (8 rows,
 // 4 columns) touch every bank equally often.
@@ -63,7 +59,7 @@ __device__ __forceinline__ bool panel_wait(const int *p, int need, unsigned long
     long long spins = 0;
     int v = 1;
     while (ld_acquire(p) < need) {
-      if (panel_failed(status)) {
+      if (factor_failed(status)) {
         v = 0;
         break;
       }
@@ -74,7 +70,7 @@ __device__ __forceinline__ bool panel_wait(const int *p, int need, unsigned long
       }
       __nanosleep(32);
     }
-    if (panel_failed(status)) v = 0;  // a failed pivot also releases its flag
+    if (factor_failed(status)) v = 0;  // a failed pivot also releases its flag
     ok = v;
   }
   __syncthreads();

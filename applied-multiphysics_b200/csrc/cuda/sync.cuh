@@ -9,6 +9,18 @@
 
 namespace amp {
 
+// Whether the factorization has failed. Another CTA may set the word at any time, so where threads of a CTA (a warp) leave
+// on it, they do so on one read: threads that each took their own could part ways before a barrier, and those left behind
+// work on what the others should have made.
+__device__ __forceinline__ bool factor_failed(const unsigned long long *status) {
+  return *(volatile const unsigned long long *)status != kStatusOk;
+}
+__device__ __forceinline__ bool cta_failed(const unsigned long long *status) {  // a barrier of the CTA
+  return __syncthreads_or(threadIdx.x == 0 && factor_failed(status));
+}
+__device__ __forceinline__ bool warp_failed(const unsigned long long *status) {
+  return __any_sync(0xffffffffu, (threadIdx.x & 31) == 0 && factor_failed(status));
+}
 
 __device__ __forceinline__ int ld_acquire(const int *p) {
   int v;

@@ -26,6 +26,7 @@
 
 #include "../host/plan.hpp"
 #include "devplan.cuh"
+#include "sync.cuh"
 #include "umma.cuh"
 
 namespace amp {
@@ -112,7 +113,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_update_mx(const MixTask *__rest
   constexpr int kN = N;
   extern __shared__ __align__(1024) uint8_t smem_mx[];
   __shared__ MxShared sh;
-  if (*(volatile unsigned long long *)status != kStatusOk) return;
+  if (cta_failed(status)) return;
   if ((int)blockIdx.x >= ntasks) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint8_t *stages = smem_mx + ((1024 - (umma::smem_u32(smem_mx) & 1023)) & 1023);  // 1 KB aligned (swizzle atom)
