@@ -521,9 +521,10 @@ __device__ __forceinline__ void front_warp_argmax(double &v, int &i) {
 // order, so every thread takes the same decision without sharing it); the interchange applied in lower storage to
 // the block's earlier columns (their rows) and to the whole trailing triangle (rows below the pivot columns
 // included); the rank-1 or rank-2 update of the trailing triangle from the unscaled column(s); then the column(s)
-// scaled in place to L. Three barriers per step. A block's L columns go to Lx once the block is done (its later
-// steps may still interchange their rows), with its pivot order; D and D(k + 1, k) as they are decided. A column
-// with no usable entry in its block keeps the static perturbation to +-tau (counted); a non-finite pivot fails.
+// scaled in place to L. Three barriers per step, one more where row im is searched (its entries belong to the triangle that
+// a faster warp goes on to interchange and update). A block's L columns go to Lx once the block is done (its later steps may
+// still interchange their rows), with its pivot order; D and D(k + 1, k) as they are decided. A column with no usable entry
+// in its block keeps the static perturbation to +-tau (counted); a non-finite pivot fails.
 template <class T, int G>
 __device__ void factor_front_bk(int s, const DevPlan &P, const double *__restrict__ values, T *__restrict__ Lx,
                                 T *__restrict__ U, double *F, unsigned long long *status, const LdltArgs<T> &la,
@@ -574,6 +575,7 @@ __device__ void factor_front_bk(int s, const DevPlan &P, const double *__restric
           step = 2;
           kp = im;
         }
+        group_sync<G>();  // every warp has read row im before anyone changes the trailing triangle
       }
       const int kk = k + step - 1;
       if (kp != kk) {  // interchange p = kk and r = kp (p < r), lower storage
