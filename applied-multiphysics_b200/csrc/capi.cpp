@@ -564,7 +564,8 @@ void enqueue_factor(amp_factor *f) {
     if (P.nflags)
       timed(f, K_DIAGINV, 0.0, 8.0 * (double)inv_elems(P),
             [&] {
-              amp::launch_diag_inv<float>(f->plan->dInvBlocks, (int)P.invBlocks.size(), dp, f->dL32, f->dInv32, st);
+              amp::launch_diag_inv<float>(f->plan->dInvBlocks, (int)P.invBlocks.size(), dp, f->dL32, f->dInv32,
+                                          f->dStatus, st);
             });
     enqueue_chain_mats<float>(f, f->dL32, f->dInv32, f->dMch32, f->dGch32);
     return;
@@ -622,7 +623,7 @@ void enqueue_factor(amp_factor *f) {
   if (P.nflags)
     timed(f, K_DIAGINV, 0.0, 16.0 * (double)inv_elems(P),
           [&] {
-            amp::launch_diag_inv<double>(f->plan->dInvBlocks, (int)P.invBlocks.size(), dp, f->dLx, f->dInv, st);
+            amp::launch_diag_inv<double>(f->plan->dInvBlocks, (int)P.invBlocks.size(), dp, f->dLx, f->dInv, f->dStatus, st);
           });
   enqueue_chain_mats<double>(f, f->dLx, f->dInv, f->dMch, f->dGch);
 }

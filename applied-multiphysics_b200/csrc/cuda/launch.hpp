@@ -55,9 +55,10 @@ void launch_update(const TileTask *tasks, int64_t ntasks, const DevPlan &P, doub
 void launch_sweep_begin(unsigned long long *status, int *tickets, int *done, int nsuper, cudaStream_t st);
 void launch_permute_in(const double *b, double *y, const int *perm, int n, int q, cudaStream_t st);
 void launch_permute_out(const double *y, double *x, const int *perm, int n, int q, cudaStream_t st);
-// inverses of the diagonal blocks (with each block's pivot order folded in when P.lpiv is set)
+// inverses of the diagonal blocks (with each block's pivot order folded in when P.lpiv is set); none after a failure
 template <class TL>
-void launch_diag_inv(const int *blocks, int nblocks, const DevPlan &P, const TL *Lx, TL *Inv, cudaStream_t st);
+void launch_diag_inv(const int *blocks, int nblocks, const DevPlan &P, const TL *Lx, TL *Inv,
+                     const unsigned long long *status, cudaStream_t st);
 // D solve of a Bunch-Kaufman factor (1 x 1 and 2 x 2 pivots), q interleaved vectors, between the sweeps
 void launch_dsolve_bk(int n, int q, const double *D, const double *Doff, double *y, cudaStream_t st);
 template <class TL>

@@ -56,7 +56,8 @@ __device__ __forceinline__ unsigned warp_flags(const int *p, int step, int n, in
 // X P_b (P_b the block's pivot order, a full w x w matrix): the forward sweep's r, taken in the original order of the
 // block's rows, becomes y_b = X P_b r, and the backward sweep's x_b = (X P_b)^T r lands in that original order, so
 // L's earlier columns keep the rows of later blocks in their original order (the interchanges are not applied to
-// the left of a block) and the sweeps need no other change.
+// the left of a block) and the sweeps need no other change. After a failed factorization nothing is done: the pivot
+// orders of the blocks that it did not reach may never have been written.
 constexpr int kInvThreads = 4 * kSB;
 template <class TL>
 constexpr int diag_inv_smem() {
@@ -64,12 +65,14 @@ constexpr int diag_inv_smem() {
 }
 template <class TL>
 __global__ void __launch_bounds__(kInvThreads) k_diag_inv(const int *__restrict__ blocks, DevPlan P,
-                                                          const TL *__restrict__ Lx, TL *__restrict__ Inv) {
+                                                          const TL *__restrict__ Lx, TL *__restrict__ Inv,
+                                                          const unsigned long long *status) {
   extern __shared__ double inv_dyn[];
   double(*Xs)[kSB] = reinterpret_cast<double(*)[kSB]>(inv_dyn);
   TL(*Ls)[kSB + 1] = reinterpret_cast<TL(*)[kSB + 1]>(inv_dyn + kSB * kSB);
   __shared__ double dinv[kSB];
   __shared__ int kOf[kSB];
+  const bool bad = threadIdx.x == 0 && factor_failed(status);  // one read for the CTA
   const int b = blocks[blockIdx.x];
   int lo = 0, hi = P.nsuper;  // supernode s with blkOff[s] <= b < blkOff[s + 1]
   while (hi - lo > 1) {
@@ -84,7 +87,7 @@ __global__ void __launch_bounds__(kInvThreads) k_diag_inv(const int *__restrict_
     const int t = e >> 6, i = e & (kSB - 1);
     if (t < w && i >= t && i < w) Ls[t][i] = __ldg(Lb + (int64_t)t * m + i);
   }
-  __syncthreads();
+  if (__syncthreads_or(bad)) return;
   if (tid < w) dinv[tid] = 1.0 / (double)Ls[tid][tid];
   __syncthreads();
   const int j = tid >> 2, p = tid & 3;
@@ -760,8 +763,9 @@ int num_sms();
 static int solve_grid(int ntasks) { return ntasks < 3 * num_sms() ? ntasks : 3 * num_sms(); }
 
 template <class TL>
-void launch_diag_inv(const int *blocks, int nblocks, const DevPlan &P, const TL *Lx, TL *Inv, cudaStream_t st) {
-  if (nblocks > 0) k_diag_inv<TL><<<nblocks, kInvThreads, diag_inv_smem<TL>(), st>>>(blocks, P, Lx, Inv);
+void launch_diag_inv(const int *blocks, int nblocks, const DevPlan &P, const TL *Lx, TL *Inv,
+                     const unsigned long long *status, cudaStream_t st) {
+  if (nblocks > 0) k_diag_inv<TL><<<nblocks, kInvThreads, diag_inv_smem<TL>(), st>>>(blocks, P, Lx, Inv, status);
 }
 template <class TL>
 void launch_chain_mats(const int2 *tasks, int ntasks, const DevPlan &P, const TL *Lx, const TL *Inv, TL *Mch, TL *Gch,
@@ -784,8 +788,10 @@ void launch_bwd_blocks(const int4 *tasks, int ntasks, int *ticket, const DevPlan
     k_bwd_blocks<TL><<<solve_grid(ntasks), 256, kBwdSmem, st>>>(tasks, ntasks, ticket, P, Lx, Inv, Gch, Dpiv, y, flags,
                                                                  hand, epoch, status);
 }
-template void launch_diag_inv<double>(const int *, int, const DevPlan &, const double *, double *, cudaStream_t);
-template void launch_diag_inv<float>(const int *, int, const DevPlan &, const float *, float *, cudaStream_t);
+template void launch_diag_inv<double>(const int *, int, const DevPlan &, const double *, double *,
+                                      const unsigned long long *, cudaStream_t);
+template void launch_diag_inv<float>(const int *, int, const DevPlan &, const float *, float *, const unsigned long long *,
+                                     cudaStream_t);
 template void launch_chain_mats<double>(const int2 *, int, const DevPlan &, const double *, const double *, double *,
                                         double *, cudaStream_t);
 template void launch_chain_mats<float>(const int2 *, int, const DevPlan &, const float *, const float *, float *,
