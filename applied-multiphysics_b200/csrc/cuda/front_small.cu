@@ -88,6 +88,7 @@ __device__ void assemble_warp(int s, const DevPlan &P, const double *__restrict_
   __syncwarp();
   // A's entries of all nc pivot columns (one contiguous CSR range): slot dst = j m + i of the L panel, each (i, j) once
   for (int p = p0 + lane; p < p1; p += 32) F[P.asmDst[p]] += (TC)(T)__ldg(values + P.asmSrc[p]);
+  __syncwarp();  // other lanes add the children to these entries
   pdl_wait();  // the children's level
   for (int qb = 0; qb < nch; qb += 32) {  // the metadata of up to 32 children, one per lane
     const int nq = min(32, nch - qb);
