@@ -884,6 +884,7 @@ int guarded(F &&fn) {
     g_err.clear();
     return fn();
   } catch (const CudaError &e) {
+    cudaGetLastError();  // this call's error (out of memory, say) is not the next launch check's
     return e.code;
   } catch (const std::bad_alloc &) {
     return fail(AMP_OOM, "host allocation failed");
