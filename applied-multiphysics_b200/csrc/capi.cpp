@@ -14,6 +14,7 @@
 #include <stdexcept>
 #include <string>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "../../include/ampsolve.h"
@@ -986,6 +987,7 @@ void upload_cx(amp_plan *pl) {
   if (pl->cxUploaded) return;
   const amp::Plan &P = pl->P;
   amp::build_dense_all(P, pl->cx);
+  std::vector<amp::CSolveLevel> levels;  // the plan's only once everything is there: an upload that throws is tried again
   for (int L = 0; L < P.nlevels; L++) {
     int maxNc = 0, maxM = 0;
     for (int i = P.lvlPtr[L]; i < P.lvlPtr[L + 1]; i++) {
@@ -993,7 +995,7 @@ void upload_cx(amp_plan *pl) {
       maxM = std::max(maxM, P.snM[P.lvlSn[i]]);
     }
     if (P.lvlPtr[L + 1] > P.lvlPtr[L])
-      pl->cxSolve.push_back(amp::csolve_level(P.lvlPtr[L], P.lvlPtr[L + 1] - P.lvlPtr[L], maxNc, maxM));
+      levels.push_back(amp::csolve_level(P.lvlPtr[L], P.lvlPtr[L + 1] - P.lvlPtr[L], maxNc, maxM));
   }
   DevMem &m = pl->mem;
   pl->dCxAsm = m.upload(pl->cx.asmTasks);
@@ -1002,6 +1004,7 @@ void upload_cx(amp_plan *pl) {
   pl->dCxStrips = m.upload(pl->cx.strips);
   pl->dCxTiles = m.upload(pl->cx.tileTasks);
   pl->dCxU = m.upload(pl->cx.uTasks);
+  pl->cxSolve = std::move(levels);
   pl->cxUploaded = true;
 }
 
