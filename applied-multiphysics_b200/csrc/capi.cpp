@@ -229,7 +229,7 @@ struct amp_factor_s {
   __nv_bfloat16 *dWhi = nullptr, *dWlo = nullptr;   // mixed LDL^T: BF16 split of L21 D
   CUtensorMap *dMaps = nullptr;                     // per supernode: TMA descriptors of the split A and B operands
   unsigned long long *dStatus = nullptr;
-  double *dLinv = nullptr;     // group panels: inverses of the 8 x 8 diagonal blocks of every pivot block (scratch)
+  double *dLinv = nullptr;     // FP64 group panels: inverses of the 8 x 8 diagonal blocks of every pivot block (scratch)
   int *dGroupFlags = nullptr;  // group panels: flags of every item, then the ticket counter of every group step
   long long waitSpins = 0;  // bound of the device waits in polls (0 = the kernels' defaults)
   bool ok = false, hasValues = false;
@@ -536,9 +536,9 @@ void enqueue_factor(amp_factor *f) {
       for (int k = P.lvlStepPtr[L]; k < P.lvlStepPtr[L + 1]; k++) {
         const amp::StepRange &sr = P.steps[k];
         timed(f, K_PANEL, sr.panelFlops, 0.0, [&] {
-          amp::launch_group_panel<float>(f->plan->dGroupItems, f->plan->dStrips + sr.strip0,
-                                         (int)(sr.strip1 - sr.strip0), tickets + sr.ticket, f->dGroupFlags, dp,
-                                         f->dL32, f->dLinv, f->dStatus, f->dShi, f->dSlo, ld32, st);
+          amp::launch_group_panel(f->plan->dGroupItems, f->plan->dStrips + sr.strip0, (int)(sr.strip1 - sr.strip0),
+                                  tickets + sr.ticket, f->dGroupFlags, dp, f->dL32, f->dStatus, f->dShi, f->dSlo, ld32,
+                                  st);
         });
         la.trsm_done();
         la.before_part_a();
@@ -596,9 +596,8 @@ void enqueue_factor(amp_factor *f) {
     for (int k = P.lvlStepPtr[L]; k < P.lvlStepPtr[L + 1]; k++) {
       const amp::StepRange &sr = P.steps[k];
       timed(f, K_PANEL, sr.panelFlops, 0.0, [&] {
-        amp::launch_group_panel<double>(f->plan->dGroupItems, f->plan->dStrips + sr.strip0,
-                                        (int)(sr.strip1 - sr.strip0), tickets + sr.ticket, f->dGroupFlags, dp, f->dLx,
-                                        f->dLinv, f->dStatus, nullptr, nullptr, ld, st);
+        amp::launch_group_panel(f->plan->dGroupItems, f->plan->dStrips + sr.strip0, (int)(sr.strip1 - sr.strip0),
+                                tickets + sr.ticket, f->dGroupFlags, dp, f->dLx, f->dLinv, f->dStatus, ld, st);
       });
       la.trsm_done();
       la.before_part_a();
@@ -1032,9 +1031,8 @@ void enqueue_cfactor(amp_factor *f) {
     for (int k = D.lvlStepPtr[L]; k < D.lvlStepPtr[L + 1]; k++) {
       const amp::StepRange &sr = D.steps[k];
       timed(f, K_PANEL, 4.0 * sr.panelFlops, 0.0, [&] {
-        amp::launch_group_panel<amp::cplx>(f->plan->dCxItems, f->plan->dCxStrips + sr.strip0,
-                                           (int)(sr.strip1 - sr.strip0), tickets + sr.ticket, f->dCxFlags, dp,
-                                           f->dLc, f->dLinv, f->dStatus, nullptr, nullptr, ld, st);
+        amp::launch_group_panel(f->plan->dCxItems, f->plan->dCxStrips + sr.strip0, (int)(sr.strip1 - sr.strip0),
+                                tickets + sr.ticket, f->dCxFlags, dp, f->dLc, f->dLinv, f->dStatus, ld, st);
       });
       if (sr.tile1 > sr.tile0)
         timed(f, K_UPDATE, 4.0 * (sr.updateFlopsA + sr.updateFlopsB), 0.0, [&] {
@@ -1401,7 +1399,7 @@ int amp_factor_create(amp_plan *pl, const amp_factor_opts *opts, amp_factor **ou
       }
       f->dTickets = f->mem.alloc<int>(2);
       f->dGroupFlags = f->mem.alloc<int>((size_t)std::max(1, P.nGroupFlags + P.nGroupTickets));
-      f->dLinv = f->mem.alloc<double>((size_t)P.nGroupFlags / 2 * amp::linv_stride(1));
+      if (!f->dL32) f->dLinv = f->mem.alloc<double>((size_t)P.nGroupFlags / 2 * amp::linv_stride(1));
       f->dDone = f->mem.alloc<int>((size_t)kSlices * std::max(1, P.nsuper));
       f->dSolveStatus = f->mem.alloc<unsigned long long>(1);
       init_device_once(pl->device);

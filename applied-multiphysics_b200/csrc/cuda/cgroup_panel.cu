@@ -87,7 +87,7 @@ __device__ __forceinline__ void load_cblock(double *S, const cplx *L, int m, int
 }
 
 // Pivot steps of eight columns: buffers of 64 rows x 8 columns, planar (row stride 10 as the real FP64 steps)
-constexpr int kRowLd = col_ld<double>();
+constexpr int kRowLd = kColLd;
 constexpr int kStepPlane = kPanel * kRowLd, kStepBuf = 2 * kStepPlane;
 __device__ __forceinline__ void cstep_tile(CTile &c, const double *P, const double *Q, int g, int t) {
   const double2 ar = *reinterpret_cast<const double2 *>(P + g * kRowLd + 2 * t);
@@ -517,10 +517,9 @@ cudaError_t init_cgroup_panel_attributes() {
   return cudaFuncSetAttribute(k_cgroup_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCGroupSmem);
 }
 
-template <>
-void launch_group_panel<cplx>(const GroupItem *items, const StripTask *strips, int nstrips, int *ticket, int *flags,
-                              const DevPlan &P, cplx *Lx, double *Linv, unsigned long long *status, __nv_bfloat16 *,
-                              __nv_bfloat16 *, const LdltArgs<cplx> &ld, cudaStream_t st) {
+void launch_group_panel(const GroupItem *items, const StripTask *strips, int nstrips, int *ticket, int *flags,
+                        const DevPlan &P, cplx *Lx, double *Linv, unsigned long long *status, const LdltArgs<cplx> &ld,
+                        cudaStream_t st) {
   if (nstrips > 0)
     k_cgroup_panel<<<(unsigned)nstrips, 256, kCGroupSmem, st>>>(items, strips, nstrips, ticket, flags, P, Lx, Linv,
                                                                status, ld);

@@ -15,23 +15,16 @@
 
 #include <algorithm>
 #include <cstdint>
-#include <type_traits>
 
 #include "../host/plan.hpp"
 #include "devplan.cuh"
 #include "launch.hpp"
 #include "pivot_steps.cuh"
+#include "small_fronts.cuh"
 #include "sync.cuh"
 
 namespace amp {
 
-// Tiny fronts come in two size classes (sorted by m within each level by the plan): m <= kTinyMid with 8 warps per
-// CTA and 16 x 16 tiles, and kTinyMid < m <= 32 with 4 warps per CTA and 32 x 32 tiles, so that the many smallest fronts
-// are not held to the shared memory of the largest.
-template <int MAXM>
-constexpr int tiny_warps() {
-  return MAXM <= kTinyMid ? 8 : 4;
-}
 // entries per lane in flight during the assembly, and CTAs per SM that the registers are held to: the m <= 16 class is
 // bound by the warps in flight (157,000 leaves of a batch: 262 us at 98 registers and two CTAs per SM)
 template <int MAXM>
@@ -43,32 +36,8 @@ constexpr int tiny_ctas() {
   return MAXM <= kTinyMid ? 4 : 5;
 }
 
-template <int G>
-__device__ __forceinline__ void group_sync() {
-  if constexpr (G == 32)
-    __syncwarp();
-  else
-    __syncthreads();
-}
-
-// |d| < tau (or NaN) becomes -tau / +tau by the sign of d; a non-finite small pivot fails (ldlt.mjs:513-522)
-template <class T>
-__device__ __forceinline__ bool small_ldlt_pivot(T &d, T tau, int &neg, int &pert) {
-  if (!(fabs(d) >= tau)) {
-    if (!isfinite(d)) return false;
-    d = d < T(0) ? -tau : tau;
-    pert++;
-  }
-  if (d < T(0)) neg++;
-  return true;
-}
-
-// Children of one front whose metadata and row maps a CTA holds at a time (fetched in parallel, applied in the
-// reference's order); a map's entries are front positions below 128
-constexpr int kChildChunk = 32;
-struct ChildMeta {
-  int muc[kChildChunk];
-  int64_t uo[kChildChunk], ea[kChildChunk];
+// The children's row maps as well; a map's entries are front positions below 128
+struct ChildMaps : ChildMeta {
   unsigned char map[kChildChunk][kSmallFront];
 };
 
@@ -78,16 +47,16 @@ struct ChildMeta {
 
 // Zero F (m x m, column-major), add A's entries of the pivot columns and the children's update matrices in the
 // reference's order. One warp, m <= 32: a lane per row of the child.
-template <class T, class TC, int kBatch>
-__device__ void assemble_warp(int s, const DevPlan &P, const double *__restrict__ values, const T *__restrict__ U,
-                              TC *F, int lane) {
+template <int kBatch>
+__device__ void assemble_warp(int s, const DevPlan &P, const double *__restrict__ values, const double *__restrict__ U,
+                              double *F, int lane) {
   const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s];
   const int q0 = P.chPtr[s], nch = P.chPtr[s + 1] - q0;
   const int p0 = P.asmColPtr[f], p1 = P.asmColPtr[f + nc];
-  for (int e = lane; e < m * m; e += 32) F[e] = TC(0);
+  for (int e = lane; e < m * m; e += 32) F[e] = 0.0;
   __syncwarp();
   // A's entries of all nc pivot columns (one contiguous CSR range): slot dst = j m + i of the L panel, each (i, j) once
-  for (int p = p0 + lane; p < p1; p += 32) F[P.asmDst[p]] += (TC)(T)__ldg(values + P.asmSrc[p]);
+  for (int p = p0 + lane; p < p1; p += 32) F[P.asmDst[p]] += __ldg(values + P.asmSrc[p]);
   __syncwarp();  // other lanes add the children to these entries
   pdl_wait();  // the children's level
   for (int qb = 0; qb < nch; qb += 32) {  // the metadata of up to 32 children, one per lane
@@ -101,16 +70,16 @@ __device__ void assemble_warp(int s, const DevPlan &P, const double *__restrict_
       uo = P.snUoff[c];
     }
     // batch (q, b0): columns [b0, b0 + kBatch) of child q, row a = lane; pos: the child row's front position
-    auto fetch = [&](int q, int b0, T(&v)[kBatch], int &mq, int &pos) {
+    auto fetch = [&](int q, int b0, double(&v)[kBatch], int &mq, int &pos) {
       mq = __shfl_sync(0xffffffffu, muc, q);
       const int64_t eq = __shfl_sync(0xffffffffu, ea, q), uq = __shfl_sync(0xffffffffu, uo, q);
       pos = lane < mq ? P.eaMap[eq + lane] : 0;
-      const T *Uc = U + uq;
+      const double *Uc = U + uq;
 #pragma unroll
       for (int i = 0; i < kBatch; i++)
-        v[i] = lane < mq && b0 + i <= lane ? Uc[(b0 + i) * mq + lane] : T(0);
+        v[i] = lane < mq && b0 + i <= lane ? Uc[(b0 + i) * mq + lane] : 0.0;
     };
-    T v[kBatch], vn[kBatch];
+    double v[kBatch], vn[kBatch];
     int mq = 0, pos = 0, mn = 0, pn = 0;
     fetch(0, 0, v, mq, pos);
     for (int q = 0, b0 = 0; q < nq;) {
@@ -119,7 +88,7 @@ __device__ void assemble_warp(int s, const DevPlan &P, const double *__restrict_
 #pragma unroll
       for (int i = 0; i < kBatch; i++) {
         const int col = __shfl_sync(0xffffffffu, pos, min(b0 + i, 31));
-        if (lane < mq && b0 + i <= lane) F[col * m + pos] += (TC)v[i];
+        if (lane < mq && b0 + i <= lane) F[col * m + pos] += v[i];
       }
       __syncwarp();
 #pragma unroll
@@ -135,9 +104,9 @@ __device__ void assemble_warp(int s, const DevPlan &P, const double *__restrict_
 
 // The same by a CTA of NT threads (m <= 128): warps over the child's columns, lanes over its rows. Ends with a barrier;
 // false (in every thread) when the factorization has failed.
-template <class T, class TC, int NT>
-__device__ bool assemble_cta(int s, const DevPlan &P, const double *__restrict__ values, const T *__restrict__ U, TC *F,
-                             ChildMeta *cm, const unsigned long long *status) {
+template <int NT>
+__device__ bool assemble_cta(int s, const DevPlan &P, const double *__restrict__ values, const double *__restrict__ U,
+                             double *F, ChildMaps *cm, const unsigned long long *status) {
   constexpr int NW = NT / 32;
   constexpr int kBatch = 16;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -153,9 +122,9 @@ __device__ bool assemble_cta(int s, const DevPlan &P, const double *__restrict__
     }
   };
   metadata(0, min(kChildChunk, nch));
-  for (int e = t; e < m * m; e += NT) F[e] = TC(0);
+  for (int e = t; e < m * m; e += NT) F[e] = 0.0;
   __syncthreads();
-  for (int p = p0 + t; p < p1; p += NT) F[P.asmDst[p]] += (TC)(T)__ldg(values + P.asmSrc[p]);
+  for (int p = p0 + t; p < p1; p += NT) F[P.asmDst[p]] += __ldg(values + P.asmSrc[p]);
   pdl_wait();  // the children's level
   const bool bad = t == 0 && factor_failed(status);  // one read for the CTA (sync.cuh), in time for the last barrier
   for (int qb = 0; qb < nch; qb += kChildChunk) {
@@ -166,20 +135,20 @@ __device__ bool assemble_cta(int s, const DevPlan &P, const double *__restrict__
     }
     // batch (q, i): rows [128 i' ..) of 4 of the warp's columns of child q: columns b = warp + NW (4 i + j), j < 4, rows
     // b + lane + 32 h, h < 4
-    auto fetch = [&](int q, int i, T(&v)[kBatch]) {
+    auto fetch = [&](int q, int i, double(&v)[kBatch]) {
       const int mq = cm->muc[q];
-      const T *Uc = U + cm->uo[q];
+      const double *Uc = U + cm->uo[q];
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         const int b = warp + NW * (4 * i + j);
 #pragma unroll
         for (int h = 0; h < 4; h++) {
           const int a = b + lane + 32 * h;
-          v[4 * j + h] = a < mq ? Uc[b * mq + a] : T(0);
+          v[4 * j + h] = a < mq ? Uc[b * mq + a] : 0.0;
         }
       }
     };
-    T v[kBatch], vn[kBatch];
+    double v[kBatch], vn[kBatch];
     fetch(0, 0, v);
     for (int e = t; e < nq * kSmallFront; e += NT) {
       const int q = e / kSmallFront, a = e % kSmallFront;
@@ -195,11 +164,11 @@ __device__ bool assemble_cta(int s, const DevPlan &P, const double *__restrict__
       for (int j = 0; j < 4; j++) {
         const int b = warp + NW * (4 * i + j);
         if (b >= mq) continue;
-        TC *col = F + map[b] * m;
+        double *col = F + map[b] * m;
 #pragma unroll
         for (int h = 0; h < 4; h++) {
           const int a = b + lane + 32 * h;
-          if (a < mq) col[map[a]] += (TC)v[4 * j + h];
+          if (a < mq) col[map[a]] += v[4 * j + h];
         }
       }
       if (qn != q) __syncthreads();  // the next child adds to the same entries from other warps
@@ -212,27 +181,26 @@ __device__ bool assemble_cta(int s, const DevPlan &P, const double *__restrict__
   return !__syncthreads_or(bad);
 }
 
-// The whole front of supernode s by one warp (m <= 32) over the shared m x m column-major tile F, in the compute type TC
-// (FP64, as the storage type T: the FP32 factors' kernels are in front_small_f32.cu).
+// The whole front of supernode s by one warp (m <= 32) over the shared m x m column-major tile F.
 //
 // Column k of the elimination is one phase with one barrier: every lane reads the pivot F(k, k) (final since the
 // previous barrier), computes the same pivot decision and scale, writes its share of L's column k straight to Lx and
 // updates its share of the trailing triangle from the unscaled column k, which nobody writes in the phase. The
 // arithmetic is the column-scaled form's: l_i = F(i, k) / r (Cholesky, r = sqrt F(k, k)) or F(i, k) / d (LDL^T), and
 // F(i, j) -= l_i (l_j d) with d = 1 for Cholesky.
-template <class T, class TC, int MAXM>
-__device__ void factor_front_warp(int s, const DevPlan &P, const double *__restrict__ values, T *__restrict__ Lx,
-                                  T *__restrict__ U, TC *F, unsigned long long *status, const LdltArgs<T> &la,
+template <int MAXM>
+__device__ void factor_front_warp(int s, const DevPlan &P, const double *__restrict__ values, double *__restrict__ Lx,
+                                  double *__restrict__ U, double *F, unsigned long long *status, const LdltArgs<double> &la,
                                   int lane) {
   const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s], mu = m - nc;
   const bool ldlt = la.scal != nullptr;
-  const TC tau = ldlt ? (TC)(T)la.scal[1] : TC(0);
-  assemble_warp<T, TC, tiny_batch<MAXM>()>(s, P, values, U, F, lane);
+  const double tau = ldlt ? la.scal[1] : 0.0;
+  assemble_warp<tiny_batch<MAXM>()>(s, P, values, U, F, lane);
   if (warp_failed(status)) return;
   int neg = 0, pert = 0;  // lane 0
-  T *Lp = Lx + P.snLxp[s];
+  double *Lp = Lx + P.snLxp[s];
   for (int k = 0; k < nc; k++) {
-    TC d = F[k * m + k], inv, dk, diag;
+    double d = F[k * m + k], inv, dk, diag;
     if (ldlt) {
       int n1 = 0, p1 = 0;
       const bool ok = small_ldlt_pivot(d, tau, n1, p1);
@@ -243,28 +211,28 @@ __device__ void factor_front_warp(int s, const DevPlan &P, const double *__restr
       if (lane == 0) {
         neg += n1;
         pert += p1;
-        la.D[f + k] = (double)(T)d;
+        la.D[f + k] = d;
       }
       dk = d;
-      inv = TC(1) / d;
-      diag = TC(1);
+      inv = 1.0 / d;
+      diag = 1.0;
     } else {
-      if (!(d > TC(0))) {
+      if (!(d > 0.0)) {
         if (lane == 0) atomicMin(status, status_word(f + k, 1, s));
         return;  // warp-uniform
       }
-      const TC r = sqrt(d);
-      dk = TC(1);
-      inv = TC(1) / r;
+      const double r = sqrt(d);
+      dk = 1.0;
+      inv = 1.0 / r;
       diag = r;
     }
-    const TC *Fk = F + k * m;
+    const double *Fk = F + k * m;
     const int i = lane;  // the lane's row
-    const TC li = i < m ? Fk[i] * inv : TC(0);
-    if (i >= k && i < m) Lp[(int64_t)k * m + i] = (T)(i == k ? diag : li);
+    const double li = i < m ? Fk[i] * inv : 0.0;
+    if (i >= k && i < m) Lp[(int64_t)k * m + i] = i == k ? diag : li;
 #pragma unroll 4
     for (int j = k + 1; j < m; j++) {
-      const TC lj = __shfl_sync(0xffffffffu, li, j) * dk;
+      const double lj = __shfl_sync(0xffffffffu, li, j) * dk;
       if (i >= j && i < m) F[j * m + i] -= li * lj;
     }
     __syncwarp();
@@ -273,14 +241,14 @@ __device__ void factor_front_warp(int s, const DevPlan &P, const double *__restr
     atomicAdd(la.counts, neg);
     atomicAdd(la.counts + 1, pert);
   }
-  T *Up = U + P.snUoff[s];
+  double *Up = U + P.snUoff[s];
   for (int jj = 0; jj < mu; jj++) {
     const int ii = jj + lane;
-    if (ii < mu) Up[(int64_t)jj * mu + ii] = (T)F[(nc + jj) * m + nc + ii];
+    if (ii < mu) Up[(int64_t)jj * mu + ii] = F[(nc + jj) * m + nc + ii];
   }
 }
 
-// The whole front of supernode s (32 < m <= MAXM, 64 or 128) by one CTA, in TC (as above). The front is assembled in
+// The whole front of supernode s (32 < m <= MAXM, 64 or 128) by one CTA. The front is assembled in
 // shared memory and then held in registers, as C fragments of its 8 x 8 tiles: eight warps own the row groups (w, and
 // for 128 rows also 15 - w), MAXM / 32 more warps take the pivot columns, a row per lane (pivot_steps.cuh). Eight pivot
 // columns per step with two barriers: the panel warps eliminate them; the others update their tiles of the next eight
@@ -289,24 +257,21 @@ __device__ void factor_front_warp(int s, const DevPlan &P, const double *__restr
 // The steps' columns stay in shared memory (over the front, which is dead by then) until they are scaled and written.
 template <int MAXM>
 constexpr int small_threads() { return 32 * (8 + MAXM / 32); }
-// shared memory (entries of TC) for fronts of at most m rows and nc pivot columns: the front, or the steps' columns over
+// shared memory (entries) for fronts of at most m rows and nc pivot columns: the front, or the steps' columns over
 // it, and three step buffers
-template <class TC>
 __host__ __device__ constexpr int small_main(int m, int nc) {
-  const int f = m * m, p = (nc + 7) / 8 * ((m + 7) / 8 * 8) * col_ld<TC>();
+  const int f = m * m, p = (nc + 7) / 8 * ((m + 7) / 8 * 8) * kColLd;
   return ((f > p ? f : p) + 3) & ~3;
 }
-template <class TC>
-constexpr int small_elems(int m, int nc) { return small_main<TC>(m, nc) + 3 * ((m + 7) / 8 * 8) * col_ld<TC>(); }
+constexpr int small_elems(int m, int nc) { return small_main(m, nc) + 3 * ((m + 7) / 8 * 8) * kColLd; }
 
-template <class T, class TC, bool LDLT, int MAXM>
+template <bool LDLT, int MAXM>
 __global__ void __launch_bounds__(small_threads<MAXM>(), MAXM == 64 ? 2 : 1)
     k_front_small(const int *__restrict__ fronts, int mainElems, DevPlan P, const double *__restrict__ values,
-                  T *__restrict__ Lx, T *__restrict__ U, unsigned long long *status, LdltArgs<T> la) {
-  using V2 = typename Vec2<TC>::type;
-  constexpr int NT = small_threads<MAXM>(), NP = MAXM / 32, CL = col_ld<TC>(), NG = MAXM / 64;
+                  double *__restrict__ Lx, double *__restrict__ U, unsigned long long *status, LdltArgs<double> la) {
+  constexpr int NT = small_threads<MAXM>(), NP = MAXM / 32, CL = kColLd, NG = MAXM / 64;
   extern __shared__ __align__(16) unsigned char fs_dyn[];
-  __shared__ ChildMeta cm;
+  __shared__ ChildMaps cm;
   __shared__ double scale[MAXM], diag[MAXM];
   __shared__ int failAt, inexact, nNeg, nPert;
   pdl_next();
@@ -314,31 +279,31 @@ __global__ void __launch_bounds__(small_threads<MAXM>(), MAXM == 64 ? 2 : 1)
   const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s], mu = m - nc;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int rows = (m + 7) & ~7, RB = rows / 8, steps = (nc + 7) / 8, pst = rows * CL;
-  TC *F = reinterpret_cast<TC *>(fs_dyn), *R = F + mainElems, *Q = R + pst, *Pc = F;  // Pc: -a of every step
-  T *Lp = Lx + P.snLxp[s];
-  T *Up = U + (mu > 0 ? P.snUoff[s] : 0);
-  const TC tau = LDLT ? (TC)(T)la.scal[1] : TC(0);
-  if (!assemble_cta<T, TC, NT>(s, P, values, U, F, &cm, status)) return;
+  double *F = reinterpret_cast<double *>(fs_dyn), *R = F + mainElems, *Q = R + pst, *Pc = F;  // Pc: -a of every step
+  double *Lp = Lx + P.snLxp[s];
+  double *Up = U + (mu > 0 ? P.snUoff[s] : 0);
+  const double tau = LDLT ? la.scal[1] : 0.0;
+  if (!assemble_cta<NT>(s, P, values, U, F, &cm, status)) return;
   // the front's tiles: row group rg[h], tile column cb
   const int rg[2] = {warp, NG == 2 ? 15 - warp : -1};
-  auto tile = [&](int rb, int cb, TC(&c)[2]) {
+  auto tile = [&](int rb, int cb, double(&c)[2]) {
     const int i = 8 * rb + g;
 #pragma unroll
     for (int u = 0; u < 2; u++) {
       const int j = 8 * cb + 2 * t + u;
-      c[u] = i < m && j <= i ? F[j * m + i] : i == j ? TC(1) : TC(0);
+      c[u] = i < m && j <= i ? F[j * m + i] : i == j ? 1.0 : 0.0;
     }
   };
-  auto hand_over = [&](int rb, const TC(&c)[2]) {
-    V2 v;
+  auto hand_over = [&](int rb, const double(&c)[2]) {
+    double2 v;
     v.x = c[0];
     v.y = c[1];
-    *reinterpret_cast<V2 *>(R + (8 * rb + g) * CL + 2 * t) = v;
+    *reinterpret_cast<double2 *>(R + (8 * rb + g) * CL + 2 * t) = v;
   };
   if (warp < 8) {
 #pragma unroll
     for (int h = 0; h < NG; h++) {
-      TC c0[2];
+      double c0[2];
       if (rg[h] < RB) {
         tile(rg[h], 0, c0);
         hand_over(rg[h], c0);
@@ -352,7 +317,7 @@ __global__ void __launch_bounds__(small_threads<MAXM>(), MAXM == 64 ? 2 : 1)
   if (warp >= 8) {
     __syncthreads();  // the front is in registers: Pc may overwrite it
     for (int k = 0; k < steps; k++) {
-      TC *Pk = Pc + k * pst, *Qk = Q + (k & 1) * pst;
+      double *Pk = Pc + k * pst, *Qk = Q + (k & 1) * pst;
       const int r = min(8 * k + 32 * (warp - 8) + lane, rows - 1), w = nc - 8 * k;
       const bool mine = 8 * k + 32 * (warp - 8) < rows;
       if (mine) {
@@ -369,7 +334,7 @@ __global__ void __launch_bounds__(small_threads<MAXM>(), MAXM == 64 ? 2 : 1)
       __syncthreads();
     }
   } else {
-    TC ca[7][2], cb[NG == 2 ? 15 : 1][2];  // at step k: the tiles (rg[h], k + 1), (rg[h], k + 2), ...
+    double ca[7][2], cb[NG == 2 ? 15 : 1][2];  // at step k: the tiles (rg[h], k + 1), (rg[h], k + 2), ...
 #pragma unroll
     for (int j = 0; j < 7; j++)
       if (rg[0] < RB && j < rg[0]) tile(rg[0], j + 1, ca[j]);
@@ -382,7 +347,7 @@ __global__ void __launch_bounds__(small_threads<MAXM>(), MAXM == 64 ? 2 : 1)
     for (int k = 0; k < steps; k++) {
       __syncthreads();
       if (inexact) __syncthreads();
-      const TC *Pk = Pc + k * pst, *Qk = Q + (k & 1) * pst;
+      const double *Pk = Pc + k * pst, *Qk = Q + (k & 1) * pst;
       const bool on0 = rg[0] > k && rg[0] < RB, on1 = NG == 2 && rg[1] > k && rg[1] < RB;
       if (on0) {
         step_tile(ca[0], Pk + 8 * rg[0] * CL, Qk + 8 * (k + 1) * CL, CL, g, t);
@@ -422,12 +387,12 @@ __global__ void __launch_bounds__(small_threads<MAXM>(), MAXM == 64 ? 2 : 1)
       }
     }
     // the update block (of a failed front too: nobody reads it)
-    auto put = [&](int rb, int tc, const TC(&c)[2]) {
+    auto put = [&](int rb, int tc, const double(&c)[2]) {
       const int i = 8 * rb + g;
 #pragma unroll
       for (int u = 0; u < 2; u++) {
         const int j = 8 * tc + 2 * t + u;
-        if (i < m && j <= i) Up[(int64_t)(j - nc) * mu + i - nc] = (T)c[u];
+        if (i < m && j <= i) Up[(int64_t)(j - nc) * mu + i - nc] = c[u];
       }
     };
     if (rg[0] < RB) {
@@ -445,12 +410,12 @@ __global__ void __launch_bounds__(small_threads<MAXM>(), MAXM == 64 ? 2 : 1)
   }
   // the pivots: test and count, the columns' scales
   if (tid < MAXM) {
-    double d = tid < nc ? -(double)Pc[(tid >> 3) * pst + tid * CL + (tid & 7)] : 1.0;
+    double d = tid < nc ? -Pc[(tid >> 3) * pst + tid * CL + (tid & 7)] : 1.0;
     bool bad = false, small = false;
     if (LDLT) {
-      small = tid < nc && !(fabs(d) >= (double)tau);
+      small = tid < nc && !(fabs(d) >= tau);
       bad = small && !isfinite(d);
-      if (small) d = d < 0.0 ? -(double)tau : (double)tau;
+      if (small) d = d < 0.0 ? -tau : tau;
       const int neg = __popc(__ballot_sync(0xffffffffu, tid < nc && d < 0.0));
       const int pert = __popc(__ballot_sync(0xffffffffu, small));
       if (lane == 0) {
@@ -475,11 +440,11 @@ __global__ void __launch_bounds__(small_threads<MAXM>(), MAXM == 64 ? 2 : 1)
     const int r = tid & (MAXM - 1);
     for (int p = tid / MAXM; p < steps && tid < NT / MAXM * MAXM; p += NT / MAXM) {
       if (r < 8 * p || r >= m) continue;
-      const TC *Pr = Pc + p * pst + r * CL;
-      TC v[8];
+      const double *Pr = Pc + p * pst + r * CL;
+      double v[8];
 #pragma unroll
       for (int u = 0; u < 8; u += 2) {
-        const V2 x = *reinterpret_cast<const V2 *>(Pr + u);
+        const double2 x = *reinterpret_cast<const double2 *>(Pr + u);
         v[u] = -x.x;
         v[u + 1] = -x.y;
       }
@@ -488,14 +453,14 @@ __global__ void __launch_bounds__(small_threads<MAXM>(), MAXM == 64 ? 2 : 1)
         const int col = 8 * p + u;
         if (r < col) continue;
         if (col < nc)
-          Lp[(int64_t)col * m + r] = (T)(r == col ? (LDLT ? 1.0 : diag[col]) : (double)v[u] * scale[col]);
+          Lp[(int64_t)col * m + r] = r == col ? (LDLT ? 1.0 : diag[col]) : v[u] * scale[col];
         else
-          Up[(int64_t)(col - nc) * mu + r - nc] = (T)v[u];
+          Up[(int64_t)(col - nc) * mu + r - nc] = v[u];
       }
     }
   }
   if (LDLT) {
-    if (tid < nc) la.D[f + tid] = (double)(T)diag[tid];
+    if (tid < nc) la.D[f + tid] = diag[tid];
     if (tid == 0 && (nNeg | nPert)) {
       atomicAdd(la.counts, nNeg);
       atomicAdd(la.counts + 1, nPert);
@@ -526,25 +491,25 @@ __device__ __forceinline__ void front_warp_argmax(double &v, int &i) {
 // a faster warp goes on to interchange and update). A block's L columns go to Lx once the block is done (its later steps may
 // still interchange their rows), with its pivot order; D and D(k + 1, k) as they are decided. A column with no usable entry
 // in its block keeps the static perturbation to +-tau (counted); a non-finite pivot fails.
-template <class T, int G>
-__device__ void factor_front_bk(int s, const DevPlan &P, const double *__restrict__ values, T *__restrict__ Lx,
-                                T *__restrict__ U, double *F, unsigned long long *status, const LdltArgs<T> &la,
-                                int t, ChildMeta *cm) {
+template <int G>
+__device__ void factor_front_bk(int s, const DevPlan &P, const double *__restrict__ values, double *__restrict__ Lx,
+                                double *__restrict__ U, double *F, unsigned long long *status, const LdltArgs<double> &la,
+                                int t, ChildMaps *cm) {
   constexpr int NW = G / 32;
   const int warp = t >> 5, lane = t & 31;
   const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s], mu = m - nc;
   const double tau = la.scal[1];
   const double alpha = 0.64038820320220756;  // (1 + sqrt(17)) / 8
   if constexpr (G == 32) {
-    assemble_warp<T, double, 16>(s, P, values, U, F, t);
+    assemble_warp<16>(s, P, values, U, F, t);
     if (warp_failed(status)) return;
   } else {
-    if (!assemble_cta<T, double, G>(s, P, values, U, F, cm, status)) return;
+    if (!assemble_cta<G>(s, P, values, U, F, cm, status)) return;
   }
   auto at = [&](int i, int j) -> double & { return F[j * m + i]; };  // entry (i, j), i >= j
   int neg = 0, pert = 0;  // thread 0
   int perm[64];           // thread 0: the current block's pivot order
-  T *Lp = Lx + P.snLxp[s];
+  double *Lp = Lx + P.snLxp[s];
   for (int c0 = 0; c0 < nc; c0 += 64) {
     const int c1 = min(nc, c0 + 64);
     if (t == 0)
@@ -667,7 +632,7 @@ __device__ void factor_front_bk(int s, const DevPlan &P, const double *__restric
       k += step;
     }
     for (int j = c0; j < c1; j++)  // the block's L columns, unit diagonal, rows in the block's pivot order
-      for (int i = j + t; i < m; i += G) Lp[(int64_t)j * m + i] = (T)(i == j ? 1.0 : at(i, j));
+      for (int i = j + t; i < m; i += G) Lp[(int64_t)j * m + i] = i == j ? 1.0 : at(i, j);
     if (t == 0)
       for (int i = 0; i < c1 - c0; i++) la.piv[f + c0 + i] = perm[i];
   }
@@ -676,59 +641,58 @@ __device__ void factor_front_bk(int s, const DevPlan &P, const double *__restric
     atomicAdd(la.counts + 1, pert);
   }
   if (mu > 0) {
-    T *Up = U + P.snUoff[s];
+    double *Up = U + P.snUoff[s];
     for (int e = t; e < mu * mu; e += G) {
       const int jj = e / mu, ii = e - jj * mu;
-      if (ii >= jj) Up[e] = (T)F[(nc + jj) * m + nc + ii];
+      if (ii >= jj) Up[e] = F[(nc + jj) * m + nc + ii];
     }
   }
 }
 
 // m <= MAXM (16 or 32): one warp per front, tiny_warps<MAXM>() fronts per CTA
 // BK: Bunch-Kaufman pivots (FP64 factors with la.piv set)
-template <class T, class TC, int MAXM, bool BK>
-__global__ void __launch_bounds__(32 * tiny_warps<MAXM>(), BK ? 1 : tiny_ctas<MAXM>()) k_front_tiny(const int *__restrict__ fronts, int count,
-                                                                         DevPlan P, const double *__restrict__ values,
-                                                                         T *__restrict__ Lx, T *__restrict__ U,
-                                                                         unsigned long long *status, LdltArgs<T> la) {
+template <int MAXM, bool BK>
+__global__ void __launch_bounds__(32 * tiny_warps<MAXM>(), BK ? 1 : tiny_ctas<MAXM>())
+    k_front_tiny(const int *__restrict__ fronts, int count, DevPlan P, const double *__restrict__ values,
+                 double *__restrict__ Lx, double *__restrict__ U, unsigned long long *status, LdltArgs<double> la) {
   constexpr int W = tiny_warps<MAXM>();
-  __shared__ TC F[W][MAXM * MAXM];
+  __shared__ double F[W][MAXM * MAXM];
   pdl_next();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int idx = blockIdx.x * W + warp;
   if (idx >= count) return;  // warp-uniform; no CTA-wide barrier follows
   if constexpr (BK)
-    factor_front_bk<T, 32>(fronts[idx], P, values, Lx, U, F[warp], status, la, lane, nullptr);
+    factor_front_bk<32>(fronts[idx], P, values, Lx, U, F[warp], status, la, lane, nullptr);
   else
-    factor_front_warp<T, TC, MAXM>(fronts[idx], P, values, Lx, U, F[warp], status, la, lane);
+    factor_front_warp<MAXM>(fronts[idx], P, values, Lx, U, F[warp], status, la, lane);
 }
 
 // 32 < m <= 128 with Bunch-Kaufman pivots: one CTA per front; dynamic shared memory = the launch's largest m squared
-template <class T>
 __global__ void __launch_bounds__(256) k_front_small_bk(const int *__restrict__ fronts, DevPlan P,
-                                                        const double *__restrict__ values, T *__restrict__ Lx,
-                                                        T *__restrict__ U, unsigned long long *status, LdltArgs<T> la) {
+                                                        const double *__restrict__ values, double *__restrict__ Lx,
+                                                        double *__restrict__ U, unsigned long long *status,
+                                                        LdltArgs<double> la) {
   extern __shared__ __align__(16) unsigned char fs_dyn[];
-  __shared__ ChildMeta cm;
+  __shared__ ChildMaps cm;
   pdl_next();
-  factor_front_bk<T, 256>(fronts[blockIdx.x], P, values, Lx, U, reinterpret_cast<double *>(fs_dyn), status, la,
+  factor_front_bk<256>(fronts[blockIdx.x], P, values, Lx, U, reinterpret_cast<double *>(fs_dyn), status, la,
                           threadIdx.x, &cm);
 }
 
-template <class T, class TC, bool LDLT>
+template <bool LDLT>
 static cudaError_t init_small() {
-  const int bytes = small_elems<TC>(kSmallFront, kSmallFront) * (int)sizeof(TC);
-  cudaError_t e = cudaFuncSetAttribute(k_front_small<T, TC, LDLT, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  const int bytes = small_elems(kSmallFront, kSmallFront) * (int)sizeof(double);
+  cudaError_t e = cudaFuncSetAttribute(k_front_small<LDLT, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        bytes);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_front_small<T, TC, LDLT, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    e = cudaFuncSetAttribute(k_front_small<LDLT, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   return e;
 }
 cudaError_t init_front_small_attributes() {
-  cudaError_t e = init_small<double, double, false>();
-  if (e == cudaSuccess) e = init_small<double, double, true>();
+  cudaError_t e = init_small<false>();
+  if (e == cudaSuccess) e = init_small<true>();
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_front_small_bk<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(k_front_small_bk, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              kSmallFront * kSmallFront * (int)sizeof(double));
   return e;
 }
@@ -750,28 +714,28 @@ static void launch_level(void (*kernel)(KA...), bool after, int grid, int thread
   cudaLaunchKernelEx(&c, kernel, KA(args)...);
 }
 
-template <class T, class TC, int MAXM, bool BK>
-static int launch_tiny(bool after, const int *fronts, int count, const DevPlan &P, const double *values, T *Lx, T *U,
-                       unsigned long long *status, const LdltArgs<T> &la, cudaStream_t st) {
+template <int MAXM, bool BK>
+static int launch_tiny(bool after, const int *fronts, int count, const DevPlan &P, const double *values, double *Lx,
+                       double *U, unsigned long long *status, const LdltArgs<double> &la, cudaStream_t st) {
   constexpr int W = tiny_warps<MAXM>();
   if (count <= 0) return 0;
-  launch_level(k_front_tiny<T, TC, MAXM, BK>, after, (count + W - 1) / W, 32 * W, 0, st, fronts, count, P, values, Lx, U, status,
+  launch_level(k_front_tiny<MAXM, BK>, after, (count + W - 1) / W, 32 * W, 0, st, fronts, count, P, values, Lx, U, status,
                la);
   return 1;
 }
 
-template <class T, class TC, bool LDLT, int MAXM>
-static int launch_small(bool after, const SmallClass &c, const DevPlan &P, const double *values, T *Lx, T *U,
-                        unsigned long long *status, const LdltArgs<T> &la, cudaStream_t st) {
+template <bool LDLT, int MAXM>
+static int launch_small(bool after, const SmallClass &c, const DevPlan &P, const double *values, double *Lx, double *U,
+                        unsigned long long *status, const LdltArgs<double> &la, cudaStream_t st) {
   if (c.count <= 0) return 0;
-  launch_level(k_front_small<T, TC, LDLT, MAXM>, after, c.count, small_threads<MAXM>(),
-               small_elems<TC>(c.maxM, c.maxNc) * sizeof(TC), st, c.sn, small_main<TC>(c.maxM, c.maxNc), P, values, Lx, U,
+  launch_level(k_front_small<LDLT, MAXM>, after, c.count, small_threads<MAXM>(),
+               small_elems(c.maxM, c.maxNc) * sizeof(double), st, c.sn, small_main(c.maxM, c.maxNc), P, values, Lx, U,
                status, la);
   return 1;
 }
-template <class T, class TC, bool LDLT, bool BK>
-static int launch_fronts_tc(const SmallFronts &fr, const DevPlan &P, const double *values, T *Lx, T *U,
-                            unsigned long long *status, const LdltArgs<T> &la, cudaStream_t st) {
+template <bool LDLT, bool BK>
+static int launch_fronts_tc(const SmallFronts &fr, const DevPlan &P, const double *values, double *Lx, double *U,
+                            unsigned long long *status, const LdltArgs<double> &la, cudaStream_t st) {
   // a class of its own only where the GPU would otherwise not hold the level's fronts at once: two launches one after
   // the other take twice a front's latency
   const int mid = fr.ntiny <= num_sms() * tiny_warps<kTinyFront>() ? 0 : fr.ntinyMid;
@@ -780,32 +744,29 @@ static int launch_fronts_tc(const SmallFronts &fr, const DevPlan &P, const doubl
     full = SmallClass{half.sn, half.count + full.count, full.maxM, std::max(half.maxNc, full.maxNc)};
     half.count = 0;
   }
-  int k = launch_tiny<T, TC, kTinyMid, BK>(fr.after, fr.tiny, mid, P, values, Lx, U, status, la, st);
-  k += launch_tiny<T, TC, kTinyFront, BK>(fr.after, fr.tiny + mid, fr.ntiny - mid, P, values, Lx, U, status, la, st);
+  int k = launch_tiny<kTinyMid, BK>(fr.after, fr.tiny, mid, P, values, Lx, U, status, la, st);
+  k += launch_tiny<kTinyFront, BK>(fr.after, fr.tiny + mid, fr.ntiny - mid, P, values, Lx, U, status, la, st);
   if constexpr (BK) {
     for (const SmallClass &c : {half, full})
       if (c.count > 0) {
-        launch_level(k_front_small_bk<T>, fr.after, c.count, 256, (size_t)c.maxM * c.maxM * sizeof(TC), st, c.sn, P, values,
+        launch_level(k_front_small_bk, fr.after, c.count, 256, (size_t)c.maxM * c.maxM * sizeof(double), st, c.sn, P, values,
                      Lx, U, status, la);
         k++;
       }
   } else {
-    k += launch_small<T, TC, LDLT, 64>(fr.after, half, P, values, Lx, U, status, la, st);
-    k += launch_small<T, TC, LDLT, 128>(fr.after, full, P, values, Lx, U, status, la, st);
+    k += launch_small<LDLT, 64>(fr.after, half, P, values, Lx, U, status, la, st);
+    k += launch_small<LDLT, 128>(fr.after, full, P, values, Lx, U, status, la, st);
   }
   return k;
 }
-template <class T>
-int launch_fronts_small(const SmallFronts &fr, const DevPlan &P, const double *values, T *Lx, T *U,
-                        unsigned long long *status, const LdltArgs<T> &la, cudaStream_t st) {
-  if constexpr (std::is_same<T, double>::value)
-    if (la.piv != nullptr)  // Bunch-Kaufman pivots (FP64)
-      return launch_fronts_tc<T, double, true, true>(fr, P, values, Lx, U, status, la, st);
+template <>
+int launch_fronts_small<double>(const SmallFronts &fr, const DevPlan &P, const double *values, double *Lx, double *U,
+                                unsigned long long *status, const LdltArgs<double> &la, cudaStream_t st) {
+  if (la.piv != nullptr)  // Bunch-Kaufman pivots (FP64)
+      return launch_fronts_tc<true, true>(fr, P, values, Lx, U, status, la, st);
   if (la.scal != nullptr)  // LDL^T: FP64 arithmetic whatever the storage
-    return launch_fronts_tc<T, double, true, false>(fr, P, values, Lx, U, status, la, st);
-  return launch_fronts_tc<T, T, false, false>(fr, P, values, Lx, U, status, la, st);
+    return launch_fronts_tc<true, false>(fr, P, values, Lx, U, status, la, st);
+  return launch_fronts_tc<false, false>(fr, P, values, Lx, U, status, la, st);
 }
-template int launch_fronts_small<double>(const SmallFronts &, const DevPlan &, const double *, double *, double *,
-                                         unsigned long long *, const LdltArgs<double> &, cudaStream_t);
 
 }  // namespace amp

@@ -6,55 +6,20 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
-#include <type_traits>
 
 #include "../host/plan.hpp"
 #include "devplan.cuh"
 #include "launch.hpp"
+#include "small_fronts.cuh"
 #include "sync.cuh"
 
 namespace amp {
 
 namespace {
 
-// Tiny fronts come in two size classes (sorted by m within each level by the plan): m <= kTinyMid with 8 warps per
-// CTA and 16 x 16 tiles, and kTinyMid < m <= 32 with 4 warps per CTA and 32 x 32 tiles, so that the many smallest fronts
-// are not held to the shared memory of the largest.
-template <int MAXM>
-constexpr int tiny_warps() {
-  return MAXM <= kTinyMid ? 8 : 4;
-}
-
-template <int G>
-__device__ __forceinline__ void group_sync() {
-  if constexpr (G == 32)
-    __syncwarp();
-  else
-    __syncthreads();
-}
-
-// |d| < tau (or NaN) becomes -tau / +tau by the sign of d; a non-finite small pivot fails (ldlt.mjs:513-522)
-template <class T>
-__device__ __forceinline__ bool small_ldlt_pivot(T &d, T tau, int &neg, int &pert) {
-  if (!(fabs(d) >= tau)) {
-    if (!isfinite(d)) return false;
-    d = d < T(0) ? -tau : tau;
-    pert++;
-  }
-  if (d < T(0)) neg++;
-  return true;
-}
-
-// Children of one front whose metadata a group holds at a time (fetched in parallel, applied in the reference's order)
-constexpr int kChildChunk = 32;
-struct ChildMeta {
-  int muc[kChildChunk];
-  int64_t ea[kChildChunk], uo[kChildChunk];
-};
-
 // Zero F (m x m), add A's entries of the pivot columns and the children's update matrices in the reference's order.
-template <class T, class TC, int G>
-__device__ void assemble_front(int s, const DevPlan &P, const double *__restrict__ values, const T *__restrict__ U,
+template <class TC, int G>
+__device__ void assemble_front(int s, const DevPlan &P, const double *__restrict__ values, const float *__restrict__ U,
                                TC *F, int t, ChildMeta *cm) {
   const int warp = t >> 5, lane = t & 31;
   const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s];
@@ -63,7 +28,7 @@ __device__ void assemble_front(int s, const DevPlan &P, const double *__restrict
   // A's entries of all nc pivot columns (one contiguous CSR range): slot dst = j m + i of the L panel, each (i, j) once
   {
     const int p0 = P.asmColPtr[f], p1 = P.asmColPtr[f + nc];
-    for (int p = p0 + t; p < p1; p += G) F[P.asmDst[p]] += (TC)(T)__ldg(values + P.asmSrc[p]);
+    for (int p = p0 + t; p < p1; p += G) F[P.asmDst[p]] += (TC)(float)__ldg(values + P.asmSrc[p]);
   }
   group_sync<G>();
   // children's update matrices, one after another (the map is injective within a child); the metadata of up to
@@ -102,7 +67,7 @@ __device__ void assemble_front(int s, const DevPlan &P, const double *__restrict
       }
       if (mq <= 0) continue;  // group-uniform
       const int *map = P.eaMap + eq;
-      const T *Uc = U + uq;
+      const float *Uc = U + uq;
       for (int e = t; e < mq * mq; e += G) {
         const int b = e / mq, a = e - b * mq;
         if (a >= b) F[map[b] * m + map[a]] += (TC)Uc[e];
@@ -113,7 +78,7 @@ __device__ void assemble_front(int s, const DevPlan &P, const double *__restrict
 }
 
 // The whole front of supernode s by a group of G threads (thread t) over the shared m x m column-major tile F, in the
-// compute type TC (the storage type T of L and U, or FP64: an FP32 LDL^T factor's small fronts are computed in FP64
+// compute type TC (FP32 as L and U, or FP64: an FP32 LDL^T factor's small fronts are computed in FP64
 // and rounded once when stored, since the indefinite factor's pivots cancel). cm: the group's child metadata (G > 32;
 // a warp passes its child metadata by shuffles).
 //
@@ -122,20 +87,20 @@ __device__ void assemble_front(int s, const DevPlan &P, const double *__restrict
 // updates its share of the trailing triangle from the unscaled column k, which nobody writes in the phase. The
 // arithmetic is the column-scaled form's: l_i = F(i, k) / r (Cholesky, r = sqrt F(k, k)) or F(i, k) / d (LDL^T), and
 // F(i, j) -= l_i (l_j d) with d = 1 for Cholesky.
-template <class T, class TC, int G>
-__device__ void factor_front(int s, const DevPlan &P, const double *__restrict__ values, T *__restrict__ Lx,
-                             T *__restrict__ U, TC *F, unsigned long long *status, const LdltArgs<T> &la, int t,
+template <class TC, int G>
+__device__ void factor_front(int s, const DevPlan &P, const double *__restrict__ values, float *__restrict__ Lx,
+                             float *__restrict__ U, TC *F, unsigned long long *status, const LdltArgs<float> &la, int t,
                              ChildMeta *cm) {
   constexpr int NW = G / 32;
   const int warp = t >> 5, lane = t & 31;
   const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s], mu = m - nc;
   const bool ldlt = la.scal != nullptr;
-  const TC tau = ldlt ? (TC)(T)la.scal[1] : TC(0);
-  assemble_front<T, TC, G>(s, P, values, U, F, t, cm);
+  const TC tau = ldlt ? (TC)(float)la.scal[1] : TC(0);
+  assemble_front<TC, G>(s, P, values, U, F, t, cm);
   // partial factorization of the nc pivot columns, one barrier per column; warps over the trailing columns j, lanes
   // over the rows i >= j
   int neg = 0, pert = 0;  // thread 0
-  T *Lp = Lx + P.snLxp[s];
+  float *Lp = Lx + P.snLxp[s];
   for (int k = 0; k < nc; k++) {
     TC d = F[k * m + k], inv, dk, diag;
     if (ldlt) {
@@ -148,7 +113,7 @@ __device__ void factor_front(int s, const DevPlan &P, const double *__restrict__
       if (t == 0) {
         neg += n1;
         pert += p1;
-        la.D[f + k] = (double)(T)d;
+        la.D[f + k] = (double)(float)d;
       }
       dk = d;
       inv = TC(1) / d;
@@ -164,8 +129,8 @@ __device__ void factor_front(int s, const DevPlan &P, const double *__restrict__
       diag = r;
     }
     const TC *Fk = F + k * m;
-    T *Lk = Lp + (int64_t)k * m;
-    for (int i = k + t; i < m; i += G) Lk[i] = (T)(i == k ? diag : Fk[i] * inv);
+    float *Lk = Lp + (int64_t)k * m;
+    for (int i = k + t; i < m; i += G) Lk[i] = (float)(i == k ? diag : Fk[i] * inv);
     const int w = m - k - 1;
     for (int jj = warp; jj < w; jj += NW) {
       const int j = k + 1 + jj;
@@ -180,40 +145,40 @@ __device__ void factor_front(int s, const DevPlan &P, const double *__restrict__
     atomicAdd(la.counts + 1, pert);
   }
   if (mu > 0) {
-    T *Up = U + P.snUoff[s];
+    float *Up = U + P.snUoff[s];
     for (int e = t; e < mu * mu; e += G) {
       const int jj = e / mu, ii = e - jj * mu;
-      if (ii >= jj) Up[e] = (T)F[(nc + jj) * m + nc + ii];
+      if (ii >= jj) Up[e] = (float)F[(nc + jj) * m + nc + ii];
     }
   }
 }
 
 
 // m <= MAXM (16 or 32): one warp per front, tiny_warps<MAXM>() fronts per CTA
-// BK: Bunch-Kaufman pivots (FP64 factors with la.piv set)
-template <class T, class TC, int MAXM>
+template <class TC, int MAXM>
 __global__ void __launch_bounds__(32 * tiny_warps<MAXM>()) k_front_tiny_f32(const int *__restrict__ fronts, int count,
                                                                          DevPlan P, const double *__restrict__ values,
-                                                                         T *__restrict__ Lx, T *__restrict__ U,
-                                                                         unsigned long long *status, LdltArgs<T> la) {
+                                                                         float *__restrict__ Lx, float *__restrict__ U,
+                                                                         unsigned long long *status, LdltArgs<float> la) {
   constexpr int W = tiny_warps<MAXM>();
   __shared__ TC F[W][MAXM * MAXM];
   if (warp_failed(status)) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int idx = blockIdx.x * W + warp;
   if (idx >= count) return;  // warp-uniform; no CTA-wide barrier follows
-  factor_front<T, TC, 32>(fronts[idx], P, values, Lx, U, F[warp], status, la, lane, nullptr);
+  factor_front<TC, 32>(fronts[idx], P, values, Lx, U, F[warp], status, la, lane, nullptr);
 }
 
 // 32 < m <= 128: one CTA per front; dynamic shared memory = the launch's largest m squared
-template <class T, class TC>
+template <class TC>
 __global__ void __launch_bounds__(256) k_front_small_f32(const int *__restrict__ fronts, int count, DevPlan P,
-                                                     const double *__restrict__ values, T *__restrict__ Lx,
-                                                     T *__restrict__ U, unsigned long long *status, LdltArgs<T> la) {
+                                                     const double *__restrict__ values, float *__restrict__ Lx,
+                                                     float *__restrict__ U, unsigned long long *status,
+                                                     LdltArgs<float> la) {
   extern __shared__ __align__(16) unsigned char fs_dyn[];
   __shared__ ChildMeta cm;
   if (cta_failed(status)) return;
-  factor_front<T, TC, 256>(fronts[blockIdx.x], P, values, Lx, U, reinterpret_cast<TC *>(fs_dyn), status, la,
+  factor_front<TC, 256>(fronts[blockIdx.x], P, values, Lx, U, reinterpret_cast<TC *>(fs_dyn), status, la,
                              threadIdx.x, &cm);
 }
 
@@ -226,12 +191,12 @@ int launch_f32(const SmallFronts &fr, const DevPlan &P, const double *values, fl
     kernel<<<(count + warps - 1) / warps, 32 * warps, 0, st>>>(fronts, count, P, values, Lx, U, status, la);
     k++;
   };
-  tiny(k_front_tiny_f32<float, TC, kTinyMid>, fr.tiny, fr.ntinyMid, tiny_warps<kTinyMid>());
-  tiny(k_front_tiny_f32<float, TC, kTinyFront>, fr.tiny + fr.ntinyMid, fr.ntiny - fr.ntinyMid, tiny_warps<kTinyFront>());
+  tiny(k_front_tiny_f32<TC, kTinyMid>, fr.tiny, fr.ntinyMid, tiny_warps<kTinyMid>());
+  tiny(k_front_tiny_f32<TC, kTinyFront>, fr.tiny + fr.ntinyMid, fr.ntiny - fr.ntinyMid, tiny_warps<kTinyFront>());
   const int small = fr.half.count + fr.full.count;  // (the two lists are one)
   if (small > 0) {
     const int maxM = fr.full.count > 0 ? fr.full.maxM : fr.half.maxM;
-    k_front_small_f32<float, TC><<<small, 256, (size_t)maxM * maxM * sizeof(TC), st>>>(fr.half.sn, small, P, values, Lx, U,
+    k_front_small_f32<TC><<<small, 256, (size_t)maxM * maxM * sizeof(TC), st>>>(fr.half.sn, small, P, values, Lx, U,
                                                                                        status, la);
     k++;
   }
@@ -241,10 +206,10 @@ int launch_f32(const SmallFronts &fr, const DevPlan &P, const double *values, fl
 }  // namespace
 
 cudaError_t init_front_small_f32_attributes() {
-  cudaError_t e = cudaFuncSetAttribute(k_front_small_f32<float, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaError_t e = cudaFuncSetAttribute(k_front_small_f32<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        kSmallFront * kSmallFront * (int)sizeof(float));
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_front_small_f32<float, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(k_front_small_f32<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              kSmallFront * kSmallFront * (int)sizeof(double));
   return e;
 }

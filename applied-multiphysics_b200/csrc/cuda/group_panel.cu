@@ -18,6 +18,7 @@
 
 #include "../host/plan.hpp"
 #include "devplan.cuh"
+#include "launch.hpp"
 #include "panel_blocks.cuh"
 #include "pivot_steps.cuh"
 
@@ -28,24 +29,23 @@ namespace {
 // Rows [i0, i0 + nr) x columns [j0, j0 + ncol) of a front's column-major block (ld m) into S; lower: only the entries
 // on and below the diagonal. The rest is zero, and with pad the diagonal entries from ncol on are one. Read through
 // L2 (another CTA of the running launch may have written them). 8 rows x 4 columns per warp access.
-template <class T>
-__device__ __forceinline__ void load_block(double *S, const T *L, int m, int i0, int nr, int j0, int ncol, bool lower,
+__device__ __forceinline__ void load_block(double *S, const double *L, int m, int i0, int nr, int j0, int ncol, bool lower,
                                            bool pad) {
   const int lane = threadIdx.x & 31, i = 8 * (threadIdx.x >> 5) + (lane >> 2), t = lane & 3;
-  T v[16];
+  double v[16];
 #pragma unroll
   for (int e = 0; e < 16; e++) {
     const int c = 4 * e + t;
-    v[e] = (i < nr && c < ncol && (!lower || c <= i)) ? __ldcg(L + (int64_t)(j0 + c) * m + i0 + i) : T(0);
+    v[e] = (i < nr && c < ncol && (!lower || c <= i)) ? __ldcg(L + (int64_t)(j0 + c) * m + i0 + i) : 0.0;
   }
 #pragma unroll
   for (int e = 0; e < 16; e++) {
     const int c = 4 * e + t;
-    S[sw(i, c)] = pad && i == c && i >= ncol ? 1.0 : (double)v[e];
+    S[sw(i, c)] = pad && i == c && i >= ncol ? 1.0 : v[e];
   }
 }
 
-// Pivot block: POTRF (or LDL^T) of the 64 x 64 diagonal block of a front, called by all 256 threads of a CTA, in TC.
+// Pivot block: POTRF (or LDL^T) of the 64 x 64 diagonal block of a front, called by all 256 threads of a CTA.
 // Ds: the updated block (lower part; identity from column w on), left unchanged; Lp: the block's
 // (0, 0) entry in the front (ld m), where the factor is written; w <= 64 its columns; scr: 11 step buffers; Linv:
 // the inverses of the eight 8 x 8 diagonal blocks of L (64 doubles each, row-major), for the strips' TRSM.
@@ -63,28 +63,27 @@ __device__ __forceinline__ void load_block(double *S, const T *L, int m, int i0,
 // diagonal, LDL^T L = a / d with a unit diagonal (D to ld.D). Returns 0, or 1 (status set for the first failing column
 // f + c0 + k, nothing written) when a pivot failed. LB (the Bunch-Kaufman fast path): returns 2, writing nothing, when
 // a multiplier |L(i, k)| of the block exceeds lbound or a pivot was perturbed.
-template <class T, class TC, bool LDLT, bool LB>
-__device__ int potrf_block(const double *Ds, double *scr, T *Lp, double *Linv, int m, int w, int f, int c0, int s,
-                           unsigned long long *status, const LdltArgs<T> &ld, double lbound) {
-  using V2 = typename Vec2<TC>::type;
-  constexpr int CL = col_ld<TC>(), kStepBuf = kPanel * CL;
+template <bool LDLT, bool LB>
+__device__ int potrf_block(const double *Ds, double *scr, double *Lp, double *Linv, int m, int w, int f, int c0, int s,
+                           unsigned long long *status, const LdltArgs<double> &ld, double lbound) {
+  constexpr int CL = kColLd, kStepBuf = kPanel * CL;
   __shared__ double scale[kPanel], diag[kPanel];
   __shared__ int failAt, redo, nNeg, nPert, inexact;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, rg = row_group(warp);
   const int nk = (w + 7) >> 3;  // steps: the columns from w on are the identity's
-  const TC tau = LDLT ? (TC)ld.scal[1] : TC(0);
-  TC *R = reinterpret_cast<TC *>(scr), *Q = R + kStepBuf, *P = R + 3 * kStepBuf;  // Q: two buffers; P: -a of every step
+  const double tau = LDLT ? ld.scal[1] : 0.0;
+  double *R = scr, *Q = R + kStepBuf, *P = R + 3 * kStepBuf;  // Q: two buffers; P: -a of every step
   const int myRow = (8 * rg + g) * CL + 2 * t;
-  auto tile = [&](int cb, TC(&c)[2]) {  // this warp's tile (rg, cb) of the block
+  auto tile = [&](int cb, double(&c)[2]) {  // this warp's tile (rg, cb) of the block
     const double2 v = pair_at(Ds, 8 * rg + g, 8 * cb + 2 * t);
-    c[0] = (TC)v.x;
-    c[1] = (TC)v.y;
+    c[0] = v.x;
+    c[1] = v.y;
   };
-  auto hand_over = [&](const TC(&c)[2]) {
-    V2 v;
+  auto hand_over = [&](const double(&c)[2]) {
+    double2 v;
     v.x = c[0];
     v.y = c[1];
-    *reinterpret_cast<V2 *>(R + myRow) = v;
+    *reinterpret_cast<double2 *>(R + myRow) = v;
   };
   auto panel = [&](auto exact) {  // the first two warps, a row per lane
     bool fine = true;
@@ -94,7 +93,7 @@ __device__ int potrf_block(const double *Ds, double *scr, T *Lp, double *Linv, i
                                                                min(8 * k + 32 * warp + lane, kPanel - 1), 8, tau);
       __syncthreads();
       if (k == 0 && warp == 1) {  // row group 1's only trailing tile
-        TC c[2];
+        double c[2];
         tile(1, c);
         step_tile(c, P + 8 * CL, Q + 8 * CL, CL, g, t);
         hand_over(c);
@@ -104,15 +103,15 @@ __device__ int potrf_block(const double *Ds, double *scr, T *Lp, double *Linv, i
     if (!fine) inexact = 1;
   };
   auto trailing = [&]() {  // the other warps
-    TC c[7][2];  // at step k: the tiles (rg, k + 1), (rg, k + 2), ...
+    double c[7][2];  // at step k: the tiles (rg, k + 1), (rg, k + 2), ...
 #pragma unroll
     for (int j = 0; j < 7; j++) {
-      c[j][0] = c[j][1] = TC(0);
+      c[j][0] = c[j][1] = 0.0;
       if (j < rg) tile(j + 1, c[j]);
     }
     for (int k = 0; k < nk; k++) {
       __syncthreads();
-      const TC *Pk = P + k * kStepBuf + 8 * rg * CL, *Qk = Q + (k & 1) * kStepBuf;
+      const double *Pk = P + k * kStepBuf + 8 * rg * CL, *Qk = Q + (k & 1) * kStepBuf;
       if (rg > k) {
         step_tile(c[0], Pk, Qk + 8 * (k + 1) * CL, CL, g, t);
         hand_over(c[0]);
@@ -129,7 +128,7 @@ __device__ int potrf_block(const double *Ds, double *scr, T *Lp, double *Linv, i
     }
   };
   for (int pass = 0; pass < 2; pass++) {
-    TC first[2];
+    double first[2];
     tile(0, first);
     hand_over(first);
     if (tid == 0) {
@@ -149,12 +148,12 @@ __device__ int potrf_block(const double *Ds, double *scr, T *Lp, double *Linv, i
   }
   // the pivots: test and count, the columns' scales
   if (tid < kPanel) {
-    double d = -(double)P[(tid >> 3) * kStepBuf + tid * CL + (tid & 7)];
+    double d = -P[(tid >> 3) * kStepBuf + tid * CL + (tid & 7)];
     bool bad = false, small = false;
     if (LDLT) {
-      small = tid < w && !(fabs(d) >= (double)tau);
+      small = tid < w && !(fabs(d) >= tau);
       bad = small && !isfinite(d);
-      if (small) d = d < 0.0 ? -(double)tau : (double)tau;
+      if (small) d = d < 0.0 ? -tau : tau;
       const int neg = __popc(__ballot_sync(0xffffffffu, tid < w && d < 0.0));
       const int pert = __popc(__ballot_sync(0xffffffffu, small));
       if (lane == 0) {
@@ -175,7 +174,7 @@ __device__ int potrf_block(const double *Ds, double *scr, T *Lp, double *Linv, i
   if (LB) {  // the multipliers a / d of the strictly lower part (a failed pivot exceeds the bound too)
     for (int e = tid; e < kPanel * kPanel; e += 256) {
       const int r = e & (kPanel - 1), j = e >> 6;
-      if (r > j && r < w && !(fabs((double)P[(j >> 3) * kStepBuf + r * CL + (j & 7)]) <= lbound * fabs(diag[j]))) redo = 1;
+      if (r > j && r < w && !(fabs(P[(j >> 3) * kStepBuf + r * CL + (j & 7)]) <= lbound * fabs(diag[j]))) redo = 1;
     }
     __syncthreads();
     if (redo) return 2;
@@ -188,22 +187,22 @@ __device__ int potrf_block(const double *Ds, double *scr, T *Lp, double *Linv, i
     const int r = tid & (kPanel - 1);
     for (int p = (tid >> 6) - 1; p < 8; p += 3) {
       if (r < 8 * p || r >= w) continue;
-      const TC *Pr = P + p * kStepBuf + r * CL;
-      T *dst = Lp + (int64_t)(8 * p) * m + r;
-      T v[8];
+      const double *Pr = P + p * kStepBuf + r * CL;
+      double *dst = Lp + (int64_t)(8 * p) * m + r;
+      double v[8];
 #pragma unroll
       for (int u = 0; u < 8; u += 2) {
-        const V2 a = *reinterpret_cast<const V2 *>(Pr + u);
-        v[u] = (T)(-(double)a.x * scale[8 * p + u]);
-        v[u + 1] = (T)(-(double)a.y * scale[8 * p + u + 1]);
+        const double2 a = *reinterpret_cast<const double2 *>(Pr + u);
+        v[u] = -a.x * scale[8 * p + u];
+        v[u + 1] = -a.y * scale[8 * p + u + 1];
       }
 #pragma unroll
       for (int u = 0; u < 8; u++)
-        if (r >= 8 * p + u) dst[(int64_t)u * m] = r > 8 * p + u ? v[u] : LDLT ? T(1) : (T)diag[r];
+        if (r >= 8 * p + u) dst[(int64_t)u * m] = r > 8 * p + u ? v[u] : LDLT ? 1.0 : diag[r];
     }
   } else {  // column j of inv(L_pp): forward substitution with the unit block, rows over the diagonal
     const int p = min(tid >> 3, nk - 1), j = tid & 7;  // (the strips use the first nk blocks)
-    const TC *Pp = P + p * kStepBuf + 8 * p * CL;
+    const double *Pp = P + p * kStepBuf + 8 * p * CL;
     double x[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) {
@@ -211,14 +210,14 @@ __device__ int potrf_block(const double *Ds, double *scr, T *Lp, double *Linv, i
 #pragma unroll
       for (int u = 0; u < i; u++) {
         const double sc = scale[8 * p + u];
-        v += ((double)Pp[i * CL + u] * (LDLT ? sc : sc * sc)) * x[u];
+        v += (Pp[i * CL + u] * (LDLT ? sc : sc * sc)) * x[u];
       }
       x[i] = i < j ? 0.0 : i == j ? 1.0 : v;  // (P holds -a)
     }
     double r2 = 0.0;  // squared norm of row j of the scaled block
 #pragma unroll
     for (int u = 0; u < 7; u++) {
-      const double a = u < j ? (double)Pp[j * CL + u] : 0.0, l = a * scale[8 * p + u];
+      const double a = u < j ? Pp[j * CL + u] : 0.0, l = a * scale[8 * p + u];
       r2 += LDLT ? fabs(a * l) : l * l;
     }
     r2 += LDLT ? fabs(diag[8 * p + j]) : diag[8 * p + j] * diag[8 * p + j];
@@ -268,7 +267,7 @@ __device__ __forceinline__ double fast_recip(double d) {
 // (Bunch and Kaufman, Math. Comp. 31, 1977). Each interchange is applied to the block's whole rows, the L columns
 // already computed included, so that P B P^T = L D L^T with L unit lower triangular (L(k + 1, k) = 0 inside a 2 x 2
 // pivot, whose off-diagonal is D(k + 1, k)). A column with no entry at or above tau keeps the reference's static
-// perturbation (|d| < tau -> -+tau, a non-finite one fails; ldlt.mjs:513-522). FP64 arithmetic for every T.
+// perturbation (|d| < tau -> -+tau, a non-finite one fails; ldlt.mjs:513-522).
 // S: 64 x 65 doubles of shared workspace (a full symmetric copy, S[j][i] = B(i, j)); Ds: the updated block (lower part),
 // overwritten by L. Writes L to Lp (ld m), D, Doff and piv, adds the inertia (a 2 x 2 pivot with a
 // negative determinant has one negative eigenvalue, with a positive one two when its diagonal is negative) and the
@@ -279,9 +278,8 @@ __device__ __forceinline__ double fast_recip(double d) {
 // pivot's columns stay unscaled in S once they are chosen. Thread (i, q) holds the entries S[q + 4 u][i] in registers and
 // stores those that the step has changed. With physical interchanges, one warp choosing and five barriers per column, the
 // panels of the edge-element system with 13 elements per edge took 4.49 ms, now 2.56 ms (a full block 67,000 clocks).
-template <class T>
-__device__ bool bk_block(double *Ds, double (*S)[kPanel + 1], T *Lp, double *Linv, int m, int w, int f, int c0, int s,
-                         unsigned long long *status, const LdltArgs<T> &ld) {
+__device__ bool bk_block(double *Ds, double (*S)[kPanel + 1], double *Lp, double *Linv, int m, int w, int f, int c0, int s,
+                         unsigned long long *status, const LdltArgs<double> &ld) {
   __shared__ int sPerm[kPanel];
   __shared__ double sD[kPanel], sE[kPanel];
   __shared__ double sT[kPanel], sG[kPanel];  // 1 x 1: 1 / d, -; 2 x 2 (k, k + 1): t / e twice, c and a
@@ -314,7 +312,7 @@ __device__ bool bk_block(double *Ds, double (*S)[kPanel + 1], T *Lp, double *Lin
     const unsigned long long xm = warp_max_key(max(x0, x1));
     const double colmax = __longlong_as_double((long long)xm), absakk = fabs(S[c][c]);
     int step = 1, r = c, posR = k;  // r: the row of the larger pivot, at position posR
-    if (colmax > 0.0 && !(absakk >= alpha * colmax)) {  // (a NaN diagonal takes the 1 x 1 path and fails below)
+    if (colmax > 0.0 && !(absakk >= alpha * colmax)) {  // (a NaN diagonal goes on too, and fails at its own turn)
       const unsigned at0 = (p0 > k && x0 == xm) ? (unsigned)p0 : ~0u, at1 = (p1 > k && x1 == xm) ? (unsigned)p1 : ~0u;
       posR = (int)__reduce_min_sync(kAll, min(at0, at1));  // the first in the pivot order
       r = row_at(posR);
@@ -419,7 +417,7 @@ __device__ bool bk_block(double *Ds, double (*S)[kPanel + 1], T *Lp, double *Lin
         x = S[sPerm[j]][ri] * sT[j];
       }
     }
-    if (i < w && j <= i) Lp[(int64_t)j * m + i] = (T)x;
+    if (i < w && j <= i) Lp[(int64_t)j * m + i] = x;
     Ds[kPanel * j + i] = x;
   }
   __syncthreads();
@@ -505,12 +503,12 @@ __device__ __forceinline__ void substitute8(const double (&c)[2], double (&w)[2]
 // releases P[b], so every waiter leaves.
 constexpr int kBlockElems = kPanel * kPanel;
 constexpr int kGroupSmem = 3 * kBlockElems * (int)sizeof(double);  // two CTAs per SM
-template <class T, bool LDLT, bool BK>
+template <bool LDLT, bool BK>
 __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restrict__ items,
                                                         const StripTask *__restrict__ strips, int nstrips, int *ticket,
-                                                        int *flags, DevPlan P, T *__restrict__ Lx,
+                                                        int *flags, DevPlan P, double *__restrict__ Lx,
                                                         double *__restrict__ Linv, unsigned long long *status,
-                                                        LdltArgs<T> ld) {
+                                                        LdltArgs<double> ld) {
   extern __shared__ __align__(16) unsigned char gp_raw[];
   double *Ls = reinterpret_cast<double *>(gp_raw);  // pivot block, rows of another diagonal strip, POTRF step buffers
   double *Xs = Ls + kBlockElems;                    // this strip's solved rows (Bunch-Kaufman: column exchange)
@@ -532,7 +530,7 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
   const int r0 = st.r0, r1 = st.r1, jd = st.diag;
   const int bmax = jd >= 0 ? jd : nb;  // pivot blocks whose rows below include this strip
   const int64_t lxp = P.snLxp[s];
-  T *L = Lx + lxp;
+  double *L = Lx + lxp;
   int *Pf = flags + it.flag0, *Df = Pf + nb;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int lr = 8 * row_group(warp) + g, row = r0 + lr;  // this lane's row of every fragment
@@ -544,12 +542,12 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
   for (int b = 0; b < bmax; b++) {
     const int c0 = g0 + b * kPanel, w = min(kPanel, g1 - c0);
     double x[8][2];  // the strip's rows of block b
-    const T *src = L + (int64_t)(c0 + 2 * t) * m + row;
+    const double *src = L + (int64_t)(c0 + 2 * t) * m + row;
 #pragma unroll
     for (int p = 0; p < 8; p++)
 #pragma unroll
       for (int u = 0; u < 2; u++)
-        x[p][u] = act && 8 * p + 2 * t + u < w ? (double)__ldcg(src + (int64_t)(8 * p + u) * m) : 0.0;
+        x[p][u] = act && 8 * p + 2 * t + u < w ? __ldcg(src + (int64_t)(8 * p + u) * m) : 0.0;
     for (int q = 0; q < b; q++) {
       const int cq = g0 + q * kPanel;
       if (b > 1) {  // read the strip's solved rows back (with one earlier block they are still in registers)
@@ -561,7 +559,7 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
             double v = 0.0;
             if (act) {
               const int64_t at = (int64_t)cc * m + row;
-              v = BK ? (double)__ldcg(ld.W + lxp + at) : (double)__ldcg(L + at);
+              v = BK ? __ldcg(ld.W + lxp + at) : __ldcg(L + at);
               if (LDLT && !BK) v *= __ldcg(ld.D + f + cc);
             }
             nx[p][u] = -v;
@@ -651,7 +649,7 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
       for (int p = 0; p < 8; p++) set_pair(Xs, lr, 8 * p + 2 * t, x[p][0], x[p][1]);
       __syncwarp();
     }
-    // x := L21's entries, rounded to the storage; nx := -W (W = x D for LDL^T)
+    // x := L21's entries; nx := -W (W = x D for LDL^T)
 #pragma unroll
     for (int p = 0; p < 8; p++)
 #pragma unroll
@@ -663,9 +661,9 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
           xv = dinv[cc] * wv + dB[cc] * Xs[sw(lr, dP[cc])];
         else if constexpr (LDLT)
           xv = wv * dinv[cc];
-        x[p][u] = (double)(T)xv;
+        x[p][u] = xv;
         nx[p][u] = BK ? -wv : LDLT ? -x[p][u] * dv[cc] : -x[p][u];
-        if (BK && act && cc < w) ld.W[lxp + (int64_t)(c0 + cc) * m + row] = (T)wv;
+        if (BK && act && cc < w) ld.W[lxp + (int64_t)(c0 + cc) * m + row] = wv;
       }
     if constexpr (BK) __syncwarp();
 #pragma unroll
@@ -679,8 +677,8 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
         if (r0 + r >= r1) continue;
         const double xv = Xs[sw(r, cc)];
         const int64_t at = (int64_t)(c0 + cc) * m + r0 + r;
-        L[at] = (T)xv;
-        if (LDLT && !BK && ld.W) ld.W[lxp + at] = (T)(xv * dv[cc]);
+        L[at] = xv;
+        if (LDLT && !BK && ld.W) ld.W[lxp + at] = xv * dv[cc];
       }
     }
     if (jd < 0) continue;
@@ -705,23 +703,22 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
   }
   if (jd >= 0) {  // this strip's own pivot block, fully updated: factor it and publish it (also after a failure)
     const int c0 = g0 + jd * kPanel, w = min(kPanel, g1 - c0);
-    T *Lp = L + (int64_t)c0 * m + c0;
+    double *Lp = L + (int64_t)c0 * m + c0;
     double *Lb = Linv + ((int64_t)(it.flag0 / 2) + jd) * linv_stride(1);
     __syncthreads();  // Ds complete (also when the strip had no earlier pivot block); Ls and Xs free
     if constexpr (BK) {
       // Bunch-Kaufman keeps every pivot of the block in place exactly when each multiplier is at most 1 / alpha in
       // magnitude and no pivot needs the perturbation: try the unpivoted LDL^T first, else redo the block with pivots
       // from its untouched entries
-      const int r = potrf_block<T, double, true, true>(Ds, Ls, Lp, Lb, m, w, f, c0, s, status, ld, 1.0 / 0.64038820320220756);
+      const int r = potrf_block<true, true>(Ds, Ls, Lp, Lb, m, w, f, c0, s, status, ld, 1.0 / 0.64038820320220756);
       if (r == 2) {
-        bk_block<T>(Ds, reinterpret_cast<double(*)[kPanel + 1]>(gp_raw), Lp, Lb, m, w, f, c0, s, status, ld);
+        bk_block(Ds, reinterpret_cast<double(*)[kPanel + 1]>(gp_raw), Lp, Lb, m, w, f, c0, s, status, ld);
       } else if (r == 0 && tid < w) {  // the identity pivot order, 1 x 1 pivots
         ld.piv[f + c0 + tid] = tid;
         ld.Doff[f + c0 + tid] = 0.0;
       }
     } else {
-      using TC = typename std::conditional<LDLT, double, T>::type;
-      potrf_block<T, TC, LDLT, false>(Ds, Ls, Lp, Lb, m, w, f, c0, s, status, ld, -1.0);
+      potrf_block<LDLT, false>(Ds, Ls, Lp, Lb, m, w, f, c0, s, status, ld, -1.0);
     }
     panel_release(Pf + jd, 1);
   }
@@ -729,34 +726,30 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
 
 }  // namespace
 
-template <class T, bool LDLT, bool BK>
+template <bool LDLT, bool BK>
 static cudaError_t init_one() {
-  return cudaFuncSetAttribute(k_group_panel<T, LDLT, BK>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupSmem);
+  return cudaFuncSetAttribute(k_group_panel<LDLT, BK>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupSmem);
 }
 cudaError_t init_group_panel_attributes() {
-  cudaError_t e = init_one<double, false, false>();
-  if (e == cudaSuccess) e = init_one<double, true, false>();
-  if (e == cudaSuccess) e = init_one<double, true, true>();
+  cudaError_t e = init_one<false, false>();
+  if (e == cudaSuccess) e = init_one<true, false>();
+  if (e == cudaSuccess) e = init_one<true, true>();
   return e;
 }
 
-template <class T>
 void launch_group_panel(const GroupItem *items, const StripTask *strips, int nstrips, int *ticket, int *flags,
-                        const DevPlan &P, T *Lx, double *Linv, unsigned long long *status, __nv_bfloat16 *,
-                        __nv_bfloat16 *, const LdltArgs<T> &ld, cudaStream_t st) {
+                        const DevPlan &P, double *Lx, double *Linv, unsigned long long *status, const LdltArgs<double> &ld,
+                        cudaStream_t st) {
   if (nstrips <= 0) return;
   auto run = [&](auto kernel) {
     kernel<<<(unsigned)nstrips, 256, kGroupSmem, st>>>(items, strips, nstrips, ticket, flags, P, Lx, Linv, status, ld);
   };
-  if constexpr (std::is_same<T, double>::value)
-    if (ld.piv) return run(k_group_panel<T, true, true>);  // Bunch-Kaufman pivot blocks
-  if (ld.scal)
-    run(k_group_panel<T, true, false>);
+  if (ld.piv)
+    run(k_group_panel<true, true>);  // Bunch-Kaufman pivot blocks
+  else if (ld.scal)
+    run(k_group_panel<true, false>);
   else
-    run(k_group_panel<T, false, false>);
+    run(k_group_panel<false, false>);
 }
-template void launch_group_panel<double>(const GroupItem *, const StripTask *, int, int *, int *, const DevPlan &,
-                                         double *, double *, unsigned long long *, __nv_bfloat16 *, __nv_bfloat16 *,
-                                         const LdltArgs<double> &, cudaStream_t);
 
 }  // namespace amp

@@ -7,7 +7,6 @@
 #include <cuda_runtime.h>
 
 #include <cfloat>
-#include <type_traits>
 
 #include "../host/plan.hpp"
 #include "devplan.cuh"
@@ -22,10 +21,10 @@ __device__ __forceinline__ double ldcg_v(const double *p) { return __ldcg(p); }
 __device__ __forceinline__ float ldcg_v(const float *p) { return __ldcg(p); }
 __device__ __forceinline__ double pivot_mag(double d) { return fabs(d); }
 __device__ __forceinline__ double pivot_mag(float d) { return fabs((double)d); }
-template <class T>
-__device__ __forceinline__ bool chol_pivot_ok(T d) { return d > T(0); }
-template <class T>
-__device__ __forceinline__ T chol_sqrt(T d) { return sqrt(d); }
+template <class TC>
+__device__ __forceinline__ bool chol_pivot_ok(TC d) { return d > TC(0); }
+template <class TC>
+__device__ __forceinline__ TC chol_sqrt(TC d) { return sqrt(d); }
 __device__ __forceinline__ double recip_nr(double d) {
   const double a = fabs(d);
   if (!(a > 1e-30 && a < 1e30)) return 1.0 / d;  // outside the float range of the first approximation
@@ -40,27 +39,22 @@ __device__ __forceinline__ double recip_nr(double d) {
 
 // Static pivot perturbation of LDL^T (ldlt.mjs:513-522): |d| < tau (or NaN) becomes -tau / +tau by the sign of d,
 // a non-finite small pivot fails the factorization. flags: bit 0 negative pivot, bit 1 perturbed. false = failure.
-template <class T>
-__device__ __forceinline__ bool ldlt_pivot(T &d, T tau, unsigned char &flags) {
+template <class TC>
+__device__ __forceinline__ bool ldlt_pivot(TC &d, TC tau, unsigned char &flags) {
   flags = 0;
   if (!(fabs(d) >= tau)) {
     if (!isfinite(d)) return false;
-    d = d < T(0) ? -tau : tau;
+    d = d < TC(0) ? -tau : tau;
     flags = 2;
   }
-  if (d < T(0)) flags |= 1;
+  if (d < TC(0)) flags |= 1;
   return true;
 }
 __device__ __forceinline__ double fast_recip(double d) { return recip_nr(d); }
 __device__ __forceinline__ float fast_recip(float d) { return __fdividef(1.0f, d); }
 
-// ---------------------------------------------------------------------------------------------------------------
-// Group panel: the pivot blocks of a group of up to kGroup 64-column blocks of a front, factored in one dataflow
-// launch (POTRF of each pivot block, TRSM of the rows below it, and the update of the group's remaining columns).
-// ---------------------------------------------------------------------------------------------------------------
-
 // Pivot block: POTRF (or LDL^T) of the 64 x 64 diagonal block of a front, called by all 256 threads of a CTA, the
-// block in registers. T = double: the FP64 factor; T = float: the mixed-precision factor. src: the updated block in
+// block in registers, in TC. src: the updated block in
 // shared memory, entry (i, j) at src[j lds + i]; Lp: the block's (0, 0) entry in the front (ld m), where the factor is
 // written; w <= 64 its columns. Thread t < 136 owns the 4 x 4 tile (ti, tj), ti >= tj, of the lower triangle.
 // Right-looking on the unscaled columns, four columns per step kb with two barriers: (1) the diagonal tile eliminates
@@ -71,17 +65,16 @@ __device__ __forceinline__ float fast_recip(float d) { return __fdividef(1.0f, d
 // scaled: Cholesky L = a / sqrt(d) with sqrt(d) on the diagonal, LDL^T L = a / d with a unit diagonal (D to ld.D).
 // Returns false (status set for the first failing column f + c0 + k) when a pivot failed; the block is then not
 // written back.
-template <class T, class TC>
-__device__ int potrf_core(const T *src, int lds, T *Lp, int m, int w, int f, int c0, int s,
-                          unsigned long long *status, const LdltArgs<T> &ld, double promoteBelow) {
+template <class TC>
+__device__ int potrf_core(const float *src, int lds, float *Lp, int m, int w, int f, int c0, int s,
+                          unsigned long long *status, const LdltArgs<float> &ld, double promoteBelow) {
   __shared__ TC col[2][4][kPanel];  // per 4-column block (double-buffered): the block's unscaled columns, by row
   __shared__ TC pd[kPanel], piv[2][4];
   __shared__ unsigned char pflag[kPanel];
   __shared__ int fail, promote;
   const int tid = threadIdx.x;
   const bool ldlt = ld.scal != nullptr;
-  using RT = typename real_of<TC>::type;
-  const RT tau = ldlt ? (RT)ld.scal[1] : RT(0);
+  const TC tau = ldlt ? (TC)ld.scal[1] : TC(0);
   // tile of this thread: row block ti, column block tj (ti >= tj), from tid by the triangular numbering
   int ti = 0;
   while ((ti + 1) * (ti + 2) / 2 <= tid) ti++;
@@ -177,12 +170,12 @@ __device__ int potrf_core(const T *src, int lds, T *Lp, int m, int w, int f, int
 #pragma unroll
       for (int r = 0; r < 4; r++) {
         const int i = 4 * ti + r;
-        if (i >= j && i < w && j < w) Lp[(int64_t)j * m + i] = (T)(i == j ? (ldlt ? TC(1) : lj) : a[r][c] * inv);
+        if (i >= j && i < w && j < w) Lp[(int64_t)j * m + i] = (float)(i == j ? (ldlt ? TC(1) : lj) : a[r][c] * inv);
       }
     }
   }
   if (ldlt) {
-    if (tid < w) ld.D[f + c0 + tid] = (typename LdltArgs<T>::DT)pd[tid];
+    if (tid < w) ld.D[f + c0 + tid] = (double)pd[tid];
     if (tid == 0) {
       int neg = 0, pert = 0;
       for (int k = 0; k < w; k++) neg += pflag[k] & 1, pert += pflag[k] >> 1;
@@ -197,20 +190,14 @@ __device__ int potrf_core(const T *src, int lds, T *Lp, int m, int w, int f, int
 // magnitude below FLT_EPSILON x max_i |A(i, i)| (a pivot with no correct FP32 digit left) is factored again from the
 // same entries (src is left unchanged) in FP64 arithmetic (stored FP32): the small-pivot blocks of the mixed-precision
 // indefinite factor get FP64 pivots. Returns false when a pivot failed (status set).
-template <class T>
-__device__ bool potrf_block(const T *src, int lds, T *Lp, int m, int w, int f, int c0, int s,
-                            unsigned long long *status, const LdltArgs<T> &ld) {
-  if constexpr (std::is_same<T, float>::value) {
-    if (ld.scal != nullptr) {
-      const double amax = ld.scal[0] > 0.0 ? ld.scal[1] / ld.scal[0] : 0.0;
-      const int r = potrf_core<float, float>(src, lds, Lp, m, w, f, c0, s, status, ld, amax * (double)FLT_EPSILON);
-      if (r != 2) return r == 0;
-      return potrf_core<float, double>(src, lds, Lp, m, w, f, c0, s, status, ld, -1.0) == 0;
-    }
-  }
-  return potrf_core<T, T>(src, lds, Lp, m, w, f, c0, s, status, ld, -1.0) == 0;
+__device__ bool potrf_block(const float *src, int lds, float *Lp, int m, int w, int f, int c0, int s,
+                            unsigned long long *status, const LdltArgs<float> &ld) {
+  if (ld.scal == nullptr) return potrf_core<float>(src, lds, Lp, m, w, f, c0, s, status, ld, -1.0) == 0;
+  const double amax = ld.scal[0] > 0.0 ? ld.scal[1] / ld.scal[0] : 0.0;
+  const int r = potrf_core<float>(src, lds, Lp, m, w, f, c0, s, status, ld, amax * (double)FLT_EPSILON);
+  if (r != 2) return r == 0;
+  return potrf_core<double>(src, lds, Lp, m, w, f, c0, s, status, ld, -1.0) == 0;
 }
-
 
 // TRSM of up to 64 rows [r0, r1) of a front (L: its column-major block, ld m) against its factored pivot block
 // [c0, c0 + w): x_k = (a_k - sum_{c<k} x_c M(k, c)) / M(k, k). Four threads per row, thread (row, q) holds columns
@@ -224,32 +211,31 @@ __device__ bool potrf_block(const T *src, int lds, T *Lp, int m, int w, int f, i
 // before it waited for the pivot block (the strip's own rows are final by then).
 // On return Ws[c][r] holds this strip's update operand (x, or x D for LDL^T) and M[c][r] the solved rows x
 // (c < w, r < r1 - r0; zero elsewhere): a diagonal strip's X_c for its own column block.
-template <class T>
-__device__ void trsm_strip(T *L, int m, int f, int c0, int w, int r0, int r1, int64_t lxp, int64_t sp,
-                           __nv_bfloat16 *Shi, __nv_bfloat16 *Slo, const LdltArgs<T> &ld, T (*M)[kPanel + 1],
-                           T (*Ws)[kPanel + 1], T *invd, T *dv, T (&x)[16]) {
+__device__ void trsm_strip(float *L, int m, int f, int c0, int w, int r0, int r1, int64_t lxp, int64_t sp,
+                           __nv_bfloat16 *Shi, __nv_bfloat16 *Slo, const LdltArgs<float> &ld, float (*M)[kPanel + 1],
+                           float (*Ws)[kPanel + 1], float *invd, float *dv, float (&x)[16]) {
   const bool ldlt = ld.scal != nullptr;
   const int tid = threadIdx.x, r = tid & (kPanel - 1), q = tid >> 6;
   {  // the pivot block: thread (r, q) loads row r of columns 16 q .. 16 q + 15 (times their pivots for LDL^T), and
      // thread r < 64 the pivot of column r, in one round trip
-    T v[16];
+    float v[16];
 #pragma unroll
     for (int u = 0; u < 16; u++) {
       const int c = 16 * q + u;
-      v[u] = (r < w && c < r) ? ldcg_v(L + (int64_t)(c0 + c) * m + c0 + r) : T(0);
+      v[u] = (r < w && c < r) ? ldcg_v(L + (int64_t)(c0 + c) * m + c0 + r) : 0.0f;
     }
     if (ldlt) {
 #pragma unroll
       for (int u = 0; u < 16; u++) {
         const int c = 16 * q + u;
-        v[u] = v[u] * (c < w ? (T)ldcg_v(ld.D + f + c0 + c) : T(1));
+        v[u] = v[u] * (c < w ? (float)ldcg_v(ld.D + f + c0 + c) : 1.0f);
       }
     }
     if (tid < kPanel) {
-      const T d = tid < w ? (ldlt ? (T)ldcg_v(ld.D + f + c0 + tid) : ldcg_v(L + (int64_t)(c0 + tid) * m + c0 + tid))
-                               : T(1);
+      const float d = tid < w ? (ldlt ? (float)ldcg_v(ld.D + f + c0 + tid) : ldcg_v(L + (int64_t)(c0 + tid) * m + c0 + tid))
+                               : 1.0f;
       dv[tid] = d;
-      invd[tid] = T(1) / d;
+      invd[tid] = 1.0f / d;
     }
 #pragma unroll
     for (int u = 0; u < 16; u++) M[r][16 * q + u] = v[u];
@@ -274,7 +260,7 @@ __device__ void trsm_strip(T *L, int m, int f, int c0, int w, int r0, int r1, in
 #pragma unroll 4
       for (int kk = 0; kk < 16; kk++) {
         const int k = 16 * p + kk;
-        const T xk = Ws[k][r];
+        const float xk = Ws[k][r];
 #pragma unroll
         for (int u = 0; u < 16; u++) x[u] -= xk * M[16 * q + u][k];
       }
@@ -285,10 +271,10 @@ __device__ void trsm_strip(T *L, int m, int f, int c0, int w, int r0, int r1, in
 #pragma unroll
   for (int u = 0; u < 16; u++) {
     const int cc = 16 * q + u;
-    T xv = x[u];
-    T wv = ldlt ? xv * dv[cc] : xv;
-    Ws[cc][r] = active && cc < w ? wv : T(0);
-    M[cc][r] = active && cc < w ? xv : T(0);  // the pivot block in M is no longer read
+    float xv = x[u];
+    float wv = ldlt ? xv * dv[cc] : xv;
+    Ws[cc][r] = active && cc < w ? wv : 0.0f;
+    M[cc][r] = active && cc < w ? xv : 0.0f;  // the pivot block in M is no longer read
     if (!active || cc >= w) continue;
     L[(int64_t)(c0 + cc) * m + row] = xv;
     if (ldlt && ld.W) ld.W[lxp + (int64_t)(c0 + cc) * m + row] = wv;
@@ -321,17 +307,16 @@ __device__ void trsm_strip(T *L, int m, int f, int c0, int w, int r0, int r1, in
 // releases P[b], so every waiter leaves.
 constexpr int kGroupSmem32 = 3 * kPanel * (kPanel + 1) * (int)sizeof(float);
 // two CTAs per SM (registers capped at 128)
-template <class T>
 __global__ void __launch_bounds__(256, 2) k_group_panel_f32(const GroupItem *__restrict__ items,
                                                      const StripTask *__restrict__ strips, int nstrips, int *ticket,
-                                                     int *flags, DevPlan P, T *__restrict__ Lx,
+                                                     int *flags, DevPlan P, float *__restrict__ Lx,
                                                      unsigned long long *status, __nv_bfloat16 *__restrict__ Shi,
-                                                     __nv_bfloat16 *__restrict__ Slo, LdltArgs<T> ld) {
+                                                     __nv_bfloat16 *__restrict__ Slo, LdltArgs<float> ld) {
   extern __shared__ __align__(16) unsigned char gp_raw[];
-  T(*M)[kPanel + 1] = reinterpret_cast<T(*)[kPanel + 1]>(gp_raw);  // pivot block (TRSM), then the X_c chunk
-  T(*Ws)[kPanel + 1] = reinterpret_cast<T(*)[kPanel + 1]>(gp_raw + kPanel * (kPanel + 1) * sizeof(T));
-  T(*Ds)[kPanel + 1] = reinterpret_cast<T(*)[kPanel + 1]>(gp_raw + 2 * kPanel * (kPanel + 1) * sizeof(T));
-  __shared__ T invd[kPanel], dv[kPanel];
+  float(*M)[kPanel + 1] = reinterpret_cast<float(*)[kPanel + 1]>(gp_raw);  // pivot block (TRSM), then the X_c chunk
+  float(*Ws)[kPanel + 1] = reinterpret_cast<float(*)[kPanel + 1]>(gp_raw + kPanel * (kPanel + 1) * sizeof(float));
+  float(*Ds)[kPanel + 1] = reinterpret_cast<float(*)[kPanel + 1]>(gp_raw + 2 * kPanel * (kPanel + 1) * sizeof(float));
+  __shared__ float invd[kPanel], dv[kPanel];
   __shared__ int sTicket;
   if (threadIdx.x == 0) sTicket = factor_failed(status) ? nstrips : atomicAdd(ticket, 1);
   __syncthreads();
@@ -344,7 +329,7 @@ __global__ void __launch_bounds__(256, 2) k_group_panel_f32(const GroupItem *__r
   const int nb = (g1 - g0 + kPanel - 1) / kPanel;
   const int r0 = st.r0, r1 = st.r1, jd = st.diag;
   const int bmax = jd >= 0 ? jd : nb;  // pivot blocks whose rows below include this strip
-  T *L = Lx + P.snLxp[s];
+  float *L = Lx + P.snLxp[s];
   int *Pf = flags + it.flag0, *Df = Pf + nb;
   const int tid = threadIdx.x, tr = tid & 15, tc = tid >> 4;
   // A diagonal strip keeps its own pivot block (columns [r0, r1), lower part) in shared memory while it updates it
@@ -352,22 +337,22 @@ __global__ void __launch_bounds__(256, 2) k_group_panel_f32(const GroupItem *__r
   if (jd >= 0) {
     for (int e = tid; e < kPanel * kPanel; e += blockDim.x) {
       const int i = e & 63, j = e >> 6;
-      Ds[j][i] = (r0 + i < r1 && j <= i) ? L[(int64_t)(r0 + j) * m + r0 + i] : T(0);
+      Ds[j][i] = (r0 + i < r1 && j <= i) ? L[(int64_t)(r0 + j) * m + r0 + i] : 0.0f;
     }
   }
   for (int b = 0; b < bmax; b++) {
     const int c0 = g0 + b * kPanel, w = min(kPanel, g1 - c0), c1 = c0 + w;
-    T x[16];  // this thread's part of the strip's rows of block b, loaded while the pivot block is not yet ready
+    float x[16];  // this thread's part of the strip's rows of block b, loaded while the pivot block is not yet ready
     {
       const int xr = r0 + (tid & (kPanel - 1)), xq = tid >> 6;
 #pragma unroll
       for (int u = 0; u < 16; u++) {
         const int c = 16 * xq + u;
-        x[u] = xr < r1 && c < w ? L[(int64_t)(c0 + c) * m + xr] : T(0);
+        x[u] = xr < r1 && c < w ? L[(int64_t)(c0 + c) * m + xr] : 0.0f;
       }
     }
     if (!panel_wait(Pf + b, 1, status, P.spin)) return;
-    trsm_strip<T>(L, m, f, c0, w, r0, r1, P.snLxp[s], P.snSp[s], Shi, Slo, ld, M, Ws, invd, dv, x);
+    trsm_strip(L, m, f, c0, w, r0, r1, P.snLxp[s], P.snSp[s], Shi, Slo, ld, M, Ws, invd, dv, x);
     if (jd >= 0) panel_release(Df + jd, b + 1);
     // Update with block b (C -= W_r X_c^T, K = w): a diagonal strip first its own pivot block (X_c = its solved rows,
     // left in M by the TRSM; into Ds), then the blocks between block b and its own; a strip below every remaining
@@ -381,17 +366,17 @@ __global__ void __launch_bounds__(256, 2) k_group_panel_f32(const GroupItem *__r
         if (!panel_wait(Df + (cb - g0) / kPanel, b + 1, status, P.spin)) return;
         for (int e = tid; e < kPanel * kPanel; e += blockDim.x) {  // X_c[k][jj] = L(cb + jj, c0 + k)
           const int k = e >> 6, jj = e & 63;
-          M[k][jj] = (k < w && jj < ncol) ? ldcg_v(L + (int64_t)(c0 + k) * m + cb + jj) : T(0);
+          M[k][jj] = (k < w && jj < ncol) ? ldcg_v(L + (int64_t)(c0 + k) * m + cb + jj) : 0.0f;
         }
         __syncthreads();
       }
-      T acc[4][4];
+      float acc[4][4];
 #pragma unroll
       for (int a = 0; a < 4; a++)
 #pragma unroll
-        for (int bb = 0; bb < 4; bb++) acc[a][bb] = T(0);
+        for (int bb = 0; bb < 4; bb++) acc[a][bb] = 0.0f;
       for (int k = 0; k < w; k++) {
-        T wv[4], xv[4];
+        float wv[4], xv[4];
 #pragma unroll
         for (int a = 0; a < 4; a++) wv[a] = Ws[k][tr + 16 * a];
 #pragma unroll
@@ -409,7 +394,7 @@ __global__ void __launch_bounds__(256, 2) k_group_panel_f32(const GroupItem *__r
           if (own) {
             if (jj <= i) Ds[jj][i] -= acc[a][bb];
           } else if (r0 + i < r1 && jj < ncol) {
-            T *cptr = L + (int64_t)(cb + jj) * m + r0 + i;
+            float *cptr = L + (int64_t)(cb + jj) * m + r0 + i;
             *cptr = *cptr - acc[a][bb];
           }
         }
@@ -419,7 +404,7 @@ __global__ void __launch_bounds__(256, 2) k_group_panel_f32(const GroupItem *__r
   if (jd >= 0) {  // this strip's own pivot block, fully updated: factor it and publish it (also after a failure)
     const int c0 = g0 + jd * kPanel, w = min(kPanel, g1 - c0);
     __syncthreads();  // Ds complete (also when the strip had no earlier pivot block)
-    potrf_block<T>(&Ds[0][0], kPanel + 1, L + (int64_t)c0 * m + c0, m, w, f, c0, s, status, ld);
+    potrf_block(&Ds[0][0], kPanel + 1, L + (int64_t)c0 * m + c0, m, w, f, c0, s, status, ld);
     panel_release(Pf + jd, 1);
   }
 }
@@ -428,15 +413,14 @@ __global__ void __launch_bounds__(256, 2) k_group_panel_f32(const GroupItem *__r
 }  // namespace
 
 cudaError_t init_group_panel_f32_attributes() {
-  return cudaFuncSetAttribute(k_group_panel_f32<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupSmem32);
+  return cudaFuncSetAttribute(k_group_panel_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupSmem32);
 }
 
-template <>
-void launch_group_panel<float>(const GroupItem *items, const StripTask *strips, int nstrips, int *ticket, int *flags,
-                               const DevPlan &P, float *Lx, double *, unsigned long long *status, __nv_bfloat16 *Shi,
-                               __nv_bfloat16 *Slo, const LdltArgs<float> &ld, cudaStream_t st) {
+void launch_group_panel(const GroupItem *items, const StripTask *strips, int nstrips, int *ticket, int *flags,
+                        const DevPlan &P, float *Lx, unsigned long long *status, __nv_bfloat16 *Shi, __nv_bfloat16 *Slo,
+                        const LdltArgs<float> &ld, cudaStream_t st) {
   if (nstrips > 0)
-    k_group_panel_f32<float><<<(unsigned)nstrips, 256, kGroupSmem32, st>>>(items, strips, nstrips, ticket, flags, P, Lx,
+    k_group_panel_f32<<<(unsigned)nstrips, 256, kGroupSmem32, st>>>(items, strips, nstrips, ticket, flags, P, Lx,
                                                                           status, Shi, Slo, ld);
 }
 

@@ -19,11 +19,17 @@ template <class T>
 void launch_assemble(const AsmTask *tasks, const ChildRange *ranges, int64_t ntasks, const DevPlan &P,
                      const value_of<T> *values, T *Lx, T *U, const unsigned long long *status, cudaStream_t st);
 // one group of pivot blocks per item: nstrips strip tasks, ticket and flags zeroed before the factorization; Linv: linv_stride
-// doubles per pivot block of the schedule (block b of an item at flag0 / 2 + b), scratch of the launches
-template <class T>
+// doubles per pivot block of the schedule (block b of an item at flag0 / 2 + b), scratch of the launches; Shi, Slo: the BF16
+// split of the FP32 factor's pivot columns
 void launch_group_panel(const GroupItem *items, const StripTask *strips, int nstrips, int *ticket, int *flags,
-                        const DevPlan &P, T *Lx, double *Linv, unsigned long long *status, __nv_bfloat16 *Shi,
-                        __nv_bfloat16 *Slo, const LdltArgs<T> &ld, cudaStream_t st);
+                        const DevPlan &P, double *Lx, double *Linv, unsigned long long *status, const LdltArgs<double> &ld,
+                        cudaStream_t st);
+void launch_group_panel(const GroupItem *items, const StripTask *strips, int nstrips, int *ticket, int *flags,
+                        const DevPlan &P, float *Lx, unsigned long long *status, __nv_bfloat16 *Shi, __nv_bfloat16 *Slo,
+                        const LdltArgs<float> &ld, cudaStream_t st);
+void launch_group_panel(const GroupItem *items, const StripTask *strips, int nstrips, int *ticket, int *flags,
+                        const DevPlan &P, cplx *Lx, double *Linv, unsigned long long *status, const LdltArgs<cplx> &ld,
+                        cudaStream_t st);
 void launch_ldlt_tau(const double *values, const DevPlan &P, double *scal, cudaStream_t st);
 // complex-symmetric update tiles (FP64 complex, CUDA cores), one CTA per tile
 void launch_update_c(const TileTask *tasks, int64_t ntasks, cplx *Lx, cplx *U, const cplx *W,

@@ -31,13 +31,8 @@ __device__ __forceinline__ bool recip_parts(double d, double &x, double &f) {
   f = fma(s, e * e, s);
   return ((unsigned)__double2hiint(d) & 0x7fffffffu) - 0x03000000u <= 0x79000000u;
 }
-// POTRF step buffers: 8 columns of 64 rows; row strides with 16-byte rows and few bank conflicts
-template <class TC>
-constexpr int col_ld() { return sizeof(TC) == 8 ? 10 : 12; }
-template <class TC>
-struct Vec2;  // two neighbouring entries
-template <>
-struct Vec2<double> { using type = double2; };
+// Row stride of the step buffers (8 columns): 16-byte rows, few bank conflicts
+constexpr int kColLd = 10;
 
 // C(g, 2 t ..) -= A(g, .) B(., 2 t ..) on an 8 x 8 tile, K = 8: P the negated rows of A, Q the rows of B^T (stride ld)
 __device__ __forceinline__ void step_tile(double (&c)[2], const double *P, const double *Q, int ld, int g, int t) {
@@ -47,44 +42,43 @@ __device__ __forceinline__ void step_tile(double (&c)[2], const double *P, const
   mma884(c, a.y, b.y);
 }
 // One pivot step for row r (one row per lane of the calling warps; rows past the block repeat its last one): the columns
-// [k8, k8 + 8) in R (row stride col_ld), their diagonal tile in R's rows k8 ... The first `pivots` columns are pivots
+// [k8, k8 + 8) in R (row stride kColLd), their diagonal tile in R's rows k8 ... The first `pivots` columns are pivots
 // (all eight unless Partial); the others only take the pivots' updates. Writes -a to Pk and a / d (0 for a column that is
 // no pivot) to Qk. LDL^T: |d| < tau counts as -+tau by d's sign (ldlt.mjs:513-522). Returns false, R being unchanged, when
 // a pivot is out of the reciprocal estimate's range (then to be repeated with Exact).
 // The chain per column is one reciprocal (the hardware estimate and three dependent products) and two products, 58
 // clocks in FP64; a step's FP64 issue takes 790 clocks of a warp alone on its scheduler. No branch inside: one around
 // the exact reciprocals made a step 1,115 clocks.
-template <bool Exact, bool LDLT, bool Partial, class TC>
-__device__ __forceinline__ bool eliminate8(const TC *R, TC *Pk, TC *Qk, int k8, int r, int pivots, TC tau) {
-  using V2 = typename Vec2<TC>::type;
-  constexpr int CL = col_ld<TC>();
-  TC dg[8][8], a[8], iv[8];
+template <bool Exact, bool LDLT, bool Partial>
+__device__ __forceinline__ bool eliminate8(const double *R, double *Pk, double *Qk, int k8, int r, int pivots, double tau) {
+  constexpr int CL = kColLd;
+  double dg[8][8], a[8], iv[8];
   bool fine = true;
 #pragma unroll
   for (int i = 0; i < 8; i++)
 #pragma unroll
     for (int j = 0; j <= i; j += 2) {
-      const V2 v = *reinterpret_cast<const V2 *>(R + (k8 + i) * CL + j);
+      const double2 v = *reinterpret_cast<const double2 *>(R + (k8 + i) * CL + j);
       dg[i][j] = v.x;
       dg[i][j + 1] = v.y;
     }
 #pragma unroll
   for (int j = 0; j < 8; j += 2) {
-    const V2 v = *reinterpret_cast<const V2 *>(R + r * CL + j);
+    const double2 v = *reinterpret_cast<const double2 *>(R + r * CL + j);
     a[j] = v.x;
     a[j + 1] = v.y;
   }
 #pragma unroll
   for (int kk = 0; kk < 8; kk++) {
-    TC d = dg[kk][kk], x, fr;
-    if (LDLT && !(fabs(d) >= tau)) d = d < TC(0) ? -tau : tau;
-    if (Partial && kk >= pivots) d = TC(1);
+    double d = dg[kk][kk], x, fr;
+    if (LDLT && !(fabs(d) >= tau)) d = d < 0.0 ? -tau : tau;
+    if (Partial && kk >= pivots) d = 1.0;
     fine &= recip_parts<Exact>(d, x, fr);
-    if (Partial && kk >= pivots) x = TC(0);
+    if (Partial && kk >= pivots) x = 0.0;
     iv[kk] = x * fr;
 #pragma unroll
     for (int j = kk + 1; j < 8; j++) {
-      const TC lj = (dg[j][kk] * x) * fr;  // the update scale; L is scaled with the exact quotient when written
+      const double lj = (dg[j][kk] * x) * fr;  // the update scale; L is scaled with the exact quotient when written
 #pragma unroll
       for (int i = j; i < 8; i++) dg[i][j] -= dg[i][kk] * lj;
       a[j] -= a[kk] * lj;
@@ -92,13 +86,13 @@ __device__ __forceinline__ bool eliminate8(const TC *R, TC *Pk, TC *Qk, int k8, 
   }
 #pragma unroll
   for (int j = 0; j < 8; j += 2) {
-    V2 v;
+    double2 v;
     v.x = -a[j];
     v.y = -a[j + 1];
-    *reinterpret_cast<V2 *>(Pk + r * CL + j) = v;
+    *reinterpret_cast<double2 *>(Pk + r * CL + j) = v;
     v.x = a[j] * iv[j];
     v.y = a[j + 1] * iv[j + 1];
-    *reinterpret_cast<V2 *>(Qk + r * CL + j) = v;
+    *reinterpret_cast<double2 *>(Qk + r * CL + j) = v;
   }
   return fine;
 }
