@@ -695,29 +695,42 @@ void device_solve(amp_factor *f, const double *dB, double *dX) {
 // the batch) and there are two or more slices, those supernodes' tasks stay single with .w = -1
 // and move all vectors at once (no chain to split, one pass over the L tile, a quarter of the tasks). Built and
 // uploaded once per plan and ns.
+// Forward, where the block tasks of a level are more than the resident CTAs, its supernodes of one pivot block and few rows
+// are one task per slice instead (kind 3): fewer hand-offs, tickets and gathers for the same work. In a smaller level the
+// supernode's tasks run side by side, and one task for all of them only takes their sum. Forward sweeps with kind 3 in every
+// level / by this rule / nowhere: elasticity with 11 elements per edge and 4 vectors 204 / 150 / 148 us, with 28 and 32
+// (FP32) 870 / 872 / 990, heat with 128 per edge and 5 vectors 305 / 250 / 253, quadratic heat with 28 and 16 vectors, five
+// sweeps, 7.47 / 7.44 / 8.51 ms, edge elements with 20 and 64 vectors 2.14 / 2.14 / 2.57 ms.
 constexpr int kWideBlocks = 2;
 static std::vector<int> expand_slices(const amp::Plan &P, const std::vector<int> &tasks, size_t ntasks, int ns,
                                       bool wide, bool forward) {
+  std::vector<char> whole(P.nsuper, 0);
+  for (int L = 0; L < P.nlevels && forward && !wide; L++) {
+    int64_t count = 0;  // the level's block tasks
+    for (int i = P.lvlPtr[L]; i < P.lvlPtr[L + 1]; i++) {
+      const int s = P.lvlSn[i], nc = P.snNc[s], m = P.snM[s];
+      if (m > amp::kTinyFront) count += (nc + 63) / 64 + (m - nc + 63) / 64;
+    }
+    if (count * ns <= amp::multi_resident()) continue;
+    for (int i = P.lvlPtr[L]; i < P.lvlPtr[L + 1]; i++) {
+      const int s = P.lvlSn[i];
+      whole[s] = P.snNc[s] <= 64 && P.snM[s] <= amp::whole_multi_rows();
+    }
+  }
   std::vector<int> out;
   out.reserve(4 * ntasks * (size_t)ns);
-  auto put = [&](int s, int blk, int kind) {
-    if (wide && (P.snNc[s] + 63) / 64 <= kWideBlocks)
-      out.insert(out.end(), {s, blk, kind, -1});
-    else
-      for (int sl = 0; sl < ns; sl++) out.insert(out.end(), {s, blk, kind, sl});
-  };
-  auto whole = [&](int s) { return forward && !wide && P.snNc[s] <= 64 && P.snM[s] <= amp::whole_multi_rows(); };
   for (size_t i = 0; i < ntasks; i++) {
-    const int *t = &tasks[4 * i];
+    const int *t = &tasks[4 * i], s = t[0];
     if (t[2] == 2)
-      out.insert(out.end(), {t[0], t[1], 2, 0});
-    else if (!whole(t[0]))
-      put(t[0], t[1], t[2]);
-    else if (t[2] == 0)  // its tasks below are part of it
-      for (int sl = 0; sl < ns; sl++) out.insert(out.end(), {t[0], 0, 3, sl});
+      out.insert(out.end(), {s, t[1], 2, 0});
+    else if (wide && (P.snNc[s] + 63) / 64 <= kWideBlocks)
+      out.insert(out.end(), {s, t[1], t[2], -1});
+    else if (!whole[s] || t[2] == 0)  // (the tasks below a whole supernode's diagonal one are part of it)
+      for (int sl = 0; sl < ns; sl++) out.insert(out.end(), {s, t[1], whole[s] ? 3 : t[2], sl});
   }
   return out;
 }
+
 static void slice_lists(amp_plan *pl, int ns) {
   std::lock_guard<std::mutex> lock(pl->slMu);
   if (pl->dFwdSl[ns - 1]) return;

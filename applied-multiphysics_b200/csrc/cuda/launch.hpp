@@ -87,6 +87,7 @@ void launch_chain_mats(const int2 *tasks, int ntasks, const DevPlan &P, const TL
 // left single with .w = -1 (the task moves every vector at once).
 int multi_max_vectors();
 int multi_slices(int q);
+int multi_resident();    // CTAs of a sweep that are resident at once
 int whole_multi_rows();  // whole-supernode tasks (kind 3) of the forward list: one pivot block, m at most this
 // wide: the list holds .w = -1 tasks (the kernels with the all-vector path)
 // Mch / Gch: the chain matrices of a Cholesky factor (launch_chain_mats), or null (LDL^T: substitution order)

@@ -30,10 +30,8 @@
 // of the quadratic heat system with 32 elements per edge (FP32 factors), five sweeps each way: forward 15.4 -> 11.6 ms,
 // backward 10.4 -> 8.7 ms; FP64 LDL^T factors of the edge-element system with 24: 5.25 -> 3.82 and 3.73 -> 3.20 ms.
 //
-// Supernodes with one pivot block and at most kWholeMulti rows (in plans that are not WIDE) are one task per slice
-// (kind 3, run_whole): their block tasks did a few products each and paid a hand-off through flags in between. A batch
-// of 64 systems of 4,225 unknowns, where most supernodes are of this size: forward 4.05 -> 2.39 ms, backward 3.10 ->
-// 2.20 ms.
+// Forward, supernodes with one pivot block and at most kWholeMulti rows are one task per slice (kind 3, run_whole) in the
+// levels that have more tasks than there are CTAs (expand_slices in capi.cpp has the rule and its times).
 //
 // Backward order: the rows below the supernode are summed from the last chunk down, each chunk after the flags of the
 // ancestor blocks that hold its rows (rowBlk), so a task works while its ancestors are still being solved (the
@@ -63,7 +61,7 @@ constexpr int ld_mk() { return chunk_k<TL>() + 4; }  // a chunk stored [m][k]: 2
 constexpr int kLdB = kQS + 4;  // B and R stored [k][n]: 20
 constexpr int kMultiThreads = 256;
 constexpr int kMultiCtas = 3;  // resident CTAs per SM of the persistent sweeps (registers capped at 80)
-constexpr int kWholeMulti = 256;  // supernodes with one pivot block and at most this many rows are one task per slice
+constexpr int kWholeMulti = 256;  // the most rows of a whole-supernode task (kind 3)
 constexpr int kRingBytes = kStages * kMB * ld_mk<double>() * (int)sizeof(double);  // the largest stage: FP64 [m][k]
 static_assert(kMB * ld_mk<float>() * 4 <= kMB * ld_mk<double>() * 8 && chunk_k<double>() * kLdKM <= kMB * ld_mk<double>() &&
                   chunk_k<float>() * kLdKM * 4 <= kMB * ld_mk<double>() * 8,
@@ -669,9 +667,8 @@ __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_fwd_multi(const i
     return true;
   };
   // kind 3: the whole supernode s (nc <= 64, m <= kWholeMulti) for vector slice sl: its front vector v (all m rows) where
-  // the ring is, y = X v[0:nc), then u = v - L[rows below, :] y in 64-row blocks. Most supernodes are this small, and
-  // one task for each replaces a diagonal task and up to four below it, whose latencies (ticket, gather, flag) were all
-  // their time.
+  // the ring is, y = X v[0:nc), then u = v - L[rows below, :] y in 64-row blocks: in place of a diagonal task and up to four
+  // below it, each with its ticket, gather and flag.
   auto run_whole = [&](const int s, const int sl) -> bool {
     const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s], mu = m - nc;
     const int vb = sl * kQS, qs = min(kQS, q - vb);
@@ -1136,9 +1133,8 @@ cudaError_t init_solve_multi_attributes() {
 int num_sms();
 int multi_max_vectors() { return kMQ; }
 int multi_slices(int q) { return (q + kQS - 1) / kQS; }
-static int multi_grid(int64_t ntasks) {
-  return ntasks < kMultiCtas * num_sms() ? (int)ntasks : kMultiCtas * num_sms();
-}
+int multi_resident() { return kMultiCtas * num_sms(); }
+static int multi_grid(int64_t ntasks) { return ntasks < multi_resident() ? (int)ntasks : multi_resident(); }
 
 template <class TL>
 void launch_fwd_multi(const int4 *tasks, int ntasks, bool wide, int *ticket, const DevPlan &P, const TL *Lx,
