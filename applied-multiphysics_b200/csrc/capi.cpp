@@ -173,7 +173,6 @@ struct amp_plan_s {
   // the multi-vector lists with every block task expanded into ns vector slices, built on first use (index ns - 1)
   int4 *dFwdSl[kSlices] = {}, *dBwdSl[kSlices] = {};
   int nFwdSl[kSlices] = {}, nBwdSl[kSlices] = {};
-  bool wideSl[kSlices] = {};  // the list holds all-vector tasks (.w = -1)
   std::mutex slMu;
   int *dTinySn = nullptr, *dSmallSn = nullptr;  // small fronts per level (whole fronts by one warp / one CTA)
   int2 *dChain = nullptr;                        // chain-matrix tasks {s, b}
@@ -690,22 +689,20 @@ void device_solve(amp_factor *f, const double *dB, double *dX) {
 
 // ---- several right-hand sides: groups of up to multi_max_vectors() vectors, interleaved ([i q + k]) -------------
 // The multi-vector task lists for ns vector slices: a block task (kind 0 / 1) is expanded into ns consecutive entries
-// with .w = the slice (the slices' chains run on different CTAs); the small-supernode tasks (kind 2) stay single.
-// When supernodes with at most kWideBlocks pivot blocks hold at least half of L (a plan of many small systems, like
-// the batch) and there are two or more slices, those supernodes' tasks stay single with .w = -1
-// and move all vectors at once (no chain to split, one pass over the L tile, a quarter of the tasks). Built and
-// uploaded once per plan and ns.
+// with .w = the slice (the slices' chains run on different CTAs); the small-supernode tasks (kind 2) stay single. Built
+// and uploaded once per plan and ns. (Tasks that moved all vectors of a small supernode at once, on the CUDA cores, were
+// slower at every size: two slices of elasticity with 8 elements per edge 287 + 434 us forward and backward, now 97 + 89;
+// of heat with 192 per edge 956 + 1,191, now 359 + 283; four of a batch of 64 such systems 2.43 + 2.23 ms, now 1.95 + 1.79.)
 // Forward, where the block tasks of a level are more than the resident CTAs, its supernodes of one pivot block and few rows
 // are one task per slice instead (kind 3): fewer hand-offs, tickets and gathers for the same work. In a smaller level the
 // supernode's tasks run side by side, and one task for all of them only takes their sum. Forward sweeps with kind 3 in every
 // level / by this rule / nowhere: elasticity with 11 elements per edge and 4 vectors 204 / 150 / 148 us, with 28 and 32
 // (FP32) 870 / 872 / 990, heat with 128 per edge and 5 vectors 305 / 250 / 253, quadratic heat with 28 and 16 vectors, five
 // sweeps, 7.47 / 7.44 / 8.51 ms, edge elements with 20 and 64 vectors 2.14 / 2.14 / 2.57 ms.
-constexpr int kWideBlocks = 2;
 static std::vector<int> expand_slices(const amp::Plan &P, const std::vector<int> &tasks, size_t ntasks, int ns,
-                                      bool wide, bool forward) {
+                                      bool forward) {
   std::vector<char> whole(P.nsuper, 0);
-  for (int L = 0; L < P.nlevels && forward && !wide; L++) {
+  for (int L = 0; L < P.nlevels && forward; L++) {
     int64_t count = 0;  // the level's block tasks
     for (int i = P.lvlPtr[L]; i < P.lvlPtr[L + 1]; i++) {
       const int s = P.lvlSn[i], nc = P.snNc[s], m = P.snM[s];
@@ -723,8 +720,6 @@ static std::vector<int> expand_slices(const amp::Plan &P, const std::vector<int>
     const int *t = &tasks[4 * i], s = t[0];
     if (t[2] == 2)
       out.insert(out.end(), {s, t[1], 2, 0});
-    else if (wide && (P.snNc[s] + 63) / 64 <= kWideBlocks)
-      out.insert(out.end(), {s, t[1], t[2], -1});
     else if (!whole[s] || t[2] == 0)  // (the tasks below a whole supernode's diagonal one are part of it)
       for (int sl = 0; sl < ns; sl++) out.insert(out.end(), {s, t[1], whole[s] ? 3 : t[2], sl});
   }
@@ -736,16 +731,8 @@ static void slice_lists(amp_plan *pl, int ns) {
   if (pl->dFwdSl[ns - 1]) return;
   const amp::Plan &P = pl->P;
   const size_t nf = (size_t)P.fwdLvlPtr[P.nlevels];
-  double lAll = 0, lSmall = 0;  // L entries (nc m per supernode): all, and in supernodes of few pivot blocks
-  for (int sn = 0; sn < P.nsuper; sn++) {
-    const double e = (double)P.snNc[sn] * P.snM[sn];
-    lAll += e;
-    if ((P.snNc[sn] + 63) / 64 <= kWideBlocks) lSmall += e;
-  }
-  const bool wide = ns > 1 && lAll > 0 && 2 * lSmall >= lAll;
-  const std::vector<int> fw = join_small(P, expand_slices(P, P.fwdTasks, nf, ns, wide, true), true);
-  const std::vector<int> bw = join_small(P, expand_slices(P, P.bwdAll, P.bwdAll.size() / 4, ns, wide, false), true);
-  pl->wideSl[ns - 1] = wide;
+  const std::vector<int> fw = join_small(P, expand_slices(P, P.fwdTasks, nf, ns, true), true);
+  const std::vector<int> bw = join_small(P, expand_slices(P, P.bwdAll, P.bwdAll.size() / 4, ns, false), true);
   pl->dBwdSl[ns - 1] = (int4 *)pl->mem.upload(bw);
   pl->nBwdSl[ns - 1] = (int)(bw.size() / 4);
   pl->nFwdSl[ns - 1] = (int)(fw.size() / 4);
@@ -767,16 +754,15 @@ void device_solve_multi_permuted(amp_factor *f, int q) {
   slice_lists(f->plan, ns);
   const int nf = f->plan->nFwdSl[ns - 1], nb = f->plan->nBwdSl[ns - 1];
   int4 *fwdTasks = f->plan->dFwdSl[ns - 1], *bwdTasks = f->plan->dBwdSl[ns - 1];
-  const bool wide = f->plan->wideSl[ns - 1];
   const double *Dp = f->kind == AMP_LDLT && !f->bk ? f->dD : nullptr;  // Bunch-Kaufman: D solve between the sweeps
   const bool chain = f->kind != AMP_LDLT;  // Cholesky: chain matrices of consecutive diagonal blocks
   timed(f, K_FORWARD, flops, lbytes, [&] {
     if (f->dL32)
-      amp::launch_fwd_multi<float>(fwdTasks, nf, wide, f->dTickets, dp, f->dL32, f->dInv32, chain ? f->dMch32 : nullptr,
+      amp::launch_fwd_multi<float>(fwdTasks, nf, f->dTickets, dp, f->dL32, f->dInv32, chain ? f->dMch32 : nullptr,
                                    f->dY, f->dT, f->dFlags,
                                    nfl, efwd, f->dDone, q, f->dSolveStatus, st);
     else
-      amp::launch_fwd_multi<double>(fwdTasks, nf, wide, f->dTickets, dp, f->dLx, f->dInv, chain ? f->dMch : nullptr,
+      amp::launch_fwd_multi<double>(fwdTasks, nf, f->dTickets, dp, f->dLx, f->dInv, chain ? f->dMch : nullptr,
                                     f->dY, f->dT, f->dFlags,
                                     nfl, efwd, f->dDone, q, f->dSolveStatus, st);
   });
@@ -785,11 +771,11 @@ void device_solve_multi_permuted(amp_factor *f, int q) {
           [&] { amp::launch_dsolve_bk(P.n, q, f->dD, f->dDoff, f->dY, st); });
   timed(f, K_BACKWARD, flops, lbytes, [&] {
     if (f->dL32)
-      amp::launch_bwd_multi<float>(bwdTasks, nb, wide, f->dTickets + 1, dp, f->dL32, f->dInv32,
+      amp::launch_bwd_multi<float>(bwdTasks, nb, f->dTickets + 1, dp, f->dL32, f->dInv32,
                                    chain ? f->dGch32 : nullptr, Dp, f->dY, f->dFlags, nfl,
                                    ebwd, q, f->dSolveStatus, st);
     else
-      amp::launch_bwd_multi<double>(bwdTasks, nb, wide, f->dTickets + 1, dp, f->dLx, f->dInv, chain ? f->dGch : nullptr,
+      amp::launch_bwd_multi<double>(bwdTasks, nb, f->dTickets + 1, dp, f->dLx, f->dInv, chain ? f->dGch : nullptr,
                                     Dp, f->dY, f->dFlags, nfl,
                                     ebwd, q, f->dSolveStatus, st);
   });

@@ -7,13 +7,10 @@
 // row lists move whole rows.
 //
 // Vector slices of 16 (ns = ceil(q / 16)), each with its own ready flags (flags[slice * nflags + block]) and done
-// counters (done[slice * nsuper + s]): the host expands the block tasks of supernodes with several pivot blocks into
-// ns consecutive tasks, one per slice (int4 .w = the slice), so the slices' dependency chains run on different CTAs;
-// a task with .w = -1 (a supernode of few pivot blocks) moves all vectors at once (below; compiled into the sweeps of
-// the WIDE instantiation only, which the host launches for plans made mostly of such supernodes: the all-vector path
-// holds more registers, and in the same kernel the sliced tasks would spill). The expanded order keeps every wait on a
-// task with a smaller ticket, and a task never computes on absent vectors. The small supernodes (kind 2, one warp
-// each, not expanded) solve all q vectors and count/release every slice.
+// counters (done[slice * nsuper + s]): the host expands the block tasks into ns consecutive tasks, one per slice (int4 .w
+// = the slice), so the slices' dependency chains run on different CTAs. The expanded order keeps every wait on a task with a
+// smaller ticket, and a task never computes on absent vectors. The small supernodes (kind 2, one warp each, not expanded)
+// solve all q vectors and count/release every slice.
 //
 // A task is a small GEMM on the FP64 tensor cores (mma.sync m16n8k16): out (64 rows x 16 vectors) = sum over a
 // reduction index of A (64 rows x a chunk, FP32 factors widened as they are read) times B (chunk x 16), 8 warps as 4
@@ -76,9 +73,7 @@ constexpr int multi_smem() {
   const int own = kRingBytes + 3 * kMB * kLdB * (int)sizeof(double);
   const int small = kSolveGroup * small_stride(kSolveGroup) * (int)sizeof(double);
   static_assert(kSolveWarps * small_stride(kSolveWarps) <= kSolveGroup * small_stride(kSolveGroup), "kind 2 tasks");
-  const int wide = (2 * 32 + kMB) * 66 * (int)sizeof(double);        // all-vector tasks (kWideSmem)
-  const int m1 = own > small ? own : small;
-  return m1 > wide ? m1 : wide;
+  return own > small ? own : small;
 }
 
 __device__ __forceinline__ void dmma16816(double (&c)[4], const double (&a)[8], const double (&b)[4]) {
@@ -149,26 +144,23 @@ __device__ __forceinline__ void ticket_loop(int *ticket, int ntasks, Run &&run) 
 }
 
 // This task's rows [r0, r0 + rows) of the front vector v_s = [y(f .. f + nc); 0] + the children's pass-up vectors (rb:
-// their 64-row block), vectors [vb, vb + qs) of q, into Rs (row r at Rs[r LDR], QW >= qs columns; zero outside): the
+// their 64-row block), vectors [vb, vb + qs) of q, into Rs (row r at Rs[r kLdB], kQS columns; zero outside): the
 // pivot rows from y, then each child's entries that map into these rows (the schedule's gatherRange), in the
 // reference's child order. Up to kGatherCh children at a time, one per thread, are waited for (their pass-up vectors of
-// slices [sl0, sl0 + nsl)), so the waits of all children overlap; a child's entries are read while the one before it is
-// added. Every task of the supernode gathers its own rows in parallel. false: a wait gave up.
+// slice sl), so the waits of all children overlap; a child's entries are read while the one before it is added. Every task of the supernode gathers its own rows in parallel. false: a wait gave up.
 constexpr int kGatherCh = 64;
 // whole: rb is not used, the rows are the whole front (r0 = 0) and every child's vector is taken whole. Rs is cleared up
 // to the next multiple of kMB rows.
-template <int QW, int LDR>
 __device__ __forceinline__ bool gather_front_rows(const DevPlan &P, int s, bool whole, int rb, int r0, int rows,
-                                                  const double *__restrict__ y,
-                                  const double *__restrict__ T, int *done, int sl0, int nsl, int q, int vb, int qs,
-                                  unsigned long long *status, double *Rs) {
+                                                  const double *__restrict__ y, const double *__restrict__ T, int *done,
+                                                  int sl, int q, int vb, int qs, unsigned long long *status, double *Rs) {
   __shared__ int2 chA[kGatherCh];
   __shared__ int64_t chMap[kGatherCh], chT[kGatherCh];
   constexpr int N = 4;  // entries per thread read ahead
   const int tid = threadIdx.x, f = P.snF[s], nc = P.snNc[s];
-  for (int e = tid; e < (rows + kMB - 1) / kMB * kMB * QW; e += blockDim.x) {
-    const int row = e / QW, k = e % QW;
-    Rs[row * LDR + k] = (row < rows && k < qs && r0 + row < nc) ? y[(int64_t)(f + r0 + row) * q + vb + k] : 0.0;
+  for (int e = tid; e < (rows + kMB - 1) / kMB * kMB * kQS; e += blockDim.x) {
+    const int row = e / kQS, k = e % kQS;
+    Rs[row * kLdB + k] = (row < rows && k < qs && r0 + row < nc) ? y[(int64_t)(f + r0 + row) * q + vb + k] : 0.0;
   }
   const int q0 = P.chPtr[s], q1 = P.chPtr[s + 1];
   const int64_t range0 = P.gatherOff[s] + (int64_t)rb * (q1 - q0);
@@ -182,20 +174,19 @@ __device__ __forceinline__ bool gather_front_rows(const DevPlan &P, int s, bool 
       chA[tid] = whole ? make_int2(0, muc) : P.gatherRange[range0 + qb - q0 + tid];
       chMap[tid] = P.eaPtr[c];
       chT[tid] = P.snTOff[c];
-      const int need = (muc + kMB - 1) / kMB;
-      for (int sl = sl0; sl < sl0 + nsl && ok; sl++) ok = wait_count(done + (int64_t)sl * P.nsuper + c, need, status, s, P.spin);
+      ok = wait_count(done + (int64_t)sl * P.nsuper + c, (muc + kMB - 1) / kMB, status, s, P.spin);
     }
     if (!__syncthreads_and(ok)) return false;  // block-uniform
-    // the first N entries per thread of child qq (row a0 + e / QW of its vector, vector e % QW), and where they go
+    // the first N entries per thread of child qq (row a0 + e / kQS of its vector, vector e % kQS), and where they go
     auto fetch = [&](int qq, double(&v)[N], int(&dst)[N]) {
       const int a0 = chA[qq].x, na = chA[qq].y - a0;
 #pragma unroll
       for (int u = 0; u < N; u++) {
-        const int e = tid + (int)blockDim.x * u, a = a0 + e / QW, k = e % QW;
+        const int e = tid + (int)blockDim.x * u, a = a0 + e / kQS, k = e % kQS;
         dst[u] = -1;
         v[u] = 0.0;
-        if (e < na * QW && k < qs) {
-          dst[u] = (P.eaMap[chMap[qq] + a] - r0) * LDR + k;
+        if (e < na * kQS && k < qs) {
+          dst[u] = (P.eaMap[chMap[qq] + a] - r0) * kLdB + k;
           v[u] = __ldcg(T + (chT[qq] + a) * q + vb + k);
         }
       }
@@ -209,9 +200,9 @@ __device__ __forceinline__ bool gather_front_rows(const DevPlan &P, int s, bool 
       for (int u = 0; u < N; u++)
         if (dst[u] >= 0) Rs[dst[u]] += v[u];
       const int a0 = chA[qq].x, na = chA[qq].y - a0;
-      for (int e = tid + (int)blockDim.x * N; e < na * QW; e += blockDim.x) {
-        const int a = a0 + e / QW, k = e % QW;
-        if (k < qs) Rs[(P.eaMap[chMap[qq] + a] - r0) * LDR + k] += __ldcg(T + (chT[qq] + a) * q + vb + k);
+      for (int e = tid + (int)blockDim.x * N; e < na * kQS; e += blockDim.x) {
+        const int a = a0 + e / kQS, k = e % kQS;
+        if (k < qs) Rs[(P.eaMap[chMap[qq] + a] - r0) * kLdB + k] += __ldcg(T + (chT[qq] + a) * q + vb + k);
       }
       __syncthreads();
 #pragma unroll
@@ -225,272 +216,6 @@ __device__ __forceinline__ bool gather_front_rows(const DevPlan &P, int s, bool 
   return true;
 }
 
-// ---- tasks of supernodes with few pivot blocks: all q vectors at once on the CUDA cores ----------------------------
-// A task of a supernode with at most two pivot blocks (list entry .w = -1) moves all q <= 64 vectors together: out
-// (64 rows x 64 vectors) = sum of A (64 x 32 L chunk) times B (32 x 64 vector chunk), both in shared memory, each
-// thread accumulating a 4 x 4 register tile in FP64. Such a task has no chain worth splitting, and one pass over
-// its L tile serves every vector. It waits for every slice of what another supernode provides (children's counts,
-// the parent's flag) and releases every slice of its own flags and counts.
-constexpr int kWKC = 32;  // reduction chunk
-constexpr int kWLd = 66;  // shared tile row stride in doubles (even: 16-byte aligned double2 reads)
-constexpr int kWideSmem = (2 * kWKC + kMB) * kWLd * (int)sizeof(double);
-// acc[i][j] += sum over kk < kc of A[kk][4 ty + i] B[kk][4 tx + j]
-__device__ __forceinline__ void mm_tile_w(const double *__restrict__ A, const double *__restrict__ B, int kc, int ty,
-                                          int tx, double (&acc)[4][4]) {
-#pragma unroll 4
-  for (int kk = 0; kk < kc; kk++) {
-    const double2 a0 = *reinterpret_cast<const double2 *>(A + kk * kWLd + 4 * ty);
-    const double2 a1 = *reinterpret_cast<const double2 *>(A + kk * kWLd + 4 * ty + 2);
-    const double2 b0 = *reinterpret_cast<const double2 *>(B + kk * kWLd + 4 * tx);
-    const double2 b1 = *reinterpret_cast<const double2 *>(B + kk * kWLd + 4 * tx + 2);
-    const double a[4] = {a0.x, a0.y, a1.x, a1.y}, b[4] = {b0.x, b0.y, b1.x, b1.y};
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-      for (int j = 0; j < 4; j++) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-  }
-}
-
-// forward: as the sliced task (diagonal y[block] = X (v[block] - L[block, 0:blk 64] y), below T[block] = v[block] -
-// L[block, 0:nc] y), every vector
-template <class TL>
-__device__ __forceinline__ bool fwd_wide_task(const int4 t, const DevPlan &P, const TL *__restrict__ Lx, const TL *__restrict__ Inv,
-                              double *__restrict__ y, double *__restrict__ T, int *flags,
-                              int nflags, int epoch, int *done, int q, int ns, unsigned long long *status,
-                              double *msm, int &waitOk) {
-  double *As = msm, *Bs = msm + kWKC * kWLd, *Rs = msm + 2 * kWKC * kWLd;
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  const int s = t.x, blk = t.y, below = t.z;
-  const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s], mu = m - nc;
-  const TL *Lp = Lx + P.snLxp[s];
-  const int r0 = below ? nc + blk * kMB : blk * kMB;
-  const int rows = below ? min(kMB, mu - blk * kMB) : min(kMB, nc - blk * kMB);
-  const int ncols = below ? nc : blk * kMB;
-  int *myflags = flags + P.blkOff[s];  // the slice-0 set: this supernode releases every slice at once
-  // this task's rows of v_s, every vector, into Rs (every slice of each child done)
-  if (!gather_front_rows<kMQ, kWLd>(P, s, false, (below ? (nc + kMB - 1) / kMB : 0) + blk, r0, rows, y, T, done, 0, ns, q, 0, q, status, Rs)) return false;
-  double acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = 0.0;
-  // L tile of a chunk: As[c][row] = L(r0 + row, cb + c); thread elements e = tid + 256 u: row = e & 63, c = e >> 6
-  TL lr[8];
-  auto loadL = [&](int cb) {
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int e = tid + kMultiThreads * u, row = e & (kMB - 1), c = e >> 6;
-      lr[u] = (row < rows && cb + c < ncols) ? Lp[(int64_t)(cb + c) * m + r0 + row] : (TL)0;
-    }
-  };
-  const int nch = (ncols + kWKC - 1) / kWKC;
-  if (nch > 0) loadL(0);
-  for (int ch = 0; ch < nch; ch++) {
-    const int cb = ch * kWKC, cw = min(kWKC, ncols - cb);
-    if ((cb & (kMB - 1)) == 0) {  // first chunk of a pivot block: its y values final?
-      if (tid == 0) waitOk = wait_flag(myflags + cb / kMB, epoch, status, s, P.spin);
-      __syncthreads();
-      if (!waitOk) return false;
-    }
-    for (int e = tid; e < kWKC * kMQ; e += kMultiThreads) {
-      const int c = e >> 6, k = e & (kMQ - 1);
-      Bs[c * kWLd + k] = (c < cw && k < q) ? __ldcg(y + (int64_t)(f + cb + c) * q + k) : 0.0;
-    }
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int e = tid + kMultiThreads * u;
-      As[(e >> 6) * kWLd + (e & (kMB - 1))] = (double)lr[u];
-    }
-    __syncthreads();
-    if (ch + 1 < nch) loadL(cb + kWKC);
-    mm_tile_w(As, Bs, cw, ty, tx, acc);
-    __syncthreads();
-  }
-  // R = v[block] - acc (the task's rows of v in Rs)
-  if (below) {
-    double *to = T + (P.snTOff[s] + (int64_t)blk * kMB) * q;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int row = 4 * ty + i;
-      if (row >= rows) continue;
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int k = 4 * tx + j;
-        if (k < q) to[(int64_t)row * q + k] = Rs[row * kWLd + k] - acc[i][j];
-      }
-    }
-    __syncthreads();
-    if (tid < ns) red_release_add(done + (int64_t)tid * P.nsuper + s, 1);  // one count per vector slice
-    return true;
-  }
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int row = 4 * ty + i;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int k = 4 * tx + j;
-      Rs[row * kWLd + k] = (row < rows && k < q) ? Rs[row * kWLd + k] - acc[i][j] : 0.0;
-      acc[i][j] = 0.0;
-    }
-  }
-  // y[block] = X R, X = L_kk^-1 (rows x rows, column-major): As[jj][i] = X(i, jb + jj)
-  const TL *X = Inv + P.invOff[P.blkOff[s] + blk];
-  for (int jb = 0; jb < rows; jb += kWKC) {
-    const int jw = min(kWKC, rows - jb);
-    __syncthreads();
-    for (int e = tid; e < kWKC * kMB; e += kMultiThreads) {
-      const int i = e & (kMB - 1), jj = e >> 6;
-      As[jj * kWLd + i] = (i < rows && jj < jw) ? (double)X[(int64_t)(jb + jj) * rows + i] : 0.0;
-    }
-    __syncthreads();
-    mm_tile_w(As, Rs + jb * kWLd, jw, ty, tx, acc);
-  }
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int row = 4 * ty + i;
-    if (row >= rows) continue;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int k = 4 * tx + j;
-      if (k < q) y[(int64_t)(f + r0 + row) * q + k] = acc[i][j];
-    }
-  }
-  __syncthreads();
-  if (tid < ns) st_release(flags + (int64_t)tid * nflags + P.blkOff[s] + blk, epoch);  // every vector slice
-  return true;
-}
-
-// backward: as the sliced task, every vector (the rows below after the parent's every slice is final)
-template <class TL>
-__device__ __forceinline__ bool bwd_wide_task(const int4 t, const DevPlan &P, const TL *__restrict__ Lx, const TL *__restrict__ Inv,
-                              const double *__restrict__ Dpiv, double *__restrict__ y, int *flags, int nflags,
-                              int epoch, int q, int ns, unsigned long long *status, double *msm, int &waitOk) {
-  double *As = msm, *Bs = msm + kWKC * kWLd, *Rs = msm + 2 * kWKC * kWLd;
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  const int s = t.x, blk = t.y;
-  const int f = P.snF[s], nc = P.snNc[s], m = P.snM[s];
-  const TL *Lp = Lx + P.snLxp[s];
-  const int *rowsOf = P.Si + P.Sp[s];
-  const int c0 = blk * kMB, w = min(kMB, nc - c0), nb = (nc + kMB - 1) / kMB;
-  int *myflags = flags + P.blkOff[s];  // the slice-0 set: this supernode releases every slice at once
-  const int par = P.snParent[s];
-  if (par >= 0) {  // the parent's every vector slice final
-    if (tid == 0) {
-      waitOk = 1;
-      for (int sl = 0; sl < ns && waitOk; sl++)
-        waitOk = wait_flag(flags + (int64_t)sl * nflags + P.blkOff[par], epoch, status, s, P.spin);
-    }
-    __syncthreads();
-    if (!waitOk) return false;
-  }
-  double acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = 0.0;
-  // chunks: ancestors rows [nc, m) in kWKC steps, then pivot blocks nb - 1 .. blk + 1 (two chunks each)
-  const int nanc = (m - nc + kWKC - 1) / kWKC;
-  const int npiv = (nb - 1 - blk) * (kMB / kWKC);
-  const int nch = nanc + npiv;
-  // chunk ch -> first row and row count
-  auto chunk = [&](int ch, int &rb, int &rw) {
-    if (ch < nanc) {
-      rb = nc + ch * kWKC;
-      rw = min(kWKC, m - rb);
-    } else {
-      const int p = ch - nanc, pb = nb - 1 - p / 2;  // pivot block, from the last down
-      rb = pb * kMB + (p & 1) * kWKC;
-      rw = max(0, min(kWKC, nc - rb));
-    }
-  };
-  // L tile: As[rr][c] = L(rb + rr, c0 + c); elements e = tid + 256 u: rr = e & 31, c = e >> 5
-  TL lr[8];
-  auto loadL = [&](int rb, int rw) {
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int e = tid + kMultiThreads * u, rr = e & (kWKC - 1), c = e >> 5;
-      lr[u] = (rr < rw && c < w) ? Lp[(int64_t)(c0 + c) * m + rb + rr] : (TL)0;
-    }
-  };
-  int rb = 0, rw = 0;
-  if (nch > 0) {
-    chunk(0, rb, rw);
-    loadL(rb, rw);
-  }
-  for (int ch = 0; ch < nch; ch++) {
-    const bool anc = ch < nanc;
-    if (!anc && ((ch - nanc) & 1) == 0) {  // first chunk of a pivot block: its x values final?
-      if (tid == 0) waitOk = wait_flag(myflags + rb / kMB, epoch, status, s, P.spin);
-      __syncthreads();
-      if (!waitOk) return false;
-    }
-    for (int e = tid; e < kWKC * kMQ; e += kMultiThreads) {
-      const int rr = e >> 6, k = e & (kMQ - 1);
-      double v = 0.0;
-      if (rr < rw && k < q) {
-        const int gi = anc ? rowsOf[rb + rr] : f + rb + rr;
-        v = __ldcg(y + (int64_t)gi * q + k);
-      }
-      Bs[rr * kWLd + k] = v;
-    }
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int e = tid + kMultiThreads * u;
-      As[(e & (kWKC - 1)) * kWLd + (e >> 5)] = (double)lr[u];
-    }
-    __syncthreads();
-    const int cw = rw;
-    if (ch + 1 < nch) {
-      chunk(ch + 1, rb, rw);
-      loadL(rb, rw);
-    }
-    mm_tile_w(As, Bs, cw, ty, tx, acc);
-    __syncthreads();
-  }
-  // R = y[block] (/ D) - acc
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int c = 4 * ty + i;
-    const double d = (Dpiv && c < w) ? Dpiv[f + c0 + c] : 1.0;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int k = 4 * tx + j;
-      double v = 0.0;
-      if (c < w && k < q) {
-        const double yv = y[(int64_t)(f + c0 + c) * q + k];
-        v = (Dpiv ? yv / d : yv) - acc[i][j];  // LDL^T: y /= D before the backward sweep (ldlt.mjs:629)
-      }
-      Rs[c * kWLd + k] = v;
-      acc[i][j] = 0.0;
-    }
-  }
-  // x[block] = X^T R: As[jj][i] = X(jb + jj, i) = Inv[i w + jb + jj]
-  const TL *X = Inv + P.invOff[P.blkOff[s] + blk];
-  for (int jb = 0; jb < w; jb += kWKC) {
-    const int jw = min(kWKC, w - jb);
-    __syncthreads();
-    for (int e = tid; e < kWKC * kMB; e += kMultiThreads) {
-      const int jj = e & (kWKC - 1), i = e >> 5;
-      As[jj * kWLd + i] = (i < w && jj < jw) ? (double)X[(int64_t)i * w + jb + jj] : 0.0;
-    }
-    __syncthreads();
-    mm_tile_w(As, Rs + jb * kWLd, jw, ty, tx, acc);
-  }
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int c = 4 * ty + i;
-    if (c >= w) continue;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int k = 4 * tx + j;
-      if (k < q) y[(int64_t)(f + c0 + c) * q + k] = acc[i][j];
-    }
-  }
-  __syncthreads();
-  if (tid < ns) st_release(flags + (int64_t)tid * nflags + P.blkOff[s] + blk, epoch);  // every vector slice
-  return true;
-}
-
 // ---- forward ------------------------------------------------------------------------------------------------------
 // task (s, blk, below) of slice sl: as k_fwd_blocks. Diagonal: y[block] = X (v[block] - L[block, 0:blk 64] y[0:blk 64]);
 // below: T[block] = v[block] - L[block, 0:nc] y[0:nc], where v[block] is the task's rows of the front vector, gathered
@@ -498,7 +223,7 @@ __device__ __forceinline__ bool bwd_wide_task(const int4 t, const DevPlan &P, co
 // diagonal task b >= 1 forms W = X (v[block] - L[block, 0:(b-1) 64] y) before its last wait and then, after block
 // b - 1's flag, y[block] = W - M_b y[block b - 1]: one 64 x 64 product per chain step instead of the block's last
 // chunk, the reduction and the inverse product.
-template <class TL, bool WIDE>
+template <class TL>
 __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_fwd_multi(const int4 *__restrict__ tasks, int ntasks, int ns,
                                                                 int *__restrict__ ticket, const __grid_constant__ DevPlan P,
                                                                 const TL *__restrict__ Lx, const TL *__restrict__ Inv,
@@ -551,7 +276,7 @@ __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_fwd_multi(const i
     };
     for (int i = 0; i < kStages - 1; i++) issue(i);
     // this task's rows of v_s (this slice) into Rs, gathered by every task of the supernode in parallel
-    if (!gather_front_rows<kQS, kLdB>(P, s, false, (below ? (nc + kMB - 1) / kMB : 0) + blk, r0, rows, y, T, done, sl, 1, q, vb,
+    if (!gather_front_rows(P, s, false, (below ? (nc + kMB - 1) / kMB : 0) + blk, r0, rows, y, T, done, sl, q, vb,
                                       qs, status, Rs))
       return bail();
     double c[4] = {0.0, 0.0, 0.0, 0.0};
@@ -692,7 +417,7 @@ __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_fwd_multi(const i
       cp_async_commit();
     };
     issue(0);
-    if (!gather_front_rows<kQS, kLdB>(P, s, true, 0, 0, m, y, T, done, sl, 1, q, vb, qs, status, V)) return bail();
+    if (!gather_front_rows(P, s, true, 0, 0, m, y, T, done, sl, q, vb, qs, status, V)) return bail();
     for (int e = tid; e < kMB * kQS; e += kMultiThreads) {  // R = v[0:nc)
       const int row = e >> 4, n = e & (kQS - 1);
       Rs[row * kLdB + n] = row < nc ? V[row * kLdB + n] : 0.0;
@@ -744,9 +469,6 @@ __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_fwd_multi(const i
       return waitOk != 0;
     }
     if (t.z == 3) return run_whole(t.x, t.w);
-    if constexpr (WIDE) {
-      if (t.w < 0) return fwd_wide_task<TL>(t, P, Lx, Inv, y, T, flags, nflags, epoch, done, q, ns, status, msm, waitOk);
-    }
     return run_slice(t, t.w);
   };
   ticket_loop(ticket, ntasks, run);
@@ -756,7 +478,7 @@ __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_fwd_multi(const i
 // task (s, blk) of slice sl: x[block] = X^T (y[block] (/ D for LDL^T) - L[rows below the block, block columns]^T
 // x[those rows]). With the chain matrices of a Cholesky factor (Gch), block b + 1 is left out of the sum and enters
 // after its flag as x[block] = W - G_b^T x[block b + 1], W = X^T (y[block] - the other rows' terms).
-template <class TL, bool WIDE>
+template <class TL>
 __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_bwd_multi(const int4 *__restrict__ tasks, int ntasks, int ns,
                                                                 int *__restrict__ ticket, const __grid_constant__ DevPlan P,
                                                                 const TL *__restrict__ Lx, const TL *__restrict__ Inv,
@@ -986,9 +708,6 @@ __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_bwd_multi(const i
       __syncthreads();
       return waitOk != 0;
     }
-    if constexpr (WIDE) {
-      if (t.w < 0) return bwd_wide_task<TL>(t, P, Lx, Inv, Dpiv, y, flags, nflags, epoch, q, ns, status, msm, waitOk);
-    }
     return run_slice(t, t.w);
   };
   ticket_loop(ticket, ntasks, run);
@@ -1115,19 +834,17 @@ __global__ void __launch_bounds__(256) k_residual_multi(int n, const int *__rest
   }
 }
 
-template <class TL, bool WIDE>
+template <class TL>
 static cudaError_t set_multi_smem() {
   cudaError_t e =
-      cudaFuncSetAttribute(k_fwd_multi<TL, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, multi_smem());
+      cudaFuncSetAttribute(k_fwd_multi<TL>, cudaFuncAttributeMaxDynamicSharedMemorySize, multi_smem());
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_bwd_multi<TL, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, multi_smem());
+    e = cudaFuncSetAttribute(k_bwd_multi<TL>, cudaFuncAttributeMaxDynamicSharedMemorySize, multi_smem());
   return e;
 }
 cudaError_t init_solve_multi_attributes() {
-  cudaError_t e = set_multi_smem<double, false>();
-  if (e == cudaSuccess) e = set_multi_smem<double, true>();
-  if (e == cudaSuccess) e = set_multi_smem<float, false>();
-  return e == cudaSuccess ? set_multi_smem<float, true>() : e;
+  const cudaError_t e = set_multi_smem<double>();
+  return e == cudaSuccess ? set_multi_smem<float>() : e;
 }
 
 int num_sms();
@@ -1137,23 +854,21 @@ int multi_resident() { return kMultiCtas * num_sms(); }
 static int multi_grid(int64_t ntasks) { return ntasks < multi_resident() ? (int)ntasks : multi_resident(); }
 
 template <class TL>
-void launch_fwd_multi(const int4 *tasks, int ntasks, bool wide, int *ticket, const DevPlan &P, const TL *Lx,
+void launch_fwd_multi(const int4 *tasks, int ntasks, int *ticket, const DevPlan &P, const TL *Lx,
                       const TL *Inv, const TL *Mch, double *y, double *T, int *flags, int nflags, int epoch, int *done,
                       int q, unsigned long long *status, cudaStream_t st) {
   const int ns = multi_slices(q);
   if (ntasks <= 0) return;
-  auto k = wide ? k_fwd_multi<TL, true> : k_fwd_multi<TL, false>;
-  k<<<multi_grid(ntasks), kMultiThreads, multi_smem(), st>>>(tasks, ntasks, ns, ticket, P, Lx, Inv, Mch, y, T,
+  k_fwd_multi<TL><<<multi_grid(ntasks), kMultiThreads, multi_smem(), st>>>(tasks, ntasks, ns, ticket, P, Lx, Inv, Mch, y, T,
                                                                   flags, nflags, epoch, done, q, status);
 }
 template <class TL>
-void launch_bwd_multi(const int4 *tasks, int ntasks, bool wide, int *ticket, const DevPlan &P, const TL *Lx,
+void launch_bwd_multi(const int4 *tasks, int ntasks, int *ticket, const DevPlan &P, const TL *Lx,
                       const TL *Inv, const TL *Gch, const double *Dpiv, double *y, int *flags, int nflags, int epoch,
                       int q, unsigned long long *status, cudaStream_t st) {
   const int ns = multi_slices(q);
   if (ntasks <= 0) return;
-  auto k = wide ? k_bwd_multi<TL, true> : k_bwd_multi<TL, false>;
-  k<<<multi_grid(ntasks), kMultiThreads, multi_smem(), st>>>(tasks, ntasks, ns, ticket, P, Lx, Inv, Gch, Dpiv, y,
+  k_bwd_multi<TL><<<multi_grid(ntasks), kMultiThreads, multi_smem(), st>>>(tasks, ntasks, ns, ticket, P, Lx, Inv, Gch, Dpiv, y,
                                                                   flags, nflags, epoch, q, status);
 }
 void launch_to_interleaved(const double *B, double *Yil, int n, int q, cudaStream_t st) {
@@ -1173,16 +888,16 @@ void launch_residual_multi(int n, const int *rowptr, const int *colidx, const do
   const int grid = (int)(want < 8 * num_sms() ? want : 8 * num_sms());
   k_residual_multi<<<grid, 256, 0, st>>>(n, rowptr, colidx, val, x, b, r, norms, q, rowGroup);
 }
-template void launch_fwd_multi<double>(const int4 *, int, bool, int *, const DevPlan &, const double *,
+template void launch_fwd_multi<double>(const int4 *, int, int *, const DevPlan &, const double *,
                                        const double *, const double *, double *, double *, int *, int, int, int *, int,
                                        unsigned long long *, cudaStream_t);
-template void launch_fwd_multi<float>(const int4 *, int, bool, int *, const DevPlan &, const float *, const float *,
+template void launch_fwd_multi<float>(const int4 *, int, int *, const DevPlan &, const float *, const float *,
                                       const float *, double *, double *, int *, int, int, int *, int,
                                       unsigned long long *, cudaStream_t);
-template void launch_bwd_multi<double>(const int4 *, int, bool, int *, const DevPlan &, const double *,
+template void launch_bwd_multi<double>(const int4 *, int, int *, const DevPlan &, const double *,
                                        const double *, const double *, const double *, double *, int *, int, int, int,
                                        unsigned long long *, cudaStream_t);
-template void launch_bwd_multi<float>(const int4 *, int, bool, int *, const DevPlan &, const float *, const float *,
+template void launch_bwd_multi<float>(const int4 *, int, int *, const DevPlan &, const float *, const float *,
                                       const float *, const double *, double *, int *, int, int, int,
                                       unsigned long long *, cudaStream_t);
 
