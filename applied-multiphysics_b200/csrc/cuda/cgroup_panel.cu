@@ -68,6 +68,20 @@ __device__ __forceinline__ void set_tile(double *S, int r, int c, const CTile &v
 }
 __device__ __forceinline__ cplx at(const double *S, int r, int c) { return cplx(S[sw(r, c)], S[kPlane + sw(r, c)]); }
 
+// c += p, p a sum of products: added to c one by one, each of a complex product's two parts would be rounded at c's size
+__device__ __forceinline__ void add_tile(CTile &c, const CTile &p) {
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    c.re[u] += p.re[u];
+    c.im[u] += p.im[u];
+  }
+}
+// a -= b c, the product rounded by itself
+__device__ __forceinline__ void csub(cplx &a, cplx b, cplx c) {
+  a.re -= fma(b.re, c.re, -(b.im * c.im));
+  a.im -= fma(b.re, c.im, b.im * c.re);
+}
+
 // as the real panel's load_block
 __device__ __forceinline__ void load_cblock(double *S, const cplx *L, int m, int i0, int nr, int j0, int ncol, bool lower,
                                             bool pad) {
@@ -94,8 +108,10 @@ __device__ __forceinline__ void cstep_tile(CTile &c, const double *P, const doub
   const double2 ai = *reinterpret_cast<const double2 *>(P + kStepPlane + g * kRowLd + 2 * t);
   const double2 br = *reinterpret_cast<const double2 *>(Q + g * kRowLd + 2 * t);
   const double2 bi = *reinterpret_cast<const double2 *>(Q + kStepPlane + g * kRowLd + 2 * t);
-  cmma(c, ar.x, ai.x, br.x, bi.x);
-  cmma(c, ar.y, ai.y, br.y, bi.y);
+  CTile p = {{0.0, 0.0}, {0.0, 0.0}};
+  cmma(p, ar.x, ai.x, br.x, bi.x);
+  cmma(p, ar.y, ai.y, br.y, bi.y);
+  add_tile(c, p);
 }
 
 // One pivot step for row r (eliminate8 in pivot_steps.cuh, complex). The plain form takes every pivot as it is, with
@@ -145,15 +161,9 @@ __device__ __forceinline__ bool celiminate8(const double *R, double *Pk, double 
       const cplx lj = dg[j][kk] * iv;
 #pragma unroll
       for (int i = j; i < 8; i++) {
-        dg[i][j].re = fma(-dg[i][kk].re, lj.re, dg[i][j].re);
-        dg[i][j].im = fma(-dg[i][kk].re, lj.im, dg[i][j].im);
-        dg[i][j].re = fma(dg[i][kk].im, lj.im, dg[i][j].re);
-        dg[i][j].im = fma(-dg[i][kk].im, lj.re, dg[i][j].im);
+        csub(dg[i][j], dg[i][kk], lj);
       }
-      a[j].re = fma(-a[kk].re, lj.re, a[j].re);
-      a[j].im = fma(-a[kk].re, lj.im, a[j].im);
-      a[j].re = fma(a[kk].im, lj.im, a[j].re);
-      a[j].im = fma(-a[kk].im, lj.re, a[j].im);
+      csub(a[j], a[kk], lj);
     }
     const cplx q = a[kk] * iv;
     Pk[r * kRowLd + kk] = -a[kk].re;
@@ -411,9 +421,23 @@ __global__ void __launch_bounds__(256, 1) k_cgroup_panel(const GroupItem *__rest
           }
       }
       if (!panel_wait(Df + b, q + 1, status, P.spin)) return;
+      if (q == 0) {  // the products are summed by themselves; after the wait's barrier nobody reads Xs any more
+#pragma unroll
+        for (int p = 0; p < 8; p++) {
+          set_tile(Xs, lr, 8 * p + 2 * t, x[p]);
+          x[p] = {{0.0, 0.0}, {0.0, 0.0}};
+        }
+      }
       load_cblock(Ls, L, m, c0, w, cq, kPanel, false, false);
       __syncthreads();
       cupdate_row_group(x, nx, Ls, g, t);
+    }
+    if (b > 0) {
+#pragma unroll
+      for (int p = 0; p < 8; p++) {
+        const CTile v = tile_at(Xs, lr, 8 * p + 2 * t);
+        add_tile(x[p], v);
+      }
     }
     if (!panel_wait(Pf + b, 1, status, P.spin)) return;  // (its barrier: every warp is done with Ls)
     load_cblock(Ls, L, m, c0, w, c0, w, true, true);
@@ -448,8 +472,10 @@ __global__ void __launch_bounds__(256, 1) k_cgroup_panel(const GroupItem *__rest
         for (int p2 = p + 1; p2 < 8; p2++) {
           if (8 * p2 >= w) break;
           const CTile l = tile_at(Ls, 8 * p2 + g, 8 * p + 2 * t);
-          cmma(x[p2], -wv.re[0], -wv.im[0], l.re[0], l.im[0]);
-          cmma(x[p2], -wv.re[1], -wv.im[1], l.re[1], l.im[1]);
+          CTile v = {{0.0, 0.0}, {0.0, 0.0}};
+          cmma(v, -wv.re[0], -wv.im[0], l.re[0], l.im[0]);
+          cmma(v, -wv.re[1], -wv.im[1], l.re[1], l.im[1]);
+          add_tile(x[p2], v);
         }
       }
     };
@@ -487,19 +513,17 @@ __global__ void __launch_bounds__(256, 1) k_cgroup_panel(const GroupItem *__rest
     panel_release(Df + jd, b + 1);
     // the strip's own pivot block: tiles (rg, 0 .. rg) of D -= W X^T
     for (int nt = 0; nt <= lr >> 3; nt++) {
-      CTile c = tile_at(Ds, lr, 8 * nt + 2 * t), c2 = {{0.0, 0.0}, {0.0, 0.0}};
+      CTile c = {{0.0, 0.0}, {0.0, 0.0}}, c2 = {{0.0, 0.0}, {0.0, 0.0}};
 #pragma unroll
       for (int q = 0; q < 8; q++) {
         const CTile v = tile_at(Xs, 8 * nt + g, 8 * q + 2 * t);
         cmma(c, nx[q].re[0], nx[q].im[0], v.re[0], v.im[0]);
         cmma(c2, nx[q].re[1], nx[q].im[1], v.re[1], v.im[1]);
       }
-#pragma unroll
-      for (int u = 0; u < 2; u++) {
-        c.re[u] += c2.re[u];
-        c.im[u] += c2.im[u];
-      }
-      set_tile(Ds, lr, 8 * nt + 2 * t, c);
+      CTile d = tile_at(Ds, lr, 8 * nt + 2 * t);
+      add_tile(c, c2);
+      add_tile(d, c);
+      set_tile(Ds, lr, 8 * nt + 2 * t, d);
     }
   }
   if (jd >= 0) {  // this strip's own pivot block, fully updated: factor it and publish it (also after a failure)

@@ -69,12 +69,10 @@ __device__ __forceinline__ cplx cldcg(const cplx *p) {
   const double2 v = __ldcg(reinterpret_cast<const double2 *>(p));
   return cplx(v.x, v.y);
 }
-// a -= b c
+// a -= b c, the product rounded by itself (its two parts, subtracted one by one, would each be rounded at a's size)
 __device__ __forceinline__ void csubmul(cplx &a, cplx b, cplx c) {
-  a.re = fma(-b.re, c.re, a.re);
-  a.im = fma(-b.re, c.im, a.im);
-  a.re = fma(b.im, c.im, a.re);
-  a.im = fma(-b.im, c.re, a.im);
+  a.re -= fma(b.re, c.re, -(b.im * c.im));
+  a.im -= fma(b.re, c.im, b.im * c.re);
 }
 // a += b c
 __device__ __forceinline__ void caddmul(cplx &a, cplx b, cplx c) {

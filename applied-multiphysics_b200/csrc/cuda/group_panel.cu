@@ -7,7 +7,7 @@
 // against it, then their update and POTRF), one CTA at a time, so a block's latency is what counts: per block POTRF
 // 11,100 clocks, the flag and the loads behind it 3,400, TRSM 2,500, the block's own update 1,600 (FP64; 33,700 / - /
 // 10,400 / 7,100 with FMA tiles and a four-thread substitution per row). A 4,096-row front's group of two blocks takes
-// 32 us (66 before), eight of them at once 63 us (110). The split: warp w
+// 32 us (66 before), eight of them at once 61 us (110). The split: warp w
 // of a strip owns 8 rows (row group rg(w)) of every 64 x 64 product, so a strip's TRSM runs inside each warp without a
 // barrier -- the C fragment of a solved 8 x 8 tile is the A fragment of the next product (its two registers are the k
 // indices 2 t and 2 t + 1, and the B fragment takes the same pair with one 16-byte load).
@@ -490,7 +490,8 @@ __device__ __forceinline__ void substitute8(const double (&c)[2], double (&w)[2]
 // One group of pivot blocks [g0, g1) of a front, a strip of up to 64 rows per CTA, CTAs ordered by an atomic ticket
 // (the diagonal strips of every item first, then the strips below the group). A strip takes the group's pivot blocks b
 // in order (a diagonal strip those before its own), left-looking:
-//   its rows of block b receive the earlier blocks q: C -= W_q X_q^T, with W_q its own solved rows and X_q the rows of
+//   its rows of block b receive the earlier blocks q: C -= sum W_q X_q^T (summed by itself, as the own block's update below:
+//   products added to C one by one would each be rounded at C's size), with W_q its own solved rows and X_q the rows of
 //   diagonal strip b, waited for by D[b] >= q + 1 (the last W_q is still in registers, earlier ones are read back);
 //   then, after P[b], they are solved against the pivot block: W = C L_bb^-T by 8 x 8 blocks with the inverses of its
 //   diagonal blocks (Cholesky X = W; LDL^T with the unit L_bb, X = W D^-1; Bunch-Kaufman the columns in the block's
@@ -566,9 +567,24 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
           }
       }
       if (!panel_wait(Df + b, q + 1, status, P.spin)) return;
+      if (q == 0) {  // the products are summed by themselves (see above); after the wait's barrier nobody reads Xs any more
+#pragma unroll
+        for (int p = 0; p < 8; p++) {
+          set_pair(Xs, lr, 8 * p + 2 * t, x[p][0], x[p][1]);
+          x[p][0] = x[p][1] = 0.0;
+        }
+      }
       load_block(Ls, L, m, c0, w, cq, kPanel, false, false);
       __syncthreads();
       update_row_group(x, nx, Ls, g, t);
+    }
+    if (b > 0) {
+#pragma unroll
+      for (int p = 0; p < 8; p++) {
+        const double2 v = pair_at(Xs, lr, 8 * p + 2 * t);
+        x[p][0] += v.x;
+        x[p][1] += v.y;
+      }
     }
     if (!panel_wait(Pf + b, 1, status, P.spin)) return;  // (its barrier: every warp is done with Ls)
     load_block(Ls, L, m, c0, w, c0, w, true, true);
@@ -687,8 +703,7 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
     for (int nt = 0; nt <= lr >> 3; nt += 2) {
       const bool two = nt + 1 <= lr >> 3;
       const int nb2 = two ? nt + 1 : nt;
-      const double2 va = pair_at(Ds, lr, 8 * nt + 2 * t), vb = pair_at(Ds, lr, 8 * nb2 + 2 * t);
-      double ca[2] = {va.x, va.y}, cb[2] = {vb.x, vb.y};
+      double ca[2] = {0.0, 0.0}, cb[2] = {0.0, 0.0};
 #pragma unroll
       for (int q = 0; q < 8; q++) {
         const double2 xa = pair_at(Xs, 8 * nt + g, 8 * q + 2 * t), xb = pair_at(Xs, 8 * nb2 + g, 8 * q + 2 * t);
@@ -697,8 +712,9 @@ __global__ void __launch_bounds__(256, 2) k_group_panel(const GroupItem *__restr
         mma884(ca, nx[q][1], xa.y);
         if (two) mma884(cb, nx[q][1], xb.y);
       }
-      set_pair(Ds, lr, 8 * nt + 2 * t, ca[0], ca[1]);
-      if (two) set_pair(Ds, lr, 8 * nt + 8 + 2 * t, cb[0], cb[1]);
+      const double2 va = pair_at(Ds, lr, 8 * nt + 2 * t), vb = pair_at(Ds, lr, 8 * nb2 + 2 * t);
+      set_pair(Ds, lr, 8 * nt + 2 * t, va.x + ca[0], va.y + ca[1]);
+      if (two) set_pair(Ds, lr, 8 * nt + 8 + 2 * t, vb.x + cb[0], vb.y + cb[1]);
     }
   }
   if (jd >= 0) {  // this strip's own pivot block, fully updated: factor it and publish it (also after a failure)
