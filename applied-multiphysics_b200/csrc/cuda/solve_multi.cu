@@ -108,6 +108,20 @@ __device__ __forceinline__ void mma_chunk(const TL *__restrict__ A, const double
   }
 }
 
+// sum += c, c = 0. The long sums over FP64 factors are taken in pieces of kFold chunks (64 columns), so that a product is
+// rounded at its piece's size. One sum over the whole reduction left the residual of solves without refinement 19% larger than
+// the two halves that the products were once split into, pieces leave it 3 to 8% larger (elasticity, quadratic heat) to 33%
+// smaller (Bunch-Kaufman), for 1 to 2% of a solve's time; pieces of one chunk took 3 to 6%, of eight no less than of four. An
+// FP32 factor's own error hides the difference (equal to four digits), so its sums stay whole.
+constexpr int kFold = 4;
+__device__ __forceinline__ void fold(double (&sum)[4], double (&c)[4]) {
+#pragma unroll
+  for (int v = 0; v < 4; v++) {
+    sum[v] += c[v];
+    c[v] = 0.0;
+  }
+}
+
 // row / vector of accumulator element v of this lane
 __device__ __forceinline__ int acc_row(int warp, int lane, int v) { return 16 * (warp & 3) + (lane >> 2) + 8 * (v >> 1); }
 __device__ __forceinline__ int acc_vec(int warp, int lane, int v) { return 8 * (warp >> 2) + 2 * (lane & 3) + (v & 1); }
@@ -279,7 +293,7 @@ __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_fwd_multi(const i
     if (!gather_front_rows(P, s, false, (below ? (nc + kMB - 1) / kMB : 0) + blk, r0, rows, y, T, done, sl, q, vb,
                                       qs, status, Rs))
       return bail();
-    double c[4] = {0.0, 0.0, 0.0, 0.0};
+    double c[4] = {0.0, 0.0, 0.0, 0.0}, sum[4] = {0.0, 0.0, 0.0, 0.0};
     // y values of a pivot block (64 x 16, four per thread): read one block ahead when that block is known final. ready:
     // the leading blocks known final, found for up to 32 blocks at a time.
     double yr[4];
@@ -329,15 +343,17 @@ __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_fwd_multi(const i
         if (ahead) load_y(cb + kMB);
       }
       issue(i + kStages - 1);
+      if (sizeof(TL) == 8 && i % kFold == 0) fold(sum, c);
       mma_chunk<true>(ring + (i % kStages) * (KC * kLdKM), Bj + (cb & (kMB - 1)) * kLdB, warp, lane, c);
     }
+    fold(sum, c);
     // R = v[block] - the sum (the task's rows of v in Rs)
     if (below) {
       double *to = T + (P.snTOff[s] + (int64_t)blk * kMB) * q + vb;
 #pragma unroll
       for (int v = 0; v < 4; v++) {
         const int row = acc_row(warp, lane, v), n = acc_vec(warp, lane, v);
-        if (row < rows && n < qs) to[(int64_t)row * q + n] = Rs[row * kLdB + n] - c[v];
+        if (row < rows && n < qs) to[(int64_t)row * q + n] = Rs[row * kLdB + n] - sum[v];
       }
       __syncthreads();
       if (tid == 0) red_release_add(mydone + s, 1);
@@ -346,8 +362,7 @@ __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_fwd_multi(const i
 #pragma unroll
     for (int v = 0; v < 4; v++) {
       const int at = acc_row(warp, lane, v) * kLdB + acc_vec(warp, lane, v);
-      Rs[at] = (acc_row(warp, lane, v) < rows && acc_vec(warp, lane, v) < qs) ? Rs[at] - c[v] : 0.0;
-      c[v] = 0.0;
+      Rs[at] = (acc_row(warp, lane, v) < rows && acc_vec(warp, lane, v) < qs) ? Rs[at] - sum[v] : 0.0;
     }
     // y[block] = X R
     for (int i = nL; i < nL + nX; i++) {
@@ -557,7 +572,7 @@ __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_bwd_multi(const i
       cp_async_commit();
     };
     for (int i = 0; i < kStages - 1; i++) issue(i);
-    double c[4] = {0.0, 0.0, 0.0, 0.0};
+    double c[4] = {0.0, 0.0, 0.0, 0.0}, sum[4] = {0.0, 0.0, 0.0, 0.0};
     // x values of a chunk (KC x 16): read one chunk ahead when its rows are known final (ready: the chunks known final,
     // found for up to eight chunks of ancestors' rows, a warp each, or 32 pivot blocks at a time); ix: the row numbers of
     // the chunk to be read next, themselves read when the one before it was
@@ -642,8 +657,10 @@ __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_bwd_multi(const i
         if (i + 2 < nS) row_index(i + 2);
       }
       issue(i + kStages - 1);
+      if (sizeof(TL) == 8 && i % kFold == 0) fold(sum, c);
       mma_chunk<false>(ring + (i % kStages) * (kMB * LD), Bi, warp, lane, c);
     }
+    fold(sum, c);
     // R = y[block] (/ D) - the sum
 #pragma unroll
     for (int v = 0; v < 4; v++) {
@@ -651,10 +668,9 @@ __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_bwd_multi(const i
       double r = 0.0;
       if (cc < w && n < qs) {
         const double yv = y[(int64_t)(f + c0 + cc) * q + vb + n];
-        r = (Dpiv ? yv / Dpiv[f + c0 + cc] : yv) - c[v];  // LDL^T: y /= D before the backward sweep (ldlt.mjs:629)
+        r = (Dpiv ? yv / Dpiv[f + c0 + cc] : yv) - sum[v];  // LDL^T: y /= D before the backward sweep (ldlt.mjs:629)
       }
       Rs[cc * kLdB + n] = r;
-      c[v] = 0.0;
     }
     // x[block] = X^T R
     for (int i = nS; i < nS + nX; i++) {
