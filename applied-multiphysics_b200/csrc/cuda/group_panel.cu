@@ -5,9 +5,9 @@
 //
 // What bounds it: the chain through the pivot blocks of the large fronts (POTRF of block b, then block b + 1's rows
 // against it, then their update and POTRF), one CTA at a time, so a block's latency is what counts: per block POTRF
-// 11,100 clocks, the flag and the loads behind it 3,400, TRSM 2,500, the block's own update 1,600 (FP64; 33,700 / - /
+// 11,200 clocks, the flag and the loads behind it 3,300, TRSM 2,500, the block's own update 1,600 (FP64; 33,700 / - /
 // 10,400 / 7,100 with FMA tiles and a four-thread substitution per row). A 4,096-row front's group of two blocks takes
-// 32 us (66 before), eight of them at once 61 us (110). The split: warp w
+// 32 us (66 before), eight of them at once 63 us (110). The split: warp w
 // of a strip owns 8 rows (row group rg(w)) of every 64 x 64 product, so a strip's TRSM runs inside each warp without a
 // barrier -- the C fragment of a solved 8 x 8 tile is the A fragment of the next product (its two registers are the k
 // indices 2 t and 2 t + 1, and the B fragment takes the same pair with one 16-byte load).
@@ -56,7 +56,7 @@ __device__ __forceinline__ void load_block(double *S, const double *L, int m, in
 // they update the rest of the triangle while the first two warps go on with step k + 1. The chain per column is one
 // reciprocal (the hardware estimate and three dependent products) and two products, 58 clocks (FP64); a step's FP64
 // issue in a panel warp takes 790 clocks alone and 1,050-1,200 beside the trailing products. The pivots are tested, the
-// columns scaled and everything written after the last step. A block takes 11,100 clocks
+// columns scaled and everything written after the last step. A block takes 11,200 clocks
 // (33,700 with 4 x 4 register tiles, a diagonal thread per step and two barriers per four columns).
 // Cholesky tests d > 0 (sparse.mjs:1151-1156); LDL^T (ldlt.mjs:450-562) perturbs |d| < tau to +-tau by the sign of d (a
 // non-finite small pivot fails) and counts negative and perturbed pivots. Cholesky L = a / sqrt(d) with sqrt(d) on the

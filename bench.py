@@ -308,13 +308,13 @@ def run_reference(args, rank):
 # DRAM bytes per launch of the roofline kernel (dram__bytes_read.sum + dram__bytes_write.sum from one ncu capture;
 # profiles/ names the command). Keyed by (workload, size, precision, kernel class).
 # DRAM bytes per launch of the dominant kernel: the largest tcgen05 update launch of an elastic3d-32 mixed factor moves
-# 169.3 MB for 26.2 GFLOP (ncu dram__bytes_read.sum + dram__bytes_write.sum), scaled by the flops of an average cfg2
+# 171.3 MB for 26.2 GFLOP (ncu dram__bytes_read.sum + dram__bytes_write.sum), scaled by the flops of an average cfg2
 # update launch (764.6 GFLOP over 183 launches)
 TRAFFIC = {
-    ("elastic3d", 40, "mixed", "update_syrk"): 169.3e6 / 26.2e9 * 764.6e9 / 183,
-    # the group panel: its longest elastic3d-32 launch moves 22.9 MB for 0.602 GFLOP, scaled by the flops of an average
+    ("elastic3d", 40, "mixed", "update_syrk"): 171.3e6 / 26.2e9 * 764.6e9 / 183,
+    # the group panel: its longest elastic3d-32 launch moves 23.2 MB for 0.603 GFLOP, scaled by the flops of an average
     # cfg2 group-panel launch (26.8 GFLOP over 157 launches)
-    ("elastic3d", 40, "mixed", "group_panel"): 22.9e6 / 0.602e9 * 26.8e9 / 157,
+    ("elastic3d", 40, "mixed", "group_panel"): 23.2e6 / 0.603e9 * 26.8e9 / 157,
 }
 
 
