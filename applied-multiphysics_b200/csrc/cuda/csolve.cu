@@ -23,6 +23,7 @@
 
 #include <cstdint>
 
+#include "cp_async.cuh"
 #include "cplx.cuh"
 #include "devplan.cuh"
 #include "launch.hpp"
@@ -112,17 +113,15 @@ __device__ __forceinline__ void stage_triangle(cplx *T, int ld, const cplx *__re
   for (int e = threadIdx.x; e < w * kCB; e += blockDim.x) {
     const int c = e >> 6, r = e & (kCB - 1);
     if (r > c && r < w)
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(T + c * ld + r)),
-                   "l"(L + (int64_t)(p0 + c) * m + p0 + r)
-                   : "memory");
+      cp_async<16>(T + c * ld + r, L + (int64_t)(p0 + c) * m + p0 + r);
   }
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
+  cp_async_commit();
 }
 __device__ __forceinline__ void staged(bool newer) {  // all but the newest staging (newer), or all
   if (newer)
-    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    cp_async_wait<1>();
   else
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    cp_async_wait<0>();
 }
 // forward operand: row `row` of columns c0 + q + 4 u (below c0 + w); ok: the row exists
 __device__ __forceinline__ void load_row(cplx (&v)[16], const cplx *__restrict__ L, int m, int row, bool ok, int c0, int w,

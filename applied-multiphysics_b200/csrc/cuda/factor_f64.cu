@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "cp_async.cuh"
 #include "devplan.cuh"
 #include "launch.hpp"
 #include "pivot_steps.cuh"
@@ -184,17 +185,6 @@ __device__ __forceinline__ void dmma_16x8x16(double (&c)[4], const double (&a)[8
         "d"(b[2]), "d"(b[3]));
 }
 
-__device__ __forceinline__ void cp_async8(void *smem, const void *gmem, bool valid) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  const int bytes = valid ? 8 : 0;  // zero-fill when out of range
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(gmem), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
 constexpr int kChunk = 32;  // pivot columns per pipeline stage
 // leading dimensions in shared memory: 4 mod 16 doubles, conflict-free fragment loads
 template <int ROWS>
@@ -212,7 +202,7 @@ __device__ __forceinline__ void stage_rows(double *dst, const double *src, int m
 #pragma unroll 8
   for (int k = kb; k < kChunk; k += STEP, p += (int64_t)STEP * m) {
     const bool ok = rowok && k0 + k < kend;
-    cp_async8(dst + k * (R + 4) + i, ok ? p : src, ok);
+    cp_async<8>(dst + k * (R + 4) + i, ok ? p : src, ok);
   }
 }
 
@@ -383,14 +373,8 @@ __global__ void __launch_bounds__(128) k_update_c(const TileTask *__restrict__ t
       for (int k = tid / TS; k < kCK; k += 128 / TS) {
         const int c = ch * kCK + k;
         const bool okA = c < t.w && i0 + i < m, okB = c < t.w && j0 + i < m;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
-                         (unsigned)__cvta_generic_to_shared(As + k * LD + i)),
-                     "l"(Ap + (okA ? (int64_t)c * m + i0 + i : 0)), "r"(okA ? 16 : 0)
-                     : "memory");
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
-                         (unsigned)__cvta_generic_to_shared(Bs + k * LD + i)),
-                     "l"(Bp + (okB ? (int64_t)c * m + j0 + i : 0)), "r"(okB ? 16 : 0)
-                     : "memory");
+        cp_async<16>(As + k * LD + i, Ap + (okA ? (int64_t)c * m + i0 + i : 0), okA);
+        cp_async<16>(Bs + k * LD + i, Bp + (okB ? (int64_t)c * m + j0 + i : 0), okB);
       }
     }
     cp_async_commit();

@@ -39,6 +39,7 @@
 #include <cstdint>
 
 #include "../host/plan.hpp"
+#include "cp_async.cuh"
 #include "devplan.cuh"
 #include "solve_small.cuh"
 #include "sync.cuh"
@@ -126,22 +127,9 @@ __device__ __forceinline__ void fold(double (&sum)[4], double (&c)[4]) {
 __device__ __forceinline__ int acc_row(int warp, int lane, int v) { return 16 * (warp & 3) + (lane >> 2) + 8 * (v >> 1); }
 __device__ __forceinline__ int acc_vec(int warp, int lane, int v) { return 8 * (warp >> 2) + 2 * (lane & 3) + (v & 1); }
 
-__device__ __forceinline__ void cp_async_el(void *smem, const void *gmem, int bytes, bool valid) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  const int n = valid ? bytes : 0;  // zero-fill when out of range
-  if (bytes == 8)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(gmem), "r"(n) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(sa), "l"(gmem), "r"(n) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
 __device__ __forceinline__ void cp_async_all() {
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  cp_async_commit();
+  cp_async_wait<0>();
 }
 
 // persistent ticket loop shared by both sweeps
@@ -283,7 +271,7 @@ __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_fwd_multi(const i
         for (int u = 0; u < KC * kMB / kMultiThreads; u++) {
           const int e = tid + kMultiThreads * u, row = e & (kMB - 1), cc = e >> 6;
           const bool ok = row < rows && k0 + cc < lim;
-          cp_async_el(dst + cc * kLdKM + row, ok ? src + (int64_t)(k0 + cc) * ld + row : src, (int)sizeof(TL), ok);
+          cp_async<sizeof(TL)>(dst + cc * kLdKM + row, ok ? src + (int64_t)(k0 + cc) * ld + row : src, ok);
         }
       }
       cp_async_commit();
@@ -426,7 +414,7 @@ __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_fwd_multi(const i
         for (int u = 0; u < KC * kMB / kMultiThreads; u++) {
           const int e = tid + kMultiThreads * u, row = e & (kMB - 1), cc = e >> 6;
           const bool ok = row < rows && k0 + cc < nc;
-          cp_async_el(dst + cc * kLdKM + row, ok ? src + (int64_t)(k0 + cc) * ld + row : src, (int)sizeof(TL), ok);
+          cp_async<sizeof(TL)>(dst + cc * kLdKM + row, ok ? src + (int64_t)(k0 + cc) * ld + row : src, ok);
         }
       }
       cp_async_commit();
@@ -566,7 +554,7 @@ __global__ void __launch_bounds__(kMultiThreads, kMultiCtas) k_bwd_multi(const i
         for (int u = 0; u < KC * kMB / kMultiThreads; u++) {
           const int e = tid + kMultiThreads * u, rr = e % KC, cc = e / KC;
           const bool ok = cc < w && k0 + rr < lim;
-          cp_async_el(dst + cc * LD + rr, ok ? src + (int64_t)cc * ld + k0 + rr : src, (int)sizeof(TL), ok);
+          cp_async<sizeof(TL)>(dst + cc * LD + rr, ok ? src + (int64_t)cc * ld + k0 + rr : src, ok);
         }
       }
       cp_async_commit();

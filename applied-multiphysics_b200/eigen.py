@@ -31,8 +31,9 @@ def shiftInvertEigen(pat, K, M, sigma: float, nWant: int, tol: float = 1e-10, bl
     """Eigenpairs of K x = lambda M x nearest sigma (EigenInput / EigenResult of eigen.ts:14-106).
 
     The explicit relative residuals of the refined pairs are checked against max(1e3 tol, 1e-9): a run whose Krylov
-    iteration reported convergence with a pair above that bound is repeated, factorization included, with the next seed, up to `attempts` runs; the result with
-    the smallest worst residual is returned, and stats["attempts"] counts the runs."""
+    iteration reported convergence with a pair above that bound is repeated, factorization included, with the next seed,
+    up to `attempts` runs; the result with the smallest worst residual is returned, and stats["attempts"] counts the
+    runs."""
     best = None
     for a in range(max(1, attempts)):
         r = _shift_invert_once(pat, K, M, sigma, nWant, tol, blockSize, maxBasis, maxRestarts, seed + a, factor, kPsd,
